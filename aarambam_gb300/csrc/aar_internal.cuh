@@ -58,6 +58,7 @@ struct Plan {
   uint32_t* d_seed = nullptr; // seed table [N][N]
   float2* d_twN = nullptr;    // exp(-2 pi i m / N), m < N
   float2* d_twH = nullptr;    // exp(-2 pi i m / (N/2)), m < N/2
+  float2* d_tw2 = nullptr;    // second-stage twiddles of the tile passes (tile.cuh)
   float* d_amp = nullptr;     // per n^2 noise amplitude
   float* d_twb = nullptr;     // per n^2 T(k) / (Dplus Beta)
   float* d_sinc = nullptr;    // per grid index: CIC window sin(x)/x
@@ -67,7 +68,7 @@ struct Plan {
   int rtab_stride = 0;
   int64_t nsq = 0;            // 3 (N/2)^2 + 1
   int qtab_m = 0;             // modes the tables were allocated for
-  // field filters of the first modal pass over (|ky|, kz, |kx|), M (N/2+1)^3
+  // field filters of the first modal pass over |ky|, kz, |kx|, M (N/2+1)^2 HP
   // floats (qcube_build); made on first use after each table change
   float* d_qcube = nullptr;
   int qcube_m = 0;
@@ -157,6 +158,7 @@ int launch_seedtable(Plan* p, uint32_t seed, uint32_t* d_out, cudaStream_t st);
 int launch_noise_fp32(Plan* p, const uint32_t* d_seed, float2* d_phik, cudaStream_t st);
 int launch_noise_fp64(Plan* p, const uint32_t* d_seed, double2* d_phik, int hp, cudaStream_t st);
 int fused_prepare(Plan* p);
+int fused_tile_r1(int N);  // first radix of the tile passes at this grid size
 int qcube_build(Plan* p);
 struct Term;
 std::vector<std::vector<Term>> regrouped_terms(const std::vector<double>& alpha, int M);

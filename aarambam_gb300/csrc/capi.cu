@@ -238,12 +238,12 @@ static void plan_release(Plan* p) {
   p->prof.clear();
   for (auto e : p->event_pool) cudaEventDestroy(e);
   p->event_pool.clear();
-  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_amp, p->d_twb, p->d_rlxpow, p->d_terms, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube};
+  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_terms, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   p->d_phik = p->d_work = nullptr;
   p->d_seed = nullptr;
-  p->d_twN = p->d_twH = nullptr;
+  p->d_twN = p->d_twH = p->d_tw2 = nullptr;
   p->d_amp = p->d_twb = nullptr;
   p->d_rlxpow = p->d_terms = nullptr;
   p->d_qtab = p->d_rtab = nullptr;
@@ -434,6 +434,15 @@ static int create(Plan* p) {
     if ((rc = plan_alloc(p, (void**)&p->d_twH, sizeof(float2) * (N / 2)))) return rc;
     AAR_CUDA_TRY(p, cudaMemcpy(p->d_twN, twN.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
     AAR_CUDA_TRY(p, cudaMemcpy(p->d_twH, twH.data(), sizeof(float2) * (N / 2), cudaMemcpyHostToDevice));
+    if (q.precision == AAR_FUSED_FP32) {
+      // second-stage twiddles of the tile passes: [r][j], r < N / R1, j < R1
+      const int R1 = fused_tile_r1(N);
+      std::vector<float2> tw2(N);
+      for (int r = 0; r < N / R1; ++r)
+        for (int j = 0; j < R1; ++j) tw2[r * R1 + j] = twN[r * j];
+      if ((rc = plan_alloc(p, (void**)&p->d_tw2, sizeof(float2) * N))) return rc;
+      AAR_CUDA_TRY(p, cudaMemcpy(p->d_tw2, tw2.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+    }
     int64_t nsq = 3LL * (N / 2) * (N / 2) + 1;
     if ((rc = plan_alloc(p, (void**)&p->d_amp, sizeof(float) * nsq))) return rc;
     if ((rc = plan_alloc(p, (void**)&p->d_twb, sizeof(float) * nsq))) return rc;

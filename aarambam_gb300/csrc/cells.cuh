@@ -73,47 +73,6 @@ struct RhoArgs {
   float A[kMaxModes], B[kMaxModes];  // (2l-1)/l, (l-1)/l
 };
 
-// Field filter q_n(k) of main.c:580-637 at K cells (n2[i] = |k|^2 in grid
-// units, > 0) in FP32: k^(s (n-3)) k^(4-ns) for n <= 3, (P_{n-1}(kbar) -
-// X0[n-1]) k^(2-ns) above, with P_l as for rho_n (RhoArgs).  With k = kF
-// sqrt(n2) and kmin = kF, kbar = -1 + c1 (n2^(s/2) - 1): for integer n2 >= 1
-// the bracket is 0 or at least 2^(s/2) - 1 ~ 0.42, so it has no cancellation
-// and the hardware base-2 logarithm and exponential (absolute error ~2^-22
-// in the exponent; ~4e-7 relative in q) replace logf / expm1f: three
-// special-function operations per cell.  The K recurrences run in lockstep
-// (K independent chains per step).
-template <int K>
-__device__ __forceinline__ void q_mode_cells(const RhoArgs& ra, int n, const int* n2, float* out) {
-  float lg[K];
-#pragma unroll
-  for (int i = 0; i < K; ++i) lg[i] = __log2f((float)n2[i]);  // log2 n2
-  if (n <= 3) {
-    const float e = ra.s * (float)(n - 3) + ra.e4;
-#pragma unroll
-    for (int i = 0; i < K; ++i) out[i] = exp2f(e * fmaf(0.5f, lg[i], ra.log2kF));
-    return;
-  }
-  float kb[K], P0[K], P1[K];
-#pragma unroll
-  for (int i = 0; i < K; ++i) {
-    kb[i] = fmaf(ra.c1, exp2f(0.5f * ra.s * lg[i]), -1.f - ra.c1);
-    P0[i] = 1.f;
-    P1[i] = kb[i];
-  }
-  for (int l = 2; l < n; ++l) {
-    const float A = ra.A[l], B = ra.B[l];
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const float Pn = A * kb[i] * P1[i] - B * P0[i];
-      P0[i] = P1[i];
-      P1[i] = Pn;
-    }
-  }
-  const float x0 = ra.x0[n - 1];
-#pragma unroll
-  for (int i = 0; i < K; ++i) out[i] = (P1[i] - x0) * exp2f(ra.e2 * fmaf(0.5f, lg[i], ra.log2kF));
-}
-
 // Neumaier's compensated step: s + c carries the running sum of the t's
 __device__ __forceinline__ void neumaier_add(float& s, float& c, float t) {
   const float u = s + t;

@@ -356,14 +356,11 @@ __device__ __forceinline__ void line_sync(int bar_id) {
 // this together; lanes with act == false (no line of their own) only take
 // part in the barriers.  bar_id names the barrier of a line spread over
 // several warps.
-// SCALE multiplies the values of the first stage as they are loaded (line
-// element t + T b + r N/R sits at v[b R + r]) by sc[b R + r] (SCALE 1) or by
-// i sc[b R + r] (SCALE 2): a per-element filter folded into the transform.
 // TWS: twiddle-table stride (tw of a line TWS times longer).  LT: tw is the
 // block's lane twiddle table in shared memory (lt_fill<N, N/T, TWS>).
-template <int N, int T, int SIGN, int S = 0, int SCALE = 0, int TWS = 1, bool LT = false>
+template <int N, int T, int SIGN, int S = 0, int TWS = 1, bool LT = false>
 __device__ __forceinline__ void line_fft_smem(float2* s, int t, const float2* __restrict__ tw, bool act,
-                                              int bar_id = 1, const float* sc = nullptr) {
+                                              int bar_id = 1) {
   constexpr int E = N / T;
   constexpr int NS = num_stages(N, E);
   if constexpr (S < NS) {
@@ -371,39 +368,19 @@ __device__ __forceinline__ void line_fft_smem(float2* s, int t, const float2* __
     constexpr int Ns = stage_span(N, E, S);
     float2 v[E];
     if (act) stage_load<N, T, R>(v, s, t);
-    if constexpr (S == 0 && SCALE != 0) {
-#pragma unroll
-      for (int i = 0; i < E; ++i)
-        v[i] = SCALE == 1 ? make_float2(v[i].x * sc[i], v[i].y * sc[i]) : make_float2(-sc[i] * v[i].y, sc[i] * v[i].x);
-    }
     line_sync<T>(bar_id);
     if (act) {
       stage_compute<N, T, R, Ns, SIGN, TWS, LT, lt_off(N, E, S)>(v, t, tw);
       stage_store<N, T, R, Ns>(v, s, t);
     }
     line_sync<T>(bar_id);
-    line_fft_smem<N, T, SIGN, S + 1, 0, TWS, LT>(s, t, tw, act, bar_id);
+    line_fft_smem<N, T, SIGN, S + 1, TWS, LT>(s, t, tw, act, bar_id);
   }
-}
-
-// Line index of the i-th value a lane holds after the first stage load.
-template <int N, int T>
-__host__ __device__ constexpr int first_load_index(int t, int i) {
-  constexpr int E = N / T;
-  constexpr int R = stage_radix(N, E, 0);
-  return t + T * (i / R) + (i % R) * (N / R);
 }
 
 // lanes per line: 16 values per lane for N >= 512, 8 below
 __host__ __device__ constexpr int lanes_for(int N) {
   return N >= 512 ? N / 16 : (N / 8 >= 1 ? (N / 8 < 32 ? N / 8 : 32) : 1);
 }
-
-// lanes per line of the strided (tile) passes: 32 values per lane for
-// N >= 512, so that a 512- or 1024-point line is two Stockham stages
-// (32 x 16, 32 x 32) instead of three, one warp per line.  (The row kernels
-// keep lanes_for: their 512-point half lines with 32 values per lane were
-// slower, 140 vs 95 ms at 1024^3.)
-__host__ __device__ constexpr int lanes_for_tile(int N) { return N >= 512 ? N / 32 : lanes_for(N); }
 
 }  // namespace aar

@@ -4,8 +4,8 @@
 // a multiple of 8 so rows are 64-byte aligned); after a c2r the same buffer
 // holds the real field as float [N][N][2 HP] (z fastest).  A 3-D transform is
 // three passes, each reading and writing a field once:
-//   x pass / y pass  -- strided complex FFTs on tiles of W consecutive kz
-//                       columns x N rows, staged through shared memory;
+//   x pass / y pass  -- strided complex FFTs on tiles of 8 consecutive kz
+//                       columns x N rows, held in registers (tile.cuh);
 //   z pass (rows)    -- the real<->half-complex transform of contiguous rows
 //                       as an N/2-point complex FFT plus the usual
 //                       even/odd split twiddle step.
@@ -33,6 +33,7 @@
 #include "fft.cuh"
 #include "rows.cuh"
 #include "spectral.cuh"
+#include "tile.cuh"
 
 namespace aar {
 
@@ -43,98 +44,6 @@ struct DevTerms {
   Term t[kMaxTerms];
 };
 size_t terms_bytes() { return sizeof(DevTerms); }
-
-// ----------------------------------------------------------- tile passes
-// Line stride of a tile in shared memory: at least the padded line length,
-// and = 2 (mod 16) float2 so that the 8 lines x 2 rows a half-warp touches
-// while moving a tile between global and shared memory fall in 32 distinct
-// banks.
-__host__ __device__ constexpr int tile_ls(int N) {
-  int base = N + N / 16;
-  return base + ((2 - base % 16) + 16) % 16;
-}
-
-template <int N, int W>
-struct AxisCfg {
-  static constexpr int T = lanes_for_tile(N);  // lanes per line
-  static constexpr int E = N / T;
-  static constexpr int THREADS = ((W * T + 31) / 32) * 32;
-  static constexpr int WARPS = THREADS / 32;
-  static constexpr int LS = tile_ls(N);  // smem line stride (float2)
-  static constexpr size_t SMEM = sizeof(float2) * (size_t)W * LS;
-  static constexpr int PER = N * W / THREADS;  // tile elements per thread
-  // resident blocks per SM aimed at: 32 values per lane need ~128 registers
-  static constexpr int MINB = E >= 32 ? (THREADS >= 256 ? 2 : 4) : THREADS >= 512 ? 2 : 4;
-};
-
-// Tile indexing.  Axis 0 (x): rows n = x, other index o = y.  Axis 1 (y):
-// rows n = y, o = x.  Column w covers kz = c0 + w.  Fields are in the
-// x-blocked row order row_of(x, y, N, kXB).
-// Tile element ownership: thread t owns column w = t % W and rows
-// n = t / W + q THREADS/W, q < PER; with THREADS/W a multiple of 16 the
-// padded shared index and the global offset are a per-thread base plus a
-// compile-time (shared) or per-launch (global) stride times q.
-template <int N, int W, int AXIS>
-struct TileAddr {
-  using C = AxisCfg<N, W>;
-  static constexpr int DN = C::THREADS / W;  // row step between a thread's elements
-  int w, n0, sbase;
-  int64_t gbase, gstep;
-  __device__ __forceinline__ TileAddr(int HP, int o, int c0) {
-    w = threadIdx.x % W;
-    n0 = threadIdx.x / W;
-    sbase = w * C::LS + spad(n0);
-    // a thread's rows n0 + q DN keep n0 % kXB, so the offsets stay affine in q
-    static_assert(DN % kXB == 0, "row step of a tile thread must be a multiple of the x block");
-    if (AXIS == 0) {
-      gbase = row_of(n0, o, N, kXB) * HP + c0 + w;
-      gstep = (int64_t)DN * N * HP;
-    } else {
-      gbase = row_of(o, n0, N, kXB) * HP + c0 + w;
-      gstep = (int64_t)DN * kXB * HP;
-    }
-  }
-  __device__ __forceinline__ int s(int q) const {
-    if constexpr (DN % 16 == 0) return sbase + q * (DN + DN / 16);
-    else return w * C::LS + spad(n0 + q * DN);
-  }
-  __device__ __forceinline__ int64_t g(int q) const { return gbase + q * gstep; }
-};
-
-// issue the asynchronous copy of a tile (rows along AXIS) into shared memory
-template <int N, int W, int AXIS>
-__device__ __forceinline__ void tile_load_async(float2* sm, const float2* __restrict__ f, int HP, int o, int c0) {
-  using C = AxisCfg<N, W>;
-  const TileAddr<N, W, AXIS> ta(HP, o, c0);
-#pragma unroll 4
-  for (int q = 0; q < C::PER; ++q) cp_async8(sm + ta.s(q), f + ta.g(q));
-}
-
-template <int N, int W, int AXIS>
-__device__ __forceinline__ void tile_store(const float2* sm, float2* __restrict__ f, int HP, int o, int c0) {
-  using C = AxisCfg<N, W>;
-  const TileAddr<N, W, AXIS> ta(HP, o, c0);
-#pragma unroll 4
-  for (int q = 0; q < C::PER; ++q) f[ta.g(q)] = sm[ta.s(q)];
-}
-
-// run the W line FFTs of a tile held in shared memory (SCALE: optional
-// per-element factors of the first stage, see line_fft_smem).  The second
-// stage reads its twiddles from the global table: a per-block shared-memory
-// lane table (fft.cuh, as the row kernels use) made every tile pass at
-// 1024^3 slower (y pass 42.7 -> 46.7 ms with the table filled by cp.async
-// while the tile loads, 49.6 filled by plain loads).
-template <int N, int W, int SIGN, int SCALE = 0>
-__device__ __forceinline__ void tile_fft(float2* sm, const float2* __restrict__ tw, const float* sc = nullptr) {
-  using C = AxisCfg<N, W>;
-  // lines spread over several warps synchronise on named barriers 1..W;
-  // barrier ids stop at 15
-  static_assert(C::T <= 32 || W <= 15, "too many multi-warp lines per tile for the named barriers");
-  int line = threadIdx.x / C::T;
-  int t = threadIdx.x % C::T;
-  bool act = line < W;
-  line_fft_smem<N, C::T, SIGN, 0, SCALE>(sm + (act ? line : 0) * C::LS, t, tw, act, 1 + (act ? line : 0), sc);
-}
 
 // Last modal step, after the forward x transform of every active slot r:
 // acc = sum_r rho_r(k) g_r(k) (rho_r computed per cell in FP32, RhoArgs;
@@ -384,7 +293,7 @@ __global__ void __launch_bounds__(256) k_rows_c2r(float2* work, int64_t fs, int 
     constexpr int h = H / 2, HO = h + h / 16;
     if (act) row_c2r_pre_fold<N>(line, lane, twN, twH, zf, f);
     __syncwarp();
-    line_fft_smem<h, 16, +1, 0, 0, 2>(line + (lane >> 4) * HO, lane & 15, twH, act);
+    line_fft_smem<h, 16, +1, 0, 2>(line + (lane >> 4) * HO, lane & 15, twH, act);
     if (act)
       for (int m = lane; m < h; m += 32) {
         const float2 e = line[spad(m)], o = line[spad(m) + HO];
@@ -654,7 +563,7 @@ __global__ void __launch_bounds__(192, 4) k_rows_lattice(const float2* __restric
     float2* line = sm + warp * C::LS;
     if (act) row_c2r_pre_fold<N>(line, lane, twN, twH, zf, work + (int64_t)warp * fs + rbase * HP);
     __syncwarp();
-    line_fft_smem<h, 16, +1, 0, 0, 2>(line + (lane >> 4) * HO, lane & 15, twH, act);
+    line_fft_smem<h, 16, +1, 0, 2>(line + (lane >> 4) * HO, lane & 15, twH, act);
   } else {
     const int sub = lane / C::T, t = lane % C::T;
     const int64_t row = rbase + sub;
@@ -701,19 +610,17 @@ __global__ void __launch_bounds__(192, 4) k_rows_lattice(const float2* __restric
 }
 
 // ----------------------------------------------------------- host side
-// Launch a persistent pass: as many blocks as fit on the device at once.
-template <int N, class Op>
+// Launch a strided pass, one block per item.
+template <int N, int AXIS, int SIGN, class Op>
 static int run_pass(Plan* p, const Op& op, int64_t nitems, cudaStream_t st, const char* name) {
-  constexpr int W = 8;
-  using A = AxisCfg<N, W>;
-  auto kern = k_pass<N, W, Op>;
-  const size_t smem = A::SMEM + ExtraSmem<Op>::value;
-  AAR_CUDA_TRY(p, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  using C = TileCfg<N>;
+  auto kern = k_pass<N, AXIS, SIGN, Op>;
+  AAR_CUDA_TRY(p, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
   if (nitems < 1) return AAR_OK;
   if (nitems > 0x7fffffff) return set_err(p, std::string(name) + ": too many work items"), AAR_ERR_ARG;
   {
     ProfScope ps_(p, name, st);
-    kern<<<(unsigned)nitems, A::THREADS, smem, st>>>(op, p->d_twN);
+    kern<<<(unsigned)nitems, C::THREADS, C::SMEM, st>>>(op, p->d_tw2);
   }
   AAR_CUDA_TRY(p, cudaGetLastError());
   p->last_launches += 1;
@@ -741,9 +648,9 @@ RhoArgs rho_args(const Plan* p) {
 
 template <int N>
 struct Launch {
-  static constexpr int W = 8;
-  static int64_t tiles(Plan* p) { return (int64_t)N * (p->HP / W); }
+  static constexpr int64_t kTiles = TileCfg<N>::TILES;
   static int64_t fstride(Plan* p) { return (int64_t)N * N * p->HP; }
+  static unsigned group(Plan* p) { return (unsigned)std::min<int64_t>(p->xpass_group, kTiles); }
   static const int* slot_map(Plan* p) {
     return (const int*)((const char*)p->d_terms + offsetof(DevTerms, tl) + offsetof(TermList, r_of_slot));
   }
@@ -759,14 +666,12 @@ struct Launch {
   // y transform of fields [first, first + nf) (or the active modal slots)
   template <int SIGN>
   static int ypass(Plan* p, float2* base, int nf, const int* map, cudaStream_t st, const char* name) {
-    AxisOp<N, W, 1, SIGN> op{base, fstride(p), tiles(p), p->HP, map};
-    return run_pass<N>(p, op, nf * tiles(p), st, name);
+    return run_pass<N, 1, SIGN>(p, AxisOp<N>{base, fstride(p), map}, nf * kTiles, st, name);
   }
   static int modal(Plan* p, const ModalArgs& a, cudaStream_t st) {
     int64_t fs = fstride(p);
-    XinvOp<N, W> xo{a, p->d_phik, p->d_work, fs, tiles(p), p->HP, rho_args(p), p->xpass_group,
-                    p->qcube_stale ? nullptr : p->d_qcube};
-    int rc = run_pass<N>(p, xo, tiles(p) * a.M, st, "modal_xinv");
+    XinvOp<N> xo{p->d_phik, p->d_work, fs, a.M, group(p), p->d_qcube};
+    int rc = run_pass<N, 0, +1>(p, xo, kTiles * a.M, st, "modal_xinv");
     if (rc) return rc;
     if ((rc = ypass<+1>(p, p->d_work, a.M, nullptr, st, "modal_ypass_inv"))) return rc;
     size_t sm_rows = row_smem(a.M + 1);
@@ -807,8 +712,8 @@ struct Launch {
   static int modal_tail(Plan* p, const ModalArgs& a, int64_t fs, cudaStream_t st) {
     int rc;
     {
-      AxisOp<N, W, 0, -1> xf{p->d_work, fs, tiles(p), p->HP, slot_map(p)};
-      if ((rc = run_pass<N>(p, xf, p->nr_active * tiles(p), st, "modal_xfwd"))) return rc;
+      AxisOp<N> xf{p->d_work, fs, slot_map(p)};
+      if ((rc = run_pass<N, 0, -1>(p, xf, p->nr_active * kTiles, st, "modal_xfwd"))) return rc;
     }
     float fnl_n3 = (float)(p->prm.fnl / ((double)N * N * N));
     if (jit_has_acc(p)) return jit_modal_acc(p, p->d_phik, p->d_work, fnl_n3, rho_args(p), st);
@@ -828,7 +733,8 @@ struct Launch {
   // kz^2) and write S to 6; psi1 (0..2) and psi2 (3..5) likewise from x
   // outputs in 0, 8 (psi1) and 3, 7 (psi2).
   static int lpt(Plan* p, const LptArgs& a, cudaStream_t st, bool rows = true) {
-    int64_t fs = fstride(p);
+    const int64_t fs = fstride(p);
+    const float kF = a.m.g.kF;
     float2* phit = p->d_work + 7 * fs;  // T/(D Beta) phi, read by the Hessian and psi1 passes
     {
       ProfScope ps_(p, "lpt_scale_twb", st);
@@ -838,10 +744,10 @@ struct Launch {
     p->last_launches += 1;
     int rc;
     {
-      LptXOp<N, W, 0> ho{a, phit, p->d_work, fs, tiles(p), p->HP, {0, 8, 6}, p->xpass_group};
-      if ((rc = run_pass<N>(p, ho, tiles(p) * 3, st, "lpt_xinv_hess"))) return rc;
-      YFanOp<N, W> yf{a, p->d_work, fs, tiles(p), p->HP, {0, 8, 8, 6, 6, 6}, {0, 1, 2, 3, 4, 5}, {0, 1, 0, 2, 1, 0}, 1};
-      if ((rc = run_pass<N>(p, yf, tiles(p) * 6, st, "lpt_ypass_inv_hess"))) return rc;
+      LptXOp<N, 0> ho{phit, p->d_work, fs, {0, 8, 6}, group(p), kF, a.isinc2};
+      if ((rc = run_pass<N, 0, +1>(p, ho, kTiles * 3, st, "lpt_xinv_hess"))) return rc;
+      YFanOp<N> yf{p->d_work, fs, {0, 8, 8, 6, 6, 6}, {0, 1, 2, 3, 4, 5}, {0, 1, 0, 2, 1, 0}, 1, kF, a.isinc2};
+      if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "lpt_ypass_inv_hess"))) return rc;
     }
     size_t sm_rows = row_smem(7);
     SourceRowOp op{6, a.m.g.kF, a.isinc2};
@@ -855,16 +761,16 @@ struct Launch {
     if ((rc = ypass<-1>(p, p->d_work + 6 * fs, 1, nullptr, st, "lpt_ypass_fwd_source"))) return rc;
     // forward x of the source in place with -1/k^2, then the displacement x passes
     {
-      XfwdInvK2Op<N, W> xs{p->d_work + 6 * fs, tiles(p), p->HP, a.m.g.kF};
-      if ((rc = run_pass<N>(p, xs, tiles(p), st, "lpt_xfwd_source"))) return rc;
+      XfwdInvK2Op<N> xs{p->d_work + 6 * fs, kF};
+      if ((rc = run_pass<N, 0, -1>(p, xs, kTiles, st, "lpt_xfwd_source"))) return rc;
     }
     {
-      LptXOp<N, W, 1> m1{a, phit, p->d_work, fs, tiles(p), p->HP, {0, 8, 0}, p->xpass_group};
-      if ((rc = run_pass<N>(p, m1, tiles(p) * 2, st, "lpt_xpsi1"))) return rc;
-      LptXOp<N, W, 1> m2{a, p->d_work + 6 * fs, p->d_work, fs, tiles(p), p->HP, {3, 7, 0}, p->xpass_group};
-      if ((rc = run_pass<N>(p, m2, tiles(p) * 2, st, "lpt_xpsi2"))) return rc;
-      YFanOp<N, W> yf{a, p->d_work, fs, tiles(p), p->HP, {0, 8, 8, 3, 7, 7}, {0, 1, 2, 3, 4, 5}, {3, 4, 3, 3, 4, 3}, 1};
-      if ((rc = run_pass<N>(p, yf, tiles(p) * 6, st, "lpt_ypass_inv_disp"))) return rc;
+      LptXOp<N, 1> m1{phit, p->d_work, fs, {0, 8, 0}, group(p), kF, a.isinc2};
+      if ((rc = run_pass<N, 0, +1>(p, m1, kTiles * 2, st, "lpt_xpsi1"))) return rc;
+      LptXOp<N, 1> m2{p->d_work + 6 * fs, p->d_work, fs, {3, 7, 0}, group(p), kF, a.isinc2};
+      if ((rc = run_pass<N, 0, +1>(p, m2, kTiles * 2, st, "lpt_xpsi2"))) return rc;
+      YFanOp<N> yf{p->d_work, fs, {0, 8, 8, 3, 7, 7}, {0, 1, 2, 3, 4, 5}, {3, 4, 3, 3, 4, 3}, 1, kF, a.isinc2};
+      if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "lpt_ypass_inv_disp"))) return rc;
     }
     // the displacement rows: here, or fused with the lattice read-out
     // (fused_rows_lattice), which leaves no real fields behind
@@ -898,6 +804,12 @@ static int dispatch_n(int N, F&& f) {
     case 1024: return f(std::integral_constant<int, 1024>{});
     default: return AAR_ERR_ARG;
   }
+}
+
+int fused_tile_r1(int N) {
+  int r1 = 0;
+  dispatch_n(N, [&](auto nc) { return r1 = TileCfg<decltype(nc)::value>::R1, AAR_OK; });
+  return r1;
 }
 
 ModalArgs modal_args(Plan* p) {
@@ -998,31 +910,29 @@ static int build_terms(Plan* p) {
   return AAR_OK;
 }
 
-// The filter cube of the first modal pass: q_p(|kx|, |ky|, kz) for
-// 0 <= |kx|, |ky|, kz <= N/2 with q_mode_cells' arithmetic, zero on the cut
-// and at k = 0 (keep_cell depends on |k_a| only).  Index ((p K + |ky|) K +
-// kz) K + |kx|, K = N/2 + 1.
-__global__ void __launch_bounds__(256) k_qcube(Grid g, RhoArgs ra, int M, float* __restrict__ q) {
-  const int K = g.N / 2 + 1;
-  const int64_t per = (int64_t)K * K * K;
+// The filter cube of the first modal pass: the plan's per-|k|^2 filters
+// (mode_tables: FP64 formulas rounded once to float) over 0 <= |kx|, |ky| <=
+// N/2 and the padded kz columns, zero on the cut, at k = 0 and on the padding
+// (keep_cell depends on |k_a| only).  Index (((p K + |ky|) NCOL + kz / 8) K +
+// |kx|) 8 + kz % 8, K = N/2 + 1, NCOL = HP / 8.
+__global__ void __launch_bounds__(256) k_qcube(Grid g, int M, const float* __restrict__ qtab, int64_t nsq,
+                                               float* __restrict__ q) {
+  const int K = g.N / 2 + 1, ncol = g.HP / 8;
+  const int64_t per = (int64_t)K * g.HP * K;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (int64_t)gridDim.x * blockDim.x) {
-    const int ax = (int)(i % K);
-    const int64_t r = i / K;
-    const int kz = (int)(r % K), ay = (int)(r / K);
-    int n2[1] = {ax * ax + ay * ay + kz * kz};
-    const bool on = n2[0] != 0 && keep_cell(g, ax, ay, kz);
-    if (!on) n2[0] = 1;
-    for (int p = 0; p < M; ++p) {
-      float v[1];
-      q_mode_cells<1>(ra, p, n2, v);
-      q[(int64_t)p * per + i] = on ? v[0] : 0.f;
-    }
+    const int64_t r = i / 8;
+    const int ax = (int)(r % K);
+    const int64_t s = r / K;
+    const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
+    const int n2 = ax * ax + ay * ay + kz * kz;
+    const bool on = kz <= g.N / 2 && n2 != 0 && keep_cell(g, ax, ay, kz);
+    for (int p = 0; p < M; ++p) q[(int64_t)p * per + i] = on ? __ldg(qtab + (int64_t)p * nsq + n2) : 0.f;
   }
 }
 
 int qcube_build(Plan* p) {
   if (!p->qcube_stale && p->d_qcube) return AAR_OK;
-  const int64_t K = p->N / 2 + 1, per = K * K * K;
+  const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
   if (!p->d_qcube || p->qcube_m != p->M) {
     if (p->d_qcube) cudaFree(p->d_qcube), p->used_bytes -= sizeof(float) * (size_t)per * p->qcube_m;
     p->d_qcube = nullptr;
@@ -1031,7 +941,7 @@ int qcube_build(Plan* p) {
     if (rc) return rc;
     p->qcube_m = p->M;
   }
-  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, rho_args(p), p->M, p->d_qcube);
+  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, p->M, p->d_qtab, p->nsq, p->d_qcube);
   AAR_CUDA_TRY(p, cudaGetLastError());
   // made on the legacy stream once per table set; runs on the caller's
   // streams read it afterwards
@@ -1266,13 +1176,12 @@ __global__ void __launch_bounds__(256) k_rows_r2c(float2* f, int HP, int64_t nro
 
 template <int N>
 struct Xform {
-  static constexpr int W = 8;
+  static constexpr int64_t tiles = TileCfg<N>::TILES;
   static int c2r(Plan* p, float2* slot, cudaStream_t st) {
     using R = RowCfg<N>;
-    int64_t tiles = (int64_t)N * (p->HP / W);
-    int rc = run_pass<N>(p, AxisOp<N, W, 0, +1>{slot, 0, tiles, p->HP, nullptr}, tiles, st, "xform_x");
+    int rc = run_pass<N, 0, +1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_x");
     if (rc) return rc;
-    if ((rc = run_pass<N>(p, AxisOp<N, W, 1, +1>{slot, 0, tiles, p->HP, nullptr}, tiles, st, "xform_y"))) return rc;
+    if ((rc = run_pass<N, 1, +1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_y"))) return rc;
     int lpb = 8 * R::LPW;
     int64_t nrows = (int64_t)N * N;
     dim3 g2((unsigned)((nrows + lpb - 1) / lpb), 1);
@@ -1296,10 +1205,9 @@ struct Xform {
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
-    int64_t tiles = (int64_t)N * (p->HP / W);
-    int rc = run_pass<N>(p, AxisOp<N, W, 1, -1>{slot, 0, tiles, p->HP, nullptr}, tiles, st, "xform_y");
+    int rc = run_pass<N, 1, -1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_y");
     if (rc) return rc;
-    return run_pass<N>(p, AxisOp<N, W, 0, -1>{slot, 0, tiles, p->HP, nullptr}, tiles, st, "xform_x");
+    return run_pass<N, 0, -1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_x");
   }
 };
 

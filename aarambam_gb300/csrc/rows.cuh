@@ -341,7 +341,7 @@ __device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs
       if constexpr (Op::kZfac) row_c2r_pre_fold<N>(line, lane, twN, twH, op.zfac(l), X);
       else row_c2r_pre_fold<N>(line, lane, twN, twH, ZFac{0, 0.f, nullptr}, X);
       __syncwarp();
-      line_fft_smem<h, 16, +1, 0, 0, 2, true>(line + half * HO, t16, lt, true);
+      line_fft_smem<h, 16, +1, 0, 2, true>(line + half * HO, t16, lt, true);
     }
     __syncthreads();
     for (int n = threadIdx.x; n < H; n += (Op::kPairs ? 2 : 1) * THREADS) {
@@ -356,7 +356,7 @@ __device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs
     __syncthreads();
     for (int l = warp; l < op.nout(); l += nwarps) {
       float2* line = sm + op.out_line(l) * C::LS;
-      line_fft_smem<h, 16, -1, 0, 0, 2, true>(line + half * HO, t16, lt, true);
+      line_fft_smem<h, 16, -1, 0, 2, true>(line + half * HO, t16, lt, true);
       row_r2c_post_fold<N>(line, work + (int64_t)op.out_slot(l) * fs + row * HP, lane, twN, twH);
       __syncwarp();
     }

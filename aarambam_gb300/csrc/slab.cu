@@ -119,9 +119,13 @@ __global__ void __launch_bounds__(256) k_slab_herm(float2* F, int nf, int64_t sf
   }
 }
 
-// Field filters q_p(k), p < M, at one cell (n2 = |k|^2 in grid units, > 0):
-// the expressions of q_mode_cells (cells.cuh) with one Legendre recurrence
-// for all modes (P_{p-1} for mode p > 3).
+// Field filters q_p(k) of main.c:580-637, p < M, at one cell (n2 = |k|^2 in
+// grid units, > 0) in FP32: k^(s (p-3)) k^(4-ns) for p <= 3, (P_{p-1}(kbar) -
+// X0[p-1]) k^(2-ns) above, one Legendre recurrence for all modes.  With k = kF
+// sqrt(n2) and kmin = kF, kbar = -1 + c1 (n2^(s/2) - 1): for integer n2 >= 1
+// the bracket is 0 or at least 2^(s/2) - 1 ~ 0.42, so it has no cancellation
+// and the hardware base-2 logarithm and exponential (absolute error ~2^-22
+// in the exponent; ~4e-7 relative in q) replace logf / expm1f.
 template <int MAXM>
 __device__ __forceinline__ void q_all_modes(const RhoArgs& ra, int M, int n2, float* q) {
   const float lg = __log2f((float)n2);
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(kProdThreads) k_slab_products(SlabTerms tm, co
 // the slot sum Neumaier-compensated in the slab's frame, then rotated by the
 // twiddle once and added to the running compensated sum (acc_s, acc_c) of
 // the slabs.  rho_r per cell with k_modal_acc's expressions, its logarithm
-// and exponentials in the base-2 hardware forms of q_mode_cells (every slab
+// and exponentials in the base-2 hardware forms of q_all_modes (every slab
 // re-evaluates them; the bracket k^s / kmin^s - 1 of kbar is 0 or at least
 // 0.42 for integer n2, no cancellation to guard).  The modes are walked in
 // one unrolled pass r = 0 .. MAXM-1 with one Legendre recurrence and a
