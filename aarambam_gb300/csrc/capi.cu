@@ -1082,6 +1082,7 @@ int aar_set_modal_partition(aar_plan* h, int32_t part, int32_t nparts) {
   p->modal_nparts = nparts;
   if (!p->have_tables) return AAR_OK;
   AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // the term list is rewritten below
+  p->qcube_stale = true;                     // the part may read other modes
   return fused_prepare(p);
 }
 
@@ -1129,9 +1130,10 @@ int aar_autotune(aar_plan* h, char* report, int32_t len, void* stream) {
   };
   const int64_t row_tiles = p->HP / 8;
   // (row kernel, blocks per SM, threads per block); 320 threads only where
-  // ten warps take the M input lines in fewer rounds than eight
+  // ten warps take the input lines in fewer rounds than eight
   std::vector<int3> rows = {{0, 2, 256}, {2, 2, 256}, {2, 3, 256}};
-  if ((p->M + 9) / 10 < (p->M + 7) / 8) rows.push_back({2, 2, 320});
+  const int nin = p->host_terms.empty() ? 0 : ((const TermList*)p->host_terms.data())->nin;
+  if ((nin + 9) / 10 < (nin + 7) / 8) rows.push_back({2, 2, 320});
   std::vector<Cand> cands;
   for (const int3& r : rows)
     for (int64_t g : {(int64_t)1, row_tiles, 4 * row_tiles}) cands.push_back(Cand{r.x, r.y, r.z, g, -1.f});

@@ -161,7 +161,7 @@ struct TermC {
   float c;
 };
 
-// modal products: lines 0..M-1 hold f_p; line r is overwritten by g_r.  The
+// modal products: the line of p holds f_p; the line of r is overwritten by g_r.  The
 // term list travels in the kernel's parameter space, so every thread reads
 // a term through the uniform constant path; each thread forms two positions
 // per term.
@@ -171,14 +171,16 @@ struct ModalRowOp {
   static constexpr int min_blocks(int n) { return n >= 1024 ? 2 : 3; }
   static constexpr bool kZfac = false;
   static constexpr bool kPairs = true;
-  int M, nr;
-  int r_of_slot[kMaxModes];
+  int ni, nr;
+  int in_mode[kMaxModes], line_in[kMaxModes];
+  int r_of_slot[kMaxModes], line_out[kMaxModes];
   int begin[kMaxModes + 1];
   TermC t[kMaxTerms];
-  __device__ int nin() const { return M; }
-  __device__ int in_slot(int l) const { return l; }
+  __device__ int nin() const { return ni; }
+  __device__ int in_slot(int l) const { return in_mode[l]; }
+  __device__ int in_line(int l) const { return line_in[l]; }
   __device__ int nout() const { return nr; }
-  __device__ int out_line(int l) const { return r_of_slot[l]; }
+  __device__ int out_line(int l) const { return line_out[l]; }
   __device__ int out_slot(int l) const { return r_of_slot[l]; }
   // Slots in descending r: g_r only needs f_p f_q with p <= q <= r, so once
   // g_r is formed nothing later reads f_r and it is stored over it at once.
@@ -219,7 +221,7 @@ struct ModalRowOp {
           acc[i].x += g1_extra[i].x;
           acc[i].y += g1_extra[i].y;
         }
-        sm[r * LS + pos[i]] = acc[i];
+        sm[line_out[s] * LS + pos[i]] = acc[i];
       }
     }
   }
@@ -239,6 +241,7 @@ struct SourceRowOp {
   __device__ ZFac zfac(int l) const { return ZFac{l == 2 || l == 4 ? 1 : l == 5 ? 2 : 0, kF, isinc2}; }
   __device__ int nin() const { return 6; }
   __device__ int in_slot(int l) const { return l; }
+  __device__ int in_line(int l) const { return l; }
   __device__ int nout() const { return 1; }
   __device__ int out_line(int) const { return 0; }
   __device__ int out_slot(int) const { return out; }
@@ -651,9 +654,6 @@ struct Launch {
   static constexpr int64_t kTiles = TileCfg<N>::TILES;
   static int64_t fstride(Plan* p) { return (int64_t)N * N * p->HP; }
   static unsigned group(Plan* p) { return (unsigned)std::min<int64_t>(p->xpass_group, kTiles); }
-  static const int* slot_map(Plan* p) {
-    return (const int*)((const char*)p->d_terms + offsetof(DevTerms, tl) + offsetof(TermList, r_of_slot));
-  }
   static constexpr size_t row_smem(int nlines) {
     return sizeof(float2) * ((size_t)nlines * RowCfg<N>::LS + row_lt_slots<N>());
   }
@@ -663,58 +663,61 @@ struct Launch {
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows<N, SourceRowOp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_rows));
     return AAR_OK;
   }
-  // y transform of fields [first, first + nf) (or the active modal slots)
-  template <int SIGN>
-  static int ypass(Plan* p, float2* base, int nf, const int* map, cudaStream_t st, const char* name) {
-    return run_pass<N, 1, SIGN>(p, AxisOp<N>{base, fstride(p), map}, nf * kTiles, st, name);
+  static Slots slots(const int* s, int n) {
+    Slots r{};
+    for (int i = 0; i < n; ++i) r.s[i] = s[i];
+    return r;
   }
-  static int modal(Plan* p, const ModalArgs& a, cudaStream_t st) {
-    int64_t fs = fstride(p);
-    XinvOp<N> xo{p->d_phik, p->d_work, fs, a.M, group(p), p->d_qcube};
-    int rc = run_pass<N, 0, +1>(p, xo, kTiles * a.M, st, "modal_xinv");
-    if (rc) return rc;
-    if ((rc = ypass<+1>(p, p->d_work, a.M, nullptr, st, "modal_ypass_inv"))) return rc;
-    size_t sm_rows = row_smem(a.M + 1);
-    if (p->jit) {
-      if ((rc = jit_modal_rows(p, p->d_work, fs, st))) return rc;
-      if ((rc = ypass<-1>(p, p->d_work, p->nr_active, slot_map(p), st, "modal_ypass_fwd"))) return rc;
-      return modal_tail(p, a, fs, st);
-    }
+  // transform of nf fields of `base` along AXIS in place
+  template <int AXIS, int SIGN>
+  static int axis_pass(Plan* p, float2* base, int nf, const Slots& sl, cudaStream_t st, const char* name) {
+    return run_pass<N, AXIS, SIGN>(p, AxisOp<N>{base, fstride(p), sl}, nf * kTiles, st, name);
+  }
+  static const TermList& terms(Plan* p) { return *(const TermList*)p->host_terms.data(); }
+  // the generic row kernel's term list as a kernel parameter
+  static ModalRowOp row_op(Plan* p) {
     static_assert(sizeof(ModalRowOp) < 32000, "kernel parameter space");
+    const TermList& tl = terms(p);
+    const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
+    constexpr int LS = RowCfg<N>::LS;
+    static_assert(kMaxModes * LS < 0x8000, "line offsets fit 15 bits");
     ModalRowOp op;
-    {
-      const TermList& tl = *(const TermList*)p->host_terms.data();
-      const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
-      constexpr int LS = RowCfg<N>::LS;
-      static_assert(kMaxModes * LS < 0x8000, "line offsets fit 15 bits");
-      op.M = a.M;
-      op.nr = tl.nr;
-      for (int i = 0; i < kMaxModes; ++i) op.r_of_slot[i] = tl.r_of_slot[i];
-      for (int i = 0; i <= kMaxModes; ++i) op.begin[i] = tl.begin[i];
-      for (int sl = 0; sl < tl.nr; ++sl)
-        for (int i = tl.begin[sl]; i < tl.begin[sl + 1]; ++i) {
-          const uint32_t early = ft[i].r != tl.r_of_slot[sl] ? 1u : 0u;
-          op.t[i].off = (uint32_t)(ft[i].p * LS) | ((uint32_t)(ft[i].q * LS) << 16) | (early << 31);
-          op.t[i].c = ft[i].c;
-        }
-    }
+    op.ni = tl.nin;
+    op.nr = tl.nr;
+    for (int i = 0; i < tl.nin; ++i) op.in_mode[i] = tl.in_mode[i], op.line_in[i] = tl.line[tl.in_mode[i]];
+    for (int i = 0; i < tl.nr; ++i) op.r_of_slot[i] = tl.r_of_slot[i], op.line_out[i] = tl.line[tl.r_of_slot[i]];
+    for (int i = 0; i <= tl.nr; ++i) op.begin[i] = tl.begin[i];
+    for (int sl = 0; sl < tl.nr; ++sl)
+      for (int i = tl.begin[sl]; i < tl.begin[sl + 1]; ++i) {
+        const uint32_t early = ft[i].r != tl.r_of_slot[sl] ? 1u : 0u;
+        op.t[i].off = (uint32_t)(tl.line[ft[i].p] * LS) | ((uint32_t)(tl.line[ft[i].q] * LS) << 16) | (early << 31);
+        op.t[i].c = ft[i].c;
+      }
+    return op;
+  }
+  static int modal_rows(Plan* p, float2* work, int64_t fs, int64_t nrows, cudaStream_t st) {
+    const ModalRowOp op = row_op(p);
+    const size_t sm_rows = row_smem(terms(p).nlines);
     {
       ProfScope ps_(p, "modal_rows", st);
-      k_rows<N, ModalRowOp><<<(unsigned)((int64_t)N * N), kRowThreads, sm_rows, st>>>(op, p->d_work, fs, p->HP, p->d_twN,
-                                                                               p->d_twH);
+      k_rows<N, ModalRowOp><<<(unsigned)nrows, kRowThreads, sm_rows, st>>>(op, work, fs, p->HP, p->d_twN, p->d_twH);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
-    if ((rc = ypass<-1>(p, p->d_work, p->nr_active, slot_map(p), st, "modal_ypass_fwd"))) return rc;
-    return modal_tail(p, a, fs, st);
+    return AAR_OK;
   }
-  // forward x of the active slots, then the accumulation into phi
-  static int modal_tail(Plan* p, const ModalArgs& a, int64_t fs, cudaStream_t st) {
-    int rc;
-    {
-      AxisOp<N> xf{p->d_work, fs, slot_map(p)};
-      if ((rc = run_pass<N, 0, -1>(p, xf, p->nr_active * kTiles, st, "modal_xfwd"))) return rc;
-    }
+  static int modal(Plan* p, const ModalArgs& a, cudaStream_t st) {
+    const int64_t fs = fstride(p);
+    const TermList& tl = terms(p);
+    const Slots in = slots(tl.in_mode, tl.nin), out = slots(tl.r_of_slot, tl.nr);
+    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), p->d_qcube};
+    int rc = run_pass<N, 0, +1>(p, xo, kTiles * tl.nin, st, "modal_xinv");
+    if (rc) return rc;
+    if ((rc = axis_pass<1, +1>(p, p->d_work, tl.nin, in, st, "modal_ypass_inv"))) return rc;
+    if ((rc = p->jit ? jit_modal_rows(p, p->d_work, fs, st) : modal_rows(p, p->d_work, fs, (int64_t)N * N, st))) return rc;
+    if ((rc = axis_pass<1, -1>(p, p->d_work, tl.nr, out, st, "modal_ypass_fwd"))) return rc;
+    // forward x of the active slots, then the accumulation into phi
+    if ((rc = axis_pass<0, -1>(p, p->d_work, tl.nr, out, st, "modal_xfwd"))) return rc;
     float fnl_n3 = (float)(p->prm.fnl / ((double)N * N * N));
     if (jit_has_acc(p)) return jit_modal_acc(p, p->d_phik, p->d_work, fnl_n3, rho_args(p), st);
     {
@@ -758,7 +761,7 @@ struct Launch {
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
-    if ((rc = ypass<-1>(p, p->d_work + 6 * fs, 1, nullptr, st, "lpt_ypass_fwd_source"))) return rc;
+    if ((rc = axis_pass<1, -1>(p, p->d_work, 1, Slots{{6}}, st, "lpt_ypass_fwd_source"))) return rc;
     // forward x of the source in place with -1/k^2, then the displacement x passes
     {
       XfwdInvK2Op<N> xs{p->d_work + 6 * fs, kF};
@@ -899,6 +902,13 @@ static int build_terms(Plan* p) {
   tl.begin[nr] = (int)flat.size();
   tl.nr = nr;
   tl.nterms = (int)flat.size();
+  bool read[kMaxModes] = {}, active[kMaxModes] = {};
+  for (const Term& t : flat) read[t.p] = read[t.q] = true;
+  for (int i = 0; i < nr; ++i) active[tl.r_of_slot[i]] = true;
+  for (int m = 0; m < M; ++m) {
+    if (read[m]) tl.in_mode[tl.nin++] = m;
+    tl.line[m] = read[m] || active[m] ? tl.nlines++ : -1;
+  }
   if (tl.nterms > kMaxTerms) return set_err(p, "too many alpha terms"), AAR_ERR_ARG;
   DevTerms* dt = (DevTerms*)p->d_terms;
   AAR_CUDA_TRY(p, cudaMemcpy(&dt->tl, &tl, sizeof(tl), cudaMemcpyHostToDevice));
@@ -914,9 +924,9 @@ static int build_terms(Plan* p) {
 // (mode_tables: FP64 formulas rounded once to float) over 0 <= |kx|, |ky| <=
 // N/2 and the padded kz columns, zero on the cut, at k = 0 and on the padding
 // (keep_cell depends on |k_a| only).  Index (((p K + |ky|) NCOL + kz / 8) K +
-// |kx|) 8 + kz % 8, K = N/2 + 1, NCOL = HP / 8.
-__global__ void __launch_bounds__(256) k_qcube(Grid g, int M, const float* __restrict__ qtab, int64_t nsq,
-                                               float* __restrict__ q) {
+// |kx|) 8 + kz % 8 for the p-th mode that the products read, K = N/2 + 1, NCOL = HP / 8.
+__global__ void __launch_bounds__(256) k_qcube(Grid g, int nin, const __grid_constant__ Slots mode,
+                                               const float* __restrict__ qtab, int64_t nsq, float* __restrict__ q) {
   const int K = g.N / 2 + 1, ncol = g.HP / 8;
   const int64_t per = (int64_t)K * g.HP * K;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (int64_t)gridDim.x * blockDim.x) {
@@ -926,22 +936,26 @@ __global__ void __launch_bounds__(256) k_qcube(Grid g, int M, const float* __res
     const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
     const int n2 = ax * ax + ay * ay + kz * kz;
     const bool on = kz <= g.N / 2 && n2 != 0 && keep_cell(g, ax, ay, kz);
-    for (int p = 0; p < M; ++p) q[(int64_t)p * per + i] = on ? __ldg(qtab + (int64_t)p * nsq + n2) : 0.f;
+    for (int c = 0; c < nin; ++c) q[(int64_t)c * per + i] = on ? __ldg(qtab + (int64_t)mode.s[c] * nsq + n2) : 0.f;
   }
 }
 
 int qcube_build(Plan* p) {
-  if (!p->qcube_stale && p->d_qcube) return AAR_OK;
+  if (p->host_terms.empty()) return AAR_OK;  // no tables yet: nothing reads filters
+  const TermList& tl = *(const TermList*)p->host_terms.data();
+  if ((!p->qcube_stale && p->d_qcube) || tl.nin == 0) return AAR_OK;
   const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
-  if (!p->d_qcube || p->qcube_m != p->M) {
+  if (!p->d_qcube || p->qcube_m != tl.nin) {
     if (p->d_qcube) cudaFree(p->d_qcube), p->used_bytes -= sizeof(float) * (size_t)per * p->qcube_m;
     p->d_qcube = nullptr;
     p->qcube_m = 0;
-    int rc = plan_alloc(p, (void**)&p->d_qcube, sizeof(float) * (size_t)per * p->M);
+    int rc = plan_alloc(p, (void**)&p->d_qcube, sizeof(float) * (size_t)per * tl.nin);
     if (rc) return rc;
-    p->qcube_m = p->M;
+    p->qcube_m = tl.nin;
   }
-  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, p->M, p->d_qtab, p->nsq, p->d_qcube);
+  Slots mode{};
+  for (int i = 0; i < tl.nin; ++i) mode.s[i] = tl.in_mode[i];
+  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, tl.nin, mode, p->d_qtab, p->nsq, p->d_qcube);
   AAR_CUDA_TRY(p, cudaGetLastError());
   // made on the legacy stream once per table set; runs on the caller's
   // streams read it afterwards
@@ -978,31 +992,7 @@ int profile_modal_rows(Plan* p, float2* work, int64_t nrows, cudaStream_t st) {
   if (p->nr_active == 0) return set_err(p, "profile rows: no modal terms"), AAR_ERR_STATE;
   const int64_t fs = nrows * p->HP;
   if (p->jit) return jit_modal_rows(p, work, fs, st, nrows);
-  return dispatch_n(p->N, [&](auto nc) {
-    constexpr int N = decltype(nc)::value;
-    ModalRowOp op;
-    const TermList& tl = *(const TermList*)p->host_terms.data();
-    const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
-    constexpr int LS = RowCfg<N>::LS;
-    op.M = p->M;
-    op.nr = tl.nr;
-    for (int i = 0; i < kMaxModes; ++i) op.r_of_slot[i] = tl.r_of_slot[i];
-    for (int i = 0; i <= kMaxModes; ++i) op.begin[i] = tl.begin[i];
-    for (int sl = 0; sl < tl.nr; ++sl)
-      for (int i = tl.begin[sl]; i < tl.begin[sl + 1]; ++i) {
-        const uint32_t early = ft[i].r != tl.r_of_slot[sl] ? 1u : 0u;
-        op.t[i].off = (uint32_t)(ft[i].p * LS) | ((uint32_t)(ft[i].q * LS) << 16) | (early << 31);
-        op.t[i].c = ft[i].c;
-      }
-    const size_t sm_rows = Launch<N>::row_smem(p->M + 1);
-    {
-      ProfScope ps_(p, "modal_rows", st);
-      k_rows<N, ModalRowOp><<<(unsigned)nrows, kRowThreads, sm_rows, st>>>(op, work, fs, p->HP, p->d_twN, p->d_twH);
-    }
-    AAR_CUDA_TRY(p, cudaGetLastError());
-    p->last_launches += 1;
-    return AAR_OK;
-  });
+  return dispatch_n(p->N, [&](auto nc) { return Launch<decltype(nc)::value>::modal_rows(p, work, fs, nrows, st); });
 }
 
 int fused_modal(Plan* p, cudaStream_t st) {
@@ -1179,9 +1169,9 @@ struct Xform {
   static constexpr int64_t tiles = TileCfg<N>::TILES;
   static int c2r(Plan* p, float2* slot, cudaStream_t st) {
     using R = RowCfg<N>;
-    int rc = run_pass<N, 0, +1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_x");
+    int rc = run_pass<N, 0, +1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_x");
     if (rc) return rc;
-    if ((rc = run_pass<N, 1, +1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_y"))) return rc;
+    if ((rc = run_pass<N, 1, +1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_y"))) return rc;
     int lpb = 8 * R::LPW;
     int64_t nrows = (int64_t)N * N;
     dim3 g2((unsigned)((nrows + lpb - 1) / lpb), 1);
@@ -1205,9 +1195,9 @@ struct Xform {
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
-    int rc = run_pass<N, 1, -1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_y");
+    int rc = run_pass<N, 1, -1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_y");
     if (rc) return rc;
-    return run_pass<N, 0, -1>(p, AxisOp<N>{slot, 0, nullptr}, tiles, st, "xform_x");
+    return run_pass<N, 0, -1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_x");
   }
 };
 

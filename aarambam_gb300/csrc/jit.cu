@@ -40,26 +40,39 @@ struct JitState {
 
 static std::string gen_source(int N, int M, int minb, int threads, int pairs, const TermList& tl,
                               const std::vector<Term>& terms) {
-  std::string s;
-  // kCoef at global scope: its symbol name is not mangled (cudaLibraryGetGlobal)
-  s += "#include \"rows.cuh\"\n";
-  s += "__constant__ float kCoef[" + std::to_string(terms.empty() ? 1 : terms.size()) + "];\n";
-  s += "namespace aar {\n";
-  s += "struct JitRowOp {\n";
+  std::string s = "struct JitRowOp {\n";
   s += "  static constexpr int min_blocks(int) { return " + std::to_string(minb) + "; }\n";
   s += "  static constexpr bool kPairs = " + std::string(pairs ? "true" : "false") + ";\n";
   s += "  static constexpr bool kZfac = false;\n";
-  s += "  __device__ int nin() const { return " + std::to_string(M) + "; }\n";
-  s += "  __device__ int in_slot(int l) const { return l; }\n";
+  // maps of the inputs and outputs to field slots and lines: the identity
+  // where it is one, else constant memory (a switch in the loops over lines
+  // cost the 512^3 rows 5.8 -> 7.2 ms)
+  std::string consts;
+  auto map = [&](const char* name, int n, auto&& value) {
+    bool id = true;
+    std::string v;
+    for (int i = 0; i < n; ++i) {
+      id = id && value(i) == i;
+      v += (i ? "," : "") + std::to_string(value(i));
+    }
+    if (!id) consts += std::string("__constant__ int k_") + name + "[] = {" + v + "};\n";
+    s += std::string("  __device__ int ") + name + "(int l) const { return " +
+         (id ? "l" : std::string("k_") + name + "[l]") + "; }\n";
+  };
+  const int nin = tl.nin;
+  s += "  __device__ int nin() const { return " + std::to_string(nin) + "; }\n";
+  map("in_slot", nin, [&](int i) { return tl.in_mode[i]; });
+  map("in_line", nin, [&](int i) { return tl.line[tl.in_mode[i]]; });
   s += "  __device__ int nout() const { return " + std::to_string(tl.nr) + "; }\n";
-  s += "  __device__ int out_line(int l) const {\n    switch (l) {\n";
-  for (int i = 0; i < tl.nr; ++i) s += "      case " + std::to_string(i) + ": return " + std::to_string(tl.r_of_slot[i]) + ";\n";
-  s += "    }\n    return 0;\n  }\n";
-  s += "  __device__ int out_slot(int l) const { return out_line(l); }\n";
+  map("out_slot", tl.nr, [&](int i) { return tl.r_of_slot[i]; });
+  map("out_line", tl.nr, [&](int i) { return tl.line[tl.r_of_slot[i]]; });
   s += "  template <int K>\n  __device__ __forceinline__ void combine(float2* sm, const int* pos, int LS) const {\n";
-  s += "    float2 f[" + std::to_string(M) + "][K];\n";
-  s += "#pragma unroll\n    for (int p = 0; p < " + std::to_string(M) + "; ++p)\n";
-  s += "#pragma unroll\n      for (int i = 0; i < K; ++i) f[p][i] = sm[p * LS + pos[i]];\n";
+  s += "    float2 f[" + std::to_string(nin) + "][K];\n";
+  for (int p = 0; p < nin; ++p)
+    s += "#pragma unroll\n    for (int i = 0; i < K; ++i) f[" + std::to_string(p) + "][i] = sm[" +
+         std::to_string(tl.line[tl.in_mode[p]]) + " * LS + pos[i]];\n";
+  int in_of[kMaxModes] = {};  // f index of a mode
+  for (int i = 0; i < nin; ++i) in_of[tl.in_mode[i]] = i;
   // one block per output slot (the counter-term f0 f2 -> g1 with its own
   // target r).  The slot's terms are factored: greedily, the field that
   // occurs in most remaining terms is taken out, g_r += f_F (sum_t c_t f_t),
@@ -86,7 +99,7 @@ static std::string gen_source(int N, int M, int minb, int threads, int pairs, co
           continue;
         }
         const int o = terms[t].p == F ? terms[t].q : terms[t].p;
-        const std::string c = "kCoef[" + std::to_string(t) + "]", fo = "f[" + std::to_string(o) + "][i]";
+        const std::string c = "kCoef[" + std::to_string(t) + "]", fo = "f[" + std::to_string(in_of[o]) + "][i]";
         if (first)
           s += "      {\n      float2 h[K];\n#pragma unroll\n      for (int i = 0; i < K; ++i) h[i] = make_float2(" + c + " * " +
                fo + ".x, " + c + " * " + fo + ".y);\n";
@@ -95,14 +108,17 @@ static std::string gen_source(int N, int M, int minb, int threads, int pairs, co
                c + ", " + fo + ".y, h[i].y); }\n";
         first = false;
       }
-      const std::string fF = "f[" + std::to_string(F) + "][i]";
+      const std::string fF = "f[" + std::to_string(in_of[F]) + "][i]";
       s += "#pragma unroll\n      for (int i = 0; i < K; ++i) { a[i].x = fmaf(" + fF + ".x, h[i].x, a[i].x); a[i].y = fmaf(" + fF +
            ".y, h[i].y, a[i].y); }\n      }\n";
       rem.swap(keep);
     }
-    s += "#pragma unroll\n      for (int i = 0; i < K; ++i) sm[" + std::to_string(r) + " * LS + pos[i]] = a[i];\n    }\n";
+    s += "#pragma unroll\n      for (int i = 0; i < K; ++i) sm[" + std::to_string(tl.line[r]) + " * LS + pos[i]] = a[i];\n    }\n";
   }
   s += "  }\n};\n}  // namespace aar\n";
+  // kCoef at global scope: its symbol name is not mangled (cudaLibraryGetGlobal)
+  s = "#include \"rows.cuh\"\n__constant__ float kCoef[" + std::to_string(terms.empty() ? 1 : terms.size()) +
+      "];\nnamespace aar {\n" + consts + s;
   s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(threads) + ", " + std::to_string(minb) +
        ") aar_modal_rows_jit(float2* work, long long fs, int HP, const float2* __restrict__ twN, "
        "const float2* __restrict__ twH) {\n";
@@ -188,13 +204,13 @@ int jit_prepare(Plan* p) {
   const int N = p->N, M = p->M;
   const int minb = p->jit_minb > 0 ? p->jit_minb : (N >= 1024 ? 2 : 3);
   // default block size: 320 threads (ten warps) at N = 1024 where they take
-  // the M input lines in fewer rounds than eight warps (measured at 1024^3,
+  // the input lines in fewer rounds than eight warps (measured at 1024^3,
   // 20 modes: 362 vs 372 ms per step); the autotuner may choose otherwise
   const int threads = p->jit_threads > 0                                   ? p->jit_threads
-                      : (N >= 1024 && (M + 9) / 10 < (M + 7) / 8) ? 320
+                      : (N >= 1024 && (tl.nin + 9) / 10 < (tl.nin + 7) / 8) ? 320
                                                                        : kRowThreadsHost;
   const int regcap = 65536 / (threads * minb);
-  const int pairs = 2 * 2 * M + 16 <= regcap * 3 / 4;  // f values of two positions fit the register budget
+  const int pairs = 2 * 2 * tl.nin + 16 <= regcap * 3 / 4;  // f values of two positions fit the register budget
   std::string key = std::to_string(N) + ":" + std::to_string(M) + ":" + std::to_string(minb) + ":" +
                     std::to_string(threads) + ":" + std::to_string(pairs) + ":";
   for (const Term& t : terms) key += std::to_string(t.p) + "," + std::to_string(t.q) + "," + std::to_string(t.r) + ";";
@@ -256,7 +272,7 @@ int jit_prepare(Plan* p) {
     j->acc_fs = (int64_t)N * N * p->HP;
     p->jit = j;
   }
-  j->smem = sizeof(float2) * ((size_t)(M + 1) * p->row_ls + p->row_lt);
+  j->smem = sizeof(float2) * ((size_t)tl.nlines * p->row_ls + p->row_lt);
   if (cudaFuncSetAttribute((const void*)j->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)j->smem) !=
       cudaSuccess) {
     cudaGetLastError();

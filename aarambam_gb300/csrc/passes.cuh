@@ -13,7 +13,8 @@
 // (included inside namespace aar)
 
 template <int N, int AXIS, int SIGN, class Op>
-__global__ void __launch_bounds__(TileCfg<N>::THREADS, TileCfg<N>::MINB) k_pass(Op op, const float2* __restrict__ tw2) {
+__global__ void __launch_bounds__(TileCfg<N>::THREADS, TileCfg<N>::MINB) k_pass(const __grid_constant__ Op op,
+                                                                                       const float2* __restrict__ tw2) {
   using C = TileCfg<N>;
   extern __shared__ float2 ex[];
   const int w = threadIdx.x % C::W, t = threadIdx.x / C::W;
@@ -43,17 +44,22 @@ __device__ __forceinline__ void tile_coords(unsigned tile, int& o, int& c0) {
   c0 = (int)(tile % TileCfg<N>::NCOL) * TileCfg<N>::W;
 }
 
-// In-place complex FFT of fields (slot_map[f] or f), items f * tiles + tile.
+// Field slots of a pass (indexed in the kernel's parameter space).
+struct Slots {
+  int s[kMaxModes];
+};
+
+// In-place complex FFT of the fields slot.s[f], items f * tiles + tile.
 template <int N>
 struct AxisOp {
   static constexpr bool kPre = false, kPost = false;
   float2* base;
   int64_t fs;
-  const int* slot_map;  // optional field indirection (active modal slots)
+  Slots slot;
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     const unsigned f = item / TileCfg<N>::TILES;
     tile_coords<N>(item - f * TileCfg<N>::TILES, o, c0);
-    c = slot_map ? slot_map[f] : (int)f;
+    c = slot.s[f];
   }
   __device__ const float2* src(int c) const { return base + (int64_t)c * fs; }
   __device__ float2* dst(int c) const { return base + (int64_t)c * fs; }
@@ -74,7 +80,8 @@ __device__ __forceinline__ void group_order(unsigned item, unsigned nc, unsigned
 }
 
 // First modal pass: phi tile times q_p(k) (zero on the cut, DC and padding
-// columns), inverse x FFT, into field p.  The factors come from the plan's
+// columns), inverse x FFT, into field p, for the modes p = mode.s[c] that the
+// products read.  The factors come from the plan's
 // filter cube (qcube_build), laid out so that a warp's 32 factors of a
 // value index are 4 rows of 8 consecutive floats; they load together with
 // the tile.
@@ -84,21 +91,22 @@ struct XinvOp {
   const float2* phi;
   float2* work;
   int64_t fs;
-  int M;
+  int nin;
+  Slots mode;
   unsigned grp;
-  const float* qcube;  // [M][|ky|][kz / 8][|kx|][8]
-  __device__ void coords(unsigned item, int& o, int& c0, int& p) const {
+  const float* qcube;  // [nin][|ky|][kz / 8][|kx|][8]
+  __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     unsigned t;
-    group_order<N>(item, (unsigned)M, grp, t, p);
+    group_order<N>(item, (unsigned)nin, grp, t, c);
     tile_coords<N>(t, o, c0);
   }
   __device__ const float2* src(int) const { return phi; }
-  __device__ float2* dst(int p) const { return work + (int64_t)p * fs; }
-  __device__ void pre(float2* v, int o, int kz, int p, int t) const {
+  __device__ float2* dst(int c) const { return work + (int64_t)mode.s[c] * fs; }
+  __device__ void pre(float2* v, int o, int kz, int c, int t) const {
     using C = TileCfg<N>;
     constexpr int K = N / 2 + 1;
     const int ay = o <= N / 2 ? o : N - o;
-    const float* q = qcube + ((((int64_t)p * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
+    const float* q = qcube + ((((int64_t)c * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
     float f[C::R1];
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) {
@@ -137,7 +145,7 @@ struct LptXOp {
     tile_coords<N>(t, o, c0);
   }
   __device__ const float2* src(int) const { return in; }
-  __device__ float2* dst(int c) const { return work + (int64_t)(c == 0 ? out[0] : c == 1 ? out[1] : out[2]) * fs; }
+  __device__ float2* dst(int c) const { return work + (int64_t)out[c] * fs; }
   __device__ void pre(float2* v, int, int kz, int c, int t) const {
     using C = TileCfg<N>;
     float f[C::R1];
@@ -178,22 +186,14 @@ struct YFanOp {
     group_order<N>(item, NC, grp, t, c);
     tile_coords<N>(t, o, c0);
   }
-  // a[c] by selects (a dynamic index into the parameter block would copy it
-  // to local memory)
-  __device__ static int at(const int* a, int c) {
-    int r = a[0];
-#pragma unroll
-    for (int j = 1; j < NC; ++j) r = c == j ? a[j] : r;
-    return r;
-  }
-  __device__ const float2* src(int c) const { return work + (int64_t)at(in, c) * fs; }
-  __device__ float2* dst(int c) const { return work + (int64_t)at(out, c) * fs; }
+  __device__ const float2* src(int c) const { return work + (int64_t)in[c] * fs; }
+  __device__ float2* dst(int c) const { return work + (int64_t)out[c] * fs; }
   __device__ void pre(float2* v, int, int, int c, int t) const {
     using C = TileCfg<N>;
     // axis_factor with its table loads issued together (a branch per value
     // left them one after another: 15.7 vs 10.2 ms for the displacements at
     // 1024^3)
-    const int ty = at(type, c);
+    const int ty = type[c];
     float f[C::R1];
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) f[i] = ty >= 3 ? __ldg(isinc2 + tile_n<N>(t, i)) : 1.f;

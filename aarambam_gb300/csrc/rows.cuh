@@ -293,7 +293,7 @@ __device__ __forceinline__ void row_r2c_post_fold(const float2* line, float2* __
 }
 
 // Generic row kernel.  For each memory row (blockIdx.x): c2r of `nin`
-// input fields (slots in_slot[]), a per-position combine step Op, r2c of
+// input fields (slots in_slot[], into lines in_line[]), a per-position combine step Op, r2c of
 // `nout` output lines into slots out_slot[].  One warp per line at a time.
 // THREADS = 256 (the library's kernels; the NVRTC kernel may use 320) with
 // two resident blocks per SM: while one block waits at a phase barrier (its
@@ -321,7 +321,7 @@ __device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs
   if constexpr (!RowFold<N>::value) {
     for (int l = 0; l < op.nin(); ++l) {
       const float2* X = work + (int64_t)op.in_slot(l) * fs + row * HP;
-      float2* line = sm + l * C::LS;
+      float2* line = sm + op.in_line(l) * C::LS;
       for (int k = threadIdx.x; k <= H; k += THREADS) cp_async8(line + spad(k), X + k);
     }
     cp_async_commit();
@@ -336,7 +336,7 @@ __device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs
     lt_fill<h, 16, 2>(sm_all, twH, threadIdx.x, THREADS);
     __syncthreads();
     for (int l = warp; l < op.nin(); l += nwarps) {
-      float2* line = sm + l * C::LS;
+      float2* line = sm + op.in_line(l) * C::LS;
       const float2* X = work + (int64_t)op.in_slot(l) * fs + row * HP;
       if constexpr (Op::kZfac) row_c2r_pre_fold<N>(line, lane, twN, twH, op.zfac(l), X);
       else row_c2r_pre_fold<N>(line, lane, twN, twH, ZFac{0, 0.f, nullptr}, X);
@@ -366,7 +366,7 @@ __device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs
   for (int l0 = warp * C::LPW; l0 < op.nin(); l0 += nwarps * C::LPW) {
     int l = l0 + sub;
     bool act = l < op.nin() && sub < C::LPW;
-    float2* line = sm + (act ? l : 0) * C::LS;
+    float2* line = sm + (act ? op.in_line(l) : 0) * C::LS;
     if (act) {
       if constexpr (Op::kZfac) row_c2r_pre_inplace<N>(line, t, C::T, twN, op.zfac(l));
       else row_c2r_pre_inplace<N>(line, t, C::T, twN);
