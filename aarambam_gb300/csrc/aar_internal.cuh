@@ -12,7 +12,6 @@
 
 namespace aar {
 
-constexpr int kRowThreadsHost = 256;  // block size of the row kernels (rows.cuh kRowThreads)
 
 // Host twin of keep_cell's cube bound.
 int host_kcut(int nsample, double box);
@@ -78,12 +77,10 @@ struct Plan {
   // modal term list (device)
   void* d_terms = nullptr;
   std::vector<char> host_terms;  // the same term list on the host (kernel parameter of the row combine)
-  int row_ls = 0;                // row-kernel line stride (float2) of this grid size
-  int row_lt = 0;                // float2 slots of the row kernels' lane twiddle table
   void* jit = nullptr;           // run-time specialised modal row kernel (jit.cu), or null
   int jit_mode = 1;              // 0 off, 1 for N >= 256, 2 always
   int jit_minb = 0;              // resident row blocks per SM of the NVRTC kernel (0: by N)
-  int jit_threads = 0;           // threads per block of the NVRTC row kernel (0: 256)
+  int jit_threads = 0;           // threads per block of the NVRTC folded row kernel (0: by the lines)
   int64_t xpass_group = 1;       // tiles per item group of the multi-output x passes (passes.cuh)
   int noise_one_draw = 0;        // noise columns one draw at a time (AAR_NOISE_ONE_DRAW=1, a check)
   std::string jit_status = "off";

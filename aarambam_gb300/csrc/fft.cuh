@@ -146,6 +146,10 @@ __host__ __device__ constexpr int num_stages(int N, int E) {
   return s;
 }
 
+// First radix of the two-stage transforms (tile.cuh, rows.cuh): N = R1 R2,
+// R2 <= R1 <= 32.
+__host__ __device__ constexpr int two_stage_r1(int N) { return N >= 512 ? 32 : N >= 128 ? 16 : N >= 32 ? 8 : 4; }
+
 // padded shared-memory index: one spare slot per 16 entries, so that the
 // first Stockham stage's stores (lane j writes j R + r, R = 8 or 16) and the
 // natural-order loads both fall on distinct banks within a half-warp
@@ -376,11 +380,6 @@ __device__ __forceinline__ void line_fft_smem(float2* s, int t, const float2* __
     line_sync<T>(bar_id);
     line_fft_smem<N, T, SIGN, S + 1, TWS, LT>(s, t, tw, act, bar_id);
   }
-}
-
-// lanes per line: 16 values per lane for N >= 512, 8 below
-__host__ __device__ constexpr int lanes_for(int N) {
-  return N >= 512 ? N / 16 : (N / 8 >= 1 ? (N / 8 < 32 ? N / 8 : 32) : 1);
 }
 
 }  // namespace aar

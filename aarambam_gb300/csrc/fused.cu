@@ -146,11 +146,39 @@ __global__ void __launch_bounds__(256) k_scale_twb(const float2* __restrict__ ph
 }
 
 // ----------------------------------------------------------- row passes
-// (rows.cuh: RowCfg, the c2r / r2c row steps and rows_body)
+// (rows.cuh: rows_pairs, rows_fold)
+template <int N>
+constexpr int pair_min_blocks(int threads) {
+  const int regs = two_stage_r1(N) == 32 ? 128 : 64;
+  return 65536 / regs / threads > 0 ? 65536 / regs / threads : 1;
+}
+constexpr int kPairThreads = 256;
 template <int N, class Op>
-__global__ void __launch_bounds__(kRowThreads, Op::min_blocks(N)) k_rows(Op op, float2* work, int64_t fs, int HP,
-                                                       const float2* __restrict__ twN, const float2* __restrict__ twH) {
-  rows_body<N>(op, work, fs, HP, twN, twH);
+__global__ void __launch_bounds__(kPairThreads, pair_min_blocks<N>(kPairThreads))
+    k_rows_pairs(const __grid_constant__ Op op, float2* work, int64_t fs, int HP, int64_t nrows, int pr,
+                 const float2* __restrict__ tw2) {
+  rows_pairs<N, Op, kPairThreads>(op, work, fs, HP, nrows, tw2, pr);
+}
+template <int N, class Op>
+__global__ void __launch_bounds__(kRowThreads, 2) k_rows_fold(const __grid_constant__ Op op, float2* work, int64_t fs,
+                                                              int HP, const float2* __restrict__ twN,
+                                                              const float2* __restrict__ twH) {
+  rows_fold<N>(op, work, fs, HP, twN, twH);
+}
+// The source rows: 6 lines per pair, PR = 32 / T pairs, 192 threads.
+constexpr int kSixThreads = 192;
+// resident blocks: 96 registers hold 32 values per lane in these kernels
+// without spills (three blocks against two with 138-146: source rows 8.9 vs
+// 10.7 ms at 1024^3, 1.10 vs 1.31 at 512^3)
+template <int N>
+constexpr int six_min_blocks() {
+  return two_stage_r1(N) == 32 ? 3 : 5;
+}
+template <int N, class Op>
+__global__ void __launch_bounds__(kSixThreads, six_min_blocks<N>())
+    k_rows_six(const __grid_constant__ Op op, float2* work, int64_t fs, int HP, int64_t nrows,
+               const float2* __restrict__ tw2) {
+  rows_pairs<N, Op, kSixThreads>(op, work, fs, HP, nrows, tw2, 32 / PairCfg<N>::T);
 }
 
 // One product term of the row combine, as a kernel parameter: the shared-
@@ -166,17 +194,15 @@ struct TermC {
 // a term through the uniform constant path; each thread forms two positions
 // per term.
 struct ModalRowOp {
-  // resident rows per SM: shared memory holds two at 1024^3 with 20 modes;
-  // below that registers decide (three rows: 80 registers, no spill)
-  static constexpr int min_blocks(int n) { return n >= 1024 ? 2 : 3; }
   static constexpr bool kZfac = false;
   static constexpr bool kPairs = true;
-  int ni, nr;
+  int ni, nr, nl;
   int in_mode[kMaxModes], line_in[kMaxModes];
   int r_of_slot[kMaxModes], line_out[kMaxModes];
   int begin[kMaxModes + 1];
   TermC t[kMaxTerms];
   __device__ int nin() const { return ni; }
+  __device__ int nlines() const { return nl; }
   __device__ int in_slot(int l) const { return in_mode[l]; }
   __device__ int in_line(int l) const { return line_in[l]; }
   __device__ int nout() const { return nr; }
@@ -230,9 +256,6 @@ struct ModalRowOp {
 // 2LPT source (main.c:1284-1294): lines 0..5 hold d00 d01 d02 d11 d12 d22;
 // the source goes to line 0, written to slot `out`.
 struct SourceRowOp {
-  // seven lines per row (at 512^3 four blocks spill a few bytes with 16
-  // values per lane and still ran faster than three: 2.33 vs 2.63 ms)
-  static constexpr int min_blocks(int) { return 4; }
   static constexpr bool kPairs = true;
   static constexpr bool kZfac = true;  // z factors of the Hessians (1, 1, kz, 1, kz, kz^2)
   int out;
@@ -240,6 +263,7 @@ struct SourceRowOp {
   const float* isinc2;
   __device__ ZFac zfac(int l) const { return ZFac{l == 2 || l == 4 ? 1 : l == 5 ? 2 : 0, kF, isinc2}; }
   __device__ int nin() const { return 6; }
+  __device__ int nlines() const { return 6; }
   __device__ int in_slot(int l) const { return l; }
   __device__ int in_line(int l) const { return l; }
   __device__ int nout() const { return 1; }
@@ -275,40 +299,38 @@ struct ZTypes {
     return i < 6 ? r : 0;
   }
 };
+constexpr int kC2rThreads = 128;
 template <int N>
-__global__ void __launch_bounds__(256) k_rows_c2r(float2* work, int64_t fs, int HP, int first, int64_t nrows,
-                                                  const float2* __restrict__ twN, const float2* __restrict__ twH,
-                                                  ZTypes zt) {
-  using C = RowCfg<N>;
-  constexpr int H = C::H;
+constexpr unsigned c2r_blocks() {  // of a field's N^2 rows
+  constexpr int rows = 2 * (kC2rThreads / PairCfg<N>::T);
+  return (unsigned)(((int64_t)N * N + rows - 1) / rows);
+}
+template <int N>
+constexpr size_t pair_line_smem(int threads) {  // one line buffer per T threads
+  return sizeof(float2) * (size_t)(threads / PairCfg<N>::T) * PairCfg<N>::LS;
+}
+template <int N>
+__global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
+    k_rows_c2r(float2* work, int64_t fs, int HP, int first, int64_t nrows, const float2* __restrict__ tw2, ZTypes zt) {
+  using C = PairCfg<N>;
   extern __shared__ float2 sm[];
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int sub = lane / C::T, t = lane % C::T;
-  int lines_per_block = (blockDim.x >> 5) * C::LPW;
-  int64_t row = (int64_t)blockIdx.x * lines_per_block + warp * C::LPW + sub;
-  bool act = row < nrows && sub < C::LPW;
-  float2* line = sm + (warp * C::LPW + sub) * C::LS;
+  const int u = threadIdx.x / C::T, t = threadIdx.x % C::T;
+  const int64_t row = 2 * ((int64_t)blockIdx.x * (kC2rThreads / C::T) + u);
+  const bool act = row < nrows;
   float2* f = work + (int64_t)(first + blockIdx.y) * fs + (act ? row : 0) * HP;
   const ZFac zf{zt.at(blockIdx.y), zt.kF, zt.isinc2};
-  if constexpr (RowFold<N>::value) {
-    // folded radix-2 (rows.cuh): the halves hold z_{2m} and z_{2m+1}; lane
-    // t writes the pair (z_{2m}, z_{2m+1}) as one 16-byte store
-    constexpr int h = H / 2, HO = h + h / 16;
-    if (act) row_c2r_pre_fold<N>(line, lane, twN, twH, zf, f);
-    __syncwarp();
-    line_fft_smem<h, 16, +1, 0, 2>(line + (lane >> 4) * HO, lane & 15, twH, act);
-    if (act)
-      for (int m = lane; m < h; m += 32) {
-        const float2 e = line[spad(m)], o = line[spad(m) + HO];
-        reinterpret_cast<float4*>(f)[m] = make_float4(e.x, e.y, o.x, o.y);
-      }
-    return;
+  float2 v[C::R1];
+  pair_spectrum<N, true>(v, f, row + 1 < nrows ? f + HP : nullptr, t, zf, act);
+  pair_fft<N, +1>(v, sm + u * C::LS, t, tw2, act);  // every lane of the line has read its rows
+  float* a = reinterpret_cast<float*>(f);
+  if (act) {
+#pragma unroll
+    for (int i = 0; i < C::R1; ++i) a[t + C::T * i] = v[i].x;
+    if (row + 1 < nrows) {
+#pragma unroll
+      for (int i = 0; i < C::R1; ++i) a[2 * HP + t + C::T * i] = v[i].y;
+    }
   }
-  if (act) row_c2r_pre<N>(f, line, t, C::T, twN, zf);
-  __syncwarp();
-  line_fft_smem<H, C::T, +1>(line, t, twH, act);
-  if (act)
-    for (int n = t; n < H; n += C::T) f[n] = line[spad(n)];
 }
 
 // ----------------------------------------------------------- 2LPT passes
@@ -536,79 +558,105 @@ __global__ void k_lattice_glass(int g, double gsp, float* glass) {
   }
 }
 
-// The six displacement rows of RPB memory rows (c2r with the z factors, as
-// k_rows_c2r; warp c takes field c), then the particles on the rows' grid
-// points: Pos / Vel from the grid values (readout_one's on-grid branch,
-// main.c:1486-1509) and IDs, written at their tiled-glass particle index.
-// Rows [row0, row0 + nrows) of the x-blocked order.
+// The six displacement rows of PR = 32 / T pairs of memory rows (c2r with the
+// z factors, as k_rows_c2r; one line per T threads), then the particles on the
+// rows' grid points: Pos / Vel from the grid values (readout_one's on-grid
+// branch, main.c:1486-1509) and IDs, written at their tiled-glass particle
+// index.  A warp's 32 consecutive grid points are 32 consecutive particles
+// unless a tile edge falls between them: their Pos and Vel go through shared
+// memory and out as whole lines (stores 12 bytes apart write every sector
+// three times).  Rows [row0, row0 + nrows) of the x-blocked order, row0 even.
 template <int N>
 struct LatticeCfg {
-  static constexpr int RPB = RowFold<N>::value ? 1 : RowCfg<N>::LPW;  // rows per block
-  static constexpr size_t SMEM = sizeof(float2) * (size_t)RPB * 6 * RowCfg<N>::LS;
+  static constexpr int PR = 32 / PairCfg<N>::T;
+  static constexpr int LINES = 6 * PR;
+  static constexpr size_t SMEM = sizeof(float2) * (size_t)LINES * PairCfg<N>::LS + sizeof(float) * kSixThreads * 6;
 };
 template <int N>
-__global__ void __launch_bounds__(192, 4) k_rows_lattice(const float2* __restrict__ work, int64_t fs, int HP,
-                                                         const float2* __restrict__ twN, const float2* __restrict__ twH,
-                                                         ZTypes zt, ReadArgs ra, int g, int tile,
-                                                         const float* __restrict__ lpa, float* pos, float* vel,
-                                                         int* ids, int64_t row0, int64_t nrows) {
-  using C = RowCfg<N>;
-  constexpr int H = C::H, RPB = LatticeCfg<N>::RPB;
-  extern __shared__ float2 sm[];  // [RPB][6][LS]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t rbase = row0 + (int64_t)blockIdx.x * RPB, rend = row0 + nrows;
-  const ZFac zf{zt.at(warp), zt.kF, zt.isinc2};
-  if constexpr (RowFold<N>::value) {
-    constexpr int h = H / 2, HO = h + h / 16;
-    const bool act = rbase < rend;
-    // (the lane twiddle table of rows_body cost more than it saved here:
-    // one row per block, 13.1 -> 14.5 ms)
-    float2* line = sm + warp * C::LS;
-    if (act) row_c2r_pre_fold<N>(line, lane, twN, twH, zf, work + (int64_t)warp * fs + rbase * HP);
-    __syncwarp();
-    line_fft_smem<h, 16, +1, 0, 2>(line + (lane >> 4) * HO, lane & 15, twH, act);
-  } else {
-    const int sub = lane / C::T, t = lane % C::T;
-    const int64_t row = rbase + sub;
-    const bool act = sub < RPB && row < rend;
-    float2* line = sm + ((act ? sub : 0) * 6 + warp) * C::LS;
-    if (act) row_c2r_pre<N>(work + (int64_t)warp * fs + row * HP, line, t, C::T, twN, zf);
-    __syncwarp();
-    line_fft_smem<H, C::T, +1>(line, t, twH, act);
+__global__ void __launch_bounds__(kSixThreads, six_min_blocks<N>())
+    k_rows_lattice(const float2* __restrict__ work, int64_t fs, int HP, const float2* __restrict__ tw2, ZTypes zt,
+                   ReadArgs ra, int g, int tile, const float* __restrict__ lpa, float* pos, float* vel, int* ids,
+                   int64_t row0, int64_t nrows) {
+  using C = PairCfg<N>;
+  using L = LatticeCfg<N>;
+  static_assert(kXB % 2 == 0, "the rows of a pair are (x, y) and (x + 1, y)");
+  extern __shared__ float2 sm[];  // [PR][6][LS], then the warps' particle staging
+  const int64_t rbase = row0 + (int64_t)blockIdx.x * (2 * L::PR), rend = row0 + nrows;
+  {
+    const int u = threadIdx.x / C::T, t = threadIdx.x % C::T;
+    const int pr = u / 6, c = u - 6 * pr;
+    const int64_t row = rbase + 2 * pr;
+    const bool act = row < rend;
+    const ZFac zf{zt.at(c), zt.kF, zt.isinc2};
+    const float2* X = work + (int64_t)c * fs + (act ? row : 0) * HP;
+    float2* ln = sm + u * C::LS;
+    float2 v[C::R1];
+    pair_spectrum<N, true>(v, X, row + 1 < rend ? X + HP : nullptr, t, zf, act);
+    pair_fft<N, +1>(v, ln, t, tw2, act);
+    if (act) {
+#pragma unroll
+      for (int i = 0; i < C::R1; ++i) ln[t + C::T * i] = v[i];
+    }
   }
   __syncthreads();
+  // a warp takes 32 consecutive grid points of a row pair at a time (N = 16:
+  // of two pairs)
   const int64_t g3 = (int64_t)g * g * g;
-  for (int q = threadIdx.x; q < RPB * N; q += blockDim.x) {
-    const int sub = q / N, z = q - sub * N;
-    const int64_t row = rbase + sub;
-    if (row >= rend) break;
-    int x, y;
-    row_xy(row, N, kXB, x, y);
-    float d[6];
+  const int lane = threadIdx.x & 31;
+  float* stp = reinterpret_cast<float*>(sm + L::LINES * C::LS) + (threadIdx.x >> 5) * 192;
+  float* stv = stp + 96;
+  for (int q0 = threadIdx.x - lane; q0 < L::PR * N; q0 += kSixThreads) {  // uniform over the warp
+    const int q = q0 + lane, pr = q / N, z = q - pr * N;
+    const int64_t row = rbase + 2 * pr;
+    const bool live = q < L::PR * N && row < rend;
+    const int tk = z / g, gk = z - tk * g;
+    int x = 0, y = 0;
+    float2 d2[6];
+    if (live) {
+      row_xy(row, N, kXB, x, y);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      float2 v;
-      if constexpr (RowFold<N>::value) {
-        // the folded transform leaves z_{2m} at m and z_{2m+1} at h + m
-        // (z_j = (x_{2j}, x_{2j+1})): x_z sits in the pair of z / 4
-        constexpr int h = H / 2, HO = h + h / 16;
-        v = sm[c * C::LS + spad(z >> 2) + (((z >> 1) & 1) ? HO : 0)];
-      } else {
-        v = sm[(sub * 6 + c) * C::LS + spad(z >> 1)];
+      for (int c = 0; c < 6; ++c) d2[c] = sm[(pr * 6 + c) * C::LS + z];
+    }
+    const float py = lpa[y], pz = lpa[z];
+    const int tj = y / g, gj = y - tj * g;
+    const bool line = N >= 32 && __all_sync(0xffffffffu, live && gk >= lane);  // one tile cell along z
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const bool on = live && row + s < rend;
+      float op[3], ov[3];
+      const int ti = (x + s) / g, gi = x + s - ti * g;
+      const int64_t n = (((int64_t)ti * tile + tj) * tile + tk) * g3 + ((int64_t)gi * g + gj) * g + gk;
+      if (on) {
+        float d[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) d[c] = s ? d2[c].y : d2[c].x;
+        const float p[3] = {lpa[x + s], py, pz};
+        move_particle(ra, p, d, d + 3, op, ov);
+        if (ids) ids[n] = (int)(n + 1);
       }
-      d[c] = (z & 1) ? v.y : v.x;
-    }
-    const float p[3] = {lpa[x], lpa[y], lpa[z]};
-    float op[3], ov[3];
-    move_particle(ra, p, d, d + 3, op, ov);
-    const int ti = x / g, gi = x - ti * g, tj = y / g, gj = y - tj * g, tk = z / g, gk = z - tk * g;
-    const int64_t n = (((int64_t)ti * tile + tj) * tile + tk) * g3 + ((int64_t)gi * g + gj) * g + gk;
+      if (line && __all_sync(0xffffffffu, on)) {
+        __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      pos[3 * n + c] = op[c];
-      vel[3 * n + c] = ov[c];
+        for (int c = 0; c < 3; ++c) {
+          stp[3 * lane + c] = op[c];
+          stv[3 * lane + c] = ov[c];
+        }
+        __syncwarp();
+        float* po = pos + 3 * (n - lane);
+        float* vo = vel + 3 * (n - lane);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          po[lane + 32 * c] = stp[lane + 32 * c];
+          vo[lane + 32 * c] = stv[lane + 32 * c];
+        }
+      } else if (on) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          pos[3 * n + c] = op[c];
+          vel[3 * n + c] = ov[c];
+        }
+      }
     }
-    if (ids) ids[n] = (int)(n + 1);
   }
 }
 
@@ -654,14 +702,25 @@ struct Launch {
   static constexpr int64_t kTiles = TileCfg<N>::TILES;
   static int64_t fstride(Plan* p) { return (int64_t)N * N * p->HP; }
   static unsigned group(Plan* p) { return (unsigned)std::min<int64_t>(p->xpass_group, kTiles); }
-  static constexpr size_t row_smem(int nlines) {
-    return sizeof(float2) * ((size_t)nlines * RowCfg<N>::LS + row_lt_slots<N>());
-  }
+  static constexpr size_t pair_smem(int lines) { return sizeof(float2) * (size_t)lines * PairCfg<N>::LS; }
+  static constexpr size_t kSixSmem = pair_smem(6 * (32 / PairCfg<N>::T));
+  // dynamic shared memory of k_rows_pairs: several row pairs up to kPairSmem,
+  // one whatever its lines
+  static constexpr size_t kPairSmem = 100 * 1024;
+  static constexpr size_t kPairSmemMax = std::max(kPairSmem, pair_smem(N < 1024 ? kMaxModes : 8));
   static int configure(Plan* p) {
-    size_t sm_rows = row_smem(kMaxModes + 1);
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows<N, ModalRowOp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_rows));
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows<N, SourceRowOp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_rows));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_pairs<N, ModalRowOp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kPairSmemMax));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_six<N, SourceRowOp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kSixSmem));
+    if constexpr (N == 1024)
+      AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_fold<N, ModalRowOp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)fold_smem(kMaxModes)));
     return AAR_OK;
+  }
+  static constexpr size_t fold_smem(int nlines) {
+    if constexpr (N == 1024) return sizeof(float2) * ((size_t)nlines * FoldCfg<N>::LS + FoldCfg<N>::LT);
+    else return 0;
   }
   static Slots slots(const int* s, int n) {
     Slots r{};
@@ -674,16 +733,18 @@ struct Launch {
     return run_pass<N, AXIS, SIGN>(p, AxisOp<N>{base, fstride(p), sl}, nf * kTiles, st, name);
   }
   static const TermList& terms(Plan* p) { return *(const TermList*)p->host_terms.data(); }
-  // the generic row kernel's term list as a kernel parameter
-  static ModalRowOp row_op(Plan* p) {
+  // the generic row kernel's term list as a kernel parameter, for lines LS
+  // float2 apart
+  static ModalRowOp row_op(Plan* p, int LS) {
     static_assert(sizeof(ModalRowOp) < 32000, "kernel parameter space");
     const TermList& tl = terms(p);
     const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
-    constexpr int LS = RowCfg<N>::LS;
-    static_assert(kMaxModes * LS < 0x8000, "line offsets fit 15 bits");
+    static_assert(kMaxModes * PairCfg<512>::LS < 0x8000 && 8 * PairCfg<1024>::LS < 0x8000 &&
+                  kMaxModes * FoldCfg<1024>::LS < 0x8000, "line offsets fit 15 bits");
     ModalRowOp op;
     op.ni = tl.nin;
     op.nr = tl.nr;
+    op.nl = tl.nlines;
     for (int i = 0; i < tl.nin; ++i) op.in_mode[i] = tl.in_mode[i], op.line_in[i] = tl.line[tl.in_mode[i]];
     for (int i = 0; i < tl.nr; ++i) op.r_of_slot[i] = tl.r_of_slot[i], op.line_out[i] = tl.line[tl.r_of_slot[i]];
     for (int i = 0; i <= tl.nr; ++i) op.begin[i] = tl.begin[i];
@@ -696,11 +757,22 @@ struct Launch {
     return op;
   }
   static int modal_rows(Plan* p, float2* work, int64_t fs, int64_t nrows, cudaStream_t st) {
-    const ModalRowOp op = row_op(p);
-    const size_t sm_rows = row_smem(terms(p).nlines);
+    const TermList& tl = terms(p);
     {
       ProfScope ps_(p, "modal_rows", st);
-      k_rows<N, ModalRowOp><<<(unsigned)nrows, kRowThreads, sm_rows, st>>>(op, work, fs, p->HP, p->d_twN, p->d_twH);
+      if (rows_use_pairs(N, tl.nlines)) {
+        // as many row pairs as give every T threads of a block a line, while
+        // two blocks' lines fit an SM
+        constexpr int slots = kPairThreads / PairCfg<N>::T;
+        int pr = std::max(1, slots / std::max(tl.nin, tl.nr));
+        while (pr > 1 && pair_smem(pr * tl.nlines) > kPairSmem) --pr;
+        k_rows_pairs<N, ModalRowOp><<<(unsigned)((nrows + 2 * pr - 1) / (2 * pr)), kPairThreads,
+                                      pair_smem(pr * tl.nlines), st>>>(row_op(p, PairCfg<N>::LS), work, fs, p->HP,
+                                                                       nrows, pr, p->d_tw2);
+      } else if constexpr (N == 1024) {
+        k_rows_fold<N, ModalRowOp><<<(unsigned)nrows, kRowThreads, fold_smem(tl.nlines), st>>>(
+            row_op(p, FoldCfg<N>::LS), work, fs, p->HP, p->d_twN, p->d_twH);
+      }
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -752,12 +824,12 @@ struct Launch {
       YFanOp<N> yf{p->d_work, fs, {0, 8, 8, 6, 6, 6}, {0, 1, 2, 3, 4, 5}, {0, 1, 0, 2, 1, 0}, 1, kF, a.isinc2};
       if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "lpt_ypass_inv_hess"))) return rc;
     }
-    size_t sm_rows = row_smem(7);
-    SourceRowOp op{6, a.m.g.kF, a.isinc2};
+    const SourceRowOp op{6, a.m.g.kF, a.isinc2};
     {
       ProfScope ps_(p, "lpt_rows_source", st);
-      k_rows<N, SourceRowOp><<<(unsigned)((int64_t)N * N), kRowThreads, sm_rows, st>>>(op, p->d_work, fs, p->HP, p->d_twN,
-                                                                                p->d_twH);
+      constexpr int rows = 2 * (32 / PairCfg<N>::T);  // of a block
+      k_rows_six<N, SourceRowOp><<<(unsigned)(((int64_t)N * N + rows - 1) / rows), kSixThreads, kSixSmem, st>>>(
+          op, p->d_work, fs, p->HP, (int64_t)N * N, p->d_tw2);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -779,15 +851,11 @@ struct Launch {
     // (fused_rows_lattice), which leaves no real fields behind
     p->disp_real = rows;
     if (!rows) return AAR_OK;
-    using R = RowCfg<N>;
-    int lines_per_block = 8 * R::LPW;
-    int64_t nrows = (int64_t)N * N;
-    dim3 grid((unsigned)((nrows + lines_per_block - 1) / lines_per_block), 6);
     const ZTypes zt{{3, 3, 4, 3, 3, 4}, a.m.g.kF, a.isinc2};
     {
       ProfScope ps_(p, "lpt_rows_c2r", st);
-      k_rows_c2r<N><<<grid, 256, sizeof(float2) * lines_per_block * R::LS, st>>>(p->d_work, fs, p->HP, 0, nrows,
-                                                                                p->d_twN, p->d_twH, zt);
+      k_rows_c2r<N><<<dim3(c2r_blocks<N>(), 6), kC2rThreads, pair_line_smem<N>(kC2rThreads), st>>>(
+          p->d_work, fs, p->HP, 0, (int64_t)N * N, p->d_tw2, zt);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -974,15 +1042,11 @@ int fused_prepare(Plan* p) {
   int rc = build_terms(p);
   if (rc) return rc;
   if ((rc = dispatch_n(p->N, [&](auto nc) {
-         p->row_ls = RowCfg<decltype(nc)::value>::LS;
-         p->row_lt = row_lt_slots<decltype(nc)::value>();
          return Launch<decltype(nc)::value>::configure(p);
        })))
     return rc;
   return jit_prepare(p);
 }
-
-static_assert(kRowThreads == kRowThreadsHost, "row kernel block size");
 
 // The plan's modal row kernel (NVRTC or generic) on nrows rows of caller
 // fields laid out with field stride nrows * HP: a harness that profiles the
@@ -1095,9 +1159,9 @@ int fused_rows_lattice(Plan* p, int g, int tile, float* d_pos, float* d_vel, int
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_lattice<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM));
     {
       ProfScope ps_(p, "lpt_rows_readout", st);
-      k_rows_lattice<N><<<(unsigned)((nrows + L::RPB - 1) / L::RPB), 192, L::SMEM, st>>>(
-          p->d_work, (int64_t)N * N * p->HP, p->HP, p->d_twN, p->d_twH, zt, read_args(p), g, tile, p->d_lpa, d_pos,
-          d_vel, d_ids, row0, nrows);
+      k_rows_lattice<N><<<(unsigned)((nrows + 2 * L::PR - 1) / (2 * L::PR)), kSixThreads, L::SMEM, st>>>(
+          p->d_work, (int64_t)N * N * p->HP, p->HP, p->d_tw2, zt, read_args(p), g, tile, p->d_lpa, d_pos, d_vel, d_ids,
+          row0, nrows);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -1145,53 +1209,46 @@ int fused_readout_glass(Plan* p, int64_t nglass, int tile, float* d_pos, float* 
 namespace aar {
 
 template <int N>
-__global__ void __launch_bounds__(256) k_rows_r2c(float2* f, int HP, int64_t nrows, const float2* __restrict__ twN,
-                                                  const float2* __restrict__ twH) {
-  using C = RowCfg<N>;
-  constexpr int H = C::H;
+__global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
+    k_rows_r2c(float2* f, int HP, int64_t nrows, const float2* __restrict__ tw2) {
+  using C = PairCfg<N>;
   extern __shared__ float2 sm[];
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int sub = lane / C::T, t = lane % C::T;
-  int lines_per_block = (blockDim.x >> 5) * C::LPW;
-  int64_t row = (int64_t)blockIdx.x * lines_per_block + warp * C::LPW + sub;
-  bool act = row < nrows && sub < C::LPW;
-  float2* line = sm + (warp * C::LPW + sub) * C::LS;
+  const int u = threadIdx.x / C::T, t = threadIdx.x % C::T;
+  const int64_t row = 2 * ((int64_t)blockIdx.x * (kC2rThreads / C::T) + u);
+  const bool act = row < nrows, two = row + 1 < nrows;
   float2* r = f + (act ? row : 0) * HP;
-  if (act)
-    for (int n = t; n < H; n += C::T) line[spad(n)] = r[n];
-  __syncwarp();
-  line_fft_smem<H, C::T, -1>(line, t, twH, act);
-  if (act) row_r2c_post<N>(line, r, t, C::T, twN);
+  const float* a = reinterpret_cast<const float*>(r);
+  float2 v[C::R1];
+#pragma unroll
+  for (int i = 0; i < C::R1; ++i) {
+    const int n = t + C::T * i;
+    v[i] = make_float2(act ? a[n] : 0.f, two ? a[2 * HP + n] : 0.f);
+  }
+  pair_fft<N, -1>(v, sm + u * C::LS, t, tw2, act);  // every lane of the line has read its rows
+  pair_split<N>(v, r, HP, t, act, two);
 }
 
 template <int N>
 struct Xform {
   static constexpr int64_t tiles = TileCfg<N>::TILES;
+  static constexpr size_t kSmem = pair_line_smem<N>(kC2rThreads);
   static int c2r(Plan* p, float2* slot, cudaStream_t st) {
-    using R = RowCfg<N>;
     int rc = run_pass<N, 0, +1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_x");
     if (rc) return rc;
     if ((rc = run_pass<N, 1, +1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_y"))) return rc;
-    int lpb = 8 * R::LPW;
-    int64_t nrows = (int64_t)N * N;
-    dim3 g2((unsigned)((nrows + lpb - 1) / lpb), 1);
     {
       ProfScope ps_(p, "xform_rows", st);
-      k_rows_c2r<N><<<g2, 256, sizeof(float2) * lpb * R::LS, st>>>(slot, 0, p->HP, 0, nrows, p->d_twN, p->d_twH,
-                                                                  ZTypes{{0, 0, 0, 0, 0, 0}, 0.f, nullptr});
+      k_rows_c2r<N><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(slot, 0, p->HP, 0, (int64_t)N * N, p->d_tw2,
+                                                                 ZTypes{{0, 0, 0, 0, 0, 0}, 0.f, nullptr});
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
     return AAR_OK;
   }
   static int r2c(Plan* p, float2* slot, cudaStream_t st) {
-    using R = RowCfg<N>;
-    int lpb = 8 * R::LPW;
-    int64_t nrows = (int64_t)N * N;
-    dim3 g2((unsigned)((nrows + lpb - 1) / lpb), 1);
     {
       ProfScope ps_(p, "xform_rows", st);
-      k_rows_r2c<N><<<g2, 256, sizeof(float2) * lpb * R::LS, st>>>(slot, p->HP, nrows, p->d_twN, p->d_twH);
+      k_rows_r2c<N><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(slot, p->HP, (int64_t)N * N, p->d_tw2);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -1252,12 +1309,9 @@ int fused_r2c(Plan* p, const float* in, float2* out, cudaStream_t st) {
 int fused_configure_xform(Plan* p) {
   return dispatch_n(p->N, [&](auto nc) {
     constexpr int N = decltype(nc)::value;
-    using R = RowCfg<N>;
-    int lpb = 8 * R::LPW;
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(float2) * lpb * R::LS)));
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(float2) * lpb * R::LS)));
+    const int smem = (int)pair_line_smem<N>(kC2rThreads);
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     return Launch<N>::configure(p);
   });
 }

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "aar_internal.cuh"
+#include "rows.cuh"
 #include "jit_embed.h"  // kEmbedFft, kEmbedRows, kEmbedCells (generated by build.py)
 #include "spectral.cuh"
 
@@ -32,16 +33,16 @@ struct JitState {
   std::string key;        // N, M and the term structure the module was made for
   size_t smem = 0;
   int nterms = 0;
-  int threads = kRowThreadsHost;  // block size the module was compiled for
+  int threads = 0;        // block size the module was compiled for
+  int pr = 0;             // row pairs per block (rows_pairs), 0: rows_fold, one row per block
   cudaKernel_t acc = nullptr;      // aar_modal_acc_jit, or null
   int acc_blocks = 0;              // its resident blocks per SM
   int64_t acc_fs = 0;              // field stride it was compiled for
 };
 
-static std::string gen_source(int N, int M, int minb, int threads, int pairs, const TermList& tl,
+static std::string gen_source(int N, int M, int minb, int threads, int pr, int pairs, const TermList& tl,
                               const std::vector<Term>& terms) {
   std::string s = "struct JitRowOp {\n";
-  s += "  static constexpr int min_blocks(int) { return " + std::to_string(minb) + "; }\n";
   s += "  static constexpr bool kPairs = " + std::string(pairs ? "true" : "false") + ";\n";
   s += "  static constexpr bool kZfac = false;\n";
   // maps of the inputs and outputs to field slots and lines: the identity
@@ -60,6 +61,7 @@ static std::string gen_source(int N, int M, int minb, int threads, int pairs, co
          (id ? "l" : std::string("k_") + name + "[l]") + "; }\n";
   };
   const int nin = tl.nin;
+  s += "  __device__ int nlines() const { return " + std::to_string(tl.nlines) + "; }\n";
   s += "  __device__ int nin() const { return " + std::to_string(nin) + "; }\n";
   map("in_slot", nin, [&](int i) { return tl.in_mode[i]; });
   map("in_line", nin, [&](int i) { return tl.line[tl.in_mode[i]]; });
@@ -120,10 +122,13 @@ static std::string gen_source(int N, int M, int minb, int threads, int pairs, co
   s = "#include \"rows.cuh\"\n__constant__ float kCoef[" + std::to_string(terms.empty() ? 1 : terms.size()) +
       "];\nnamespace aar {\n" + consts + s;
   s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(threads) + ", " + std::to_string(minb) +
-       ") aar_modal_rows_jit(float2* work, long long fs, int HP, const float2* __restrict__ twN, "
-       "const float2* __restrict__ twH) {\n";
-  s += "  aar::rows_body<" + std::to_string(N) + ", aar::JitRowOp, " + std::to_string(threads) +
-       ">(aar::JitRowOp{}, work, fs, HP, twN, twH);\n}\n";
+       ") aar_modal_rows_jit(float2* work, long long fs, int HP, long long nrows, const float2* __restrict__ twN, "
+       "const float2* __restrict__ twH, const float2* __restrict__ tw2) {\n";
+  const std::string targs = std::to_string(N) + ", aar::JitRowOp, " + std::to_string(threads);
+  if (pr)
+    s += "  aar::rows_pairs<" + targs + ">(aar::JitRowOp{}, work, fs, HP, nrows, tw2, " + std::to_string(pr) + ");\n}\n";
+  else
+    s += "  aar::rows_fold<" + targs + ">(aar::JitRowOp{}, work, fs, HP, twN, twH);\n}\n";
   return s;
 }
 
@@ -202,24 +207,39 @@ int jit_prepare(Plan* p) {
   const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
   std::vector<Term> terms(ft, ft + tl.nterms);
   const int N = p->N, M = p->M;
-  const int minb = p->jit_minb > 0 ? p->jit_minb : (N >= 1024 ? 2 : 3);
-  // default block size: 320 threads (ten warps) at N = 1024 where they take
-  // the input lines in fewer rounds than eight warps (measured at 1024^3,
-  // 20 modes: 362 vs 372 ms per step); the autotuner may choose otherwise
-  const int threads = p->jit_threads > 0                                   ? p->jit_threads
-                      : (N >= 1024 && (tl.nin + 9) / 10 < (tl.nin + 7) / 8) ? 320
-                                                                       : kRowThreadsHost;
+  int minb, threads, pr = 0;
+  size_t smem;
+  if (rows_use_pairs(N, tl.nlines)) {
+    // a line per T threads: as many row pairs as fill 192 threads within 72
+    // KB, one or more rounds of at most 512 threads where a pair has more lines
+    const int R1 = two_stage_r1(N), T = N / R1, m = std::max(tl.nin, tl.nr);
+    const size_t pair = sizeof(float2) * (size_t)tl.nlines * (N + T);
+    pr = std::max(1, 192 / (m * T));
+    while (pr > 1 && pr * pair > 72 * 1024) --pr;
+    const int want = pr * m * T, rounds = (want + 511) / 512;
+    threads = ((want + rounds - 1) / rounds + 31) / 32 * 32;
+    minb = p->jit_minb > 0 ? p->jit_minb : std::max(1, 65536 / (R1 == 32 ? 112 : 64) / threads);
+    minb = std::min(minb, 65536 / 64 / threads);
+    smem = pr * pair;
+  } else {
+    minb = p->jit_minb > 0 ? p->jit_minb : 2;
+    // 320 threads (ten warps) where they take the input lines in fewer rounds
+    // than eight warps (measured at 1024^3, 20 modes: 362 vs 372 ms per step);
+    // the autotuner may choose otherwise
+    threads = p->jit_threads > 0 ? p->jit_threads : (tl.nin + 9) / 10 < (tl.nin + 7) / 8 ? 320 : kRowThreads;
+    smem = sizeof(float2) * ((size_t)tl.nlines * FoldCfg<1024>::LS + FoldCfg<1024>::LT);
+  }
   const int regcap = 65536 / (threads * minb);
   const int pairs = 2 * 2 * tl.nin + 16 <= regcap * 3 / 4;  // f values of two positions fit the register budget
   std::string key = std::to_string(N) + ":" + std::to_string(M) + ":" + std::to_string(minb) + ":" +
-                    std::to_string(threads) + ":" + std::to_string(pairs) + ":";
+                    std::to_string(threads) + ":" + std::to_string(pr) + ":" + std::to_string(pairs) + ":";
   for (const Term& t : terms) key += std::to_string(t.p) + "," + std::to_string(t.q) + "," + std::to_string(t.r) + ";";
   std::vector<float> coef(terms.size());
   for (size_t i = 0; i < terms.size(); ++i) coef[i] = terms[i].c;
   JitState* j = (JitState*)p->jit;
   if (!j || j->key != key) {
     jit_free(p);
-    const std::string src = "#include \"cells.cuh\"\n" + gen_source(N, M, minb, threads, pairs, tl, terms) +
+    const std::string src = "#include \"cells.cuh\"\n" + gen_source(N, M, minb, threads, pr, pairs, tl, terms) +
                             gen_acc(N, p->HP, tl);
     nvrtcProgram prog;
     const char* hdrs[3] = {kEmbedFft, kEmbedRows, kEmbedCells};
@@ -262,6 +282,7 @@ int jit_prepare(Plan* p) {
     j->key = key;
     j->nterms = (int)terms.size();
     j->threads = threads;
+    j->pr = pr;
     // the accumulation kernel is optional: without it the generic one runs
     if (cudaLibraryGetKernel(&j->acc, j->lib, "aar_modal_acc_jit") != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&j->acc_blocks, (const void*)j->acc, 256, 0) != cudaSuccess ||
@@ -272,7 +293,7 @@ int jit_prepare(Plan* p) {
     j->acc_fs = (int64_t)N * N * p->HP;
     p->jit = j;
   }
-  j->smem = sizeof(float2) * ((size_t)tl.nlines * p->row_ls + p->row_lt);
+  j->smem = smem;
   if (cudaFuncSetAttribute((const void*)j->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)j->smem) !=
       cudaSuccess) {
     cudaGetLastError();
@@ -287,13 +308,15 @@ int jit_prepare(Plan* p) {
 
 int jit_modal_rows(Plan* p, float2* work, int64_t fs, cudaStream_t st, int64_t nrows) {
   JitState* j = (JitState*)p->jit;
-  long long fsl = fs;
-  int hp = p->HP;
-  void* args[] = {&work, &fsl, &hp, &p->d_twN, &p->d_twH};
   if (nrows < 0) nrows = (int64_t)p->N * p->N;
+  long long fsl = fs, nr = nrows;
+  int hp = p->HP;
+  void* args[] = {&work, &fsl, &hp, &nr, &p->d_twN, &p->d_twH, &p->d_tw2};
+  const int64_t rows = j->pr ? 2 * j->pr : 1;  // of a block
   {
     ProfScope ps_(p, "modal_rows", st);
-    AAR_CUDA_TRY(p, cudaLaunchKernel((const void*)j->kern, dim3((unsigned)nrows), dim3(j->threads), args, j->smem, st));
+    AAR_CUDA_TRY(p, cudaLaunchKernel((const void*)j->kern, dim3((unsigned)((nrows + rows - 1) / rows)),
+                                     dim3(j->threads), args, j->smem, st));
   }
   p->last_launches += 1;
   return AAR_OK;

@@ -168,7 +168,7 @@ struct LptXOp {
 };
 
 // Inverse y pass fanning fields out: item (tile, c), c < NC: field in[c]
-// times the y factor type[c] (axis_factor), inverse y FFT, into out[c].
+// times the y factor type[c] (axis_table, axis_poly), inverse y FFT, into out[c].
 // Outputs never alias an input that another item still reads (an in-place
 // output reads only its own input).
 template <int N>
@@ -190,18 +190,16 @@ struct YFanOp {
   __device__ float2* dst(int c) const { return work + (int64_t)out[c] * fs; }
   __device__ void pre(float2* v, int, int, int c, int t) const {
     using C = TileCfg<N>;
-    // axis_factor with its table loads issued together (a branch per value
-    // left them one after another: 15.7 vs 10.2 ms for the displacements at
-    // 1024^3)
+    // (a branch and a load per value left the loads one after another: 15.7
+    // vs 9.9 ms for the displacements at 1024^3)
     const int ty = type[c];
     float f[C::R1];
 #pragma unroll
-    for (int i = 0; i < C::R1; ++i) f[i] = ty >= 3 ? __ldg(isinc2 + tile_n<N>(t, i)) : 1.f;
+    for (int i = 0; i < C::R1; ++i) f[i] = axis_table(ty, isinc2, tile_n<N>(t, i));
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) {
       const float k = (float)(i < C::R1 / 2 ? tile_n<N>(t, i) : tile_n<N>(t, i) - N);
-      const float a = ty == 1 ? k : ty == 2 ? k * k : ty == 4 ? kF * k : 1.f;
-      v[i] = cscale(v[i], a * f[i]);
+      v[i] = cscale(v[i], axis_poly(ty, k, kF) * f[i]);
     }
   }
 };

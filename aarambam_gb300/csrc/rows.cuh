@@ -21,123 +21,236 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // Per-axis real factor of the 2LPT y pass and c2r rows (index k along the
 // axis; y uses the signed index, z the column index kz = 0..N/2): 0: 1,
-// 1: k, 2: k^2, 3: 1/sinc^2, 4: kF k / sinc^2 (isinc2 = 1/sinc^2 per grid
-// index gi).
-__device__ __forceinline__ float axis_factor(int type, int k, float kF, const float* __restrict__ isinc2, int gi) {
-  if (type == 0) return 1.f;
-  if (type == 1) return (float)k;
-  if (type == 2) return (float)k * (float)k;
-  const float is2 = __ldg(isinc2 + gi);
-  return type == 3 ? is2 : kF * (float)k * is2;
+// 1: k, 2: k^2, 3: 1/sinc^2, 4: kF k / sinc^2, as the product of a table value
+// (isinc2 = 1/sinc^2 per grid index; types 3 and 4) and a polynomial.  A
+// thread's table loads go out together, without a branch per value.
+__device__ __forceinline__ float axis_table(int type, const float* __restrict__ isinc2, int gi) {
+  return type >= 3 ? __ldg(isinc2 + gi) : 1.f;
+}
+__device__ __forceinline__ float axis_poly(int type, float k, float kF) {
+  return type == 1 ? k : type == 2 ? k * k : type == 4 ? kF * k : 1.f;
 }
 
-// z factor of a row's spectrum, applied as the c2r pre-step reads X_k
+// z factor of a row's spectrum, applied as the c2r reads X_k
 struct ZFac {
-  int type;  // axis_factor type, 0 = none
+  int type;  // 0 = none
   float kF;
   const float* isinc2;
-  __device__ __forceinline__ float at(int k) const { return axis_factor(type, k, kF, isinc2, k); }
 };
 
 // Row layout: complex row X[0..N/2] at field + m HP, m the row's memory
 // index (the plan's row order maps (x, y) to m); the real row x[0..N-1]
-// occupies the same bytes (float2 z_n = (x_{2n}, x_{2n+1})).  The row steps
-// are the same for every row, so the kernels run over memory rows.
+// occupies the same bytes.  The row steps are the same for every row, so the
+// kernels run over memory rows.
+
+// ---------------------------------------------------------------------
+// Rows in pairs.  Two real rows a, b travel as one complex line a + i b: its
+// N-point spectrum is C_k = A_k + i B_k, C_{N-k} = conj A_k + i conj B_k, so
+// a c2r of both is one complex inverse transform of C and an r2c of both one
+// forward transform and C's even / odd split -- no half-length twiddle steps.
+// The rows of a pair are neighbours of the same field (memory rows m, m + 1),
+// so both have the same magnitude and the FP32 rounding of the line is that
+// of each row.
+//
+// A line is transformed by T threads with R1 = N / T values each in two
+// register stages and one exchange through the line's own shared memory
+// (R1 R2 = N, T = R2; fft.cuh: two_stage_r1): lane t holds C_{t + T i}, i < R1,
+// before and after, so the partner C_{N-k} of k = t + T i is value R1 - 1 - i
+// of lane T - t: a shuffle (lane 0 has its own partners).  The samples come
+// out at positions t + T i again, and go through shared memory once for the
+// pointwise combine, which needs every line at one position.
+//
+// What bounds it: instruction issue (FP32) and shared-memory wavefronts, then
+// HBM.  Measured against half-length transforms of single rows staged in
+// shared memory (folded radix 2 at N = 1024): modal rows 5.81 -> 3.90 ms
+// (512^3, 12 modes), 0.82 -> 0.48 (256^3, 13 modes), 0.089 -> 0.019 (128^3,
+// generic kernel, 3 read modes); source rows 10.3 -> 9.0 (1024^3), 2.34 ->
+// 1.10 (512^3), 0.317 -> 0.115 (256^3); displacement rows 12.9 -> 9.3
+// (1024^3); rows with the lattice read-out 13.3 -> 12.9 (1024^3), 2.47 -> 1.65
+// (512^3).
 template <int N>
-struct RowCfg {
-  static constexpr int H = N / 2;             // complex FFT length
-  // 16 values per lane from H = 256 up (two stages of 16 x 16 at H = 256,
-  // measured 6.2 vs 7.3 ms for the modal rows at 512^3; at H = 128 eight
-  // lanes per line made the 256^3 batch slower, 139 vs 127 ms)
-  static constexpr int T = H == 256 ? 16 : lanes_for(H);
-  static constexpr int LPW = 32 / T;
-  static constexpr int LS = spad_len(H);
+struct PairCfg {
+  static constexpr int R1 = two_stage_r1(N);
+  static constexpr int R2 = N / R1;
+  static constexpr int T = R2;           // threads per line
+  static constexpr int G = R1 / T;       // second-stage DFTs per thread
+  static constexpr int LPW = 32 / T;     // lines per warp
+  static constexpr int LS = N + T;       // exchange entries of a line
+  static constexpr int HR = R1 / 2;
 };
 
-// load X_k (k = 0..N/2) of a row and form Z_k = E_k + i O_k for the
-// inverse half-length FFT (FFTW c2r semantics: Im X_0, Im X_{N/2} dropped)
-template <int N>
-__device__ __forceinline__ void row_c2r_pre(const float2* __restrict__ X, float2* line, int t, int T,
-                                            const float2* __restrict__ twN, ZFac zf = ZFac{0, 0.f, nullptr}) {
-  constexpr int H = N / 2;
-  for (int k = t; k <= H / 2; k += T) {
-    int k2 = H - k;
-    float2 a = X[k], b = X[k2];
-    if (zf.type) {
-      a = cscale(a, zf.at(k));
-      b = cscale(b, zf.at(k2));
+// The modal rows' path: pairs, except at N = 1024 with more than 8 lines,
+// where a block of a row pair leaves too few warps on the SM for its 32
+// values per lane (1024^3, NVRTC kernel, pairs against one folded row per
+// block: 4 modes 7.5 / 10.7 ms, 6 12.4 / 14.6, 8 17.1 / 18.7, 10 28.7 / 27.2,
+// 13 36.6 / 36.0).
+__host__ __device__ constexpr bool rows_use_pairs(int N, int nlines) { return N < 1024 || nlines <= 8; }
+
+// The transform of a lane's line values, v[i] = x[t + T i] in and out
+// (reordered), through the line buffer ln.  tw2[r R1 + j] = exp(-2 pi i r j /
+// N).  The T lanes of a line call it together (whole warps); lanes without a
+// line (act false) take part in the barriers only.  Conflict-free: the first
+// stage's stores are R1 + 1 (odd) entries apart between lanes, its loads
+// contiguous.
+template <int N, int SIGN>
+__device__ __forceinline__ void pair_fft(float2* v, float2* ln, int t, const float2* __restrict__ tw2, bool act) {
+  using C = PairCfg<N>;
+  DFT<C::R1, SIGN>::run(v);
+  __syncwarp();  // the line's earlier readers are done
+  if (act) {
+#pragma unroll
+    for (int r = 0; r < C::R1; ++r) ln[t * (C::R1 + 1) + r] = v[r];
+  }
+  __syncwarp();
+  float2 u[C::R1];
+  if (act) {
+#pragma unroll
+    for (int b = 0; b < C::G; ++b)
+#pragma unroll
+      for (int r = 0; r < C::R2; ++r) u[b * C::R2 + r] = ln[r * (C::R1 + 1) + t + C::T * b];
+  }
+#pragma unroll
+  for (int b = 0; b < C::G; ++b) {
+#pragma unroll
+    for (int r = 1; r < C::R2; ++r)
+      u[b * C::R2 + r] = cmul(u[b * C::R2 + r], tw_load<SIGN>(tw2 + t + C::T * b, r * C::R1));
+    DFT<C::R2, SIGN>::run(u + b * C::R2);
+  }
+  __syncwarp();  // the exchange has been read
+#pragma unroll
+  for (int b = 0; b < C::G; ++b)
+#pragma unroll
+    for (int r = 0; r < C::R2; ++r) v[b + C::G * r] = u[b * C::R2 + r];
+}
+
+// Lane t's line values C_{t + T i} of the pair's half spectra A, B (B null:
+// zero), with the z factor of the field.  FFTW c2r: Im X_0, Im X_{N/2} of
+// each row are dropped.
+template <int N, bool ZF>
+__device__ __forceinline__ void pair_spectrum(float2* v, const float2* __restrict__ A, const float2* __restrict__ B,
+                                              int t, ZFac zf, bool act) {
+  using C = PairCfg<N>;
+  float2 a[C::HR], b[C::HR];
+  float2 ah = make_float2(0.f, 0.f), bh = ah;
+#pragma unroll
+  for (int i = 0; i < C::HR; ++i) {
+    a[i] = act ? A[t + C::T * i] : make_float2(0.f, 0.f);
+    b[i] = act && B ? B[t + C::T * i] : make_float2(0.f, 0.f);
+  }
+  if (act && t == 0) {
+    ah = A[N / 2];
+    if (B) bh = B[N / 2];
+  }
+  if constexpr (ZF) {
+    float f[C::HR];
+#pragma unroll
+    for (int i = 0; i < C::HR; ++i) f[i] = axis_table(zf.type, zf.isinc2, t + C::T * i);
+    const float fh = axis_table(zf.type, zf.isinc2, N / 2) * axis_poly(zf.type, (float)(N / 2), zf.kF);
+#pragma unroll
+    for (int i = 0; i < C::HR; ++i) {
+      f[i] *= axis_poly(zf.type, (float)(t + C::T * i), zf.kF);
+      a[i] = cscale(a[i], f[i]);
+      b[i] = cscale(b[i], f[i]);
     }
-    if (k == 0) {
-      a.y = 0.f;
-      b.y = 0.f;
-    }
-    // E_k = X_k + conj(X_{H-k}); O_k = (X_k - conj(X_{H-k})) e^{+2 pi i k / N}
-    float2 w = __ldg(twN + k);
-    w.y = -w.y;
-    float2 e = make_float2(a.x + b.x, a.y - b.y);
-    float2 d = make_float2(a.x - b.x, a.y + b.y);
-    float2 o = cmul(d, w);
-    line[spad(k)] = make_float2(e.x - o.y, e.y + o.x);
-    if (k2 != k && k2 < H) {
-      // Z_{H-k}: E = X_{H-k} + conj(X_k), O = (X_{H-k} - conj(X_k)) e^{+2 pi i (H-k)/N}
-      float2 w2 = __ldg(twN + k2);
-      w2.y = -w2.y;
-      float2 e2 = make_float2(b.x + a.x, b.y - a.y);
-      float2 d2 = make_float2(b.x - a.x, b.y + a.y);
-      float2 o2 = cmul(d2, w2);
-      line[spad(k2)] = make_float2(e2.x - o2.y, e2.y + o2.x);
-    }
+    ah.x *= fh;
+    bh.x *= fh;
+  }
+  float2 u[C::HR];  // conj A + i conj B: the value at N - k
+#pragma unroll
+  for (int i = 0; i < C::HR; ++i) {
+    v[i] = make_float2(a[i].x - b[i].y, a[i].y + b[i].x);
+    u[i] = make_float2(a[i].x + b[i].y, b[i].x - a[i].y);
+  }
+  if (t == 0) v[0] = make_float2(a[0].x, b[0].x);
+  const int lane = threadIdx.x & 31;
+  const int src = (lane & ~(C::T - 1)) | ((C::T - t) & (C::T - 1));
+#pragma unroll
+  for (int i = 0; i < C::HR; ++i) {
+    const float2 w = make_float2(__shfl_sync(0xffffffffu, u[i].x, src), __shfl_sync(0xffffffffu, u[i].y, src));
+    const float2 own = i + 1 < C::HR ? u[i + 1 < C::HR ? i + 1 : 0] : make_float2(ah.x, bh.x);
+    v[C::R1 - 1 - i] = t == 0 ? own : w;
   }
 }
 
-// The same pre-step in place, on X_0..X_{N/2} already staged in `line`
-// (element k at spad(k)): each lane rewrites the pair (k, H - k) it reads.
+// Half spectra of the pair from lane t's transformed values C_{t + T i}, into
+// X (row a) and X + HP (row b, when two).
 template <int N>
-__device__ __forceinline__ void row_c2r_pre_inplace(float2* line, int t, int T, const float2* __restrict__ twN,
-                                                    ZFac zf = ZFac{0, 0.f, nullptr}) {
-  constexpr int H = N / 2;
-  for (int k = t; k <= H / 2; k += T) {
-    int k2 = H - k;
-    float2 a = line[spad(k)], b = line[spad(k2)];
-    if (zf.type) {
-      a = cscale(a, zf.at(k));
-      b = cscale(b, zf.at(k2));
+__device__ __forceinline__ void pair_split(const float2* v, float2* __restrict__ X, int HP, int t, bool act, bool two) {
+  using C = PairCfg<N>;
+  const int lane = threadIdx.x & 31;
+  const int src = (lane & ~(C::T - 1)) | ((C::T - t) & (C::T - 1));
+#pragma unroll
+  for (int i = 0; i < C::HR; ++i) {
+    const float2 c = v[i];
+    float2 p = make_float2(__shfl_sync(0xffffffffu, v[C::R1 - 1 - i].x, src),
+                           __shfl_sync(0xffffffffu, v[C::R1 - 1 - i].y, src));
+    if (t == 0) p = v[i == 0 ? 0 : C::R1 - i];
+    if (act) {
+      X[t + C::T * i] = make_float2(0.5f * (c.x + p.x), 0.5f * (c.y - p.y));
+      if (two) X[HP + t + C::T * i] = make_float2(0.5f * (c.y + p.y), 0.5f * (p.x - c.x));
     }
-    if (k == 0) {
-      a.y = 0.f;
-      b.y = 0.f;
-    }
-    float2 w = __ldg(twN + k);
-    w.y = -w.y;
-    float2 e = make_float2(a.x + b.x, a.y - b.y);
-    float2 d = make_float2(a.x - b.x, a.y + b.y);
-    float2 o = cmul(d, w);
-    line[spad(k)] = make_float2(e.x - o.y, e.y + o.x);
-    if (k2 != k && k2 < H) {
-      float2 w2 = __ldg(twN + k2);
-      w2.y = -w2.y;
-      float2 e2 = make_float2(b.x + a.x, b.y - a.y);
-      float2 d2 = make_float2(b.x - a.x, b.y + a.y);
-      float2 o2 = cmul(d2, w2);
-      line[spad(k2)] = make_float2(e2.x - o2.y, e2.y + o2.x);
-    }
+  }
+  if (act && t == 0) {
+    X[N / 2] = make_float2(v[C::HR].x, 0.f);
+    if (two) X[HP + N / 2] = make_float2(v[C::HR].y, 0.f);
   }
 }
 
-// after the forward half-length FFT of z_n = (x_{2n}, x_{2n+1}) in `line`,
-// write X_k = (Z_k + conj Z_{H-k})/2 - i e^{-2 pi i k/N} (Z_k - conj Z_{H-k})/2
-template <int N>
-__device__ __forceinline__ void row_r2c_post(const float2* line, float2* __restrict__ X, int t, int T,
-                                             const float2* __restrict__ twN) {
-  constexpr int H = N / 2;
-  for (int k = t; k <= H; k += T) {
-    float2 z = line[spad(k % H)], zc = line[spad((H - k) % H)];
-    zc.y = -zc.y;
-    float2 e = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
-    float2 d = make_float2(0.5f * (z.x - zc.x), 0.5f * (z.y - zc.y));
-    float2 w = (k < H) ? __ldg(twN + k) : make_float2(-1.f, 0.f);
-    float2 od = cmul(d, w);  // e^{-2 pi i k/N} d
-    X[k] = make_float2(e.x + od.y, e.y - od.x);  // e - i od
+// Row kernel on pairs: block b takes the PR row pairs from memory row 2 PR b
+// on.  Phase 1: inverse transforms of every (pair, input) line, one line per
+// T threads; phase 2: the combine, a float2 position holding the two rows'
+// samples; phase 3: forward transforms of every (pair, output) line.
+template <int N, class Op, int THREADS>
+__device__ __forceinline__ void rows_pairs(const Op& op, float2* work, int64_t fs, int HP, int64_t nrows,
+                                           const float2* __restrict__ tw2, const int PR) {
+  using C = PairCfg<N>;
+  extern __shared__ float2 sm_all[];
+  float2* sm = sm_all;  // [PR][op.nlines()][LS]
+  const int64_t row0 = (int64_t)blockIdx.x * (2 * PR);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane / C::T, t = lane % C::T;
+  constexpr int STEP = THREADS / 32 * C::LPW;
+  const int stride = op.nlines() * C::LS;  // of a row pair
+  for (int u0 = warp * C::LPW; u0 < PR * op.nin(); u0 += STEP) {
+    const int u = u0 + sub, pr = PR == 1 ? 0 : u / op.nin(), l = PR == 1 ? u : u - pr * op.nin();
+    const int64_t row = row0 + 2 * pr;
+    const bool act = u < PR * op.nin() && row < nrows;
+    float2* ln = sm + (act ? pr * stride + op.in_line(l) * C::LS : 0);
+    const float2* X = work + (act ? (int64_t)op.in_slot(l) * fs + row * HP : 0);
+    float2 v[C::R1];
+    ZFac zf{0, 0.f, nullptr};
+    if constexpr (Op::kZfac) zf = op.zfac(act ? l : 0);
+    pair_spectrum<N, Op::kZfac>(v, X, row + 1 < nrows ? X + HP : nullptr, t, zf, act);
+    pair_fft<N, +1>(v, ln, t, tw2, act);
+    if (act) {
+#pragma unroll
+      for (int i = 0; i < C::R1; ++i) ln[t + C::T * i] = v[i];
+    }
+  }
+  __syncthreads();
+  constexpr int K = Op::kPairs ? 2 : 1;
+  for (int n = threadIdx.x; n < PR * N; n += K * THREADS) {
+    const int o0 = (PR == 1 ? 0 : n / N * stride) + n % N;
+    if (K == 2 && n + THREADS < PR * N) {
+      const int m = n + THREADS;
+      const int pos[2] = {o0, (PR == 1 ? 0 : m / N * stride) + m % N};
+      op.template combine<2>(sm, pos, C::LS);
+    } else {
+      const int pos[1] = {o0};
+      op.template combine<1>(sm, pos, C::LS);
+    }
+  }
+  __syncthreads();
+  for (int u0 = warp * C::LPW; u0 < PR * op.nout(); u0 += STEP) {
+    const int u = u0 + sub, pr = PR == 1 ? 0 : u / op.nout(), l = PR == 1 ? u : u - pr * op.nout();
+    const int64_t row = row0 + 2 * pr;
+    const bool act = u < PR * op.nout() && row < nrows;
+    float2* ln = sm + (act ? pr * stride + op.out_line(l) * C::LS : 0);
+    float2 v[C::R1];
+#pragma unroll
+    for (int i = 0; i < C::R1; ++i) v[i] = act ? ln[t + C::T * i] : make_float2(0.f, 0.f);
+    pair_fft<N, -1>(v, ln, t, tw2, act);
+    pair_split<N>(v, work + (act ? (int64_t)op.out_slot(l) * fs + row * HP : 0), HP, t, act, row + 1 < nrows);
   }
 }
 
@@ -159,18 +272,14 @@ __device__ __forceinline__ void row_r2c_post(const float2* line, float2* __restr
 // the h-point transforms, Z_k = E_k + e^{-2 pi i k/H} O_k and Z_{k+h} =
 // E_k - e^{-2 pi i k/H} O_k, then the post-step X_k from Z_k, Z_{H-k}.
 template <int N>
-struct RowFold {
-  static constexpr bool value = N == 1024;
+struct FoldCfg {
+  static_assert(N == 1024, "folded rows: one warp per 512-point half line");
+  static constexpr int LS = spad_len(N / 2);
+  // float2 slots of the lane twiddle table (fft.cuh) of the H/2-point
+  // half-line transforms, at the start of the shared memory, filled once per
+  // block (the modal rows at 1024^3 with 20 modes 67.9 -> 60.8 ms)
+  static constexpr int LT = lt_slots(N / 4, 16);
 };
-
-// float2 slots of the lane twiddle table (fft.cuh) of the folded rows'
-// H/2-point half-line transforms, at the start of their shared memory
-// (filled once per block of M + R lines: the modal rows at 1024^3 with 20
-// modes 67.9 -> 60.8 ms, the source rows 11.1 -> 10.6 ms)
-template <int N>
-__host__ __device__ constexpr int row_lt_slots() {
-  return RowFold<N>::value ? lt_slots(N / 4, 16) : 0;
-}
 
 // Z_j of the c2r pre-step from a = X_j, b = X_{H-j}, w = e^{+2 pi i j/N}:
 // E + i O with E = a + conj b, O = (a - conj b) w
@@ -200,7 +309,7 @@ __device__ __forceinline__ float2 post1(float2 z, float2 zr, float2 w) {
 // from the quad at k2 (k2 = k, or Q for lane 0's first quad).
 template <int N>
 __device__ __forceinline__ void row_c2r_pre_fold(float2* line, int lane, const float2* __restrict__ twN,
-                                                 const float2* __restrict__ twH, ZFac zf,
+                                                 const float2* __restrict__ twH,
                                                  const float2* __restrict__ src) {
   constexpr int H = N / 2, h = H / 2, Q = H / 4;
   static_assert(Q % 32 == 0, "folded rows: whole rounds of quads");
@@ -228,16 +337,6 @@ __device__ __forceinline__ void row_c2r_pre_fold(float2* line, int lane, const f
     const float2 wk = __ldg(twN + k), vk = __ldg(twH + k);
     const float2 w2 = l0 ? wQ : wk, v2 = l0 ? vQ : vk;
     float2 a2 = l0 ? xq : a, b2 = l0 ? x3q : b, c2 = l0 ? xq : c, d2 = l0 ? x3q : d;
-    if (zf.type) {
-      a = cscale(a, zf.at(k));
-      b = cscale(b, zf.at(H - k));
-      c = cscale(c, zf.at(h - k));
-      d = cscale(d, zf.at(h + k));
-      a2 = l0 ? cscale(a2, zf.at(Q)) : a;
-      b2 = l0 ? cscale(b2, zf.at(H - Q)) : b;
-      c2 = l0 ? cscale(c2, zf.at(Q)) : c;
-      d2 = l0 ? cscale(d2, zf.at(H - Q)) : d;
-    }
     if (k == 0) {  // FFTW c2r: Im X_0, Im X_{N/2} dropped
       a.y = 0.f;
       b.y = 0.f;
@@ -292,90 +391,33 @@ __device__ __forceinline__ void row_r2c_post_fold(const float2* line, float2* __
   }
 }
 
-// Generic row kernel.  For each memory row (blockIdx.x): c2r of `nin`
-// input fields (slots in_slot[], into lines in_line[]), a per-position combine step Op, r2c of
-// `nout` output lines into slots out_slot[].  One warp per line at a time.
-// THREADS = 256 (the library's kernels; the NVRTC kernel may use 320) with
-// two resident blocks per SM: while one block waits at a phase barrier (its
-// last round of lines keeps only some warps busy) the other block's warps
-// issue.
+// One row per block, folded (N = 1024): c2r of the input fields into their
+// lines, one warp per line at a time, the combine, r2c of the output lines.
+// For plans whose lines of a row pair do not leave room for two resident
+// blocks (rows_use_pairs); 256 threads, or 320 where ten warps take the
+// input lines in fewer rounds than eight, two resident blocks per SM.
 constexpr int kRowThreads = 256;
 template <int N, class Op, int THREADS = kRowThreads>
-__device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs, int HP,
+__device__ __forceinline__ void rows_fold(const Op& op, float2* work, int64_t fs, int HP,
                                           const float2* __restrict__ twN, const float2* __restrict__ twH) {
-  using C = RowCfg<N>;
-  constexpr int H = C::H;
+  using C = FoldCfg<N>;
+  constexpr int H = N / 2, h = H / 2, HO = h + h / 16;  // spad(h + i) = spad(i) + HO
   extern __shared__ float2 sm_all[];
-  float2* sm = sm_all + row_lt_slots<N>();  // line buffers after the lane twiddles
-  int64_t row = blockIdx.x;
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float2* sm = sm_all + C::LT;  // line buffers after the lane twiddles
+  const int64_t row = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int nwarps = THREADS / 32;
-  int sub = lane / C::T, t = lane % C::T;
-  // phase 0: stage X_0..X_{N/2} of every input line at once (one exposed
-  // memory latency per row instead of one per line; staging round by round
-  // with a barrier per round measured slower: 148 vs 141 ms at 1024^3).
-  // The folded rows read X in their pre-step straight from global memory
-  // (staged: 83.6 vs 73.4 ms at 1024^3); the other sizes keep the staging
-  // (reading in the pre-step: 7.44 vs 7.27 ms for the modal rows at 512^3
-  // with 8 values per lane, 7.29 vs 6.21 ms with 16).
-  if constexpr (!RowFold<N>::value) {
-    for (int l = 0; l < op.nin(); ++l) {
-      const float2* X = work + (int64_t)op.in_slot(l) * fs + row * HP;
-      float2* line = sm + op.in_line(l) * C::LS;
-      for (int k = threadIdx.x; k <= H; k += THREADS) cp_async8(line + spad(k), X + k);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-  }
-  if constexpr (RowFold<N>::value) {
-    static_assert(C::T == 32 && H == 512, "folded rows: one warp per 512-point half line");
-    constexpr int h = H / 2, HO = h + h / 16;  // spad(h + i) = spad(i) + HO
-    const int half = lane >> 4, t16 = lane & 15;
-    const float2* lt = sm_all;
-    lt_fill<h, 16, 2>(sm_all, twH, threadIdx.x, THREADS);
-    __syncthreads();
-    for (int l = warp; l < op.nin(); l += nwarps) {
-      float2* line = sm + op.in_line(l) * C::LS;
-      const float2* X = work + (int64_t)op.in_slot(l) * fs + row * HP;
-      if constexpr (Op::kZfac) row_c2r_pre_fold<N>(line, lane, twN, twH, op.zfac(l), X);
-      else row_c2r_pre_fold<N>(line, lane, twN, twH, ZFac{0, 0.f, nullptr}, X);
-      __syncwarp();
-      line_fft_smem<h, 16, +1, 0, 2, true>(line + half * HO, t16, lt, true);
-    }
-    __syncthreads();
-    for (int n = threadIdx.x; n < H; n += (Op::kPairs ? 2 : 1) * THREADS) {
-      if (Op::kPairs && n + THREADS < H) {
-        const int pos[2] = {spad(n), spad(n + THREADS)};
-        op.template combine<2>(sm, pos, C::LS);
-      } else {
-        const int pos[1] = {spad(n)};
-        op.template combine<1>(sm, pos, C::LS);
-      }
-    }
-    __syncthreads();
-    for (int l = warp; l < op.nout(); l += nwarps) {
-      float2* line = sm + op.out_line(l) * C::LS;
-      line_fft_smem<h, 16, -1, 0, 2, true>(line + half * HO, t16, lt, true);
-      row_r2c_post_fold<N>(line, work + (int64_t)op.out_slot(l) * fs + row * HP, lane, twN, twH);
-      __syncwarp();
-    }
-    return;
-  }
-  // phase 1: inverse transforms
-  for (int l0 = warp * C::LPW; l0 < op.nin(); l0 += nwarps * C::LPW) {
-    int l = l0 + sub;
-    bool act = l < op.nin() && sub < C::LPW;
-    float2* line = sm + (act ? op.in_line(l) : 0) * C::LS;
-    if (act) {
-      if constexpr (Op::kZfac) row_c2r_pre_inplace<N>(line, t, C::T, twN, op.zfac(l));
-      else row_c2r_pre_inplace<N>(line, t, C::T, twN);
-    }
+  const int half = lane >> 4, t16 = lane & 15;
+  const float2* lt = sm_all;
+  lt_fill<h, 16, 2>(sm_all, twH, threadIdx.x, THREADS);
+  __syncthreads();
+  for (int l = warp; l < op.nin(); l += nwarps) {
+    float2* line = sm + op.in_line(l) * C::LS;
+    row_c2r_pre_fold<N>(line, lane, twN, twH, work + (int64_t)op.in_slot(l) * fs + row * HP);
     __syncwarp();
-    line_fft_smem<H, C::T, +1>(line, t, twH, act);
+    line_fft_smem<h, 16, +1, 0, 2, true>(line + half * HO, t16, lt, true);
   }
   __syncthreads();
-  // phase 2: per position combine (in place in the line buffers)
   for (int n = threadIdx.x; n < H; n += (Op::kPairs ? 2 : 1) * THREADS) {
     if (Op::kPairs && n + THREADS < H) {
       const int pos[2] = {spad(n), spad(n + THREADS)};
@@ -386,13 +428,10 @@ __device__ __forceinline__ void rows_body(const Op& op, float2* work, int64_t fs
     }
   }
   __syncthreads();
-  // phase 3: forward transforms of the output lines
-  for (int l0 = warp * C::LPW; l0 < op.nout(); l0 += nwarps * C::LPW) {
-    int l = l0 + sub;
-    bool act = l < op.nout() && sub < C::LPW;
-    float2* line = sm + (act ? op.out_line(l) : 0) * C::LS;
-    line_fft_smem<H, C::T, -1>(line, t, twH, act);
-    if (act) row_r2c_post<N>(line, work + (int64_t)op.out_slot(l) * fs + row * HP, t, C::T, twN);
+  for (int l = warp; l < op.nout(); l += nwarps) {
+    float2* line = sm + op.out_line(l) * C::LS;
+    line_fft_smem<h, 16, -1, 0, 2, true>(line + half * HO, t16, lt, true);
+    row_r2c_post_fold<N>(line, work + (int64_t)op.out_slot(l) * fs + row * HP, lane, twN, twH);
     __syncwarp();
   }
 }

@@ -33,7 +33,7 @@ namespace aar {
 template <int N>
 struct TileCfg {
   static constexpr int W = 8;
-  static constexpr int R1 = N >= 512 ? 32 : N >= 128 ? 16 : N >= 32 ? 8 : 4;
+  static constexpr int R1 = two_stage_r1(N);
   static constexpr int R2 = N / R1;
   static constexpr int T = R2;       // threads per line
   static constexpr int G = R1 / T;   // second-stage DFTs per thread
