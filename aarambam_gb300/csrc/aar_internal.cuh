@@ -72,8 +72,7 @@ struct Plan {
   float* d_qcube = nullptr;
   int qcube_m = 0;
   bool qcube_stale = true;
-  void* d_rlxpow = nullptr;   // skip-ahead powers (U576[32])
-  int rlx_seg = 0;            // refills per seed-table thread
+  void* d_rlxpow = nullptr;   // skip-ahead powers (seedtable_powers)
   // modal term list (device)
   void* d_terms = nullptr;
   std::vector<char> host_terms;  // the same term list on the host (kernel parameter of the row combine)
@@ -151,7 +150,9 @@ size_t terms_bytes();
 const char* set_err(Plan* p, const std::string& e);
 
 // launchers (return 0 or an error code; errors leave a message on the plan)
-int launch_seedtable(Plan* p, uint32_t seed, uint32_t* d_out, cudaStream_t st);
+int launch_seedtable(Plan* p, uint32_t* d_out, cudaStream_t st);
+struct U576;
+void seedtable_powers(std::vector<U576>& pw);
 int launch_noise_fp32(Plan* p, const uint32_t* d_seed, float2* d_phik, cudaStream_t st);
 int launch_noise_fp64(Plan* p, const uint32_t* d_seed, double2* d_phik, int hp, cudaStream_t st);
 int fused_prepare(Plan* p);

@@ -410,18 +410,11 @@ static int create(Plan* p) {
 
   int rc;
   if ((rc = plan_alloc(p, (void**)&p->d_seed, sizeof(uint32_t) * (size_t)N * N))) return rc;
-  // ranlux skip-ahead: seed-table threads own rlx_seg refills; powers
-  // (b^{-202 rlx_seg})^{2^i} mod m, i < 32
-  p->rlx_seg = 8;
   {
-    std::vector<U576> pw(32);
-    U576 a = modpow576(u576_binv(), (uint64_t)kRlxLux * p->rlx_seg);
-    for (int i = 0; i < 32; ++i) {
-      pw[i] = a;
-      a = modmul576(a, a);
-    }
-    if ((rc = plan_alloc(p, &p->d_rlxpow, sizeof(U576) * 32))) return rc;
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_rlxpow, pw.data(), sizeof(U576) * 32, cudaMemcpyHostToDevice));
+    std::vector<U576> pw;  // ranlux skip-ahead
+    seedtable_powers(pw);
+    if ((rc = plan_alloc(p, &p->d_rlxpow, sizeof(U576) * pw.size()))) return rc;
+    AAR_CUDA_TRY(p, cudaMemcpy(p->d_rlxpow, pw.data(), sizeof(U576) * pw.size(), cudaMemcpyHostToDevice));
   }
   if (is_fp32(q)) {
     std::vector<float2> twN(N), twH(N / 2);
@@ -506,7 +499,7 @@ static int ready(Plan* p) {
 }
 
 static int run_noise(Plan* p, cudaStream_t st) {
-  int rc = launch_seedtable(p, (uint32_t)p->prm.seed, p->d_seed, st);
+  int rc = launch_seedtable(p, p->d_seed, st);
   if (rc) return rc;
   return launch_noise_fp32(p, p->d_seed, p->d_phik, st);
 }
@@ -628,7 +621,7 @@ int aar_set_seed(aar_plan* h, int32_t seed) {
 int aar_seedtable(aar_plan* h, uint32_t* d_out, void* stream) {
   if (!h || !d_out) return AAR_ERR_ARG;
   h->p.last_launches = 0;
-  return launch_seedtable(&h->p, (uint32_t)h->p.prm.seed, d_out, S(stream));
+  return launch_seedtable(&h->p, d_out, S(stream));
 }
 
 int aar_stage_noise(aar_plan* h, void* stream) {

@@ -2,10 +2,10 @@
 //
 // Seed table (Aarambam/LPT/Basis/main.c:317-349): one ranlxd1 stream seeded
 // with Seed delivers N^2 uniforms, stored as (unsigned)(0x7fffffff * u) in
-// eight "shell" segments per i < N/2.  The stream is split into segments of
-// rlx_seg refills; each thread rebuilds its segment's starting state with the
-// exact skip-ahead of ranlux.cuh and scatters its draws (the shell order is a
-// permutation of the table, so the scatter has no write conflicts).
+// eight "shell" segments per i < N/2.  One thread takes one refill (12
+// draws): it rebuilds the refill's starting state with the exact skip-ahead of
+// ranlux.cuh and scatters its draws (the shell order is a permutation of the
+// table, so the scatter has no write conflicts).
 //
 // Noise (main.c:382-524): one thread per (i, j) column reseeds ranlxd1 with
 // seedtable[i][j] and draws (phase, amplitude) pairs for k < N/2, skipping the
@@ -18,19 +18,20 @@
 
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "aar_internal.cuh"
 #include "ranlux.cuh"
 
 namespace aar {
 
-__device__ __forceinline__ int64_t shell_pos(int64_t d, int N) {
+__device__ __forceinline__ int shell_pos(int d, int N) {
   // draws before shell i: 4 i^2; segment lengths i, i+1, i, i+1, ...
-  int64_t i = (int64_t)sqrt((double)d) / 2;
+  int i = (int)sqrtf((float)d) / 2;
   while (4 * (i + 1) * (i + 1) <= d) ++i;
   while (4 * i * i > d) --i;
-  int64_t o = d - 4 * i * i;
-  int64_t n = N;
+  int o = d - 4 * i * i;
+  const int n = N;
   if (o < i) return i * n + o;
   o -= i;
   if (o < i + 1) return o * n + i;
@@ -48,36 +49,63 @@ __device__ __forceinline__ int64_t shell_pos(int64_t d, int N) {
   return (n - 1 - o) * n + (n - 1 - i);
 }
 
-__global__ void k_seedtable(uint32_t seed, int N, int seg, const U576* __restrict__ pw, int npw,
-                            uint32_t* __restrict__ table) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t total = (int64_t)N * N;
-  int64_t d0 = g * 12 * seg;
+// What bounds it: the latency of one thread's chain of 576-bit products and
+// of the 202 steps, at every grid size (N^2 / 12 threads).  So the chain is
+// short: the seeded state and its residue come from the host, the power of
+// the g-th refill is a product of at most three table entries (g's base-256
+// digits; the binary powers took up to 17), and a thread does one refill.
+// N = 64 0.023 ms, N = 1024 0.065 ms; with 8 refills per thread, seeding on
+// the device and binary powers 0.137 and 0.161 ms.
+struct SeedStart {
+  Rlx s;   // the seeded state
+  U576 r;  // its residue
+};
+__global__ void __launch_bounds__(32) k_seedtable(const __grid_constant__ SeedStart st, int N,
+                                                  const U576* __restrict__ pw, uint32_t* __restrict__ table) {
+  const int g = blockIdx.x * 32 + threadIdx.x;
+  const int total = N * N, d0 = 12 * g;
   if (d0 >= total) return;
   Rlx s;
-  rlx_seed(s, seed);
-  if (g > 0) {
-    U576 r = rlx_window_residue(s);
-    for (int b = 0; b < npw; ++b)
-      if ((g >> b) & 1) r = modmul576(r, pw[b]);
+  if (g == 0) {
+    s = st.s;
+  } else {
+    U576 r = st.r;
+    for (int l = 0, h = g; h; ++l, h >>= 8)
+      if (h & 255) r = modmul576(r, pw[l * kRlxRadix + (h & 255)]);
     rlx_from_residue(r, s);
   }
-  int64_t d1 = d0 + 12 * (int64_t)seg;
-  if (d1 > total) d1 = total;
-  for (int64_t d = d0; d < d1; ++d) {
-    double u = (double)rlx_next48(s) * 3.5527136788005009e-15;  // 2^-48
-    table[shell_pos(d, N)] = __double2uint_rz(__dmul_rn(2147483647.0, u));
+  rlx_refill(s);
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    if (d0 + i >= total) break;
+    const double u = (double)s.x[i] * 3.5527136788005009e-15;  // 2^-48
+    table[shell_pos(d0 + i, N)] = __double2uint_rz(__dmul_rn(2147483647.0, u));
   }
 }
 
-int launch_seedtable(Plan* p, uint32_t seed, uint32_t* d_out, cudaStream_t st) {
-  int64_t total = (int64_t)p->N * p->N;
-  int64_t draws_per = 12 * (int64_t)p->rlx_seg;
-  int64_t nthr = (total + draws_per - 1) / draws_per;
-  int bs = 64;
-  { ProfScope ps_(p, "seedtable", st);
-  k_seedtable<<<(unsigned)((nthr + bs - 1) / bs), bs, 0, st>>>(seed, p->N, p->rlx_seg, (const U576*)p->d_rlxpow,
-                                                                 32, d_out);
+// Table of the skip-ahead powers, level l, digit d: b^{-202 d 256^l} mod m.
+void seedtable_powers(std::vector<U576>& pw) {
+  static_assert(kRlxRadix == 256 && kRlxLevels == 3, "the threads' numbers have three base-256 digits");
+  pw.assign(kRlxLevels * kRlxRadix, u576_one());
+  U576 a = modpow576(u576_binv(), (uint64_t)kRlxLux);
+  for (int l = 0; l < kRlxLevels; ++l) {
+    for (int d = 1; d < kRlxRadix; ++d) pw[l * kRlxRadix + d] = modmul576(pw[l * kRlxRadix + d - 1], a);
+    a = modmul576(pw[l * kRlxRadix + kRlxRadix - 1], a);
+  }
+}
+
+static void run_seedtable(Plan* p, uint32_t* d_out, cudaStream_t st) {
+  SeedStart s0;
+  rlx_seed(s0.s, (uint32_t)p->prm.seed);
+  s0.r = rlx_window_residue(s0.s);
+  const int64_t nthr = ((int64_t)p->N * p->N + 11) / 12;
+  k_seedtable<<<(unsigned)((nthr + 31) / 32), 32, 0, st>>>(s0, p->N, (const U576*)p->d_rlxpow, d_out);
+}
+
+int launch_seedtable(Plan* p, uint32_t* d_out, cudaStream_t st) {
+  {
+    ProfScope ps_(p, "seedtable", st);
+    run_seedtable(p, d_out, st);
   }
   AAR_CUDA_TRY(p, cudaGetLastError());
   p->last_launches += 1;
@@ -333,10 +361,7 @@ int noalloc_gaussian(Plan* p, void* d_out, cudaStream_t st) {
   int rc = noalloc_scratch(p, &seed);
   if (rc) return rc;
   const int64_t total = (int64_t)N * N;
-  const int64_t draws_per = 12 * (int64_t)p->rlx_seg;
-  const int64_t nthr = (total + draws_per - 1) / draws_per;
-  k_seedtable<<<(unsigned)((nthr + 63) / 64), 64, 0, st>>>((uint32_t)p->prm.seed, N, p->rlx_seg,
-                                                           (const U576*)p->d_rlxpow, 32, seed);
+  run_seedtable(p, seed, st);
   AAR_CUDA_TRY(p, cudaGetLastError());
   const int hp = N / 2 + 1;
   const bool fp64 = is_plain(p->prm);

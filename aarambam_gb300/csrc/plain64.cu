@@ -467,7 +467,7 @@ int plain_run(Plan* p, const float* d_lagr, int64_t npart, float* d_pos, float* 
     return AAR_OK;
   };
   // noise
-  if ((rc = launch_seedtable(p, (uint32_t)p->prm.seed, p->d_seed, st))) return rc;
+  if ((rc = launch_seedtable(p, p->d_seed, st))) return rc;
   if ((rc = launch_noise_fp64(p, p->d_seed, phi, s->H, st))) return rc;
   AAR_CUDA_TRY(p, cudaMemsetAsync(acc, 0, sizeof(double2) * s->nc, st));
   auto A = [&](int i, int j, int k) { return p->alpha[((size_t)i * M + j) * M + k]; };

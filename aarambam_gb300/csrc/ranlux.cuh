@@ -30,6 +30,9 @@
 namespace aar {
 
 constexpr int kRlxLux = 202;  // ranlxd1
+// skip-ahead powers: kRlxLevels base-kRlxRadix digits of the refill number
+// (Nmesh <= 4096: N^2 / 12 refills < 2^24)
+constexpr int kRlxRadix = 256, kRlxLevels = 3;
 constexpr uint64_t kMask48 = (uint64_t(1) << 48) - 1;
 
 struct Rlx {
