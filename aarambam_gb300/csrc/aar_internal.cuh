@@ -73,9 +73,7 @@ struct Plan {
   int qcube_m = 0;
   bool qcube_stale = true;
   void* d_rlxpow = nullptr;   // skip-ahead powers (seedtable_powers)
-  // modal term list (device)
-  void* d_terms = nullptr;
-  std::vector<char> host_terms;  // the same term list on the host (kernel parameter of the row combine)
+  std::vector<char> host_terms;  // the modal term list (a TermList, then its Terms)
   void* jit = nullptr;           // run-time specialised modal row kernel (jit.cu), or null
   int jit_mode = 1;              // 0 off, 1 for N >= 256, 2 always
   int jit_minb = 0;              // resident row blocks per SM of the NVRTC kernel (0: by N)
@@ -145,7 +143,6 @@ struct ProfScope {
 };
 
 int plan_alloc(Plan* p, void** ptr, size_t bytes);
-size_t terms_bytes();
 
 const char* set_err(Plan* p, const std::string& e);
 
@@ -201,10 +198,6 @@ int noalloc_gaussian(Plan* p, void* d_out, cudaStream_t st);
 int jit_prepare(Plan* p);
 int jit_modal_rows(Plan* p, float2* work, int64_t fs, cudaStream_t st, int64_t nrows = -1);
 int profile_modal_rows(Plan* p, float2* work, int64_t nrows, cudaStream_t st);
-// the specialised modal accumulation of the same module; false when the
-// plan has none (the generic k_modal_acc runs)
-bool jit_has_acc(const Plan* p);
-int jit_modal_acc(Plan* p, float2* phi, const float2* work, float fnl_n3, const RhoArgs& ra, cudaStream_t st);
 void jit_free(Plan* p);
 int adj_spectral(Plan* p, int op, int comp, int mode, const float2* in, float2* out, int accumulate,
                  cudaStream_t st);

@@ -238,14 +238,14 @@ static void plan_release(Plan* p) {
   p->prof.clear();
   for (auto e : p->event_pool) cudaEventDestroy(e);
   p->event_pool.clear();
-  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_terms, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube};
+  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   p->d_phik = p->d_work = nullptr;
   p->d_seed = nullptr;
   p->d_twN = p->d_twH = p->d_tw2 = nullptr;
   p->d_amp = p->d_twb = nullptr;
-  p->d_rlxpow = p->d_terms = nullptr;
+  p->d_rlxpow = nullptr;
   p->d_qtab = p->d_rtab = nullptr;
   p->d_sinc = p->d_isinc2 = nullptr;
   p->d_qcube = nullptr;
@@ -573,13 +573,11 @@ int aar_set_tables(aar_plan* h, const double* alpha, const double* x0, int32_t M
   plain_free(p);  // plain-form tables are rebuilt on the next run
   int rc;
   if (p->prm.precision == AAR_SLAB_FP32) {
-    if (!p->d_terms && (rc = plan_alloc(p, &p->d_terms, terms_bytes()))) return rc;
     if ((rc = build_term_list(p))) return rc;
   }
   if (p->prm.precision == AAR_FUSED_FP32) {
     p->qcube_stale = true;  // rebuilt on first use (ensure_fields)
     if ((rc = mode_tables(p))) return rc;
-    if (!p->d_terms && (rc = plan_alloc(p, &p->d_terms, terms_bytes()))) return rc;
     if ((rc = fused_prepare(p))) return rc;
     if ((rc = fused_configure_xform(p))) return rc;
   }

@@ -38,93 +38,6 @@
 namespace aar {
 
 
-// term list in plan-owned device memory (read uniformly by all threads)
-struct DevTerms {
-  TermList tl;
-  Term t[kMaxTerms];
-};
-size_t terms_bytes() { return sizeof(DevTerms); }
-
-// Last modal step, after the forward x transform of every active slot r:
-// acc = sum_r rho_r(k) g_r(k) (rho_r computed per cell in FP32, RhoArgs;
-// Neumaier-compensated in registers), then phi <- phi + fnl_n3 * acc,
-// DC = 0 (main.c:1101-1126).
-// One thread per half-spectrum element (padding columns are not touched);
-// cut cells keep phi as it is.  A streaming kernel: the R slot reads of a
-// thread are independent, so many are in flight per SM.  (Measured: pairs of
-// cells per thread with 16-byte loads were slower, 36.5 vs 30.8 ms at
-// 1024^3; so was the slot list as a kernel parameter, 39.0 ms, and the rho
-// row read with 16-byte loads into registers and the slots walked with
-// compile-time indices, 38.0 ms.  Gathering rho_r from a per-|k|^2 table,
-// one load per slot, left the kernel waiting on those loads: 31.4 ms.  The
-// slot loads issued in chunks of eight ahead of their sums: 48 registers,
-// five blocks per SM, 34.5 vs 28.9 ms.)
-template <int N>
-__global__ void __launch_bounds__(256) k_modal_acc(ModalArgs a, float2* phi, const float2* __restrict__ work,
-                                                   int64_t fs, int HP, float fnl_n3, const DevTerms* __restrict__ dt,
-                                                   const RhoArgs ra) {
-  constexpr int K = N / 2 + 1;  // kz = 0 .. N/2 of a row
-  constexpr int64_t total = (int64_t)N * N * K;
-  // the active slots and their field bases, once per block
-  __shared__ int rs[kMaxModes];
-  __shared__ const float2* base[kMaxModes];
-  const int nr = dt->tl.nr;
-  if (threadIdx.x < nr) {
-    const int r = dt->tl.r_of_slot[threadIdx.x];
-    rs[threadIdx.x] = r;
-    base[threadIdx.x] = work + (int64_t)r * fs;
-  }
-  __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / K;
-    const int kz = (int)(i - row * K);
-    const int64_t e = row * HP + kz;
-    int x, y;
-    row_xy(row, N, kXB, x, y);
-    const int kx = sidx(x, N), ky = sidx(y, N);
-    const int n2 = kx * kx + ky * ky + kz * kz;
-    if (n2 == 0) {
-      phi[e] = make_float2(0.f, 0.f);
-      continue;
-    }
-    if (!keep_cell(a.g, kx, ky, kz)) continue;
-    const float lnn2 = logf((float)n2);
-    const float kbar = -1.f + ra.c1 * expm1f(0.5f * ra.s * lnn2);
-    const float L = ra.log2kF + lnn2 * 0.72134752044448170368f;  // log2 k = log2 kF + ln(n2) / (2 ln 2)
-    const float inv_k2 = ra.inv_kF2 / (float)n2;
-    float P0 = 1.f, P1 = kbar;  // P_{deg-1}, P_deg
-    int deg = 1;
-    float sx = 0.f, sy = 0.f, cx = 0.f, cy = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < nr; ++k) {
-      const int r = rs[k];
-      const float2 v = __ldg(base[k] + e);
-      float rho;
-      if (r <= 3) {
-        rho = r == 3 ? 1.f : exp2f(ra.s * (float)(r - 3) * L);
-      } else {
-        while (deg < r - 1) {
-          ++deg;
-          const float Pn = ra.A[deg] * kbar * P1 - ra.B[deg] * P0;
-          P0 = P1;
-          P1 = Pn;
-        }
-        rho = (P1 - ra.x0[r - 1]) * inv_k2;
-      }
-      const float tx = v.x * rho, ty = v.y * rho;
-      const float ux = sx + tx, uy = sy + ty;
-      cx += (fabsf(sx) >= fabsf(tx)) ? (sx - ux) + tx : (tx - ux) + sx;
-      cy += (fabsf(sy) >= fabsf(ty)) ? (sy - uy) + ty : (ty - uy) + sy;
-      sx = ux;
-      sy = uy;
-    }
-    float2 ph = phi[e];
-    ph.x += fnl_n3 * (sx + cx);
-    ph.y += fnl_n3 * (sy + cy);
-    phi[e] = ph;
-  }
-}
-
 // phi_T = T(k)/(D Beta) phi on every half-spectrum cell (padding columns
 // are not touched): the factor the Hessians and psi1 share.
 template <int N>
@@ -782,20 +695,32 @@ struct Launch {
     const int64_t fs = fstride(p);
     const TermList& tl = terms(p);
     const Slots in = slots(tl.in_mode, tl.nin), out = slots(tl.r_of_slot, tl.nr);
-    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), p->d_qcube};
+    Slots in_line{}, out_line{};
+    for (int i = 0; i < tl.nin; ++i) in_line.s[i] = tl.line[tl.in_mode[i]];
+    for (int i = 0; i < tl.nr; ++i) out_line.s[i] = tl.line[tl.r_of_slot[i]];
+    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), in_line, p->d_qcube};
     int rc = run_pass<N, 0, +1>(p, xo, kTiles * tl.nin, st, "modal_xinv");
     if (rc) return rc;
     if ((rc = axis_pass<1, +1>(p, p->d_work, tl.nin, in, st, "modal_ypass_inv"))) return rc;
     if ((rc = p->jit ? jit_modal_rows(p, p->d_work, fs, st) : modal_rows(p, p->d_work, fs, (int64_t)N * N, st))) return rc;
     if ((rc = axis_pass<1, -1>(p, p->d_work, tl.nr, out, st, "modal_ypass_fwd"))) return rc;
-    // forward x of the active slots, then the accumulation into phi
-    if ((rc = axis_pass<0, -1>(p, p->d_work, tl.nr, out, st, "modal_xfwd"))) return rc;
-    float fnl_n3 = (float)(p->prm.fnl / ((double)N * N * N));
-    if (jit_has_acc(p)) return jit_modal_acc(p, p->d_phik, p->d_work, fnl_n3, rho_args(p), st);
+    const RhoArgs ra = rho_args(p);
+    const AccScale sc{(float)(p->prm.primordial_index - 4), ra.log2kF, (float)(p->prm.fnl / ((double)N * N * N))};
+    // one slot: 2.83 ms against k_xacc's 4.39 at 1024^3, whose registers leave
+    // one block per SM; with 16 values per lane and fewer k_xacc is as fast
+    // (0.0122 against 0.0132 ms at 128^3)
+    if constexpr (TileCfg<N>::R1 == 32) {
+      if (tl.nr == 1) {
+        const int64_t plane = (int64_t)(N / 2 + 1) * p->HP * (N / 2 + 1);
+        const XaddOp<N> xo1{a.g, p->d_phik, p->d_work + out.s[0] * fs, p->d_qcube + out_line.s[0] * plane, sc};
+        return run_pass<N, 0, -1>(p, xo1, kTiles, st, "modal_xacc");
+      }
+    }
+    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, out_line, p->d_qcube, sc};
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XaccCfg<N>::SMEM));
     {
-      ProfScope ps_(p, "modal_acc", st);
-      k_modal_acc<N><<<(unsigned)(p->num_sms * 8), 256, 0, st>>>(a, p->d_phik, p->d_work, fs, p->HP, fnl_n3,
-                                                             (const DevTerms*)p->d_terms, rho_args(p));
+      ProfScope ps_(p, "modal_xacc", st);
+      k_xacc<N><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -937,7 +862,7 @@ std::vector<int> modal_partition(const std::vector<std::vector<Term>>& by_r, int
   return part;
 }
 
-// The plan's term list (device and host copies): the regrouped terms, or
+// The plan's term list: the regrouped terms, or
 // with a modal partition only the slots of the plan's part.  A split keeps
 // the counter-term f_0 f_2 -> g_1 with the part of r = 1: as a term read
 // before g_2 replaces f_2 when r = 2 is in the same part, else as an
@@ -978,9 +903,6 @@ static int build_terms(Plan* p) {
     tl.line[m] = read[m] || active[m] ? tl.nlines++ : -1;
   }
   if (tl.nterms > kMaxTerms) return set_err(p, "too many alpha terms"), AAR_ERR_ARG;
-  DevTerms* dt = (DevTerms*)p->d_terms;
-  AAR_CUDA_TRY(p, cudaMemcpy(&dt->tl, &tl, sizeof(tl), cudaMemcpyHostToDevice));
-  if (!flat.empty()) AAR_CUDA_TRY(p, cudaMemcpy(dt->t, flat.data(), sizeof(Term) * flat.size(), cudaMemcpyHostToDevice));
   p->host_terms.assign((const char*)&tl, (const char*)&tl + sizeof(tl));
   p->host_terms.insert(p->host_terms.end(), (const char*)flat.data(), (const char*)(flat.data() + flat.size()));
   p->nterms = tl.nterms;
@@ -992,8 +914,9 @@ static int build_terms(Plan* p) {
 // (mode_tables: FP64 formulas rounded once to float) over 0 <= |kx|, |ky| <=
 // N/2 and the padded kz columns, zero on the cut, at k = 0 and on the padding
 // (keep_cell depends on |k_a| only).  Index (((p K + |ky|) NCOL + kz / 8) K +
-// |kx|) 8 + kz % 8 for the p-th mode that the products read, K = N/2 + 1, NCOL = HP / 8.
-__global__ void __launch_bounds__(256) k_qcube(Grid g, int nin, const __grid_constant__ Slots mode,
+// |kx|) 8 + kz % 8, p the row-kernel line of a read mode or active r (TermList),
+// K = N/2 + 1, NCOL = HP / 8.
+__global__ void __launch_bounds__(256) k_qcube(Grid g, int nl, const __grid_constant__ Slots mode,
                                                const float* __restrict__ qtab, int64_t nsq, float* __restrict__ q) {
   const int K = g.N / 2 + 1, ncol = g.HP / 8;
   const int64_t per = (int64_t)K * g.HP * K;
@@ -1004,26 +927,27 @@ __global__ void __launch_bounds__(256) k_qcube(Grid g, int nin, const __grid_con
     const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
     const int n2 = ax * ax + ay * ay + kz * kz;
     const bool on = kz <= g.N / 2 && n2 != 0 && keep_cell(g, ax, ay, kz);
-    for (int c = 0; c < nin; ++c) q[(int64_t)c * per + i] = on ? __ldg(qtab + (int64_t)mode.s[c] * nsq + n2) : 0.f;
+    for (int c = 0; c < nl; ++c) q[(int64_t)c * per + i] = on ? __ldg(qtab + (int64_t)mode.s[c] * nsq + n2) : 0.f;
   }
 }
 
 int qcube_build(Plan* p) {
   if (p->host_terms.empty()) return AAR_OK;  // no tables yet: nothing reads filters
   const TermList& tl = *(const TermList*)p->host_terms.data();
-  if ((!p->qcube_stale && p->d_qcube) || tl.nin == 0) return AAR_OK;
+  if ((!p->qcube_stale && p->d_qcube) || tl.nlines == 0) return AAR_OK;
   const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
-  if (!p->d_qcube || p->qcube_m != tl.nin) {
+  if (!p->d_qcube || p->qcube_m != tl.nlines) {
     if (p->d_qcube) cudaFree(p->d_qcube), p->used_bytes -= sizeof(float) * (size_t)per * p->qcube_m;
     p->d_qcube = nullptr;
     p->qcube_m = 0;
-    int rc = plan_alloc(p, (void**)&p->d_qcube, sizeof(float) * (size_t)per * tl.nin);
+    int rc = plan_alloc(p, (void**)&p->d_qcube, sizeof(float) * (size_t)per * tl.nlines);
     if (rc) return rc;
-    p->qcube_m = tl.nin;
+    p->qcube_m = tl.nlines;
   }
   Slots mode{};
-  for (int i = 0; i < tl.nin; ++i) mode.s[i] = tl.in_mode[i];
-  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, tl.nin, mode, p->d_qtab, p->nsq, p->d_qcube);
+  for (int m = 0; m < p->M; ++m)
+    if (tl.line[m] >= 0) mode.s[tl.line[m]] = m;
+  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, tl.nlines, mode, p->d_qtab, p->nsq, p->d_qcube);
   AAR_CUDA_TRY(p, cudaGetLastError());
   // made on the legacy stream once per table set; runs on the caller's
   // streams read it afterwards

@@ -94,7 +94,8 @@ struct XinvOp {
   int nin;
   Slots mode;
   unsigned grp;
-  const float* qcube;  // [nin][|ky|][kz / 8][|kx|][8]
+  Slots line;          // a mode's plane of the cube
+  const float* qcube;  // [line][|ky|][kz / 8][|kx|][8]
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     unsigned t;
     group_order<N>(item, (unsigned)nin, grp, t, c);
@@ -106,7 +107,7 @@ struct XinvOp {
     using C = TileCfg<N>;
     constexpr int K = N / 2 + 1;
     const int ay = o <= N / 2 ? o : N - o;
-    const float* q = qcube + ((((int64_t)c * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
+    const float* q = qcube + ((((int64_t)line.s[c] * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
     float f[C::R1];
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) {
@@ -231,5 +232,174 @@ struct XfwdInvK2Op {
         const float g = n2 ? -1.f / (kF * kF * (float)n2) : 0.f;
         v[b * C::R2 + r] = cscale(v[b * C::R2 + r], g);
       }
+  }
+};
+
+// k^(ns - 4) Fnl / N^3 at a cell of |k|^2 = n2 (grid units): the factor of the
+// modal sum's cube-weighted terms (rho_r = q_r k^(ns - 4))
+struct AccScale {
+  float e, log2kF, fnl_n3;  // e = ns - 4
+  __device__ __forceinline__ float at(int n2) const {
+    return fnl_n3 * exp2f(e * fmaf(0.5f, log2f((float)n2), log2kF));
+  }
+};
+
+// Last modal step: forward x pass of every active slot and the accumulation,
+// phi <- phi + fnl_n3 sum_r rho_r(k) g_r(k), DC = 0 (main.c:825-867,
+// 1101-1126).  rho_r = q_r k^(ns - 4) for every r (main.c:580-637, 833-860), so
+// the sum takes the filter cube's factors and one power of k at its end.  One
+// block per tile walks the slots: the tile of the next slot comes in through
+// shared memory (from N = 256 on) while one is transformed, the compensated
+// sums (two_sum2) stay in registers -- the transformed slots never go back to
+// memory, where a forward x pass and a pointwise accumulation moved them
+// three more times.  Cut cells keep phi.
+//
+// What bounds it: instruction issue of the 8 (N >= 512) to 16 warps that
+// 32 values, their sums and compensations leave room for.  Against the forward
+// x pass and the specialised pointwise accumulation: 0.39 -> 0.23 ms (256^3, 12
+// slots), 0.71 -> 0.33 (256^3, 19), 3.39 -> 1.95 (512^3, 11), 48.1 -> 35.0
+// (1024^3, 19).
+template <int N>
+struct XaccArgs {
+  Grid g;
+  float2* phi;
+  const float2* work;
+  int64_t fs;
+  int nr;
+  Slots slot, line;  // field and cube plane of an active r
+  const float* qcube;
+  AccScale sc;
+};
+template <int N>
+struct XaccCfg {
+  using C = TileCfg<N>;
+  static constexpr bool kStaged = N >= 256;
+  static constexpr int K = N / 2 + 1;
+  static constexpr size_t QROWS = (size_t)K * C::W;  // floats of a plane's column block
+  static constexpr size_t SMEM = C::SMEM + (kStaged ? sizeof(float2) * N * C::W + 2 * sizeof(float) * QROWS : 0);
+  static constexpr int MINB = C::R1 == 32 ? 256 / C::THREADS : C::R1 == 16 ? 512 / C::THREADS : 8;
+};
+template <int N>
+__global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
+    k_xacc(const __grid_constant__ XaccArgs<N> a, const float2* __restrict__ tw2) {
+  using C = TileCfg<N>;
+  using X = XaccCfg<N>;
+  extern __shared__ float2 ex[];
+  const int w = threadIdx.x % C::W, t = threadIdx.x / C::W;
+  int o, c0;
+  tile_coords<N>(blockIdx.x, o, c0);
+  const int64_t base = TileMap<N, 0>(o, c0, t, w).base;
+  const int ay = o <= N / 2 ? o : N - o;
+  const float* qb = a.qcube + ((int64_t)ay * C::NCOL + c0 / C::W) * X::QROWS;
+  constexpr int64_t plane = (int64_t)X::K * C::NCOL * X::QROWS;
+  float2* stage = ex + C::SMEM / sizeof(float2);
+  float* qs = reinterpret_cast<float*>(stage + N * C::W);  // two buffers
+  auto issue = [&](int s) {
+    tile_stage_load<N, 0>(stage, a.work + (int64_t)a.slot.s[s] * a.fs, o, c0);
+    const float* q = qb + a.line.s[s] * plane;
+    float* d = qs + (s & 1) * X::QROWS;
+    for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
+    cp_async_commit();
+  };
+  float2 sum[C::R1], cmp[C::R1];
+#pragma unroll
+  for (int i = 0; i < C::R1; ++i) sum[i] = cmp[i] = make_float2(0.f, 0.f);
+  if constexpr (X::kStaged) issue(0);
+#pragma unroll 1
+  for (int s = 0; s < a.nr; ++s) {
+    float2 v[C::R1];
+    const float* q;
+    if constexpr (X::kStaged) {
+      cp_async_wait<0>();
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < C::R1; ++r) v[r] = stage[tile_n<N>(t, r) * C::W + w];
+      __syncthreads();  // the stage is free, and the exchange of the slot before has been read
+      if (s + 1 < a.nr) issue(s + 1);
+      q = qs + (s & 1) * X::QROWS + w;
+    } else {
+      const float2* src = a.work + (int64_t)a.slot.s[s] * a.fs + base;
+#pragma unroll
+      for (int r = 0; r < C::R1; ++r) v[r] = src[TileMap<N, 0>::off(C::T * r)];
+      if (s) __syncthreads();  // the exchange has been read
+      q = qb + a.line.s[s] * plane + w;
+    }
+    tile_fft2<N, -1>(v, ex, t, w, tw2);
+#pragma unroll
+    for (int b = 0; b < C::G; ++b)
+#pragma unroll
+      for (int r = 0; r < C::R2; ++r) {
+        const int i = tile_out_i<N>(b, r), n = tile_n<N>(t, i);
+        const float f = q[(i < C::R1 / 2 ? n : N - n) * C::W];
+        two_sum2(sum[i], cmp[i], cscale(v[b * C::R2 + r], f));
+      }
+  }
+  const int kz = c0 + w;
+  if (kz > N / 2) return;
+  const int ky = sidx(o, N);
+  float2* phi = a.phi + base;
+  float2 u[C::R1];  // all loads first: behind one another's stores they cost 9 ms at 1024^3
+#pragma unroll
+  for (int i = 0; i < C::R1; ++i) u[i] = phi[TileMap<N, 0>::off(C::T * i)];
+#pragma unroll
+  for (int i = 0; i < C::R1; ++i) {
+    const int n = tile_n<N>(t, i);
+    const int kx = i < C::R1 / 2 ? n : n - N;
+    const int n2 = kx * kx + ky * ky + kz * kz;
+    const float g = a.sc.at(n2);
+    const float2 d = add2(sum[i], cmp[i]);
+    float2 r = make_float2(fmaf(g, d.x, u[i].x), fmaf(g, d.y, u[i].y));
+    if (!keep_cell(a.g, kx, ky, kz)) r = u[i];
+    if (n2 == 0) r = make_float2(0.f, 0.f);
+    phi[TileMap<N, 0>::off(C::T * i)] = r;
+  }
+}
+
+// The same with a single active r (Local templates): nothing to accumulate,
+// so a pass of its own with the plain passes' occupancy.
+template <int N>
+struct XaddOp {
+  static constexpr bool kPre = false, kPost = true;
+  Grid g;
+  float2* phi;
+  const float2* slot;
+  const float* q;  // the cube's plane of r
+  AccScale sc;
+  __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
+    tile_coords<N>(item, o, c0);
+    c = 0;
+  }
+  __device__ const float2* src(int) const { return slot; }
+  __device__ float2* dst(int) const { return phi; }
+  __device__ void post(float2* v, int o, int kz, int, int t) const {
+    using C = TileCfg<N>;
+    constexpr int K = N / 2 + 1;
+    const int ay = o <= N / 2 ? o : N - o, ky = sidx(o, N);
+    const float* qb = q + (((int64_t)ay * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
+    const float2* ph = phi + TileMap<N, 0>(o, kz, t, 0).base;
+    constexpr int H = 8 < C::R1 ? 8 : C::R1;  // values whose loads go out together
+#pragma unroll
+    for (int h = 0; h < C::R1; h += H) {
+      float2 u[H];
+      float f[H];
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        const int i = h + j, n = tile_n<N>(t, i);
+        u[j] = ph[TileMap<N, 0>::off(C::T * i)];
+        f[j] = __ldg(qb + (i < C::R1 / 2 ? n : N - n) * C::W);
+      }
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        const int i = h + j, n = tile_n<N>(t, i);
+        const int kx = i < C::R1 / 2 ? n : n - N;
+        const int n2 = kx * kx + ky * ky + kz * kz;
+        float2& x = v[(i % C::G) * C::R2 + i / C::G];  // tile_out_i
+        const float s = sc.at(n2);
+        float2 r = make_float2(fmaf(s, x.x * f[j], u[j].x), fmaf(s, x.y * f[j], u[j].y));
+        if (kz > N / 2 || !keep_cell(g, kx, ky, kz)) r = u[j];
+        if (n2 == 0) r = make_float2(0.f, 0.f);
+        x = r;
+      }
+    }
   }
 };

@@ -7,18 +7,6 @@
 
 namespace aar {
 
-// asynchronous global -> shared copies (sm_80+ cp.async), 8 bytes each
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int K>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory");
-}
-
-
 // Per-axis real factor of the 2LPT y pass and c2r rows (index k along the
 // axis; y uses the signed index, z the column index kz = 0..N/2): 0: 1,
 // 1: k, 2: k^2, 3: 1/sinc^2, 4: kF k / sinc^2, as the product of a table value

@@ -30,6 +30,17 @@
 
 namespace aar {
 
+// asynchronous global -> shared copy of 16 bytes (cp.async), past L1
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int K>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory");
+}
+
 template <int N>
 struct TileCfg {
   static constexpr int W = 8;
@@ -97,6 +108,44 @@ __device__ __forceinline__ void tile_fft2(float2* v, float2* ex, int t, int w, c
     for (int r = 1; r < C::R2; ++r) v[b * C::R2 + r] = cmul(v[b * C::R2 + r], tw_load<SIGN>(tw, r * C::R1));
     DFT<C::R2, SIGN>::run(v + b * C::R2);
   }
+}
+
+// Issue the asynchronous copy of a tile into shared memory as [n][W] (its
+// 64-byte row segments as they lie in memory).
+template <int N, int AXIS>
+__device__ __forceinline__ void tile_stage_load(float2* stage, const float2* __restrict__ f, int o, int c0) {
+  using C = TileCfg<N>;
+  constexpr int ROWS = C::THREADS / 4;  // rows of one copy per thread
+  static_assert(ROWS % kXB == 0 && N % ROWS == 0);
+  const int n = threadIdx.x >> 2, part = (threadIdx.x & 3) * 2;
+  const float2* src = f + TileMap<N, AXIS>(o, c0, n, part).base;
+  float2* dst = stage + n * C::W + part;
+#pragma unroll
+  for (int j = 0; j < N / ROWS; ++j) cp_async16(dst + j * ROWS * C::W, src + TileMap<N, AXIS>::off(j * ROWS));
+}
+
+// Packed FP32 sums of a complex value's two parts (one issue slot each; the
+// FP32 pipe takes as long as two scalar ones).
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return reinterpret_cast<float2&>(r);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return reinterpret_cast<float2&>(r);
+}
+// Knuth's two-sum: s + c carries the running sum of the t's, the rounding
+// error of s + t exactly (as Neumaier's step, without its comparison)
+__device__ __forceinline__ void two_sum2(float2& s, float2& c, float2 t) {
+  const float2 u = add2(s, t), b = sub2(u, s);
+  c = add2(c, add2(sub2(s, sub2(u, b)), sub2(t, b)));
+  s = u;
 }
 
 }  // namespace aar

@@ -71,3 +71,19 @@ def test_passes_match_plain_fp64(cuda, N, sphere, nsample, tab, M):
     assert rel(g.spectrum(), plain.spectrum()) < 1e-6
     for i, want in enumerate(lpt_fields(g, g.spectrum().to(torch.complex128))):
         assert rel(g.field(i), want) < (1e-6 if i < 3 else 2e-4), i
+
+
+@pytest.mark.parametrize("N", [64, 512])
+def test_single_slot_matches_plain_fp64(cuda, N):
+    """One active r (an exact Local table): the pass that adds it straight to
+    the potential from N = 512 on, the accumulating one below."""
+    alpha, x0 = np.zeros((6, 6, 6)), np.linspace(1.0, 0.5, 6)
+    for t in ((0, 0, 3), (0, 3, 0), (3, 0, 0)):
+        alpha[t] = 1.0
+    cfg = make_cfg(N, 500.0, 8, 1000.0, 6, "", 512, Nsample=N - 6)
+    lagr = torch.rand((10, 3), generator=torch.Generator(device="cuda").manual_seed(1), device=cuda) * 499.0
+    plain = ICGenerator(cfg, alpha, x0, *bbks(), precision="fp64_regrouped")
+    plain.run(lagr)
+    g = ICGenerator(cfg, alpha, x0, *bbks())
+    g.run(lagr)
+    assert rel(g.spectrum(), plain.spectrum()) < 1e-6
