@@ -222,9 +222,19 @@ template <int N>
 constexpr size_t pair_line_smem(int threads) {  // one line buffer per T threads
   return sizeof(float2) * (size_t)(threads / PairCfg<N>::T) * PairCfg<N>::LS;
 }
+// Start of memory row m's row in the caller's natural order, in rows
 template <int N>
+__device__ __forceinline__ int64_t nat_row(int64_t m) {
+  int x, y;
+  row_xy(m, N, kXB, x, y);
+  return (int64_t)x * N + y;
+}
+// NAT: the real rows go to `nat` in the caller's natural order, real
+// [N][N][N], else in place of the spectra.
+template <int N, bool NAT>
 __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
-    k_rows_c2r(float2* work, int64_t fs, int HP, int first, int64_t nrows, const float2* __restrict__ tw2, ZTypes zt) {
+    k_rows_c2r(float2* work, int64_t fs, int HP, int first, int64_t nrows, const float2* __restrict__ tw2, ZTypes zt,
+               float* nat) {
   using C = PairCfg<N>;
   extern __shared__ float2 sm[];
   const int u = threadIdx.x / C::T, t = threadIdx.x % C::T;
@@ -235,13 +245,14 @@ __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
   float2 v[C::R1];
   pair_spectrum<N, true>(v, f, row + 1 < nrows ? f + HP : nullptr, t, zf, act);
   pair_fft<N, +1>(v, sm + u * C::LS, t, tw2, act);  // every lane of the line has read its rows
-  float* a = reinterpret_cast<float*>(f);
   if (act) {
+    float* a = NAT ? nat + nat_row<N>(row) * N : reinterpret_cast<float*>(f);
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) a[t + C::T * i] = v[i].x;
     if (row + 1 < nrows) {
+      float* b = NAT ? nat + nat_row<N>(row + 1) * N : a + 2 * HP;
 #pragma unroll
-      for (int i = 0; i < C::R1; ++i) a[2 * HP + t + C::T * i] = v[i].y;
+      for (int i = 0; i < C::R1; ++i) b[t + C::T * i] = v[i].y;
     }
   }
 }
@@ -779,8 +790,8 @@ struct Launch {
     const ZTypes zt{{3, 3, 4, 3, 3, 4}, a.m.g.kF, a.isinc2};
     {
       ProfScope ps_(p, "lpt_rows_c2r", st);
-      k_rows_c2r<N><<<dim3(c2r_blocks<N>(), 6), kC2rThreads, pair_line_smem<N>(kC2rThreads), st>>>(
-          p->d_work, fs, p->HP, 0, (int64_t)N * N, p->d_tw2, zt);
+      k_rows_c2r<N, false><<<dim3(c2r_blocks<N>(), 6), kC2rThreads, pair_line_smem<N>(kC2rThreads), st>>>(
+          p->d_work, fs, p->HP, 0, (int64_t)N * N, p->d_tw2, zt, nullptr);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -1132,75 +1143,84 @@ int fused_readout_glass(Plan* p, int64_t nglass, int tile, float* d_pos, float* 
 // ----------------------------------------------------------- standalone 3-D transforms
 namespace aar {
 
+// r2c of the caller's natural-order real field `nat` into a plan field
 template <int N>
 __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
-    k_rows_r2c(float2* f, int HP, int64_t nrows, const float2* __restrict__ tw2) {
+    k_rows_r2c(const float* __restrict__ nat, float2* f, int HP, int64_t nrows, const float2* __restrict__ tw2) {
   using C = PairCfg<N>;
   extern __shared__ float2 sm[];
   const int u = threadIdx.x / C::T, t = threadIdx.x % C::T;
   const int64_t row = 2 * ((int64_t)blockIdx.x * (kC2rThreads / C::T) + u);
   const bool act = row < nrows, two = row + 1 < nrows;
-  float2* r = f + (act ? row : 0) * HP;
-  const float* a = reinterpret_cast<const float*>(r);
+  const float* a = nat + nat_row<N>(act ? row : 0) * N;
+  const float* b = nat + nat_row<N>(two ? row + 1 : 0) * N;
   float2 v[C::R1];
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) {
     const int n = t + C::T * i;
-    v[i] = make_float2(act ? a[n] : 0.f, two ? a[2 * HP + n] : 0.f);
+    v[i] = make_float2(act ? a[n] : 0.f, two ? b[n] : 0.f);
   }
-  pair_fft<N, -1>(v, sm + u * C::LS, t, tw2, act);  // every lane of the line has read its rows
-  pair_split<N>(v, r, HP, t, act, two);
+  pair_fft<N, -1>(v, sm + u * C::LS, t, tw2, act);
+  pair_split<N>(v, f + (act ? row : 0) * HP, HP, t, act, two);
 }
 
+// The 3-D transforms of a caller's field through work slot 0: the first pass
+// reads the caller's order, the last one writes it (with copies between the
+// two orders before and after an r2c and a c2r at 512^3 took 3.5 ms, now 1.2).
 template <int N>
 struct Xform {
   static constexpr int64_t tiles = TileCfg<N>::TILES;
   static constexpr size_t kSmem = pair_line_smem<N>(kC2rThreads);
-  static int c2r(Plan* p, float2* slot, cudaStream_t st) {
-    int rc = run_pass<N, 0, +1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_x");
+  static int c2r(Plan* p, const float2* in, float* out, cudaStream_t st) {
+    float2* slot = p->d_work;
+    int rc = run_pass<N, 0, +1>(p, XNatInOp<N>{in, slot}, tiles, st, "xform_x");
     if (rc) return rc;
     if ((rc = run_pass<N, 1, +1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_y"))) return rc;
     {
       ProfScope ps_(p, "xform_rows", st);
-      k_rows_c2r<N><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(slot, 0, p->HP, 0, (int64_t)N * N, p->d_tw2,
-                                                                 ZTypes{{0, 0, 0, 0, 0, 0}, 0.f, nullptr});
+      k_rows_c2r<N, true><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(slot, 0, p->HP, 0, (int64_t)N * N, p->d_tw2,
+                                                                       ZTypes{{0, 0, 0, 0, 0, 0}, 0.f, nullptr}, out);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
     return AAR_OK;
   }
-  static int r2c(Plan* p, float2* slot, cudaStream_t st) {
+  static int r2c(Plan* p, const float* in, float2* out, cudaStream_t st) {
+    float2* slot = p->d_work;
     {
       ProfScope ps_(p, "xform_rows", st);
-      k_rows_r2c<N><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(slot, p->HP, (int64_t)N * N, p->d_tw2);
+      k_rows_r2c<N><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(in, slot, p->HP, (int64_t)N * N, p->d_tw2);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
     int rc = run_pass<N, 1, -1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_y");
     if (rc) return rc;
-    return run_pass<N, 0, -1>(p, AxisOp<N>{slot, 0, Slots{}}, tiles, st, "xform_x");
+    return run_pass<N, 0, -1>(p, XNatOutOp<N>{slot, out}, tiles, st, "xform_x");
   }
 };
 
 // Row copy between row orders: row (x, y) of src (order src_xb, ld src_ld
-// elements) to row (x, y) of dst, the first ncols elements of each row.
-// Moves fields between the caller's natural [x][y] buffers and the plan's
-// x-blocked ones.
+// elements) to row (x, y) of dst, the first ncols elements of each row, a warp
+// per row.  Moves fields between the caller's natural [x][y] buffers and the
+// plan's x-blocked ones.
 template <class T>
-__global__ void k_copy_rows(T* __restrict__ dst, int64_t dst_ld, int dst_xb, const T* __restrict__ src, int64_t src_ld,
-                            int src_xb, int N, int ncols) {
-  const int64_t total = (int64_t)N * N * ncols;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / ncols;
-    const int c = (int)(i - r * ncols);
-    const int x = (int)(r / N), y = (int)(r % N);
-    dst[row_of(x, y, N, dst_xb) * dst_ld + c] = src[row_of(x, y, N, src_xb) * src_ld + c];
+__global__ void __launch_bounds__(256) k_copy_rows(T* __restrict__ dst, int64_t dst_ld, int dst_xb,
+                                                   const T* __restrict__ src, int64_t src_ld, int src_xb, int N,
+                                                   int ncols) {
+  const int lane = threadIdx.x & 31;
+  const int64_t rows = (int64_t)N * N, step = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += step) {
+    const int x = (int)(r / N), y = (int)(r - (int64_t)x * N);
+    T* d = dst + row_of(x, y, N, dst_xb) * dst_ld;
+    const T* s = src + row_of(x, y, N, src_xb) * src_ld;
+#pragma unroll 4
+    for (int c = lane; c < ncols; c += 32) d[c] = s[c];
   }
 }
 
 int copy_rows(Plan* p, void* dst, int64_t dst_ld, int dst_xb, const void* src, int64_t src_ld, int src_xb, int ncols,
               size_t elem, cudaStream_t st) {
-  const unsigned nb = (unsigned)(p->num_sms * 8);
+  const unsigned nb = (unsigned)std::min<int64_t>(((int64_t)p->N * p->N + 7) / 8, (int64_t)p->num_sms * 8);
   if (elem == sizeof(float2))
     k_copy_rows<float2><<<nb, 256, 0, st>>>((float2*)dst, dst_ld, dst_xb, (const float2*)src, src_ld, src_xb, p->N,
                                             ncols);
@@ -1211,30 +1231,21 @@ int copy_rows(Plan* p, void* dst, int64_t dst_ld, int dst_xb, const void* src, i
   return AAR_OK;
 }
 
-// unnormalised FFTW-convention transforms through work slot 0
+// unnormalised FFTW-convention transforms
 int fused_c2r(Plan* p, const float2* in, float* out, cudaStream_t st) {
-  int N = p->N, H = N / 2 + 1;
-  float2* slot = p->d_work;
-  int rc = copy_rows(p, slot, p->HP, kXB, in, H, 1, H, sizeof(float2), st);
-  if (rc) return rc;
-  if ((rc = dispatch_n(N, [&](auto nc) { return Xform<decltype(nc)::value>::c2r(p, slot, st); }))) return rc;
-  return copy_rows(p, out, N, 1, slot, 2 * p->HP, kXB, N, sizeof(float), st);
+  return dispatch_n(p->N, [&](auto nc) { return Xform<decltype(nc)::value>::c2r(p, in, out, st); });
 }
 
 int fused_r2c(Plan* p, const float* in, float2* out, cudaStream_t st) {
-  int N = p->N, H = N / 2 + 1;
-  float2* slot = p->d_work;
-  int rc = copy_rows(p, slot, 2 * p->HP, kXB, in, N, 1, N, sizeof(float), st);
-  if (rc) return rc;
-  if ((rc = dispatch_n(N, [&](auto nc) { return Xform<decltype(nc)::value>::r2c(p, slot, st); }))) return rc;
-  return copy_rows(p, out, H, 1, slot, p->HP, kXB, H, sizeof(float2), st);
+  return dispatch_n(p->N, [&](auto nc) { return Xform<decltype(nc)::value>::r2c(p, in, out, st); });
 }
 
 int fused_configure_xform(Plan* p) {
   return dispatch_n(p->N, [&](auto nc) {
     constexpr int N = decltype(nc)::value;
     const int smem = (int)pair_line_smem<N>(kC2rThreads);
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     return Launch<N>::configure(p);
   });

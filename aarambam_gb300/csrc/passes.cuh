@@ -6,6 +6,8 @@
 //   src(c), dst(c)          its input and output fields
 //   pre(v, ...)             spectral factors on the loaded values (kPre)
 //   post(v, ...)            factors on the transformed values (kPost)
+// and may name its input (kNatIn) or output (kNatOut) as a caller's field in
+// natural order.
 // Consecutive items run at the same time on consecutive blocks, so items
 // that share an input tile (one phi tile for the M filters, the 2LPT
 // components) are next to each other and hit L2.
@@ -22,20 +24,35 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, TileCfg<N>::MINB) k_pass(
   op.coords(blockIdx.x, o, c0, c);
   const TileMap<N, AXIS> tm(o, c0, t, w);
   float2 v[C::R1];
-  const float2* src = op.src(c) + tm.base;
+  if constexpr (requires { Op::kNatIn; }) {
+    static_assert(AXIS == 0);
+    const bool in = c0 + w <= N / 2;
+    const float2* src = op.src(c) + NatMap<N>::base(o, c0, t, w);
 #pragma unroll
-  for (int r = 0; r < C::R1; ++r) v[r] = src[TileMap<N, AXIS>::off(C::T * r)];
+    for (int r = 0; r < C::R1; ++r) v[r] = in ? src[NatMap<N>::off(C::T * r)] : make_float2(0.f, 0.f);
+  } else {
+    const float2* src = op.src(c) + tm.base;
+#pragma unroll
+    for (int r = 0; r < C::R1; ++r) v[r] = src[TileMap<N, AXIS>::off(C::T * r)];
+  }
   if constexpr (Op::kPre) op.pre(v, o, c0 + w, c, t);
   tile_fft2<N, SIGN>(v, ex, t, w, tw2);
   if constexpr (Op::kPost) op.post(v, o, c0 + w, c, t);
-  float2* dst = op.dst(c) + tm.base;
-  // opaque: an in-place pass would otherwise keep its R1 load addresses live
-  // for the stores (and spill values at 32 per thread)
-  asm volatile("" : "+l"(dst));
+  if constexpr (requires { Op::kNatOut; }) {
+    static_assert(AXIS == 0);
+    if (c0 + w > N / 2) return;
+    float2* dst = op.dst(c) + NatMap<N>::base(o, c0, t, w);
 #pragma unroll
-  for (int b = 0; b < C::G; ++b)
+    for (int b = 0; b < C::G; ++b)
 #pragma unroll
-    for (int r = 0; r < C::R2; ++r) dst[TileMap<N, AXIS>::off(C::T * b + C::R1 * r)] = v[b * C::R2 + r];
+      for (int r = 0; r < C::R2; ++r) dst[NatMap<N>::off(C::T * b + C::R1 * r)] = v[b * C::R2 + r];
+  } else {
+    float2* dst = op.dst(c) + tm.base;
+#pragma unroll
+    for (int b = 0; b < C::G; ++b)
+#pragma unroll
+      for (int r = 0; r < C::R2; ++r) dst[TileMap<N, AXIS>::off(C::T * b + C::R1 * r)] = v[b * C::R2 + r];
+  }
 }
 
 template <int N>
@@ -63,6 +80,33 @@ struct AxisOp {
   }
   __device__ const float2* src(int c) const { return base + (int64_t)c * fs; }
   __device__ float2* dst(int c) const { return base + (int64_t)c * fs; }
+};
+
+// x pass from a caller's natural-order spectrum into a plan field, and from a
+// plan field into one.
+template <int N>
+struct XNatInOp {
+  static constexpr bool kPre = false, kPost = false, kNatIn = true;
+  const float2* in;
+  float2* out;
+  __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
+    tile_coords<N>(item, o, c0);
+    c = 0;
+  }
+  __device__ const float2* src(int) const { return in; }
+  __device__ float2* dst(int) const { return out; }
+};
+template <int N>
+struct XNatOutOp {
+  static constexpr bool kPre = false, kPost = false, kNatOut = true;
+  const float2* in;
+  float2* out;
+  __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
+    tile_coords<N>(item, o, c0);
+    c = 0;
+  }
+  __device__ const float2* src(int) const { return in; }
+  __device__ float2* dst(int) const { return out; }
 };
 
 // Item order of the passes that write several output fields from one input

@@ -73,6 +73,17 @@ struct TileMap {
   static __device__ __forceinline__ int64_t off(int dn) { return (int64_t)dn * STEP; }  // dn a multiple of kXB
 };
 
+// The same in the caller's natural order, complex [N][N][N/2+1] (x passes): its
+// row segments start on any 8 bytes.
+template <int N>
+struct NatMap {
+  static constexpr int K = N / 2 + 1;
+  static __device__ __forceinline__ int64_t base(int o, int c0, int t, int w) {
+    return ((int64_t)t * N + o) * K + c0 + w;
+  }
+  static __device__ __forceinline__ int64_t off(int dn) { return (int64_t)dn * N * K; }
+};
+
 // Line index of value i of thread t before a transform (x[t + T i]) and, at
 // v[b R2 + r], after it (X[t + T b + R1 r]): the same indices, value i = b +
 // (R1 / T) r.
