@@ -33,7 +33,8 @@ EXPORTS = [
     "aar_stage_readout", "aar_stage_readout_glass", "aar_copy_spectrum", "aar_copy_field", "aar_gaussian_spectrum_noalloc", "aar_c2r", "aar_r2c", "aar_last_launch_count", "aar_profile_enable", "aar_profile_report",
     "aar_last_error", "aar_plan_destroy", "aar_version",
     "aar_batch_create", "aar_batch_run", "aar_batch_launch_count", "aar_batch_last_error", "aar_batch_destroy",
-    "aar_set_spectrum", "aar_adj_spectral", "aar_adj_source", "aar_adj_products", "aar_set_jit", "aar_jit_status",
+    "aar_set_spectrum", "aar_adj_spectral", "aar_adj_source", "aar_adj_products",
+    "aar_adj_displacement", "aar_adj_gradient_scratch_bytes", "aar_adj_gradient", "aar_set_jit", "aar_jit_status",
     "aar_tetra_covariance_scratch_bytes", "aar_tetra_covariance", "aar_tetra_QS", "aar_tetra_residual",
     "aar_tetra_modes_ld", "aar_tetra_modes", "aar_modes_covariance_scratch_bytes", "aar_modes_covariance",
     "aar_modes_project", "aar_modes_residual",
@@ -133,6 +134,10 @@ def load(build_if_missing: bool = False):
     L.aar_adj_spectral.argtypes = [vp, i32, i32, i32, vp, vp, i32, vp]
     L.aar_adj_source.argtypes = [vp, vp, vp, vp, vp]
     L.aar_adj_products.argtypes = [vp, vp, vp, vp, vp, vp]
+    L.aar_adj_displacement.argtypes = [vp, vp, vp, vp, vp, vp]
+    L.aar_adj_gradient_scratch_bytes.argtypes = [vp]
+    L.aar_adj_gradient_scratch_bytes.restype = C.c_size_t
+    L.aar_adj_gradient.argtypes = [vp, vp, vp, vp, vp, vp, vp, C.c_size_t, vp]
     # Decomposer (device pointers; tetrapyd arguments as tetrapyd.c's)
     tetra = [vp, vp, vp, vp, i32, vp, vp, vp, i32, vp, i32, i32]
     L.aar_tetra_covariance_scratch_bytes.argtypes = [i32, i32]

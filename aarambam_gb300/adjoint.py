@@ -18,11 +18,10 @@ dis2 /= N^3).  Inputs:
          AlphaTable rows, main.c:233-241), and the gradient is returned there.
 
 The backward pass is the transpose of every step (aarambam_gb300/csrc/
-adjoint.cu has the per-cell factors and the real-space products); it runs the
-plan's own FFTs and recomputes the M filtered fields f_p and the six
-Hessians from the saved spectra instead of storing them (memory: the noise,
-the Gaussian and the total potential spectra are saved; the backward holds
-about 2M + 12 fields at its peak).
+chain.cuh); it runs the plan's own FFT passes and recomputes the M filtered
+fields f_p and the six Hessians from the saved spectra instead of storing them
+(memory: the Gaussian and the total potential spectra are saved; the backward
+holds max(2M, 9) + 2 fields of scratch).
 """
 from __future__ import annotations
 
@@ -85,18 +84,14 @@ class _Ops:
 class _Displacement(torch.autograd.Function):
     @staticmethod
     def forward(ctx, w_hat, alpha, gen):
-        ops = _Ops(gen)
         N = gen.N
         ctx.w_dtype = w_hat.dtype
         w_hat = w_hat.to(torch.complex64).contiguous()
         gen.set_tables(alpha.detach().double().cpu().numpy())
-        phig = ops.spec(GAUSS, 0, FWD, w_hat)
-        ops.set_spectrum(phig)
-        gen.stage("modal")
-        phi = gen.spectrum()
-        gen.stage("lpt")
-        f = [gen.field(i) for i in range(6)]
-        disp = torch.stack(f[:3]) - (3.0 / 7.0) / float(N) ** 3 * torch.stack(f[3:])
+        phig, phi = torch.empty_like(w_hat), torch.empty_like(w_hat)
+        disp = torch.empty((3, N, N, N), dtype=torch.float32, device=gen.device)
+        check(gen.L, gen.h, gen.L.aar_adj_displacement(gen.h, _ptr(w_hat), _ptr(disp), _ptr(phig), _ptr(phi),
+                                                       gen._stream()))
         ctx.gen = gen
         ctx.save_for_backward(phig, phi)
         ctx.alpha_dtype, ctx.alpha_device = alpha.dtype, alpha.device
@@ -105,35 +100,14 @@ class _Displacement(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gdisp):
         gen = ctx.gen
-        ops = _Ops(gen)
         phig, phi = ctx.saved_tensors
-        N, M = gen.N, gen.n_modes
+        M = gen.n_modes
         gdisp = gdisp.to(torch.float32).contiguous()
-        # ZA and 2LPT read-outs: psi1 and -(3/7)/N^3 psi2
-        gphi = torch.zeros_like(phi)
-        gsrc = torch.zeros_like(phi)
-        c2 = -(3.0 / 7.0) / float(N) ** 3
-        for a in range(3):
-            ops.spec(PSI1, a, CT_W, ops.r2c(gdisp[a].contiguous()), out=gphi)
-            ops.spec(PSI2, a, CT_W, ops.r2c((c2 * gdisp[a]).contiguous()), out=gsrc)
-        gS = ops.c2r(ops.spec(ONE, 0, CT_INV_W, gsrc))
-        del gsrc
-        # source S(d) with the Hessians recomputed from phi
-        d = torch.stack([ops.c2r(ops.spec(HESS, ab, FWD, phi)) for ab in range(6)])
-        gd = ops.source_adj(d, gS)
-        del d, gS
-        for ab in range(6):
-            ops.spec(HESS, ab, CT_W, ops.r2c(gd[ab].contiguous()), out=gphi)
-        del gd
-        # modal part: phi = phig + sum_r rho_r r2c(g_r), g_r = sum alpha' f_p f_q
-        gg = torch.stack([ops.c2r(ops.spec(RHO, r, CT_INV_W, gphi)) for r in range(M)])
-        f = torch.stack([ops.c2r(ops.spec(Q, p, FWD, phig)) for p in range(M)])
-        gf, galpha = ops.products_adj(f, gg)
-        del f, gg
-        gphig = gphi
-        for p in range(M):
-            ops.spec(Q, p, CT_W, ops.r2c(gf[p].contiguous()), out=gphig)
-        gw = ops.spec(GAUSS, 0, CT, gphig)
+        gw = torch.empty_like(phig)
+        galpha = torch.empty((M, M, M), dtype=torch.float64, device=gdisp.device)
+        scratch = torch.empty(gen.L.aar_adj_gradient_scratch_bytes(gen.h), dtype=torch.uint8, device=gdisp.device)
+        check(gen.L, gen.h, gen.L.aar_adj_gradient(gen.h, _ptr(phig), _ptr(phi), _ptr(gdisp), _ptr(gw), _ptr(galpha),
+                                                   _ptr(scratch), scratch.numel(), gen._stream()))
         return gw.to(ctx.w_dtype), galpha.to(device=ctx.alpha_device, dtype=ctx.alpha_dtype), None
 
 

@@ -72,6 +72,15 @@ struct Plan {
   float* d_qcube = nullptr;
   int qcube_m = 0;
   bool qcube_stale = true;
+  // gradient (chain.cuh): the cube of all modes where the one above is not,
+  // and the products' tables, made on the first gradient after a table change
+  float* d_qfull = nullptr;
+  int qfull_m = 0;
+  bool qfull_stale = true;
+  void* d_chain = nullptr;
+  size_t chain_bytes = 0;
+  int chain_nent = 0, chain_ngrp = 0;
+  bool chain_stale = true;
   void* d_rlxpow = nullptr;   // skip-ahead powers (seedtable_powers)
   std::vector<char> host_terms;  // the modal term list (a TermList, then its Terms)
   void* jit = nullptr;           // run-time specialised modal row kernel (jit.cu), or null
@@ -191,6 +200,11 @@ void slab_free(Plan* p);
 int fused_c2r(Plan* p, const float2* in, float* out, cudaStream_t st);
 int fused_r2c(Plan* p, const float* in, float2* out, cudaStream_t st);
 int fused_configure_xform(Plan* p);
+// the differentiable chain and its transpose (chain.cuh)
+size_t chain_scratch_bytes(const Plan* p);
+int chain_forward(Plan* p, const float2* w, float* disp, float2* phig, float2* phi, cudaStream_t st);
+int chain_backward(Plan* p, const float2* phig, const float2* phi, const float* gdisp, float2* gw, double* galpha,
+                   float2* scratch, cudaStream_t st);
 // row copy between row orders (row_of), ncols elements of `elem` bytes per row
 int copy_rows(Plan* p, void* dst, int64_t dst_ld, int dst_xb, const void* src, int64_t src_ld, int src_xb, int ncols,
               size_t elem, cudaStream_t st);

@@ -238,7 +238,7 @@ static void plan_release(Plan* p) {
   p->prof.clear();
   for (auto e : p->event_pool) cudaEventDestroy(e);
   p->event_pool.clear();
-  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube};
+  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_qfull, p->d_chain};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   p->d_phik = p->d_work = nullptr;
@@ -248,9 +248,11 @@ static void plan_release(Plan* p) {
   p->d_rlxpow = nullptr;
   p->d_qtab = p->d_rtab = nullptr;
   p->d_sinc = p->d_isinc2 = nullptr;
-  p->d_qcube = nullptr;
-  p->qcube_m = 0;
-  p->qcube_stale = true;
+  p->d_qcube = p->d_qfull = nullptr;
+  p->qcube_m = p->qfull_m = 0;
+  p->qcube_stale = p->qfull_stale = p->chain_stale = true;
+  p->d_chain = nullptr;
+  p->chain_bytes = 0;
   p->d_io = nullptr;
   p->io_cap = 0;
   p->d_adj_scratch = nullptr;
@@ -1228,6 +1230,29 @@ int aar_adj_products(aar_plan* h, const float* d_f, const float* d_gg, float* d_
   int rc = adj_ready(&h->p);
   if (rc) return rc;
   return adj_products(&h->p, d_f, d_gg, d_gf, d_galpha, S(stream));
+}
+
+int aar_adj_displacement(aar_plan* h, const void* d_w, float* d_disp, void* d_phig, void* d_phi, void* stream) {
+  if (!h || !d_w || !d_disp || !d_phig || !d_phi) return AAR_ERR_ARG;
+  int rc = adj_ready(&h->p);
+  if (rc) return rc;
+  h->p.last_launches = 0;
+  return chain_forward(&h->p, (const float2*)d_w, d_disp, (float2*)d_phig, (float2*)d_phi, S(stream));
+}
+
+size_t aar_adj_gradient_scratch_bytes(const aar_plan* h) {
+  return h && h->p.prm.precision == AAR_FUSED_FP32 && h->p.have_tables ? chain_scratch_bytes(&h->p) : 0;
+}
+
+int aar_adj_gradient(aar_plan* h, const void* d_phig, const void* d_phi, const float* d_gdisp, void* d_gw,
+                     double* d_galpha, void* d_scratch, size_t scratch_bytes, void* stream) {
+  if (!h || !d_phig || !d_phi || !d_gdisp || !d_gw || !d_galpha || !d_scratch) return AAR_ERR_ARG;
+  int rc = adj_ready(&h->p);
+  if (rc) return rc;
+  if (scratch_bytes < chain_scratch_bytes(&h->p)) return set_err(&h->p, "gradient scratch too small"), AAR_ERR_ARG;
+  h->p.last_launches = 0;
+  return chain_backward(&h->p, (const float2*)d_phig, (const float2*)d_phi, d_gdisp, (float2*)d_gw, d_galpha,
+                        (float2*)d_scratch, S(stream));
 }
 
 // ------------------------------------------------------------- batches

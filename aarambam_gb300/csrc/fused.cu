@@ -727,11 +727,11 @@ struct Launch {
         return run_pass<N, 0, -1>(p, xo1, kTiles, st, "modal_xacc");
       }
     }
-    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, out_line, p->d_qcube, sc};
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XaccCfg<N>::SMEM));
+    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, out_line, p->d_qcube, sc, nullptr, nullptr};
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XaccCfg<N>::SMEM));
     {
       ProfScope ps_(p, "modal_xacc", st);
-      k_xacc<N><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);
+      k_xacc<N, false><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -918,6 +918,7 @@ static int build_terms(Plan* p) {
   p->host_terms.insert(p->host_terms.end(), (const char*)flat.data(), (const char*)(flat.data() + flat.size()));
   p->nterms = tl.nterms;
   p->nr_active = nr;
+  p->chain_stale = p->qfull_stale = true;
   return AAR_OK;
 }
 
@@ -942,27 +943,37 @@ __global__ void __launch_bounds__(256) k_qcube(Grid g, int nl, const __grid_cons
   }
 }
 
-int qcube_build(Plan* p) {
-  if (p->host_terms.empty()) return AAR_OK;  // no tables yet: nothing reads filters
-  const TermList& tl = *(const TermList*)p->host_terms.data();
-  if ((!p->qcube_stale && p->d_qcube) || tl.nlines == 0) return AAR_OK;
+// The cube of n modes into `cube` (plan-owned, `have` planes of it allocated)
+static int make_cube(Plan* p, int n, const Slots& mode, float*& cube, int& have) {
   const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
-  if (!p->d_qcube || p->qcube_m != tl.nlines) {
-    if (p->d_qcube) cudaFree(p->d_qcube), p->used_bytes -= sizeof(float) * (size_t)per * p->qcube_m;
-    p->d_qcube = nullptr;
-    p->qcube_m = 0;
-    int rc = plan_alloc(p, (void**)&p->d_qcube, sizeof(float) * (size_t)per * tl.nlines);
+  if (!cube || have != n) {
+    if (cube) {
+      AAR_CUDA_TRY(p, cudaDeviceSynchronize());
+      cudaFree(cube), p->used_bytes -= sizeof(float) * (size_t)per * have;
+    }
+    cube = nullptr;
+    have = 0;
+    int rc = plan_alloc(p, (void**)&cube, sizeof(float) * (size_t)per * n);
     if (rc) return rc;
-    p->qcube_m = tl.nlines;
+    have = n;
   }
-  Slots mode{};
-  for (int m = 0; m < p->M; ++m)
-    if (tl.line[m] >= 0) mode.s[tl.line[m]] = m;
-  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, tl.nlines, mode, p->d_qtab, p->nsq, p->d_qcube);
+  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, n, mode, p->d_qtab, p->nsq, cube);
   AAR_CUDA_TRY(p, cudaGetLastError());
   // made on the legacy stream once per table set; runs on the caller's
   // streams read it afterwards
   AAR_CUDA_TRY(p, cudaDeviceSynchronize());
+  return AAR_OK;
+}
+
+int qcube_build(Plan* p) {
+  if (p->host_terms.empty()) return AAR_OK;  // no tables yet: nothing reads filters
+  const TermList& tl = *(const TermList*)p->host_terms.data();
+  if ((!p->qcube_stale && p->d_qcube) || tl.nlines == 0) return AAR_OK;
+  Slots mode{};
+  for (int m = 0; m < p->M; ++m)
+    if (tl.line[m] >= 0) mode.s[tl.line[m]] = m;
+  int rc = make_cube(p, tl.nlines, mode, p->d_qcube, p->qcube_m);
+  if (rc) return rc;
   p->qcube_stale = false;
   return AAR_OK;
 }
@@ -1143,17 +1154,20 @@ int fused_readout_glass(Plan* p, int64_t nglass, int tile, float* d_pos, float* 
 // ----------------------------------------------------------- standalone 3-D transforms
 namespace aar {
 
-// r2c of the caller's natural-order real field `nat` into a plan field
-template <int N>
+// r2c of real fields into plan fields fs apart, blockIdx.y of them: NAT, the
+// caller's natural-order ones at `nat`, N^3 apart, else in place
+template <int N, bool NAT>
 __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
-    k_rows_r2c(const float* __restrict__ nat, float2* f, int HP, int64_t nrows, const float2* __restrict__ tw2) {
+    k_rows_r2c(const float* nat, float2* f, int64_t fs, int HP, int64_t nrows, const float2* __restrict__ tw2) {
   using C = PairCfg<N>;
   extern __shared__ float2 sm[];
   const int u = threadIdx.x / C::T, t = threadIdx.x % C::T;
   const int64_t row = 2 * ((int64_t)blockIdx.x * (kC2rThreads / C::T) + u);
   const bool act = row < nrows, two = row + 1 < nrows;
-  const float* a = nat + nat_row<N>(act ? row : 0) * N;
-  const float* b = nat + nat_row<N>(two ? row + 1 : 0) * N;
+  f += blockIdx.y * fs + (act ? row : 0) * HP;
+  if (NAT) nat += blockIdx.y * ((int64_t)N * N * N);
+  const float* a = NAT ? nat + nat_row<N>(act ? row : 0) * N : reinterpret_cast<const float*>(f);
+  const float* b = NAT ? nat + nat_row<N>(two ? row + 1 : 0) * N : a + (two ? 2 * HP : 0);
   float2 v[C::R1];
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) {
@@ -1161,7 +1175,7 @@ __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
     v[i] = make_float2(act ? a[n] : 0.f, two ? b[n] : 0.f);
   }
   pair_fft<N, -1>(v, sm + u * C::LS, t, tw2, act);
-  pair_split<N>(v, f + (act ? row : 0) * HP, HP, t, act, two);
+  pair_split<N>(v, f, HP, t, act, two);
 }
 
 // The 3-D transforms of a caller's field through work slot 0: the first pass
@@ -1189,7 +1203,7 @@ struct Xform {
     float2* slot = p->d_work;
     {
       ProfScope ps_(p, "xform_rows", st);
-      k_rows_r2c<N><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(in, slot, p->HP, (int64_t)N * N, p->d_tw2);
+      k_rows_r2c<N, true><<<c2r_blocks<N>(), kC2rThreads, kSmem, st>>>(in, slot, 0, p->HP, (int64_t)N * N, p->d_tw2);
     }
     AAR_CUDA_TRY(p, cudaGetLastError());
     p->last_launches += 1;
@@ -1240,13 +1254,240 @@ int fused_r2c(Plan* p, const float* in, float2* out, cudaStream_t st) {
   return dispatch_n(p->N, [&](auto nc) { return Xform<decltype(nc)::value>::r2c(p, in, out, st); });
 }
 
+#include "chain.cuh"
+
+// Device tables of the chain's products (entries, groups) and the sums; made
+// once per table set.
+struct ChainTables {
+  AdjEntry* ent;
+  AdjGroup* grp;
+  double* sum;
+  int nent, ngrp;
+};
+static int chain_tables(Plan* p, ChainTables& ct, cudaStream_t st) {
+  const int M = p->M, ntrip = chain_ntrip(M);
+  if (!p->d_chain || p->chain_stale) {
+    const TermList& tl = *(const TermList*)p->host_terms.data();
+    const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
+    std::vector<std::vector<AdjEntry>> by((size_t)M * M);  // [p][r]
+    for (int i = 0; i < tl.nterms; ++i) {
+      if (ft[i].c == 0.f) continue;
+      by[(size_t)ft[i].p * M + ft[i].r].push_back(AdjEntry{ft[i].c, ft[i].q});
+      by[(size_t)ft[i].q * M + ft[i].r].push_back(AdjEntry{ft[i].c, ft[i].p});
+    }
+    std::vector<AdjEntry> ent;
+    std::vector<AdjGroup> grp;
+    for (int i = 0; i < M * M; ++i) {
+      if (by[i].empty()) continue;
+      grp.push_back(AdjGroup{i / M, i % M, (int)ent.size(), (int)(ent.size() + by[i].size())});
+      ent.insert(ent.end(), by[i].begin(), by[i].end());
+    }
+    const size_t o_grp = sizeof(double) * ntrip, o_ent = o_grp + sizeof(AdjGroup) * grp.size();
+    const size_t need = o_ent + sizeof(AdjEntry) * ent.size();
+    AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // an earlier pass may still read the old tables
+    if (p->chain_bytes < need) {
+      if (p->d_chain) cudaFree(p->d_chain), p->used_bytes -= p->chain_bytes;
+      p->d_chain = nullptr;
+      p->chain_bytes = 0;
+      int rc = plan_alloc(p, &p->d_chain, need);
+      if (rc) return rc;
+      p->chain_bytes = need;
+    }
+    std::vector<char> host(need - o_grp);
+    std::copy(grp.begin(), grp.end(), (AdjGroup*)host.data());
+    std::copy(ent.begin(), ent.end(), (AdjEntry*)(host.data() + (o_ent - o_grp)));
+    AAR_CUDA_TRY(p, cudaMemcpy((char*)p->d_chain + o_grp, host.data(), host.size(), cudaMemcpyHostToDevice));
+    p->chain_nent = (int)ent.size();
+    p->chain_ngrp = (int)grp.size();
+    p->chain_stale = false;
+  }
+  ct.sum = (double*)p->d_chain;
+  ct.grp = (AdjGroup*)(ct.sum + ntrip);
+  ct.ent = (AdjEntry*)(ct.grp + p->chain_ngrp);
+  ct.nent = p->chain_nent;
+  ct.ngrp = p->chain_ngrp;
+  AAR_CUDA_TRY(p, cudaMemsetAsync(ct.sum, 0, sizeof(double) * ntrip, st));
+  return AAR_OK;
+}
+
+// The filter cube of all M modes (the products' gradients need the ones that
+// the products do not read, too): the plan's own where its lines are all
+// modes, else a second one made on the first gradient after a table change.
+static int chain_cube(Plan* p, const float*& cube, Slots& plane) {
+  const TermList& tl = *(const TermList*)p->host_terms.data();
+  for (int m = 0; m < p->M; ++m) plane.s[m] = tl.nlines == p->M ? tl.line[m] : m;
+  cube = p->d_qcube;
+  if (tl.nlines == p->M) return AAR_OK;
+  if (p->qfull_stale || !p->d_qfull) {
+    Slots mode{};
+    for (int m = 0; m < p->M; ++m) mode.s[m] = m;
+    int rc = make_cube(p, p->M, mode, p->d_qfull, p->qfull_m);
+    if (rc) return rc;
+    p->qfull_stale = false;
+  }
+  cube = p->d_qfull;
+  return AAR_OK;
+}
+
+// Fields of the gradient's scratch: G, T, then the larger of the Hessian
+// stage's nine and the products' 2 M.
+static int chain_fields(int M) { return 2 + std::max(9, 2 * M); }
+
+template <int N>
+struct Chain {
+  using L = Launch<N>;
+  static constexpr int64_t kTiles = TileCfg<N>::TILES;
+  static constexpr size_t kLineSmem = pair_line_smem<N>(kC2rThreads);
+  static unsigned cells(Plan* p) { return (unsigned)(p->num_sms * 8); }
+  static int done(Plan* p) {
+    AAR_CUDA_TRY(p, cudaGetLastError());
+    p->last_launches += 1;
+    return AAR_OK;
+  }
+  static Slots run(int first, int n) {
+    Slots s{};
+    for (int i = 0; i < n; ++i) s.s[i] = first + i;
+    return s;
+  }
+  static int forward(Plan* p, const float2* w, float* disp, float2* phig, float2* phi, cudaStream_t st) {
+    int rc;
+    k_chain_gauss<N><<<cells(p), 256, 0, st>>>(p->grid, p->d_amp, w, p->d_phik, phig);
+    if ((rc = done(p)) || (rc = fused_modal(p, st))) return rc;
+    if ((rc = copy_rows(p, phi, N / 2 + 1, 1, p->d_phik, p->HP, kXB, N / 2 + 1, sizeof(float2), st))) return rc;
+    if ((rc = fused_lpt(p, st))) return rc;
+    k_chain_disp<N><<<dim3(cells(p), 3), 256, 0, st>>>((const float*)p->d_work, 2 * L::fstride(p), p->HP,
+                                                       (float)(-(3.0 / 7.0) / ((double)N * N * N)), disp);
+    return done(p);
+  }
+  static int backward(Plan* p, const float2* phig, const float2* phi, const float* gdisp, float2* gw, double* galpha,
+                      float2* scratch, cudaStream_t st) {
+    const int64_t fs = L::fstride(p), rows = (int64_t)N * N;
+    const int M = p->M;
+    float2 *G = scratch, *T = scratch + fs, *W = scratch + 2 * fs;
+    const LptArgs a = lpt_args(p);
+    const float kF = a.m.g.kF;
+    const ZTypes none{{0, 0, 0, 0, 0, 0}, 0.f, nullptr};
+    const RhoArgs ra = rho_args(p);
+    const AccScale sc{(float)(p->prm.primordial_index - 4), ra.log2kF, (float)(p->prm.fnl / ((double)N * N * N))};
+    ChainTables ct;
+    Slots plane{};
+    const float* cube = nullptr;
+    int rc;
+    if ((rc = chain_tables(p, ct, st)) || (rc = chain_cube(p, cube, plane))) return rc;
+    // displacement fields
+    k_rows_r2c<N, true><<<dim3(c2r_blocks<N>(), 3), kC2rThreads, kLineSmem, st>>>(gdisp, W, fs, p->HP, rows, p->d_tw2);
+    if ((rc = done(p))) return rc;
+    if ((rc = L::template axis_pass<1, -1>(p, W, 3, run(0, 3), st, "grad_y"))) return rc;
+    if ((rc = L::template axis_pass<0, -1>(p, W, 3, run(0, 3), st, "grad_x"))) return rc;
+    k_chain_div<N><<<cells(p), 256, 0, st>>>(a, W, fs, (float)(-(3.0 / 7.0) / ((double)N * N * N)), G, T);
+    if ((rc = done(p))) return rc;
+    if ((rc = L::template axis_pass<0, +1>(p, T, 1, run(0, 1), st, "grad_x"))) return rc;
+    if ((rc = L::template axis_pass<1, +1>(p, T, 1, run(0, 1), st, "grad_y"))) return rc;
+    // the source, its Hessians made again from phi
+    k_chain_twb<N><<<cells(p), 256, 0, st>>>(p->HP, p->d_twb, phi, W + 7 * fs);
+    if ((rc = done(p))) return rc;
+    const LptXOp<N, 0> ho{W + 7 * fs, W, fs, {0, 8, 6}, 1, kF, a.isinc2};
+    if ((rc = run_pass<N, 0, +1>(p, ho, kTiles * 3, st, "grad_xhess"))) return rc;
+    const YFanOp<N> yf{W, fs, {0, 8, 8, 6, 6, 6}, {0, 1, 2, 3, 4, 5}, {0, 1, 0, 2, 1, 0}, 1, kF, a.isinc2};
+    if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "grad_yhess"))) return rc;
+    {
+      ProfScope ps_(p, "grad_rows_source", st);
+      constexpr int per = 2 * (32 / PairCfg<N>::T);  // rows of a block
+      constexpr size_t smem = L::pair_smem(7 * (32 / PairCfg<N>::T));
+      AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_source_adj<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      k_rows_source_adj<N><<<(unsigned)((rows + per - 1) / per), kSevenThreads, smem, st>>>(
+          SourceAdjRowOp{-1, kF, a.isinc2}, W, fs, p->HP, rows, p->d_tw2);
+    }
+    if ((rc = done(p))) return rc;
+    if ((rc = run_pass<N, 1, -1>(p, YAdjOp<N>{W, fs, Slots{{0, 1, 0, 2, 1, 0}}}, kTiles * 6, st, "grad_y"))) return rc;
+    if ((rc = run_pass<N, 0, -1>(p, XSumOp<N>{W, fs, {0, 1, 3}, {1, 2, 3}}, kTiles * 3, st, "grad_x"))) return rc;
+    k_chain_hess<N><<<cells(p), 256, 0, st>>>(a, W, fs, sc, G, T);
+    if ((rc = done(p))) return rc;
+    // the modal products, their fields made again from phig
+    const XinvOp<N> xg{T, W, fs, M, run(M, M), 1, plane, cube};
+    if ((rc = run_pass<N, 0, +1>(p, xg, kTiles * M, st, "grad_xinv"))) return rc;
+    const XinvNatOp<N> xf{{phig, W, fs, M, run(0, M), 1, plane, cube}};
+    if ((rc = run_pass<N, 0, +1>(p, xf, kTiles * M, st, "grad_xinv"))) return rc;
+    for (int h = 0; h < 2; ++h)
+      if ((rc = L::template axis_pass<1, +1>(p, W, M, run(h * M, M), st, "grad_y"))) return rc;
+    {
+      ProfScope ps_(p, "grad_rows", st);
+      k_rows_c2r<N, false><<<dim3(c2r_blocks<N>(), 2 * M), kC2rThreads, kLineSmem, st>>>(W, fs, p->HP, 0, rows, p->d_tw2,
+                                                                                        none, nullptr);
+    }
+    if ((rc = done(p))) return rc;
+    {
+      ProfScope ps_(p, "grad_sums", st);
+      // r in as few blocks of at most 16 as hold them, the threads in as many
+      // shares of a chunk as the items leave
+      const int nrb = (M + 15) / 16, rb = (M + nrb - 1) / nrb;
+      const int items = M * (M + 1) / 2 * nrb, share = items <= 32 ? 4 : items <= 64 ? 2 : 1;
+      const size_t smem = sizeof(double) * ((share * chain_ntrip(M) + 1) / 2 * 2) + sizeof(float) * 2 * M * kChainLd;
+      const unsigned blocks = (unsigned)std::min<int64_t>((int64_t)N * N * N / kChainChunk, (int64_t)p->num_sms * 8);
+      auto go = [&](auto rbc) {
+        auto kern = k_chain_sums<N, decltype(rbc)::value>;
+        AAR_CUDA_TRY(p, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<blocks, kChainThreads, smem, st>>>((const float*)W, 2 * fs, p->HP, M, share, ct.sum);
+        return AAR_OK;
+      };
+      if ((rc = rb <= 4 ? go(std::integral_constant<int, 4>{})
+                : rb <= 8 ? go(std::integral_constant<int, 8>{})
+                : rb <= 12 ? go(std::integral_constant<int, 12>{})
+                           : go(std::integral_constant<int, 16>{})))
+        return rc;
+    }
+    if ((rc = done(p))) return rc;
+    {
+      ProfScope ps_(p, "grad_gf", st);
+      const size_t smem = sizeof(float2) * 2 * M * kChainThreads + sizeof(AdjEntry) * ((ct.nent + 1) / 2 * 2) +
+                          sizeof(AdjGroup) * ct.ngrp;
+      AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_chain_gf<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const int64_t n2 = (int64_t)N * N * N / 2;
+      k_chain_gf<N><<<(unsigned)std::min<int64_t>((n2 + kChainThreads - 1) / kChainThreads, (int64_t)p->num_sms * 16),
+                      kChainThreads, smem, st>>>((float*)W, 2 * fs, p->HP, M, ct.ent, ct.nent, ct.grp, ct.ngrp);
+    }
+    if ((rc = done(p))) return rc;
+    const int counter = M > 2 && p->alpha[(size_t)1 * M + 2] != 0;
+    k_chain_galpha<<<1, 256, 0, st>>>(ct.sum, M, counter, galpha);
+    if ((rc = done(p))) return rc;
+    {
+      ProfScope ps_(p, "grad_rows", st);
+      k_rows_r2c<N, false><<<dim3(c2r_blocks<N>(), M), kC2rThreads, kLineSmem, st>>>(nullptr, W, fs, p->HP, rows, p->d_tw2);
+    }
+    if ((rc = done(p))) return rc;
+    if ((rc = L::template axis_pass<1, -1>(p, W, M, run(0, M), st, "grad_y"))) return rc;
+    const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), plane, cube, sc, p->d_amp, gw};
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)XaccCfg<N>::SMEM));
+    {
+      ProfScope ps_(p, "grad_xacc", st);
+      k_xacc<N, true><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);
+    }
+    return done(p);
+  }
+};
+
+size_t chain_scratch_bytes(const Plan* p) {
+  return sizeof(float2) * (size_t)p->N * p->N * p->HP * chain_fields(p->M);
+}
+int chain_forward(Plan* p, const float2* w, float* disp, float2* phig, float2* phi, cudaStream_t st) {
+  return dispatch_n(p->N, [&](auto nc) { return Chain<decltype(nc)::value>::forward(p, w, disp, phig, phi, st); });
+}
+int chain_backward(Plan* p, const float2* phig, const float2* phi, const float* gdisp, float2* gw, double* galpha,
+                   float2* scratch, cudaStream_t st) {
+  return dispatch_n(p->N, [&](auto nc) {
+    return Chain<decltype(nc)::value>::backward(p, phig, phi, gdisp, gw, galpha, scratch, st);
+  });
+}
+
 int fused_configure_xform(Plan* p) {
   return dispatch_n(p->N, [&](auto nc) {
     constexpr int N = decltype(nc)::value;
     const int smem = (int)pair_line_smem<N>(kC2rThreads);
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     return Launch<N>::configure(p);
   });
 }

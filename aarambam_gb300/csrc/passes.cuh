@@ -55,6 +55,16 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, TileCfg<N>::MINB) k_pass(
   }
 }
 
+__device__ __forceinline__ float half_weight(int kz, int N) { return kz == 0 || kz == N / 2 ? 1.f : 2.f; }
+
+// Noise amplitude of the cells the draw writes (main.c:405-459), else 0
+__device__ __forceinline__ float gauss_amp(const Grid& g, const float* __restrict__ amp, int x, int y, int kx, int ky,
+                                           int kz) {
+  const int N = g.N, n2 = kx * kx + ky * ky + kz * kz;
+  const bool on = x != N / 2 && y != N / 2 && kz < N / 2 && n2 != 0 && keep_cell(g, kx, ky, kz);
+  return on ? __ldg(amp + n2) : 0.f;
+}
+
 template <int N>
 __device__ __forceinline__ void tile_coords(unsigned tile, int& o, int& c0) {
   o = (int)(tile / TileCfg<N>::NCOL);
@@ -162,6 +172,11 @@ struct XinvOp {
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) v[i] = cscale(v[i], f[i]);
   }
+};
+
+template <int N>
+struct XinvNatOp : XinvOp<N> {  // phi in the caller's natural order
+  static constexpr bool kNatIn = true;
 };
 
 // 2LPT x passes.  The spectral factors of main.c:1180-1368 are products of
@@ -298,6 +313,8 @@ struct AccScale {
 // memory, where a forward x pass and a pointwise accumulation moved them
 // three more times.  Cut cells keep phi.
 //
+// GRAD: the last step of the transposed chain (chain.cuh) instead.
+//
 // What bounds it: instruction issue of the 8 (N >= 512) to 16 warps that
 // 32 values, their sums and compensations leave room for.  Against the forward
 // x pass and the specialised pointwise accumulation: 0.39 -> 0.23 ms (256^3, 12
@@ -313,6 +330,10 @@ struct XaccArgs {
   Slots slot, line;  // field and cube plane of an active r
   const float* qcube;
   AccScale sc;
+  // gradient form (k_xacc<N, true>): gw = amp (phi + w sum) in natural order,
+  // w = 1 on the kz = 0 and N/2 planes, else 2
+  const float* amp;
+  float2* gw;
 };
 template <int N>
 struct XaccCfg {
@@ -323,7 +344,7 @@ struct XaccCfg {
   static constexpr size_t SMEM = C::SMEM + (kStaged ? sizeof(float2) * N * C::W + 2 * sizeof(float) * QROWS : 0);
   static constexpr int MINB = C::R1 == 32 ? 256 / C::THREADS : C::R1 == 16 ? 512 / C::THREADS : 8;
 };
-template <int N>
+template <int N, bool GRAD>
 __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
     k_xacc(const __grid_constant__ XaccArgs<N> a, const float2* __restrict__ tw2) {
   using C = TileCfg<N>;
@@ -390,8 +411,13 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
     const int n = tile_n<N>(t, i);
     const int kx = i < C::R1 / 2 ? n : n - N;
     const int n2 = kx * kx + ky * ky + kz * kz;
-    const float g = a.sc.at(n2);
     const float2 d = add2(sum[i], cmp[i]);
+    if constexpr (GRAD) {
+      const float h = half_weight(kz, N), m = gauss_amp(a.g, a.amp, n, o, kx, ky, kz);
+      a.gw[NatMap<N>::base(o, c0, n, w)] = make_float2(m * fmaf(h, d.x, u[i].x), m * fmaf(h, d.y, u[i].y));
+      continue;
+    }
+    const float g = a.sc.at(n2);
     float2 r = make_float2(fmaf(g, d.x, u[i].x), fmaf(g, d.y, u[i].y));
     if (!keep_cell(a.g, kx, ky, kz)) r = u[i];
     if (n2 == 0) r = make_float2(0.f, 0.f);

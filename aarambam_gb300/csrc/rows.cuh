@@ -161,9 +161,10 @@ __device__ __forceinline__ void pair_spectrum(float2* v, const float2* __restric
 }
 
 // Half spectra of the pair from lane t's transformed values C_{t + T i}, into
-// X (row a) and X + HP (row b, when two).
-template <int N>
-__device__ __forceinline__ void pair_split(const float2* v, float2* __restrict__ X, int HP, int t, bool act, bool two) {
+// X (row a) and X + HP (row b, when two), with the z factor of the field (ZF).
+template <int N, bool ZF = false>
+__device__ __forceinline__ void pair_split(const float2* v, float2* __restrict__ X, int HP, int t, bool act, bool two,
+                                           ZFac zf = ZFac{0, 0.f, nullptr}) {
   using C = PairCfg<N>;
   const int lane = threadIdx.x & 31;
   const int src = (lane & ~(C::T - 1)) | ((C::T - t) & (C::T - 1));
@@ -173,14 +174,16 @@ __device__ __forceinline__ void pair_split(const float2* v, float2* __restrict__
     float2 p = make_float2(__shfl_sync(0xffffffffu, v[C::R1 - 1 - i].x, src),
                            __shfl_sync(0xffffffffu, v[C::R1 - 1 - i].y, src));
     if (t == 0) p = v[i == 0 ? 0 : C::R1 - i];
+    const float h = ZF ? 0.5f * axis_poly(zf.type, (float)(t + C::T * i), zf.kF) : 0.5f;  // types 0..2
     if (act) {
-      X[t + C::T * i] = make_float2(0.5f * (c.x + p.x), 0.5f * (c.y - p.y));
-      if (two) X[HP + t + C::T * i] = make_float2(0.5f * (c.y + p.y), 0.5f * (p.x - c.x));
+      X[t + C::T * i] = make_float2(h * (c.x + p.x), h * (c.y - p.y));
+      if (two) X[HP + t + C::T * i] = make_float2(h * (c.y + p.y), h * (p.x - c.x));
     }
   }
   if (act && t == 0) {
-    X[N / 2] = make_float2(v[C::HR].x, 0.f);
-    if (two) X[HP + N / 2] = make_float2(v[C::HR].y, 0.f);
+    const float h = ZF ? axis_poly(zf.type, (float)(N / 2), zf.kF) : 1.f;
+    X[N / 2] = make_float2(h * v[C::HR].x, 0.f);
+    if (two) X[HP + N / 2] = make_float2(h * v[C::HR].y, 0.f);
   }
 }
 
@@ -238,7 +241,9 @@ __device__ __forceinline__ void rows_pairs(const Op& op, float2* work, int64_t f
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) v[i] = act ? ln[t + C::T * i] : make_float2(0.f, 0.f);
     pair_fft<N, -1>(v, ln, t, tw2, act);
-    pair_split<N>(v, work + (act ? (int64_t)op.out_slot(l) * fs + row * HP : 0), HP, t, act, row + 1 < nrows);
+    float2* X = work + (act ? (int64_t)op.out_slot(l) * fs + row * HP : 0);
+    if constexpr (requires { Op::kZfacOut; }) pair_split<N, true>(v, X, HP, t, act, row + 1 < nrows, op.zfac(act ? l : 0));
+    else pair_split<N>(v, X, HP, t, act, row + 1 < nrows);
   }
 }
 

@@ -350,6 +350,23 @@ int aar_adj_source(aar_plan* plan, const float* d_hess, const float* d_gsource, 
    main.c:1045-1050 included); synchronises the stream. */
 int aar_adj_products(aar_plan* plan, const float* d_f, const float* d_gg, float* d_gf, double* d_galpha, void* stream);
 
+/* The whole differentiable chain, as aar_adj_spectral (GAUSS) of the noise w,
+   aar_set_spectrum, aar_stage_modal and aar_stage_lpt, in one call: d_disp,
+   float32 [3][N][N][N], the displacement psi1 - (3/7) psi2 / N^3 on the grid;
+   d_phig and d_phi, complex [N][N][N/2+1], the Gaussian and the total
+   potential. */
+int aar_adj_displacement(aar_plan* plan, const void* d_w, float* d_disp, void* d_phig, void* d_phi, void* stream);
+/* Its transpose at (d_phig, d_phi): from d_gdisp [3][N][N][N] the noise
+   gradient d_gw, complex [N][N][N/2+1], and d_galpha, FP64 [M][M][M], the
+   gradient with respect to alpha at every sorted index p <= q <= r.  Device
+   scratch from the caller (aar_adj_gradient_scratch_bytes with the plan's
+   present tables; 0 before tables are set); the plan's own spectrum and fields
+   are not touched.  The first call after a table change makes the plan's
+   gradient tables and synchronises the device. */
+size_t aar_adj_gradient_scratch_bytes(const aar_plan* plan);
+int aar_adj_gradient(aar_plan* plan, const void* d_phig, const void* d_phi, const float* d_gdisp, void* d_gw,
+                     double* d_galpha, void* d_scratch, size_t scratch_bytes, void* stream);
+
 /* ---- batches (no counterpart in the reference, whose executable makes one
    realisation per process) ----
    Several fused plans (realisations with their own seed, coefficient table,
