@@ -10,7 +10,8 @@
 // Noise (main.c:382-524): one thread per (i, j) column reseeds ranlxd1 with
 // seedtable[i][j] and draws (phase, amplitude) pairs for k < N/2, skipping the
 // Nyquist indices and DC after the draws, keeping the cube/sphere cut, and
-// writing the k = 0 plane with its Hermitian partner.  The fused plan's
+// writing the k = 0 plane with its Hermitian partner (k_noise32: the lanes of a
+// warp share its columns' cells).  The fused plan's
 // spectrum is written in its x-blocked row order; the plain form and the
 // caller's buffers in the natural one.
 #include <cuda_runtime.h>
@@ -18,6 +19,7 @@
 
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "aar_internal.cuh"
@@ -125,11 +127,15 @@ struct NoiseArgs {
   const float* amp;
 };
 
-// -ln(u) for u = U 2^-48 in (0, 1), FP32 with the small-(1-u) branch exact
+// -ln(u) for u = U 2^-48 in (0, 1), FP32: U = f + l with f its nearest float
+// and l the exact rest (|l| <= 2^-25 f), so ln u = ln(f 2^-48) + l / f to
+// 2^-50; for u next to 1, where ln f cancels or vanishes, l / f carries the
+// digits of 1 - u.
 __device__ __forceinline__ float neg_log_u48(uint64_t U) {
-  if (U < (uint64_t(1) << 47)) return -logf((float)U * 3.5527136788005009e-15f);  // u < 1/2
-  float oneminus = (float)((uint64_t(1) << 48) - U) * 3.5527137e-15f;
-  return -log1pf(-oneminus);
+  const float h = (float)(uint32_t)(U >> 24), g = (float)(uint32_t)(U & 0xFFFFFFu);
+  const float f = fmaf(h, 16777216.f, g);
+  const float l = g - fmaf(-h, 16777216.f, f);
+  return -(logf(f * 3.5527136788005009e-15f) + __fdividef(l, f));
 }
 
 // cos / sin of 2 pi u (+ pi when flipped) for u = U 2^-48, FP32: the exact
@@ -148,72 +154,98 @@ __device__ __forceinline__ void sincos_u48(uint64_t U, bool flip, float& c, floa
   }
 }
 
-// One cell (i, j, k) of a column from its two uniforms U1 (phase), U2
-// (amplitude): the Nyquist / DC skips after the draws, the cut, the
-// Hermitian pair of the k = 0 plane (main.c:396-459).  FP64: the amplitude
-// and phase by the reference's FP64 formula (main.c:443-459); OUT64: double2
-// output (the plain forms), else float2 (the fused form, FP64 math rounded at
-// the end when FP64).
-template <bool FP64, bool OUT64>
-__device__ __forceinline__ void noise_cell(const NoiseArgs& a, int i, int j, int k, uint64_t U1, uint64_t U2, double fx,
-                                           double fy, void* __restrict__ out, int HP) {
+// Where cell (i, j, k) of a column goes and with what: the k = 0 plane is
+// Hermitian, its cell (i, j) drawn for i = 0, j < N/2 and for 0 < i < N/2 and
+// conjugated into (-i, -j) (main.c:463-520).  c1 < 0: the cell belongs to its
+// partner's column.
+__device__ __forceinline__ void noise_place(const NoiseArgs& a, int i, int j, int k, int HP, int64_t& c1, int64_t& c2) {
   const int N = a.g.N;
-  if (i == N / 2 || j == N / 2) return;
-  if (i == 0 && j == 0 && k == 0) return;
-  const int kx = sidx(i, N), ky = sidx(j, N);
-  if (!keep_cell(a.g, kx, ky, k)) return;
-  const double box = a.g.box;
-  double re, im;
-  float rf = 0.f, imf = 0.f;
-  if (FP64) {
-    double fz = __ddiv_rn(__dmul_rn((double)(2 * k), kPi), box);
-    double k2 = __dadd_rn(__dadd_rn(__dmul_rn(fx, fx), __dmul_rn(fy, fy)), __dmul_rn(fz, fz));
-    double km = sqrt(k2);
-    double phase = __dmul_rn(__dmul_rn((double)U1 * 3.5527136788005009e-15, 2.0), kPi);
-    if (a.phase_flip) phase = __dadd_rn(phase, kPi);
-    double ampl = (double)U2 * 3.5527136788005009e-15;
-    double phig = noise_osc(a.prm, a.anorm * exp(a.ns * log(km)), km);
-    if (!a.fixed_amp) phig *= -log(ampl);
-    phig = sqrt(phig) * a.fac * a.beta / k2;
-    double sn, cs;
-    sincos(phase, &sn, &cs);
-    re = phig * cs;
-    im = phig * sn;
-    rf = (float)re;
-    imf = (float)im;
-  } else {
-    int n2 = kx * kx + ky * ky + k * k;
-    float amp = __ldg(a.amp + n2);
-    if (!a.fixed_amp) amp *= sqrtf(neg_log_u48(U2));
-    float c, sn;
-    sincos_u48(U1, a.phase_flip != 0, c, sn);
-    rf = amp * c;
-    imf = amp * sn;
-    re = rf;
-    im = imf;
-  }
-  int64_t c1 = -1, c2 = -1;
+  c1 = c2 = -1;
   if (k > 0) {
     c1 = row_of(i, j, N, a.xb) * HP + k;
   } else if (i == 0) {
     if (j >= N / 2) return;
     c1 = row_of(0, j, N, a.xb) * HP;
-    c2 = row_of(0, N - j, N, a.xb) * HP;
+    if (j > 0) c2 = row_of(0, N - j, N, a.xb) * HP;
   } else {
     if (i >= N / 2) return;
-    int ii = N - i, jj = (N - j) % N;
     c1 = row_of(i, j, N, a.xb) * HP;
-    c2 = row_of(ii, jj, N, a.xb) * HP;
+    c2 = row_of(N - i, (N - j) % N, N, a.xb) * HP;
   }
+}
+
+// One cell by the reference's FP64 formula (main.c:443-459) from its two
+// uniforms U1 (phase), U2 (amplitude), into a buffer that starts at zero: the
+// Nyquist / DC skips after the draws, the cut.  OUT64: double2 output (the
+// plain forms), else float2.
+template <bool OUT64>
+__device__ __forceinline__ void noise_cell64(const NoiseArgs& a, int i, int j, int k, uint64_t U1, uint64_t U2, double fx,
+                                             double fy, void* __restrict__ out, int HP) {
+  const int N = a.g.N;
+  if (i == N / 2 || j == N / 2) return;
+  if (i == 0 && j == 0 && k == 0) return;
+  const int kx = sidx(i, N), ky = sidx(j, N);
+  if (!keep_cell(a.g, kx, ky, k)) return;
+  const double fz = __ddiv_rn(__dmul_rn((double)(2 * k), kPi), a.g.box);
+  const double k2 = __dadd_rn(__dadd_rn(__dmul_rn(fx, fx), __dmul_rn(fy, fy)), __dmul_rn(fz, fz));
+  const double km = sqrt(k2);
+  double phase = __dmul_rn(__dmul_rn((double)U1 * 3.5527136788005009e-15, 2.0), kPi);
+  if (a.phase_flip) phase = __dadd_rn(phase, kPi);
+  const double ampl = (double)U2 * 3.5527136788005009e-15;
+  double phig = noise_osc(a.prm, a.anorm * exp(a.ns * log(km)), km);
+  if (!a.fixed_amp) phig *= -log(ampl);
+  phig = sqrt(phig) * a.fac * a.beta / k2;
+  double sn, cs;
+  sincos(phase, &sn, &cs);
+  const double re = phig * cs, im = phig * sn;
+  int64_t c1, c2;
+  noise_place(a, i, j, k, HP, c1, c2);
+  if (c1 < 0) return;
   if (OUT64) {
     double2* o = (double2*)out;
     o[c1] = make_double2(re, im);
     if (c2 >= 0) o[c2] = make_double2(re, -im);
   } else {
     float2* o = (float2*)out;
-    o[c1] = make_float2(rf, imf);
-    if (c2 >= 0) o[c2] = make_float2(rf, -imf);
+    o[c1] = make_float2((float)re, (float)im);
+    if (c2 >= 0) o[c2] = make_float2((float)re, -(float)im);
   }
+}
+
+// The drawn value of a cell of |k|^2 = n2 in FP32
+__device__ __forceinline__ float2 noise_draw32(const NoiseArgs& a, int n2, uint64_t U1, uint64_t U2) {
+  float amp = __ldg(a.amp + n2);
+  if (!a.fixed_amp) amp *= sqrtf(neg_log_u48(U2));
+  float c, sn;
+  sincos_u48(U1, a.phase_flip != 0, c, sn);
+  return make_float2(amp * c, amp * sn);
+}
+
+// One cell in FP32 from the per-|k|^2 amplitudes, zero where nothing is drawn:
+// every cell k < N/2 of the spectrum is written by exactly one column, so the
+// buffer needs no clearing.
+__device__ __forceinline__ void noise_cell32(const NoiseArgs& a, int i, int j, int k, uint64_t U1, uint64_t U2,
+                                             float2* __restrict__ o, int HP) {
+  const int N = a.g.N;
+  const int kx = sidx(i, N), ky = sidx(j, N), n2 = kx * kx + ky * ky + k * k;
+  float2 r = make_float2(0.f, 0.f);
+  if (i != N / 2 && j != N / 2 && n2 != 0 && keep_cell(a.g, kx, ky, k)) r = noise_draw32(a, n2, U1, U2);
+  int64_t c1, c2;
+  noise_place(a, i, j, k, HP, c1, c2);
+  if (c1 < 0) {
+    // (N/2, j, 0) and (0, N/2, 0) are their own or each other's partners: zero
+    if (i != N / 2 && !(i == 0 && j == N / 2)) return;
+    c1 = row_of(i, j, N, a.xb) * HP;
+  }
+  o[c1] = r;
+  if (c2 >= 0) o[c2] = make_float2(r.x, -r.y);
+}
+
+template <bool FP64, bool OUT64>
+__device__ __forceinline__ void noise_cell(const NoiseArgs& a, int i, int j, int k, uint64_t U1, uint64_t U2, double fx,
+                                           double fy, void* __restrict__ out, int HP) {
+  if constexpr (FP64) noise_cell64<OUT64>(a, i, j, k, U1, U2, fx, fy, out, HP);
+  else noise_cell32(a, i, j, k, U1, U2, (float2*)out, HP);
 }
 
 // The rest of a column from cell k on with the generator as it stands:
@@ -233,26 +265,24 @@ __device__ __noinline__ void noise_column_rest(NoiseArgs a, Rlx s, int i, int j,
   }
 }
 
-// One thread per (i, j) column.  A refill of ranlxd1 gives 12 uniforms, the
-// (U1, U2) pairs of six cells while no U2 is zero: the column runs in blocks
-// of six cells reading the refilled state at compile-time indices (it stays
-// in registers), and a block with a zero U2 hands the column from its first
-// draw to noise_column_rest.  Same draws, same cells as one draw at a time.
-template <bool FP64, bool OUT64 = FP64>
-__global__ void k_noise(NoiseArgs a, const uint32_t* __restrict__ seedtable, void* __restrict__ out, int HP) {
+// The FP64 amplitudes: one thread per (i, j) column.  A refill of ranlxd1 gives
+// 12 uniforms, the (U1, U2) pairs of six cells while no U2 is zero: the column
+// runs in blocks of six cells reading the refilled state at compile-time
+// indices (it stays in registers), and a block with a zero U2 hands the column
+// from its first draw to noise_column_rest.  Same draws, same cells as one
+// draw at a time.
+template <bool OUT64>
+__global__ void k_noise64(NoiseArgs a, const uint32_t* __restrict__ seedtable, void* __restrict__ out, int HP) {
   const int N = a.g.N;
   int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= (int64_t)N * N) return;
   const int i = (int)(col / N), j = (int)(col % N);
   Rlx s;
   rlx_seed(s, seedtable[col]);
-  double fx = 0, fy = 0;
-  if (FP64) {
-    fx = __ddiv_rn(__dmul_rn((double)(2 * sidx(i, N)), kPi), a.g.box);
-    fy = __ddiv_rn(__dmul_rn((double)(2 * sidx(j, N)), kPi), a.g.box);
-  }
+  const double fx = __ddiv_rn(__dmul_rn((double)(2 * sidx(i, N)), kPi), a.g.box);
+  const double fy = __ddiv_rn(__dmul_rn((double)(2 * sidx(j, N)), kPi), a.g.box);
   if (a.one_draw) {
-    noise_column_rest<FP64, OUT64>(a, s, i, j, 0, fx, fy, out, HP);
+    noise_column_rest<true, OUT64>(a, s, i, j, 0, fx, fy, out, HP);
     return;
   }
   for (int k = 0; k < N / 2; k += 6) {
@@ -262,12 +292,105 @@ __global__ void k_noise(NoiseArgs a, const uint32_t* __restrict__ seedtable, voi
 #pragma unroll
     for (int c = 0; c < 6; ++c) zero |= c < nk && s.x[2 * c + 1] == 0;
     if (zero) {
-      noise_column_rest<FP64, OUT64>(a, s, i, j, k, fx, fy, out, HP);
+      noise_column_rest<true, OUT64>(a, s, i, j, k, fx, fy, out, HP);
       return;
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c)
-      if (c < nk) noise_cell<FP64, OUT64>(a, i, j, k + c, s.x[2 * c], s.x[2 * c + 1], fx, fy, out, HP);
+      if (c < nk) noise_cell64<OUT64>(a, i, j, k + c, s.x[2 * c], s.x[2 * c + 1], fx, fy, out, HP);
+  }
+}
+
+// The FP32 amplitudes: a warp takes COLS consecutive columns, a lane each for
+// the generator.  Two refills give a column's next twelve cells; their uniforms
+// cross the warp through shared memory so that all 32 lanes form the cells, 12
+// consecutive lanes a column's (96-byte runs), and N/2 .. HP - 1 are cleared at
+// the end.  A column with a zero U2, which shifts the pairing of its later
+// draws (probability 2^-48 per draw), leaves the warp and is made from its
+// start by noise_column_rest.
+//
+// What bounds it: the generator's serial steps -- their latency while there
+// are few columns, their issue with many -- and the cells' logarithm, sine and
+// cosine.  A column per thread, each storing 8 bytes a row, on a cleared
+// buffer: 8.2 ms at 1024^3 with the clearing, this form 7.0; 1.15 -> 0.99 at
+// 512^3, 0.060 -> 0.049 at 128^3, 0.035 -> 0.023 at 64^3.
+constexpr int kNoiseWarps = 4;
+template <int COLS>
+__global__ void __launch_bounds__(32 * kNoiseWarps, 6) k_noise32(const __grid_constant__ NoiseArgs a,
+                                                             const uint32_t* __restrict__ seedtable,
+                                                             float2* __restrict__ out, int HP) {
+  constexpr int LD = 25;  // odd: the columns' 8-byte rows fall on different banks
+  __shared__ uint64_t raw_all[kNoiseWarps][COLS * LD];
+  __shared__ int64_t base_all[kNoiseWarps][COLS];  // a column's row in `out`
+  __shared__ int kk_all[kNoiseWarps][COLS];        // kx^2 + ky^2, negative: nothing drawn in the column
+  __shared__ int kxy_all[kNoiseWarps][COLS];       // kx, ky of the sphere's cut, 16 bits each
+  const int N = a.g.N, lane = threadIdx.x & 31;
+  uint64_t* raw = raw_all[threadIdx.x >> 5];
+  const int64_t col0 = ((int64_t)blockIdx.x * kNoiseWarps + (threadIdx.x >> 5)) * COLS, ncol = (int64_t)N * N;
+  if (col0 >= ncol) return;
+  const int here = (int)min((int64_t)COLS, ncol - col0);  // N not a multiple of 8: a short last warp
+  const bool own = lane < here;
+  const int oi = (int)((unsigned)(col0 + lane) / (unsigned)N), oj = (int)(col0 + lane) - oi * N;
+  int64_t* base = base_all[threadIdx.x >> 5];
+  int* kk = kk_all[threadIdx.x >> 5];
+  int* kxy = kxy_all[threadIdx.x >> 5];
+  if (own) {
+    const int kx = sidx(oi, N), ky = sidx(oj, N);
+    const bool in = oi != N / 2 && oj != N / 2 && (a.g.sphere || (abs(kx) <= a.g.kcut && abs(ky) <= a.g.kcut));
+    base[lane] = row_of(oi, oj, N, a.xb) * HP;
+    kk[lane] = in ? kx * kx + ky * ky : -1;
+    kxy[lane] = (kx & 0xffff) | (int)((unsigned)ky << 16);
+  }
+  Rlx s;
+  rlx_seed(s, own ? seedtable[col0 + lane] : 1u);
+  if (a.one_draw) {
+    if (own) noise_column_rest<false, false>(a, s, oi, oj, 0, 0, 0, out, HP);
+  } else {
+    unsigned dead = 0;  // columns that left the warp
+    for (int k = 0; k < N / 2; k += 12) {
+      const int nk = min(12, N / 2 - k);
+      bool zero = false;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        rlx_refill(s);
+        if (own) {
+#pragma unroll
+          for (int c = 0; c < 12; ++c) raw[lane * LD + 12 * h + c] = s.x[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) zero |= 6 * h + c < nk && s.x[2 * c + 1] == 0;
+      }
+      dead |= __ballot_sync(0xffffffffu, own && zero);  // also orders the stores before the loads
+      __syncwarp();
+#pragma unroll 2
+      for (int q = lane; q < here * 12; q += 32) {
+        const int cl = q / 12, c = q - 12 * cl;
+        if (c >= nk || (dead >> cl) & 1u) continue;
+        const uint64_t U1 = raw[cl * LD + 2 * c], U2 = raw[cl * LD + 2 * c + 1];
+        const int kz = k + c;
+        if (kz == 0) {
+          const unsigned col = (unsigned)(col0 + cl);
+          noise_cell32(a, (int)(col / N), (int)(col % N), 0, U1, U2, out, HP);
+          continue;
+        }
+        const int k2 = kk[cl], n2 = k2 + kz * kz;
+        bool on = k2 >= 0;
+        if (!a.g.sphere) on = on && kz <= a.g.kcut;
+        else if (on) on = keep_cell(a.g, (int)(short)kxy[cl], kxy[cl] >> 16, kz);
+        out[base[cl] + kz] = on ? noise_draw32(a, n2, U1, U2) : make_float2(0.f, 0.f);
+      }
+      __syncwarp();
+    }
+    if (own && (dead >> lane) & 1u) {
+      rlx_seed(s, seedtable[col0 + lane]);
+      noise_column_rest<false, false>(a, s, oi, oj, 0, 0, 0, out, HP);
+    }
+  }
+  __syncwarp();
+  const int tail = HP - N / 2;  // the kz = N/2 plane and the padding columns
+  for (int q = lane; q < here * tail; q += 32) {
+    const int cl = q / tail;
+    out[base[cl] + N / 2 + (q - cl * tail)] = make_float2(0.f, 0.f);
   }
 }
 
@@ -287,16 +410,32 @@ static NoiseArgs noise_args(Plan* p, int xb) {
   return a;
 }
 
+// The FP32 form's Gaussian spectrum, row order xb, into out (rows of hp)
+static int run_noise32(Plan* p, const uint32_t* d_seed, float2* out, int hp, int xb, cudaStream_t st) {
+  const int64_t cols = (int64_t)p->N * p->N;
+  if (p->prm.noise_fp64) {
+    AAR_CUDA_TRY(p, cudaMemsetAsync(out, 0, sizeof(float2) * (size_t)cols * hp, st));
+    k_noise64<false><<<(unsigned)((cols + 127) / 128), 128, 0, st>>>(noise_args(p, xb), d_seed, out, hp);
+    return AAR_OK;
+  }
+  // columns per warp: fewer lanes run the generator where there are few warps
+  // to hide its latency, at the price of its issue slots: 64^3 0.0226 ms with
+  // 8, 0.0275 with 16; 128^3 0.049 with 16, 0.058 with 32
+  auto go = [&](auto c) {
+    constexpr int COLS = decltype(c)::value, per = COLS * kNoiseWarps;
+    k_noise32<COLS><<<(unsigned)((cols + per - 1) / per), 32 * kNoiseWarps, 0, st>>>(noise_args(p, xb), d_seed, out, hp);
+  };
+  if (p->N <= 64) go(std::integral_constant<int, 8>{});
+  else if (p->N <= 128) go(std::integral_constant<int, 16>{});
+  else go(std::integral_constant<int, 32>{});
+  return AAR_OK;
+}
+
 int launch_noise_fp32(Plan* p, const uint32_t* d_seed, float2* d_phik, cudaStream_t st) {
-  size_t bytes = sizeof(float2) * (size_t)p->N * p->N * p->HP;
-  AAR_CUDA_TRY(p, cudaMemsetAsync(d_phik, 0, bytes, st));
-  int64_t cols = (int64_t)p->N * p->N;
-  int bs = 128;
-  { ProfScope ps_(p, "noise", st);
-  if (p->prm.noise_fp64)
-    k_noise<true, false><<<(unsigned)((cols + bs - 1) / bs), bs, 0, st>>>(noise_args(p, kXB), d_seed, d_phik, p->HP);
-  else
-    k_noise<false><<<(unsigned)((cols + bs - 1) / bs), bs, 0, st>>>(noise_args(p, kXB), d_seed, d_phik, p->HP);
+  {
+    ProfScope ps_(p, "noise", st);
+    int rc = run_noise32(p, d_seed, d_phik, p->HP, kXB, st);
+    if (rc) return rc;
   }
   AAR_CUDA_TRY(p, cudaGetLastError());
   p->last_launches += 1;
@@ -309,7 +448,7 @@ int launch_noise_fp64(Plan* p, const uint32_t* d_seed, double2* d_phik, int hp, 
   int64_t cols = (int64_t)p->N * p->N;
   int bs = 128;
   { ProfScope ps_(p, "noise", st);
-  k_noise<true><<<(unsigned)((cols + bs - 1) / bs), bs, 0, st>>>(noise_args(p, 1), d_seed, d_phik, hp);
+  k_noise64<true><<<(unsigned)((cols + bs - 1) / bs), bs, 0, st>>>(noise_args(p, 1), d_seed, d_phik, hp);
   }
   AAR_CUDA_TRY(p, cudaGetLastError());
   p->last_launches += 1;
@@ -364,15 +503,12 @@ int noalloc_gaussian(Plan* p, void* d_out, cudaStream_t st) {
   run_seedtable(p, seed, st);
   AAR_CUDA_TRY(p, cudaGetLastError());
   const int hp = N / 2 + 1;
-  const bool fp64 = is_plain(p->prm);
-  AAR_CUDA_TRY(p, cudaMemsetAsync(d_out, 0, (fp64 ? sizeof(double2) : sizeof(float2)) * (size_t)total * hp, st));
-  const unsigned nb = (unsigned)((total + 127) / 128);
-  if (fp64)
-    k_noise<true><<<nb, 128, 0, st>>>(noise_args(p, 1), seed, d_out, hp);
-  else if (p->prm.noise_fp64)
-    k_noise<true, false><<<nb, 128, 0, st>>>(noise_args(p, 1), seed, d_out, hp);
-  else
-    k_noise<false><<<nb, 128, 0, st>>>(noise_args(p, 1), seed, d_out, hp);
+  if (is_plain(p->prm)) {
+    AAR_CUDA_TRY(p, cudaMemsetAsync(d_out, 0, sizeof(double2) * (size_t)total * hp, st));
+    k_noise64<true><<<(unsigned)((total + 127) / 128), 128, 0, st>>>(noise_args(p, 1), seed, d_out, hp);
+  } else if ((rc = run_noise32(p, seed, (float2*)d_out, hp, 1, st))) {
+    return rc;
+  }
   AAR_CUDA_TRY(p, cudaGetLastError());
   p->last_launches = 2;
   return AAR_OK;

@@ -41,20 +41,30 @@ struct Rlx {
   int pos;
 };
 
+// the low 12 bits of v reversed
+AAR_HD uint32_t rev12(uint32_t v) {
+#ifdef __CUDA_ARCH__
+  return __brev(v) >> 20;
+#else
+  uint32_t r = 0;
+  for (int i = 0; i < 12; ++i) r |= ((v >> i) & 1u) << (11 - i);
+  return r;
+#endif
+}
+
+// Twelve bits of the recurrence at a time (the window holds bits n .. n + 30,
+// so bits n + 31 .. n + 42 follow from it at once), four times per word; bit
+// by bit the 576 steps were a fifth of the noise kernel at 128^3.
 AAR_HD void rlx_seed(Rlx& s, uint32_t seed) {
   if (seed == 0) seed = 1;
-  uint32_t bits = seed & 0x7FFFFFFFu;  // 31-bit register, bit k = seed bit k
-  int ib = 0, jb = 18;
-  for (int w = 0; w < 12; ++w) {
+  uint32_t w = seed & 0x7FFFFFFFu;  // bit k = seed bit k
+  for (int i = 0; i < 12; ++i) {
     uint64_t word = 0;
-    for (int l = 0; l < 48; ++l) {
-      uint32_t bi = (bits >> ib) & 1u, bj = (bits >> jb) & 1u;
-      word = (word << 1) | (bi ^ 1u);
-      bits ^= (bj << ib);
-      ib = (ib == 30) ? 0 : ib + 1;
-      jb = (jb == 30) ? 0 : jb + 1;
+    for (int l = 0; l < 4; ++l) {
+      word = (word << 12) | rev12((w & 0xFFFu) ^ 0xFFFu);
+      w = (w >> 12) | (((w ^ (w >> 18)) & 0xFFFu) << 19);
     }
-    s.x[w] = word;
+    s.x[i] = word;
   }
   s.carry = 0;
   s.pos = 12;
