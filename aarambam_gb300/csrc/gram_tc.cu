@@ -197,50 +197,93 @@ __global__ void __launch_bounds__(256) k_tetra_modes(Tetra a, long long ldq, dou
     qrow[t] = t < a.npts ? q_rows(r1, r2, r3, a.i1[t], a.i2[t], a.i3[t]) : 0.0;
 }
 
+// The bits of |x| as an integer, which orders non-negative doubles; 0 for NaN
+// (fmax drops it).
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  return b > 0x7ff0000000000000ull ? 0ull : b;
+}
+__device__ __forceinline__ unsigned long long max64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+
 // Row maxima of |w Q| (rowmax[n]) and |Q| (rowmax[nm + n]) over t < npts, as
-// the bit patterns of non-negative doubles.
+// the bit patterns of non-negative doubles.  The maxima are taken on the
+// integers: with two FP64 maxima per point beside the product, GB300's FP64
+// rate (two operations per clock and SM) bound the kernel (with the digit
+// pass, whose conversions were FP64 and 64-bit, 15.3 ms at 1540 modes x 289,750
+// points; now 5.9 ms together).
 __global__ void __launch_bounds__(256) k_modes_rowmax(const double* __restrict__ Q, long long ldq,
                                                       const double* __restrict__ w, int npts, int nm,
                                                       unsigned long long* __restrict__ rowmax) {
   const int n = blockIdx.y;
   const double* qrow = Q + (size_t)n * ldq;
-  double mA = 0.0, mB = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npts; t += gridDim.x * blockDim.x) {
-    const double q = qrow[t];
-    mB = fmax(mB, fabs(q));
-    mA = fmax(mA, fabs(q * w[t]));
+  unsigned long long mA = 0, mB = 0;
+  const int step = gridDim.x * blockDim.x;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; t + 3 * step < npts; t += 4 * step) {  // four loads of each in flight
+    double q[4], v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = qrow[t + j * step], v[j] = w[t + j * step];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      mB = max64(mB, abs_bits(q[j]));
+      mA = max64(mA, abs_bits(q[j] * v[j]));
+    }
+  }
+  for (; t < npts; t += step) {
+    mB = max64(mB, abs_bits(qrow[t]));
+    mA = max64(mA, abs_bits(qrow[t] * w[t]));
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
-    mA = fmax(mA, __shfl_xor_sync(0xffffffffu, mA, o));
-    mB = fmax(mB, __shfl_xor_sync(0xffffffffu, mB, o));
+    mA = max64(mA, __shfl_xor_sync(0xffffffffu, mA, o));
+    mB = max64(mB, __shfl_xor_sync(0xffffffffu, mB, o));
   }
-  __shared__ double sA[8], sB[8];
   if ((threadIdx.x & 31) == 0) {
-    sA[threadIdx.x >> 5] = mA;
-    sB[threadIdx.x >> 5] = mB;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) {
-      mA = fmax(mA, sA[i]);
-      mB = fmax(mB, sB[i]);
-    }
-    atomicMax(rowmax + n, (unsigned long long)__double_as_longlong(mA));
-    atomicMax(rowmax + nm + n, (unsigned long long)__double_as_longlong(mB));
+    atomicMax(rowmax + n, mA);
+    atomicMax(rowmax + nm + n, mB);
   }
 }
 
-// The eight digits of x (|x| <= 2^e) as floats d_s 2^(-8 s), s = 0 most significant.
-__device__ __forceinline__ void to_digits(double x, int e, float (&d)[kDig]) {
-  long long v = __double2ll_rn(scalbn(x, 62 - e));
-#pragma unroll
-  for (int s = kDig - 1; s >= 1; --s) {
-    const long long lo = ((v + 128) & 255) - 128;
-    d[s] = scalbnf((float)lo, -8 * s);
-    v = (v - lo) >> 8;
+// rint(x 2^(62 - e)) for |x| <= 2^e, to nearest even, on the integers (as
+// __double2ll_rn(scalbn(x, 62 - e)), whose FP64 steps run at a small fraction
+// of the integer rate).
+__host__ __device__ __forceinline__ long long scaled_int(unsigned long long bits, int e) {
+  const int ex = (int)(bits >> 52) & 0x7ff;
+  const unsigned long long m = (bits & 0xfffffffffffffull) | (ex ? 0x10000000000000ull : 0ull);
+  const int sh = (ex ? ex : 1) - 1075 + 62 - e;  // value = m 2^sh
+  unsigned long long v;
+  if (sh >= 0) {
+    v = m << sh;
+  } else if (sh < -54) {
+    v = 0;  // below a quarter
+  } else {
+    const int s = -sh;
+    const unsigned long long rest = m & ((1ull << s) - 1), half = 1ull << (s - 1);
+    v = m >> s;
+    v += rest > half || (rest == half && (v & 1));
   }
-  d[0] = (float)v;
+  return bits >> 63 ? -(long long)v : (long long)v;
+}
+
+// The eight digits of x (|x| <= 2^e) as floats d_s 2^(-8 s), s = 0 most
+// significant.  v + 128 (1 + 2^8 + ... + 2^48) has the balanced digits' carries
+// in it: its low seven bytes are d_7 .. d_1 plus 128, the eighth is d_0.  A byte
+// b becomes (b - 128) 2^(-8 s) as the float 2^23 + b (its bits put together)
+// in one exact multiply-add.
+__device__ __forceinline__ void to_digits(double x, int e, float (&d)[kDig]) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+  long long v;
+  if (((bits >> 52) & 0x7ff) != 0x7ff) v = scaled_int(bits, e);
+  else v = __double2ll_rn(scalbn(x, 62 - e));  // infinities and NaN as the conversion has them
+  const unsigned long long u = (unsigned long long)v + 0x0080808080808080ull;
+  const uint32_t lo = (uint32_t)u, hi = (uint32_t)(u >> 32) ^ 0x80000000u;
+#pragma unroll
+  for (int s = 0; s < kDig; ++s) {
+    const int k = kDig - 1 - s;  // byte of u
+    const float f = __uint_as_float(__byte_perm(k < 4 ? lo : hi, 0x4B000000u, 0x7540u | (k & 3)));
+    const float p = 1.f / (float)(1ull << (8 * s));
+    d[s] = fmaf(f, p, -8388736.f * p);  // 2^23 + 128
+  }
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
