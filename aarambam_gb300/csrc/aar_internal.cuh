@@ -72,6 +72,8 @@ struct Plan {
   float* d_qcube = nullptr;
   int qcube_m = 0;
   bool qcube_stale = true;
+  float* d_tcube = nullptr;  // T/(D Beta) likewise (tcube_build), after each transfer change
+  bool tcube_stale = true;
   // gradient (chain.cuh): the cube of all modes where the one above is not,
   // and the products' tables, made on the first gradient after a table change
   float* d_qfull = nullptr;
@@ -164,6 +166,7 @@ int launch_noise_fp64(Plan* p, const uint32_t* d_seed, double2* d_phik, int hp, 
 int fused_prepare(Plan* p);
 int fused_tile_r1(int N);  // first radix of the tile passes at this grid size
 int qcube_build(Plan* p);
+int tcube_build(Plan* p);
 struct Term;
 std::vector<std::vector<Term>> regrouped_terms(const std::vector<double>& alpha, int M);
 std::vector<int> modal_partition(const std::vector<std::vector<Term>>& by_r, int nparts);

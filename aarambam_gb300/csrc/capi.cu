@@ -212,6 +212,10 @@ static int set_transfer(Plan* p, const double* k, const double* t, int n) {
     }
     AAR_CUDA_TRY(p, cudaMemcpy(p->d_amp, amp.data(), sizeof(float) * nsq, cudaMemcpyHostToDevice));
     AAR_CUDA_TRY(p, cudaMemcpy(p->d_twb, twb.data(), sizeof(float) * nsq, cudaMemcpyHostToDevice));
+    // a cube that exists follows at once (a captured run reads it); the first
+    // is made with the fields
+    p->tcube_stale = true;
+    if (p->d_tcube) return tcube_build(p);
   }
   return AAR_OK;
 }
@@ -238,7 +242,7 @@ static void plan_release(Plan* p) {
   p->prof.clear();
   for (auto e : p->event_pool) cudaEventDestroy(e);
   p->event_pool.clear();
-  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_qfull, p->d_chain};
+  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_tcube, p->d_qfull, p->d_chain};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   p->d_phik = p->d_work = nullptr;
@@ -248,7 +252,8 @@ static void plan_release(Plan* p) {
   p->d_rlxpow = nullptr;
   p->d_qtab = p->d_rtab = nullptr;
   p->d_sinc = p->d_isinc2 = nullptr;
-  p->d_qcube = p->d_qfull = nullptr;
+  p->d_qcube = p->d_tcube = p->d_qfull = nullptr;
+  p->tcube_stale = true;
   p->qcube_m = p->qfull_m = 0;
   p->qcube_stale = p->qfull_stale = p->chain_stale = true;
   p->d_chain = nullptr;
@@ -292,8 +297,8 @@ static void plan_release(Plan* p) {
 
 static bool pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
-// Work fields: the path needs max(M, 8) (2LPT: six Hessians, the source and
-// T/(D Beta) phi); the standalone transforms (M = 0) need one.
+// Work fields: the path needs max(M, 9) (2LPT: six displacement fields, the
+// source and two x outputs); the standalone transforms (M = 0) need one.
 static int alloc_fused(Plan* p, int M) {
   int N = p->N;
   size_t fbytes = sizeof(float2) * (size_t)N * N * p->HP;
@@ -491,7 +496,8 @@ static int ensure_fields(Plan* p) {
   }
   int rc = alloc_fused(p, p->M);
   if (rc) return rc;
-  return qcube_build(p);
+  if ((rc = qcube_build(p))) return rc;
+  return tcube_build(p);
 }
 
 static int ready(Plan* p) {

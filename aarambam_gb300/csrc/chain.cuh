@@ -83,19 +83,6 @@ __global__ void __launch_bounds__(256) k_chain_div(LptArgs a, const float2* __re
   }
 }
 
-// T/(D Beta) phi of a natural-order phi into a plan field
-template <int N>
-__global__ void __launch_bounds__(256) k_chain_twb(int HP, const float* __restrict__ twb,
-                                                   const float2* __restrict__ phi, float2* __restrict__ out) {
-  constexpr int64_t total = (int64_t)N * N * (N / 2 + 1);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int x, y, kz;
-    const int64_t e = spec_cell<N>(i, HP, x, y, kz);
-    const int kx = sidx(x, N), ky = sidx(y, N);
-    out[e] = cscale(phi[nat_cell<N>(x, y, kz)], __ldg(twb + kx * kx + ky * ky + kz * kz));
-  }
-}
-
 // Transpose of the 2LPT source rows: lines 0..5 the Hessians d00 d01 d02 d11
 // d12 d22 (z factors as SourceRowOp), line 6 the source gradient g; the six
 // gradients over the Hessians' lines and fields, their z factors again on the

@@ -38,26 +38,6 @@
 namespace aar {
 
 
-// phi_T = T(k)/(D Beta) phi on every half-spectrum cell (padding columns
-// are not touched): the factor the Hessians and psi1 share.
-template <int N>
-__global__ void __launch_bounds__(256) k_scale_twb(const float2* __restrict__ phi, float2* out, int HP,
-                                                   const float* __restrict__ twb) {
-  constexpr int K = N / 2 + 1;
-  constexpr int64_t total = (int64_t)N * N * K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / K;
-    const int kz = (int)(i - row * K);
-    const int64_t e = row * HP + kz;
-    int x, y;
-    row_xy(row, N, kXB, x, y);
-    const int kx = sidx(x, N), ky = sidx(y, N);
-    const float t = __ldg(twb + kx * kx + ky * ky + kz * kz);
-    const float2 v = phi[e];
-    out[e] = make_float2(v.x * t, v.y * t);
-  }
-}
-
 // ----------------------------------------------------------- row passes
 // (rows.cuh: rows_pairs, rows_fold)
 template <int N>
@@ -737,25 +717,18 @@ struct Launch {
     p->last_launches += 1;
     return AAR_OK;
   }
-  // 2LPT (main.c:1180-1431).  Work slots: 7 = T/(D Beta) phi; Hessians
-  // d_ab in 0..5 (00 01 02 11 12 22) via x outputs P = -kF^2 kx^2 phi_T -> 0,
-  // Q = -kF^2 kx phi_T -> 8, R = -kF^2 phi_T -> 6 and the y fan-out (xy, yz:
-  // ky; yy: ky^2); the source rows apply the z factors (xz, yz: kz; zz:
-  // kz^2) and write S to 6; psi1 (0..2) and psi2 (3..5) likewise from x
-  // outputs in 0, 8 (psi1) and 3, 7 (psi2).
+  // 2LPT (main.c:1180-1431).  Work slots: Hessians d_ab in 0..5 (00 01 02 11
+  // 12 22) via x outputs P = -kF^2 kx^2 phi_T -> 0, Q = -kF^2 kx phi_T -> 8, R =
+  // -kF^2 phi_T -> 6 (phi_T = T/(D Beta) phi) and the y fan-out (xy, yz: ky;
+  // yy: ky^2); the source rows apply the z factors (xz, yz: kz; zz: kz^2) and
+  // write S to 6; psi1 (0..2) and psi2 (3..5) likewise from x outputs in 0, 8
+  // (psi1) and 3, 7 (psi2).
   static int lpt(Plan* p, const LptArgs& a, cudaStream_t st, bool rows = true) {
     const int64_t fs = fstride(p);
     const float kF = a.m.g.kF;
-    float2* phit = p->d_work + 7 * fs;  // T/(D Beta) phi, read by the Hessian and psi1 passes
-    {
-      ProfScope ps_(p, "lpt_scale_twb", st);
-      k_scale_twb<N><<<(unsigned)(p->num_sms * 8), 256, 0, st>>>(p->d_phik, phit, p->HP, p->d_twb);
-    }
-    AAR_CUDA_TRY(p, cudaGetLastError());
-    p->last_launches += 1;
     int rc;
     {
-      LptXOp<N, 0> ho{phit, p->d_work, fs, {0, 8, 6}, group(p), kF, a.isinc2};
+      LptXOp<N, 0> ho{p->d_phik, nullptr, p->d_work, fs, {0, 8, 6, 0}, group(p), kF, a.isinc2, p->d_tcube, p->d_twb};
       if ((rc = run_pass<N, 0, +1>(p, ho, kTiles * 3, st, "lpt_xinv_hess"))) return rc;
       YFanOp<N> yf{p->d_work, fs, {0, 8, 8, 6, 6, 6}, {0, 1, 2, 3, 4, 5}, {0, 1, 0, 2, 1, 0}, 1, kF, a.isinc2};
       if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "lpt_ypass_inv_hess"))) return rc;
@@ -776,10 +749,8 @@ struct Launch {
       if ((rc = run_pass<N, 0, -1>(p, xs, kTiles, st, "lpt_xfwd_source"))) return rc;
     }
     {
-      LptXOp<N, 1> m1{phit, p->d_work, fs, {0, 8, 0}, group(p), kF, a.isinc2};
-      if ((rc = run_pass<N, 0, +1>(p, m1, kTiles * 2, st, "lpt_xpsi1"))) return rc;
-      LptXOp<N, 1> m2{p->d_work + 6 * fs, p->d_work, fs, {3, 7, 0}, group(p), kF, a.isinc2};
-      if ((rc = run_pass<N, 0, +1>(p, m2, kTiles * 2, st, "lpt_xpsi2"))) return rc;
+      LptXOp<N, 1> mo{p->d_phik, p->d_work + 6 * fs, p->d_work, fs, {0, 8, 3, 7}, group(p), kF, a.isinc2, p->d_tcube, p->d_twb};
+      if ((rc = run_pass<N, 0, +1>(p, mo, kTiles * 4, st, "lpt_xpsi"))) return rc;
       YFanOp<N> yf{p->d_work, fs, {0, 8, 8, 3, 7, 7}, {0, 1, 2, 3, 4, 5}, {3, 4, 3, 3, 4, 3}, 1, kF, a.isinc2};
       if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "lpt_ypass_inv_disp"))) return rc;
     }
@@ -965,14 +936,54 @@ static int make_cube(Plan* p, int n, const Slots& mode, float*& cube, int& have)
   return AAR_OK;
 }
 
+// The transfer cube of the 2LPT x passes: T/(D Beta) in the filter cube's
+// layout, no cut, zero on the padding columns.  It takes an eighth of a field
+// that a caller's memory limit does not know of, so plans with a limit, and
+// those whose device has no room, read the per-|n|^2 table in its place.
+__global__ void __launch_bounds__(256) k_tcube(Grid g, const float* __restrict__ twb, float* __restrict__ q) {
+  const int K = g.N / 2 + 1, ncol = g.HP / 8;
+  const int64_t per = (int64_t)K * g.HP * K;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / 8;
+    const int ax = (int)(r % K);
+    const int64_t s = r / K;
+    const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
+    q[i] = kz <= g.N / 2 ? __ldg(twb + ax * ax + ay * ay + kz * kz) : 0.f;
+  }
+}
+
+int tcube_build(Plan* p) {
+  if (!p->tcube_stale || !p->have_transfer) return AAR_OK;
+  const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
+  p->tcube_stale = false;
+  if (p->prm.mem_limit_bytes > 0) return AAR_OK;
+  if (!p->d_tcube && plan_alloc(p, (void**)&p->d_tcube, sizeof(float) * (size_t)per)) return AAR_OK;
+  k_tcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, p->d_twb, p->d_tcube);
+  AAR_CUDA_TRY(p, cudaGetLastError());
+  AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // as make_cube
+  return AAR_OK;
+}
+
+// Planes of the filter cube: the lines that the products read first, then the
+// modes that only their gradients read.
+static Slots cube_planes(const Plan* p, const TermList& tl) {
+  Slots plane{};
+  for (int m = 0, n = tl.nlines; m < p->M; ++m) plane.s[m] = tl.line[m] >= 0 ? tl.line[m] : n++;
+  return plane;
+}
+
+// The lines' planes; all M in a plan with a memory limit, which leaves the
+// gradient no second cube to allocate (chain_cube).
 int qcube_build(Plan* p) {
   if (p->host_terms.empty()) return AAR_OK;  // no tables yet: nothing reads filters
   const TermList& tl = *(const TermList*)p->host_terms.data();
-  if ((!p->qcube_stale && p->d_qcube) || tl.nlines == 0) return AAR_OK;
+  const int n = p->prm.mem_limit_bytes > 0 ? p->M : tl.nlines;
+  if ((!p->qcube_stale && p->d_qcube) || n == 0) return AAR_OK;
+  const Slots plane = cube_planes(p, tl);
   Slots mode{};
   for (int m = 0; m < p->M; ++m)
-    if (tl.line[m] >= 0) mode.s[tl.line[m]] = m;
-  int rc = make_cube(p, tl.nlines, mode, p->d_qcube, p->qcube_m);
+    if (plane.s[m] < n) mode.s[plane.s[m]] = m;
+  int rc = make_cube(p, n, mode, p->d_qcube, p->qcube_m);
   if (rc) return rc;
   p->qcube_stale = false;
   return AAR_OK;
@@ -1311,16 +1322,15 @@ static int chain_tables(Plan* p, ChainTables& ct, cudaStream_t st) {
 }
 
 // The filter cube of all M modes (the products' gradients need the ones that
-// the products do not read, too): the plan's own where its lines are all
-// modes, else a second one made on the first gradient after a table change.
+// the products do not read, too): the plan's own where it holds them all, else
+// a second one made on the first gradient after a table change.
 static int chain_cube(Plan* p, const float*& cube, Slots& plane) {
-  const TermList& tl = *(const TermList*)p->host_terms.data();
-  for (int m = 0; m < p->M; ++m) plane.s[m] = tl.nlines == p->M ? tl.line[m] : m;
+  plane = cube_planes(p, *(const TermList*)p->host_terms.data());
   cube = p->d_qcube;
-  if (tl.nlines == p->M) return AAR_OK;
+  if (p->qcube_m == p->M && !p->qcube_stale) return AAR_OK;
   if (p->qfull_stale || !p->d_qfull) {
     Slots mode{};
-    for (int m = 0; m < p->M; ++m) mode.s[m] = m;
+    for (int m = 0; m < p->M; ++m) mode.s[plane.s[m]] = m;
     int rc = make_cube(p, p->M, mode, p->d_qfull, p->qfull_m);
     if (rc) return rc;
     p->qfull_stale = false;
@@ -1384,9 +1394,7 @@ struct Chain {
     if ((rc = L::template axis_pass<0, +1>(p, T, 1, run(0, 1), st, "grad_x"))) return rc;
     if ((rc = L::template axis_pass<1, +1>(p, T, 1, run(0, 1), st, "grad_y"))) return rc;
     // the source, its Hessians made again from phi
-    k_chain_twb<N><<<cells(p), 256, 0, st>>>(p->HP, p->d_twb, phi, W + 7 * fs);
-    if ((rc = done(p))) return rc;
-    const LptXOp<N, 0> ho{W + 7 * fs, W, fs, {0, 8, 6}, 1, kF, a.isinc2};
+    const LptXNatOp<N> ho{{phi, nullptr, W, fs, {0, 8, 6, 0}, 1, kF, a.isinc2, p->d_tcube, p->d_twb}};
     if ((rc = run_pass<N, 0, +1>(p, ho, kTiles * 3, st, "grad_xhess"))) return rc;
     const YFanOp<N> yf{W, fs, {0, 8, 8, 6, 6, 6}, {0, 1, 2, 3, 4, 5}, {0, 1, 0, 2, 1, 0}, 1, kF, a.isinc2};
     if ((rc = run_pass<N, 1, +1>(p, yf, kTiles * 6, st, "grad_yhess"))) return rc;

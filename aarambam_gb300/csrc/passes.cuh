@@ -180,51 +180,76 @@ struct XinvNatOp : XinvOp<N> {  // phi in the caller's natural order
 };
 
 // 2LPT x passes.  The spectral factors of main.c:1180-1368 are products of
-// one factor per axis, except 1/k^2 of psi2, which the forward x pass of the
-// source applies (XfwdInvK2Op); so an x pass writes one field per distinct
-// x factor and a fan-out y pass (YFanOp) and the c2r rows (ZFac) apply the
-// rest.  KIND 0, Hessians d_ab = -k_a k_b T/(D Beta) phi: x factors -kF^2 kx^2,
-// -kF^2 kx, -kF^2 (3 outputs).  KIND 1, displacements i k_a smth on
-// T/(D Beta) phi (psi1) or on -S/k^2 (psi2), smth = [sinc_x sinc_y sinc_z]^-2:
-// x factors i kF kx / sinc_x^2 and i / sinc_x^2 (2 outputs).  Items in
-// group_order over the outputs.
+// one factor per axis, except T/(D Beta), which the transfer cube brings (laid
+// out as the filter cube, so phi needs no scaled copy), and 1/k^2 of psi2,
+// which the forward x pass of the source applies (XfwdInvK2Op); so an x pass
+// writes one field per distinct x factor and a fan-out y pass (YFanOp) and
+// the c2r rows (ZFac) apply the rest.  KIND 0, Hessians d_ab = -k_a k_b T/(D
+// Beta) phi: x factors -kF^2 kx^2, -kF^2 kx, -kF^2 (3 outputs).  KIND 1,
+// displacements i k_a smth on T/(D Beta) phi (psi1, outputs 0 and 1) and on
+// -S/k^2 (psi2, 2 and 3), smth = [sinc_x sinc_y sinc_z]^-2: x factors
+// i kF kx / sinc_x^2 and i / sinc_x^2.  Items in group_order over the outputs.
+// Bound by the fields' bytes.  A scaled copy of phi and two passes for the
+// displacements took 13.7 ms at 1024^3 and 1.72 at 512^3; these two passes take
+// 11.4 and 1.30, and 16.3 and 1.83 where the factor is read by |n|^2 (a
+// gather: neighbouring kz lie 2 kz + 1 entries apart).
 template <int N, int KIND>
 struct LptXOp {
   static constexpr bool kPre = true, kPost = false;
-  static constexpr int NC = KIND == 0 ? 3 : 2;
-  const float2* in;
+  static constexpr int NC = KIND == 0 ? 3 : 4;
+  const float2* phi;
+  const float2* s;  // psi2's input
   float2* work;
   int64_t fs;
-  int out[3];
+  int out[4];
   unsigned grp;
   float kF;
   const float* isinc2;
+  const float* tcube;  // [|ky|][kz / 8][|kx|][8], zero on the padding columns; null: twb by |n|^2
+  const float* twb;
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     unsigned t;
     group_order<N>(item, NC, grp, t, c);
     tile_coords<N>(t, o, c0);
   }
-  __device__ const float2* src(int) const { return in; }
+  __device__ const float2* src(int c) const { return KIND == 1 && c >= 2 ? s : phi; }
   __device__ float2* dst(int c) const { return work + (int64_t)out[c] * fs; }
-  __device__ void pre(float2* v, int, int kz, int c, int t) const {
+  __device__ void pre(float2* v, int o, int kz, int c, int t) const {
     using C = TileCfg<N>;
+    constexpr int K = N / 2 + 1;
+    const int ay = o <= N / 2 ? o : N - o;
+    const float* q = tcube + (((int64_t)ay * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
+    const bool psi2 = KIND == 1 && c >= 2;
     float f[C::R1];
+    if (psi2 || kz > N / 2) {
+#pragma unroll
+      for (int i = 0; i < C::R1; ++i) f[i] = kz <= N / 2 ? 1.f : 0.f;
+    } else {
+      const int b = ay * ay + kz * kz;
+#pragma unroll
+      for (int i = 0; i < C::R1; ++i) {
+        const int n = tile_n<N>(t, i), ax = i < C::R1 / 2 ? n : N - n;
+        f[i] = tcube ? __ldg(q + ax * C::W) : __ldg(twb + b + ax * ax);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) {
       const int n = tile_n<N>(t, i);
       const float kx = (float)(i < C::R1 / 2 ? n : n - N);
       if (KIND == 0) {
-        f[i] = c == 0 ? -kF * kF * kx * kx : c == 1 ? -kF * kF * kx : -kF * kF;
+        f[i] *= c == 0 ? -kF * kF * kx * kx : c == 1 ? -kF * kF * kx : -kF * kF;
+        v[i] = make_float2(v[i].x * f[i], v[i].y * f[i]);
       } else {
         const float is2 = __ldg(isinc2 + n);
-        f[i] = c == 0 ? kF * kx * is2 : is2;
+        f[i] *= (c & 1) == 0 ? kF * kx * is2 : is2;
+        v[i] = make_float2(-f[i] * v[i].y, f[i] * v[i].x);
       }
-      if (kz > N / 2) f[i] = 0.f;
     }
-#pragma unroll
-    for (int i = 0; i < C::R1; ++i)
-      v[i] = KIND == 0 ? make_float2(v[i].x * f[i], v[i].y * f[i]) : make_float2(-f[i] * v[i].y, f[i] * v[i].x);
   }
+};
+template <int N>
+struct LptXNatOp : LptXOp<N, 0> {  // phi in the caller's natural order
+  static constexpr bool kNatIn = true;
 };
 
 // Inverse y pass fanning fields out: item (tile, c), c < NC: field in[c]

@@ -84,3 +84,17 @@ def test_chain_matches_building_blocks(cuda, N, M, alpha, sphere, nsample):
     assert rel(at.grad, rga.cpu()) < 2e-5
     assert torch.equal(at.grad != 0, rga.cpu() != 0)
     assert torch.count_nonzero(wt.grad[rgw == 0]) == 0
+
+
+@pytest.mark.parametrize("N,M,alpha", [(16, 4, one_term(4)), (64, 5, sparse_alpha(5, 3, [0, 2, 4])), (256, 4, one_term(4))])
+def test_memory_limit_changes_no_bit(cuda, N, M, alpha):
+    """A plan with a memory limit keeps no transfer cube and all modes' planes
+    in the filter cube: the same factors from other places."""
+    def results(limit):
+        gen = ICGenerator(make_cfg(N, 500.0, 3, 100.0, M, "", 512), alpha, np.linspace(1.0, 0.5, M), *bbks(),
+                          mem_limit_bytes=limit)
+        w = white_noise(N, 7, cuda).requires_grad_(True)
+        disp = displacement(gen, w, torch.tensor(alpha, dtype=torch.float64))
+        disp.square().sum().backward()
+        return disp.detach(), gen.spectrum(), w.grad
+    assert all(torch.equal(a, b) for a, b in zip(results(0), results(1 << 40)))
