@@ -168,6 +168,8 @@ int fused_tile_r1(int N);  // first radix of the tile passes at this grid size
 int qcube_build(Plan* p);
 int tcube_build(Plan* p);
 struct Term;
+struct TermF;
+void factor_terms(const Term* t, std::vector<int> rem, int M, std::vector<TermF>& out);
 std::vector<std::vector<Term>> regrouped_terms(const std::vector<double>& alpha, int M);
 std::vector<int> modal_partition(const std::vector<std::vector<Term>>& by_r, int nparts);
 int fused_modal(Plan* p, cudaStream_t st);

@@ -37,7 +37,6 @@
 
 namespace aar {
 
-
 // ----------------------------------------------------------- row passes
 // (rows.cuh: rows_pairs, rows_fold)
 template <int N>
@@ -46,8 +45,15 @@ constexpr int pair_min_blocks(int threads) {
   return 65536 / regs / threads > 0 ? 65536 / regs / threads : 1;
 }
 constexpr int kPairThreads = 256;
+// Modal rows at radix 16 (N = 128, 256): 80 registers and three blocks; the 64 of
+// four blocks spill 380 bytes a thread (128^3, 3 read modes: 19 vs 15 us with
+// events), and two blocks measured the same as three.
+template <int N>
+constexpr int modal_min_blocks() {
+  return two_stage_r1(N) == 16 ? 3 : pair_min_blocks<N>(kPairThreads);
+}
 template <int N, class Op>
-__global__ void __launch_bounds__(kPairThreads, pair_min_blocks<N>(kPairThreads))
+__global__ void __launch_bounds__(kPairThreads, modal_min_blocks<N>())
     k_rows_pairs(const __grid_constant__ Op op, float2* work, int64_t fs, int HP, int64_t nrows, int pr,
                  const float2* __restrict__ tw2) {
   rows_pairs<N, Op, kPairThreads>(op, work, fs, HP, nrows, tw2, pr);
@@ -74,18 +80,23 @@ __global__ void __launch_bounds__(kSixThreads, six_min_blocks<N>())
   rows_pairs<N, Op, kSixThreads>(op, work, fs, HP, nrows, tw2, 32 / PairCfg<N>::T);
 }
 
-// One product term of the row combine, as a kernel parameter: the shared-
-// memory offsets of lines p and q, and bit 31 set for the counter-term that
-// is evaluated early into g_1 (see ModalRowOp).
+// A term in factored order (factor_terms) as a kernel parameter: the shared-
+// memory offsets of the lines of f_o and f_F, and bit 31 at its group's end.
 struct TermC {
-  uint32_t off;  // p LS | (q LS) << 16 | early << 31
+  uint32_t off;  // o LS | (F LS) << 16 | end << 31
   float c;
 };
 
 // modal products: the line of p holds f_p; the line of r is overwritten by g_r.  The
 // term list travels in the kernel's parameter space, so every thread reads
 // a term through the uniform constant path; each thread forms two positions
-// per term.
+// per term.  Bound by issue slots (60-70 % issued at 128^3), most of them
+// addresses and loop control: in factored order a term takes one field's load
+// and one multiply-add per component and a group one more of each, where f_p,
+// f_q and three operations were taken for every term (10 modes: 173 -> 145 us
+// at 128^3, two runs at a time; 25 -> 21 us at 64^3).  Two neighbouring
+// positions in one 16-byte access take a fifth fewer instructions but leave
+// half the warps without work at 64^3 (26 us) and gain nothing at 128^3.
 struct ModalRowOp {
   static constexpr bool kZfac = false;
   static constexpr bool kPairs = true;
@@ -93,6 +104,7 @@ struct ModalRowOp {
   int in_mode[kMaxModes], line_in[kMaxModes];
   int r_of_slot[kMaxModes], line_out[kMaxModes];
   int begin[kMaxModes + 1];
+  TermC early;  // the counter-term, c = 0 where there is none
   TermC t[kMaxTerms];
   __device__ int nin() const { return ni; }
   __device__ int nlines() const { return nl; }
@@ -104,44 +116,51 @@ struct ModalRowOp {
   // Slots in descending r: g_r only needs f_p f_q with p <= q <= r, so once
   // g_r is formed nothing later reads f_r and it is stored over it at once.
   // (The counter-term f_0 f_2 -> g_1 reads f_2 after g_2 has replaced it;
-  // that term is evaluated first, in the pass for r = 2, into a register.)
+  // that term is evaluated first, into registers.)
   template <int K>
   __device__ void combine(float2* sm, const int* pos, int LS) const {
     float2 g1_extra[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) g1_extra[i] = make_float2(0.f, 0.f);
-    for (int s = nr - 1; s >= 0; --s) {
-      const int r = r_of_slot[s];
-      float2 acc[K];
+    if (early.c != 0.f) {
+      const int po = (int)(early.off & 0xFFFFu), qo = (int)(early.off >> 16);
 #pragma unroll
-      for (int i = 0; i < K; ++i) acc[i] = make_float2(0.f, 0.f);
+      for (int i = 0; i < K; ++i) {
+        const float2 fp = sm[po + pos[i]], fq = sm[qo + pos[i]];
+        g1_extra[i] = make_float2(early.c * fp.x * fq.x, early.c * fp.y * fq.y);
+      }
+    }
+    for (int s = nr - 1; s >= 0; --s) {
+      float2 acc[K], h[K];
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        acc[i] = r_of_slot[s] == 1 ? g1_extra[i] : make_float2(0.f, 0.f);
+        h[i] = make_float2(0.f, 0.f);
+      }
       const int tb = begin[s], te = begin[s + 1];
-#pragma unroll 2
+#pragma unroll 4
       for (int ti = tb; ti < te; ++ti) {
         const TermC tm = t[ti];
-        const int po = (int)(tm.off & 0xFFFFu), qo = (int)((tm.off >> 16) & 0x7FFFu);
-        const bool early = (tm.off >> 31) != 0u;
+        const int oo = (int)(tm.off & 0xFFFFu);
 #pragma unroll
         for (int i = 0; i < K; ++i) {
-          const float2 fp = sm[po + pos[i]], fq = sm[qo + pos[i]];
-          const float vx = tm.c * fp.x * fq.x, vy = tm.c * fp.y * fq.y;
-          if (early) {
-            g1_extra[i].x += vx;
-            g1_extra[i].y += vy;
-          } else {
-            acc[i].x += vx;
-            acc[i].y += vy;
+          const float2 fo = sm[oo + pos[i]];
+          h[i].x = fmaf(tm.c, fo.x, h[i].x);
+          h[i].y = fmaf(tm.c, fo.y, h[i].y);
+        }
+        if ((tm.off >> 31) != 0u) {
+          const int Fo = (int)((tm.off >> 16) & 0x7FFFu);
+#pragma unroll
+          for (int i = 0; i < K; ++i) {
+            const float2 fF = sm[Fo + pos[i]];
+            acc[i].x = fmaf(fF.x, h[i].x, acc[i].x);
+            acc[i].y = fmaf(fF.y, h[i].y, acc[i].y);
+            h[i] = make_float2(0.f, 0.f);
           }
         }
       }
 #pragma unroll
-      for (int i = 0; i < K; ++i) {
-        if (r == 1) {
-          acc[i].x += g1_extra[i].x;
-          acc[i].y += g1_extra[i].y;
-        }
-        sm[line_out[s] * LS + pos[i]] = acc[i];
-      }
+      for (int i = 0; i < K; ++i) sm[line_out[s] * LS + pos[i]] = acc[i];
     }
   }
 };
@@ -239,7 +258,6 @@ __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
 
 // ----------------------------------------------------------- 2LPT passes
 
-__device__ __forceinline__ float sincf(float x) { return x == 0.f ? 1.f : sinf(x) / x; }
 
 #include "passes.cuh"
 
@@ -651,13 +669,21 @@ struct Launch {
     op.nl = tl.nlines;
     for (int i = 0; i < tl.nin; ++i) op.in_mode[i] = tl.in_mode[i], op.line_in[i] = tl.line[tl.in_mode[i]];
     for (int i = 0; i < tl.nr; ++i) op.r_of_slot[i] = tl.r_of_slot[i], op.line_out[i] = tl.line[tl.r_of_slot[i]];
-    for (int i = 0; i <= tl.nr; ++i) op.begin[i] = tl.begin[i];
-    for (int sl = 0; sl < tl.nr; ++sl)
+    op.early = {0u, 0.f};
+    const TermF* tf = (const TermF*)(ft + tl.nterms);
+    auto term = [&](int o, int F, bool end, float c) {
+      return TermC{(uint32_t)(tl.line[o] * LS) | ((uint32_t)(tl.line[F] * LS) << 16) | (end ? 1u << 31 : 0u), c};
+    };
+    int n = 0;
+    for (int sl = 0; sl < tl.nr; ++sl) {
+      op.begin[sl] = n;
       for (int i = tl.begin[sl]; i < tl.begin[sl + 1]; ++i) {
-        const uint32_t early = ft[i].r != tl.r_of_slot[sl] ? 1u : 0u;
-        op.t[i].off = (uint32_t)(tl.line[ft[i].p] * LS) | ((uint32_t)(tl.line[ft[i].q] * LS) << 16) | (early << 31);
-        op.t[i].c = ft[i].c;
+        const TermF& f = tf[i];
+        if (f.t >= 0) op.t[n++] = term(f.o, f.F, f.end, ft[f.t].c);
+        else op.early = term(ft[~f.t].p, ft[~f.t].q, false, ft[~f.t].c);
       }
+    }
+    op.begin[tl.nr] = n;
     return op;
   }
   static int modal_rows(Plan* p, float2* work, int64_t fs, int64_t nrows, cudaStream_t st) {
@@ -844,6 +870,27 @@ std::vector<int> modal_partition(const std::vector<std::vector<Term>>& by_r, int
   return part;
 }
 
+// The terms `rem` of one target in factored order: greedily, the field that
+// occurs in most remaining terms is taken out, g_r += f_F (sum_t c_t f_o), so a
+// term costs one multiply-add and a group one more (at 20 modes 212 operations
+// for the 134 terms instead of 268).
+void factor_terms(const Term* t, std::vector<int> rem, int M, std::vector<TermF>& out) {
+  while (!rem.empty()) {
+    std::vector<int> cnt(M, 0), keep;
+    for (int i : rem) {
+      cnt[t[i].p] += 1;
+      if (t[i].q != t[i].p) cnt[t[i].q] += 1;
+    }
+    const int F = (int)(std::max_element(cnt.begin(), cnt.end()) - cnt.begin());
+    for (int i : rem) {
+      if (t[i].p != F && t[i].q != F) keep.push_back(i);
+      else out.push_back({i, t[i].p == F ? t[i].q : t[i].p, F, 0});
+    }
+    out.back().end = 1;
+    rem.swap(keep);
+  }
+}
+
 // The plan's term list: the regrouped terms, or
 // with a modal partition only the slots of the plan's part.  A split keeps
 // the counter-term f_0 f_2 -> g_1 with the part of r = 1: as a term read
@@ -887,6 +934,18 @@ static int build_terms(Plan* p) {
   if (tl.nterms > kMaxTerms) return set_err(p, "too many alpha terms"), AAR_ERR_ARG;
   p->host_terms.assign((const char*)&tl, (const char*)&tl + sizeof(tl));
   p->host_terms.insert(p->host_terms.end(), (const char*)flat.data(), (const char*)(flat.data() + flat.size()));
+  // the generic row kernel's order: a slot's own terms factored, then the
+  // counter-term of g_1 among those of r = 2, as ~index
+  std::vector<TermF> fac;
+  for (int i = 0; i < nr; ++i) {
+    std::vector<int> own;
+    for (int t = tl.begin[i]; t < tl.begin[i + 1]; ++t)
+      if (flat[t].r == tl.r_of_slot[i]) own.push_back(t);
+    factor_terms(flat.data(), own, M, fac);
+    for (int t = tl.begin[i]; t < tl.begin[i + 1]; ++t)
+      if (flat[t].r != tl.r_of_slot[i]) fac.push_back({~t, 0, 0, 0});
+  }
+  p->host_terms.insert(p->host_terms.end(), (const char*)fac.data(), (const char*)(fac.data() + fac.size()));
   p->nterms = tl.nterms;
   p->nr_active = nr;
   p->chain_stale = p->qfull_stale = true;
@@ -1025,11 +1084,9 @@ int fused_modal(Plan* p, cudaStream_t st) {
 LptArgs lpt_args(Plan* p) {
   LptArgs a;
   a.m = modal_args(p);
-  a.inv_Dbeta = (float)(1.0 / (p->Dplus * p->Beta));
   a.twb = p->d_twb;
   a.sinc = p->d_sinc;
   a.isinc2 = p->d_isinc2;
-  a.box_over_2n = (float)(p->prm.box / 2 / p->N);
   return a;
 }
 

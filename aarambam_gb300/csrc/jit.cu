@@ -73,44 +73,29 @@ static std::string gen_source(int N, int M, int minb, int threads, int pr, int p
   int in_of[kMaxModes] = {};  // f index of a mode
   for (int i = 0; i < nin; ++i) in_of[tl.in_mode[i]] = i;
   // one block per output slot (the counter-term f0 f2 -> g1 with its own
-  // target r).  The slot's terms are factored: greedily, the field that
-  // occurs in most remaining terms is taken out, g_r += f_F (sum_t c_t f_t),
-  // so a term costs one multiply-add and a group one more (at 20 modes 212
-  // operations for the 134 terms instead of 268).
+  // target r), its terms in factored order.
   for (int sl = 0; sl < tl.nr; ++sl) {
     const int r = tl.r_of_slot[sl];
     s += "    {\n      float2 a[K];\n#pragma unroll\n      for (int i = 0; i < K; ++i) a[i] = make_float2(0.f, 0.f);\n";
-    std::vector<size_t> rem;
+    std::vector<int> own;
     for (size_t t = 0; t < terms.size(); ++t)
-      if (terms[t].r == r) rem.push_back(t);
-    while (!rem.empty()) {
-      std::vector<int> cnt(M, 0);
-      for (size_t t : rem) {
-        cnt[terms[t].p] += 1;
-        if (terms[t].q != terms[t].p) cnt[terms[t].q] += 1;
-      }
-      const int F = (int)(std::max_element(cnt.begin(), cnt.end()) - cnt.begin());
-      std::vector<size_t> keep;
-      bool first = true;
-      for (size_t t : rem) {
-        if (terms[t].p != F && terms[t].q != F) {
-          keep.push_back(t);
-          continue;
-        }
-        const int o = terms[t].p == F ? terms[t].q : terms[t].p;
-        const std::string c = "kCoef[" + std::to_string(t) + "]", fo = "f[" + std::to_string(in_of[o]) + "][i]";
-        if (first)
-          s += "      {\n      float2 h[K];\n#pragma unroll\n      for (int i = 0; i < K; ++i) h[i] = make_float2(" + c + " * " +
-               fo + ".x, " + c + " * " + fo + ".y);\n";
-        else
-          s += "#pragma unroll\n      for (int i = 0; i < K; ++i) { h[i].x = fmaf(" + c + ", " + fo + ".x, h[i].x); h[i].y = fmaf(" +
-               c + ", " + fo + ".y, h[i].y); }\n";
-        first = false;
-      }
-      const std::string fF = "f[" + std::to_string(in_of[F]) + "][i]";
+      if (terms[t].r == r) own.push_back((int)t);
+    std::vector<TermF> fac;
+    factor_terms(terms.data(), own, M, fac);
+    bool first = true;
+    for (const TermF& t : fac) {
+      const std::string c = "kCoef[" + std::to_string(t.t) + "]", fo = "f[" + std::to_string(in_of[t.o]) + "][i]";
+      if (first)
+        s += "      {\n      float2 h[K];\n#pragma unroll\n      for (int i = 0; i < K; ++i) h[i] = make_float2(" + c + " * " + fo +
+             ".x, " + c + " * " + fo + ".y);\n";
+      else
+        s += "#pragma unroll\n      for (int i = 0; i < K; ++i) { h[i].x = fmaf(" + c + ", " + fo + ".x, h[i].x); h[i].y = fmaf(" + c +
+             ", " + fo + ".y, h[i].y); }\n";
+      first = t.end;
+      if (!t.end) continue;
+      const std::string fF = "f[" + std::to_string(in_of[t.F]) + "][i]";
       s += "#pragma unroll\n      for (int i = 0; i < K; ++i) { a[i].x = fmaf(" + fF + ".x, h[i].x, a[i].x); a[i].y = fmaf(" + fF +
            ".y, h[i].y, a[i].y); }\n      }\n";
-      rem.swap(keep);
     }
     s += "#pragma unroll\n      for (int i = 0; i < K; ++i) sm[" + std::to_string(tl.line[r]) + " * LS + pos[i]] = a[i];\n    }\n";
   }

@@ -10,6 +10,12 @@ struct Term {      // one product f_p f_q with coefficient c into g_r
   float c;
 };
 
+// A term in factored order (factor_terms): h += c_t f_o, and at the end of its
+// group g_r += f_F h.
+struct TermF {
+  int t, o, F, end;
+};
+
 constexpr int kMaxTerms = 2048;
 
 struct TermList {
@@ -34,11 +40,9 @@ struct ModalArgs {
 
 struct LptArgs {
   ModalArgs m;        // grid and k helpers
-  float inv_Dbeta;    // 1 / (Dplus Beta)
   const float* twb;   // per n^2: T(k) / (Dplus Beta)
   const float* sinc;  // per grid index: sin(x)/x, x = k Box / 2N (1 at k = 0)
   const float* isinc2;  // per grid index: 1 / sinc^2
-  float box_over_2n;
 };
 
 ModalArgs modal_args(Plan* p);
