@@ -2,7 +2,9 @@
 // Gaussian potential -> modal non-Gaussian potential -> ZA + 2LPT
 // displacements.  The transforms of the chain are the plan's own (aar_c2r /
 // aar_r2c); these kernels are the per-cell spectral factors and the
-// real-space products, forward (for recomputation) and transposed.
+// real-space products, forward (for recomputation) and transposed, one C call
+// each.  The autograd function runs the chain in one call each way (chain.cuh);
+// these stay as its building blocks and the form its tests compare it with.
 //
 // Transposes of the FFTW-convention transforms on half spectra (kz = 0..N/2):
 // a c2r sums w(kz) Re(X_k e^{i k.x}) with w = 1 on the kz = 0 and N/2 planes

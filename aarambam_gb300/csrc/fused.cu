@@ -93,10 +93,11 @@ struct TermC {
 // per term.  Bound by issue slots (60-70 % issued at 128^3), most of them
 // addresses and loop control: in factored order a term takes one field's load
 // and one multiply-add per component and a group one more of each, where f_p,
-// f_q and three operations were taken for every term (10 modes: 173 -> 145 us
-// at 128^3, two runs at a time; 25 -> 21 us at 64^3).  Two neighbouring
+// f_q and three operations were taken for every term (six templates of 6-20
+// modes at 128^3, in one graph: 1038 -> 871 us of this kernel; a 64^3 run of 10
+// modes 152 -> 145 us).  Two neighbouring
 // positions in one 16-byte access take a fifth fewer instructions but leave
-// half the warps without work at 64^3 (26 us) and gain nothing at 128^3.
+// half the warps without work at 64^3 (21 -> 26 us) and gain nothing at 128^3.
 struct ModalRowOp {
   static constexpr bool kZfac = false;
   static constexpr bool kPairs = true;
@@ -256,9 +257,7 @@ __global__ void __launch_bounds__(kC2rThreads, pair_min_blocks<N>(kC2rThreads))
   }
 }
 
-// ----------------------------------------------------------- 2LPT passes
-
-
+// ----------------------------------------------------------- strided passes
 #include "passes.cuh"
 
 // ----------------------------------------------------------- read-out

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kProdThreads) k_slab_products(SlabTerms tm, co
 // acc(k) += e^{-2 pi i kx s / N} sum_r rho_r(k) G_{r,s}(kx mod L, ky, kz):
 // the slot sum Neumaier-compensated in the slab's frame, then rotated by the
 // twiddle once and added to the running compensated sum (acc_s, acc_c) of
-// the slabs.  rho_r per cell with k_modal_acc's expressions, its logarithm
+// the slabs.  rho_r per cell with the filter tables' expressions, its logarithm
 // and exponentials in the base-2 hardware forms of q_all_modes (every slab
 // re-evaluates them; the bracket k^s / kmin^s - 1 of kbar is 0 or at least
 // 0.42 for integer n2, no cancellation to guard).  The modes are walked in
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) k_slab_acc_modal(SlabGeo a, RhoArgs ra, S
 }
 
 // phi <- phi + fnl_n3 (sum + compensation) on kept cells, DC = 0
-// (main.c:1101-1126, as k_modal_acc ends).
+// (main.c:1101-1126, as k_xacc ends).
 __global__ void __launch_bounds__(256) k_slab_combine(Grid g, int N, int HP, float2* phi, const float2* __restrict__ acc_s,
                                                       const float2* __restrict__ acc_c, float fnl_n3) {
   const int H = N / 2 + 1;

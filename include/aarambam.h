@@ -404,9 +404,9 @@ void aar_batch_destroy(aar_batch* batch);
 int aar_modal_partition(const double* alpha_sym, int32_t n_modes, int32_t nparts, int32_t* part_of_r);
 int aar_set_modal_partition(aar_plan* plan, int32_t part, int32_t nparts);
 
-/* Run-time specialised modal row and accumulation kernels (no counterpart
-   in the reference): mode 0 off, 1 (default) for Nmesh >= 256, 2 always.
-   Both are compiled with NVRTC for the plan's alpha-term structure when the tables
+/* Run-time specialised modal row kernel (no counterpart in the reference):
+   mode 0 off, 1 (default) for Nmesh >= 256, 2 always.  It is
+   compiled with NVRTC for the plan's alpha-term structure when the tables
    are set (a new table with the same nonzero pattern only updates its
    coefficients); when compiling or loading fails the generic kernel stays
    in use and aar_jit_status says why ("on", "off" or the reason). */
