@@ -79,8 +79,10 @@ class ICGenerator:
             msg = self.L.aar_last_error(h) if h else b"plan creation failed"
             self.close()
             raise AarError(rc, msg.decode() if msg else "")
-        self._alpha = np.ascontiguousarray(alpha, dtype=np.float64)
-        self._x0 = np.ascontiguousarray(x0, dtype=np.float64)
+        # copies: set_tables compares with what the plan holds, so a table that
+        # its owner changes in place must not change here with it
+        self._alpha = np.array(alpha, dtype=np.float64, order="C")
+        self._x0 = np.array(x0, dtype=np.float64, order="C")
         M = self._alpha.shape[0]
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(self._alpha), _dptr(self._x0), M))
         kk = np.ascontiguousarray(k, dtype=np.float64)
@@ -130,10 +132,10 @@ class ICGenerator:
 
     def set_tables(self, alpha: np.ndarray, x0: np.ndarray = None) -> None:
         """Replace the coefficient tables (no-op when they are unchanged)."""
-        alpha = np.ascontiguousarray(alpha, dtype=np.float64)
-        x0 = self._x0 if x0 is None else np.ascontiguousarray(x0, dtype=np.float64)
-        if alpha.shape == self._alpha.shape and np.array_equal(alpha, self._alpha) and np.array_equal(x0, self._x0):
+        x0 = self._x0 if x0 is None else x0
+        if np.array_equal(alpha, self._alpha) and np.array_equal(x0, self._x0):
             return
+        alpha, x0 = np.array(alpha, dtype=np.float64, order="C"), np.array(x0, dtype=np.float64, order="C")
         self._alpha, self._x0 = alpha, x0
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(self._alpha), _dptr(self._x0), alpha.shape[0]))
 
