@@ -136,8 +136,8 @@ class ICGenerator:
         if np.array_equal(alpha, self._alpha) and np.array_equal(x0, self._x0):
             return
         alpha, x0 = np.array(alpha, dtype=np.float64, order="C"), np.array(x0, dtype=np.float64, order="C")
+        check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(alpha), _dptr(x0), alpha.shape[0]))
         self._alpha, self._x0 = alpha, x0
-        check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(self._alpha), _dptr(self._x0), alpha.shape[0]))
 
     def set_jit(self, mode: int) -> str:
         """Run-time specialised modal row kernel: 0 off, 1 for N >= 256 (the

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+from aarambam_gb300 import _lib
 from aarambam_gb300.ic import ICGenerator
 
 
@@ -42,3 +43,14 @@ def test_a_table_changed_in_place_is_set_again(make):
     g.set_tables(alpha.copy(), x0.copy())  # unchanged: not set again
     assert len(g.L.given) == 3
     assert g.L.given[1][0][0, 0, 1] == 7.0 and g.L.given[1][1][1] == 0.5 and g.L.given[2][1][1] == 0.25
+
+
+def test_a_refused_table_is_not_taken_for_the_plan_s():
+    alpha, x0 = np.ones((2, 2, 2)), np.array([1.0, 0.5])
+    g = generator(alpha, x0)
+    g.L.rc = 1
+    with pytest.raises(_lib.AarError):
+        g.set_tables(2 * alpha)
+    g.L.rc = 0
+    g.set_tables(2 * alpha)
+    assert len(g.L.given) == 2 and g.L.given[1][0][0, 0, 0] == 2.0
