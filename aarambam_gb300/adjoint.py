@@ -32,7 +32,7 @@ import torch
 
 from . import _lib
 from ._lib import check
-from .ic import ICGenerator, _ptr
+from .ic import ICGenerator, _dense, _ptr
 
 ONE, GAUSS, Q, RHO = _lib.AAR_ADJ_OP_ONE, _lib.AAR_ADJ_OP_GAUSS, _lib.AAR_ADJ_OP_Q, _lib.AAR_ADJ_OP_RHO
 HESS, PSI1, PSI2 = _lib.AAR_ADJ_OP_HESS, _lib.AAR_ADJ_OP_PSI1, _lib.AAR_ADJ_OP_PSI2
@@ -86,7 +86,7 @@ class _Displacement(torch.autograd.Function):
     def forward(ctx, w_hat, alpha, gen):
         N = gen.N
         ctx.w_dtype = w_hat.dtype
-        w_hat = w_hat.to(torch.complex64).contiguous()
+        w_hat = _dense(w_hat, torch.complex64)
         gen.set_tables(alpha.detach().double().cpu().numpy())
         phig, phi = torch.empty_like(w_hat), torch.empty_like(w_hat)
         disp = torch.empty((3, N, N, N), dtype=torch.float32, device=gen.device)
@@ -102,7 +102,7 @@ class _Displacement(torch.autograd.Function):
         gen = ctx.gen
         phig, phi = ctx.saved_tensors
         M = gen.n_modes
-        gdisp = gdisp.to(torch.float32).contiguous()
+        gdisp = _dense(gdisp, torch.float32)
         gw = torch.empty_like(phig)
         galpha = torch.empty((M, M, M), dtype=torch.float64, device=gdisp.device)
         scratch = torch.empty(gen.L.aar_adj_gradient_scratch_bytes(gen.h), dtype=torch.uint8, device=gdisp.device)

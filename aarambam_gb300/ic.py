@@ -47,6 +47,12 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
+def _dense(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """t as plain contiguous memory of dtype: a conjugate or negated view
+    (x.conj(), its imag) says so in a flag, which the address does not carry."""
+    return t.to(dtype).resolve_conj().resolve_neg().contiguous()
+
+
 def _dptr(a: np.ndarray):
     return np.ascontiguousarray(a, dtype=np.float64).ctypes.data_as(C.POINTER(C.c_double))
 
@@ -193,13 +199,13 @@ class ICGenerator:
         return out
 
     def c2r(self, spec: torch.Tensor) -> torch.Tensor:
-        spec = spec.to(torch.complex64).contiguous()
+        spec = _dense(spec, torch.complex64)
         out = torch.empty((self.N, self.N, self.N), dtype=torch.float32, device=self.device)
         check(self.L, self.h, self.L.aar_c2r(self.h, _ptr(spec), _ptr(out), self._stream()))
         return out
 
     def r2c(self, real: torch.Tensor) -> torch.Tensor:
-        real = real.to(torch.float32).contiguous()
+        real = _dense(real, torch.float32)
         out = torch.empty((self.N, self.N, self.N // 2 + 1), dtype=torch.complex64, device=self.device)
         check(self.L, self.h, self.L.aar_r2c(self.h, _ptr(real), _ptr(out), self._stream()))
         return out
@@ -211,11 +217,11 @@ class ICGenerator:
 
     def set_spectrum(self, spec: torch.Tensor) -> None:
         """Replace the plan's potential spectrum (complex [N, N, N/2+1])."""
-        spec = spec.to(torch.complex64).contiguous()
+        spec = _dense(spec, torch.complex64)
         check(self.L, self.h, self.L.aar_set_spectrum(self.h, _ptr(spec), self._stream()))
 
     def readout(self, lagr: torch.Tensor, pos: torch.Tensor = None, vel: torch.Tensor = None):
-        lagr = lagr.contiguous()
+        lagr = lagr.resolve_neg().contiguous()
         pos = torch.empty_like(lagr) if pos is None else pos
         vel = torch.empty_like(lagr) if vel is None else vel
         check(self.L, self.h, self.L.aar_stage_readout(self.h, _ptr(lagr), lagr.shape[0], _ptr(pos), _ptr(vel),
@@ -224,7 +230,7 @@ class ICGenerator:
 
     def run(self, lagr: torch.Tensor, pos: torch.Tensor = None, vel: torch.Tensor = None):
         """Whole path on device-resident Lagrangian positions float32 [n, 3]."""
-        lagr = lagr.contiguous()
+        lagr = lagr.resolve_neg().contiguous()
         pos = torch.empty_like(lagr) if pos is None else pos
         vel = torch.empty_like(lagr) if vel is None else vel
         check(self.L, self.h, self.L.aar_run(self.h, _ptr(lagr), lagr.shape[0], _ptr(pos), _ptr(vel),
