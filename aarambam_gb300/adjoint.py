@@ -92,7 +92,7 @@ class _Displacement(torch.autograd.Function):
         disp = torch.empty((3, N, N, N), dtype=torch.float32, device=gen.device)
         check(gen.L, gen.h, gen.L.aar_adj_displacement(gen.h, _ptr(w_hat), _ptr(disp), _ptr(phig), _ptr(phi),
                                                        gen._stream()))
-        ctx.gen = gen
+        ctx.gen, ctx.tables = gen, gen.tables
         ctx.save_for_backward(phig, phi)
         ctx.alpha_dtype, ctx.alpha_device = alpha.dtype, alpha.device
         return disp
@@ -101,13 +101,20 @@ class _Displacement(torch.autograd.Function):
     def backward(ctx, gdisp):
         gen = ctx.gen
         phig, phi = ctx.saved_tensors
-        M = gen.n_modes
         gdisp = _dense(gdisp, torch.float32)
         gw = torch.empty_like(phig)
-        galpha = torch.empty((M, M, M), dtype=torch.float64, device=gdisp.device)
-        scratch = torch.empty(gen.L.aar_adj_gradient_scratch_bytes(gen.h), dtype=torch.uint8, device=gdisp.device)
-        check(gen.L, gen.h, gen.L.aar_adj_gradient(gen.h, _ptr(phig), _ptr(phi), _ptr(gdisp), _ptr(gw), _ptr(galpha),
-                                                   _ptr(scratch), scratch.numel(), gen._stream()))
+        # at the forward pass's tables, which a later forward pass may have
+        # replaced in the plan; the plan goes back to those it holds now
+        held = gen.tables
+        gen.set_tables(*ctx.tables)
+        try:
+            M = gen.n_modes
+            galpha = torch.empty((M, M, M), dtype=torch.float64, device=gdisp.device)
+            scratch = torch.empty(gen.L.aar_adj_gradient_scratch_bytes(gen.h), dtype=torch.uint8, device=gdisp.device)
+            check(gen.L, gen.h, gen.L.aar_adj_gradient(gen.h, _ptr(phig), _ptr(phi), _ptr(gdisp), _ptr(gw),
+                                                       _ptr(galpha), _ptr(scratch), scratch.numel(), gen._stream()))
+        finally:
+            gen.set_tables(*held)
         return gw.to(ctx.w_dtype), galpha.to(device=ctx.alpha_device, dtype=ctx.alpha_dtype), None
 
 

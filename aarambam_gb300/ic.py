@@ -53,6 +53,13 @@ def _dense(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return t.to(dtype).resolve_conj().resolve_neg().contiguous()
 
 
+def _kept(a) -> np.ndarray:
+    """An own float64 copy that nothing writes to."""
+    a = np.array(a, dtype=np.float64, order="C")
+    a.setflags(write=False)
+    return a
+
+
 def _dptr(a: np.ndarray):
     return np.ascontiguousarray(a, dtype=np.float64).ctypes.data_as(C.POINTER(C.c_double))
 
@@ -87,8 +94,7 @@ class ICGenerator:
             raise AarError(rc, msg.decode() if msg else "")
         # copies: set_tables compares with what the plan holds, so a table that
         # its owner changes in place must not change here with it
-        self._alpha = np.array(alpha, dtype=np.float64, order="C")
-        self._x0 = np.array(x0, dtype=np.float64, order="C")
+        self._alpha, self._x0 = _kept(alpha), _kept(x0)
         M = self._alpha.shape[0]
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(self._alpha), _dptr(self._x0), M))
         kk = np.ascontiguousarray(k, dtype=np.float64)
@@ -136,12 +142,18 @@ class ICGenerator:
     def n_modes(self) -> int:
         return self._alpha.shape[0]
 
+    @property
+    def tables(self) -> tuple:
+        """(alpha, x0) that the plan holds, read-only."""
+        return self._alpha, self._x0
+
     def set_tables(self, alpha: np.ndarray, x0: np.ndarray = None) -> None:
         """Replace the coefficient tables (no-op when they are unchanged)."""
         x0 = self._x0 if x0 is None else x0
-        if np.array_equal(alpha, self._alpha) and np.array_equal(x0, self._x0):
+        if (alpha is self._alpha or np.array_equal(alpha, self._alpha)) and \
+                (x0 is self._x0 or np.array_equal(x0, self._x0)):
             return
-        alpha, x0 = np.array(alpha, dtype=np.float64, order="C"), np.array(x0, dtype=np.float64, order="C")
+        alpha, x0 = _kept(alpha), _kept(x0)
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(alpha), _dptr(x0), alpha.shape[0]))
         self._alpha, self._x0 = alpha, x0
 
