@@ -60,6 +60,13 @@ def _kept(a) -> np.ndarray:
     return a
 
 
+def _check_tables(alpha: np.ndarray, x0: np.ndarray) -> None:
+    """The library reads M^3 and M values from their addresses, M the first
+    extent of alpha."""
+    if alpha.ndim == 0 or alpha.size < alpha.shape[0] ** 3 or x0.size < alpha.shape[0]:
+        raise ValueError(f"expected alpha [M, M, M] and x0 [M], got {alpha.shape} and {x0.shape}")
+
+
 def _dptr(a: np.ndarray):
     return np.ascontiguousarray(a, dtype=np.float64).ctypes.data_as(C.POINTER(C.c_double))
 
@@ -70,6 +77,10 @@ class ICGenerator:
     def __init__(self, cfg: dict, alpha: np.ndarray, x0: np.ndarray, k: np.ndarray, T: np.ndarray,
                  precision: str = "fp32", device=None, mem_limit_bytes: int = 0, noise_fp64: bool = False,
                  nslab: int = 8):
+        # copies: set_tables compares with what the plan holds, so a table that
+        # its owner changes in place must not change here with it
+        self._alpha, self._x0 = _kept(alpha), _kept(x0)
+        _check_tables(self._alpha, self._x0)
         self.L = _lib.load()
         self.cfg = dict(cfg)
         self.N = int(cfg["Nmesh"])
@@ -92,9 +103,6 @@ class ICGenerator:
             msg = self.L.aar_last_error(h) if h else b"plan creation failed"
             self.close()
             raise AarError(rc, msg.decode() if msg else "")
-        # copies: set_tables compares with what the plan holds, so a table that
-        # its owner changes in place must not change here with it
-        self._alpha, self._x0 = _kept(alpha), _kept(x0)
         M = self._alpha.shape[0]
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(self._alpha), _dptr(self._x0), M))
         kk = np.ascontiguousarray(k, dtype=np.float64)
@@ -154,6 +162,7 @@ class ICGenerator:
                 (x0 is self._x0 or np.array_equal(x0, self._x0)):
             return
         alpha, x0 = _kept(alpha), _kept(x0)
+        _check_tables(alpha, x0)
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(alpha), _dptr(x0), alpha.shape[0]))
         self._alpha, self._x0 = alpha, x0
 

@@ -54,3 +54,13 @@ def test_a_refused_table_is_not_taken_for_the_plan_s():
     g.L.rc = 0
     g.set_tables(2 * alpha)
     assert len(g.L.given) == 2 and g.L.given[1][0][0, 0, 0] == 2.0
+
+
+@pytest.mark.parametrize("alpha,x0", [(np.ones((3, 3, 3)), None), (np.ones((3, 3, 2)), np.ones(3)), (np.ones((2, 2)), None)])
+def test_tables_that_are_too_short_are_refused(alpha, x0):
+    """Before the library reads past their end: x0 of two modes beside an alpha
+    of three, an alpha that is not a cube."""
+    g = generator(np.ones((2, 2, 2)), np.array([1.0, 0.5]))
+    with pytest.raises(ValueError):
+        g.set_tables(alpha, x0)
+    assert len(g.L.given) == 1 and g.n_modes == 2
