@@ -1256,6 +1256,8 @@ int aar_adj_gradient(aar_plan* h, const void* d_phig, const void* d_phi, const f
   int rc = adj_ready(&h->p);
   if (rc) return rc;
   if (scratch_bytes < chain_scratch_bytes(&h->p)) return set_err(&h->p, "gradient scratch too small"), AAR_ERR_ARG;
+  // the accumulating pass stages its tiles in 16-byte copies
+  if ((uintptr_t)d_scratch % 16) return set_err(&h->p, "gradient scratch must be 16-byte aligned"), AAR_ERR_ARG;
   h->p.last_launches = 0;
   return chain_backward(&h->p, (const float2*)d_phig, (const float2*)d_phi, d_gdisp, (float2*)d_gw, d_galpha,
                         (float2*)d_scratch, S(stream));

@@ -359,9 +359,9 @@ int aar_adj_displacement(aar_plan* plan, const void* d_w, float* d_disp, void* d
 /* Its transpose at (d_phig, d_phi): from d_gdisp [3][N][N][N] the noise
    gradient d_gw, complex [N][N][N/2+1], and d_galpha, FP64 [M][M][M], the
    gradient with respect to alpha at every sorted index p <= q <= r.  Device
-   scratch from the caller (aar_adj_gradient_scratch_bytes with the plan's
-   present tables; 0 before tables are set); the plan's own spectrum and fields
-   are not touched.  The first call after a table change makes the plan's
+   scratch from the caller, 16-byte aligned (aar_adj_gradient_scratch_bytes with
+   the plan's present tables; 0 before tables are set); the plan's own spectrum
+   and fields are not touched.  The first call after a table change makes the plan's
    gradient tables and synchronises the device. */
 size_t aar_adj_gradient_scratch_bytes(const aar_plan* plan);
 int aar_adj_gradient(aar_plan* plan, const void* d_phig, const void* d_phi, const float* d_gdisp, void* d_gw,

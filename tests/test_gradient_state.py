@@ -1,9 +1,11 @@
 """What a gradient takes from its plan and from its caller: the table of its own
-forward pass, whatever table the plan holds by then."""
+forward pass, whatever table the plan holds by then, and scratch that its 16-byte
+copies can read."""
 import numpy as np
 import pytest
 import torch
 
+from aarambam_gb300 import _lib
 from aarambam_gb300.adjoint import displacement, white_noise
 from aarambam_gb300.ic import ICGenerator
 from tests.common import bbks, make_cfg
@@ -53,3 +55,25 @@ def test_backward_after_another_forward(cuda, N):
     for (w, a), (gw, ga) in zip(got, want):
         assert torch.equal(w.grad, gw)
         assert rel(a.grad, ga) < 1e-12  # FP64 sums in another order
+
+
+def gradient(g, phig, phi, gd, scratch, gw, galpha):
+    return g.L.aar_adj_gradient(g.h, *(t.data_ptr() for t in (phig, phi, gd, gw, galpha, scratch)), scratch.numel(),
+                                g._stream())
+
+
+def test_misaligned_scratch_is_refused(cuda):
+    """On the host, before anything is launched."""
+    N = 16
+    g = generator(N, symmetric(4, [(0, 0, 3, 1.0)]))
+    phi, gd = white_noise(N, 7, cuda), torch.randn((3, N, N, N), device=cuda)
+    gw, galpha = torch.zeros_like(phi), torch.zeros((4, 4, 4), dtype=torch.float64, device=cuda)
+    need = g.L.aar_adj_gradient_scratch_bytes(g.h)
+    scratch = torch.empty(need + 16, dtype=torch.uint8, device=cuda)
+    assert gradient(g, phi, phi, gd, scratch[8:], gw, galpha) == _lib.AAR_ERR_ARG
+    assert b"16-byte" in g.L.aar_last_error(g.h)
+    torch.cuda.synchronize()
+    assert not gw.any() and not galpha.any()
+    assert gradient(g, phi, phi, gd, scratch[16:], gw, galpha) == _lib.AAR_OK
+    torch.cuda.synchronize()
+    assert gw.any() and galpha.any()
