@@ -1325,17 +1325,16 @@ int fused_r2c(Plan* p, const float* in, float2* out, cudaStream_t st) {
 
 #include "chain.cuh"
 
-// Device tables of the chain's products (entries, groups) and the sums; made
-// once per table set.
+// Device tables of the chain's products (entries, groups); made once per table
+// set.
 struct ChainTables {
   AdjEntry* ent;
   AdjGroup* grp;
-  double* sum;
   int nent, ngrp;
 };
-static int chain_tables(Plan* p, ChainTables& ct, cudaStream_t st) {
-  const int M = p->M, ntrip = chain_ntrip(M);
-  if (!p->d_chain || p->chain_stale) {
+static int chain_tables(Plan* p, ChainTables& ct) {
+  const int M = p->M;
+  if (p->chain_stale) {
     const TermList& tl = *(const TermList*)p->host_terms.data();
     const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
     std::vector<std::vector<AdjEntry>> by((size_t)M * M);  // [p][r]
@@ -1351,8 +1350,7 @@ static int chain_tables(Plan* p, ChainTables& ct, cudaStream_t st) {
       grp.push_back(AdjGroup{i / M, i % M, (int)ent.size(), (int)(ent.size() + by[i].size())});
       ent.insert(ent.end(), by[i].begin(), by[i].end());
     }
-    const size_t o_grp = sizeof(double) * ntrip, o_ent = o_grp + sizeof(AdjGroup) * grp.size();
-    const size_t need = o_ent + sizeof(AdjEntry) * ent.size();
+    const size_t o_ent = sizeof(AdjGroup) * grp.size(), need = o_ent + sizeof(AdjEntry) * ent.size();
     AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // an earlier pass may still read the old tables
     if (p->chain_bytes < need) {
       if (p->d_chain) cudaFree(p->d_chain), p->used_bytes -= p->chain_bytes;
@@ -1362,20 +1360,18 @@ static int chain_tables(Plan* p, ChainTables& ct, cudaStream_t st) {
       if (rc) return rc;
       p->chain_bytes = need;
     }
-    std::vector<char> host(need - o_grp);
+    std::vector<char> host(need);
     std::copy(grp.begin(), grp.end(), (AdjGroup*)host.data());
-    std::copy(ent.begin(), ent.end(), (AdjEntry*)(host.data() + (o_ent - o_grp)));
-    AAR_CUDA_TRY(p, cudaMemcpy((char*)p->d_chain + o_grp, host.data(), host.size(), cudaMemcpyHostToDevice));
+    std::copy(ent.begin(), ent.end(), (AdjEntry*)(host.data() + o_ent));
+    if (need) AAR_CUDA_TRY(p, cudaMemcpy(p->d_chain, host.data(), need, cudaMemcpyHostToDevice));
     p->chain_nent = (int)ent.size();
     p->chain_ngrp = (int)grp.size();
     p->chain_stale = false;
   }
-  ct.sum = (double*)p->d_chain;
-  ct.grp = (AdjGroup*)(ct.sum + ntrip);
+  ct.grp = (AdjGroup*)p->d_chain;
   ct.ent = (AdjEntry*)(ct.grp + p->chain_ngrp);
   ct.nent = p->chain_nent;
   ct.ngrp = p->chain_ngrp;
-  AAR_CUDA_TRY(p, cudaMemsetAsync(ct.sum, 0, sizeof(double) * ntrip, st));
   return AAR_OK;
 }
 
@@ -1398,7 +1394,9 @@ static int chain_cube(Plan* p, const float*& cube, Slots& plane) {
 }
 
 // Fields of the gradient's scratch: G, T, then the larger of the Hessian
-// stage's nine and the products' 2 M.
+// stage's nine and the products' 2 M; the sums of the products follow them (in
+// the caller's scratch, not the plan's memory: calls on different streams may
+// overlap).
 static int chain_fields(int M) { return 2 + std::max(9, 2 * M); }
 
 template <int N>
@@ -1437,11 +1435,13 @@ struct Chain {
     const ZTypes none{{0, 0, 0, 0, 0, 0}, 0.f, nullptr};
     const RhoArgs ra = rho_args(p);
     const AccScale sc{(float)(p->prm.primordial_index - 4), ra.log2kF, (float)(p->prm.fnl / ((double)N * N * N))};
+    double* sum = (double*)(scratch + chain_fields(M) * fs);
     ChainTables ct;
     Slots plane{};
     const float* cube = nullptr;
     int rc;
-    if ((rc = chain_tables(p, ct, st)) || (rc = chain_cube(p, cube, plane))) return rc;
+    if ((rc = chain_tables(p, ct)) || (rc = chain_cube(p, cube, plane))) return rc;
+    AAR_CUDA_TRY(p, cudaMemsetAsync(sum, 0, sizeof(double) * chain_ntrip(M), st));
     // displacement fields
     k_rows_r2c<N, true><<<dim3(c2r_blocks<N>(), 3), kC2rThreads, kLineSmem, st>>>(gdisp, W, fs, p->HP, rows, p->d_tw2);
     if ((rc = done(p))) return rc;
@@ -1493,7 +1493,7 @@ struct Chain {
       auto go = [&](auto rbc) {
         auto kern = k_chain_sums<N, decltype(rbc)::value>;
         AAR_CUDA_TRY(p, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<blocks, kChainThreads, smem, st>>>((const float*)W, 2 * fs, p->HP, M, share, ct.sum);
+        kern<<<blocks, kChainThreads, smem, st>>>((const float*)W, 2 * fs, p->HP, M, share, sum);
         return AAR_OK;
       };
       if ((rc = rb <= 4 ? go(std::integral_constant<int, 4>{})
@@ -1514,7 +1514,7 @@ struct Chain {
     }
     if ((rc = done(p))) return rc;
     const int counter = M > 2 && p->alpha[(size_t)1 * M + 2] != 0;
-    k_chain_galpha<<<1, 256, 0, st>>>(ct.sum, M, counter, galpha);
+    k_chain_galpha<<<1, 256, 0, st>>>(sum, M, counter, galpha);
     if ((rc = done(p))) return rc;
     {
       ProfScope ps_(p, "grad_rows", st);
@@ -1534,7 +1534,7 @@ struct Chain {
 };
 
 size_t chain_scratch_bytes(const Plan* p) {
-  return sizeof(float2) * (size_t)p->N * p->N * p->HP * chain_fields(p->M);
+  return sizeof(float2) * (size_t)p->N * p->N * p->HP * chain_fields(p->M) + sizeof(double) * chain_ntrip(p->M);
 }
 int chain_forward(Plan* p, const float2* w, float* disp, float2* phig, float2* phi, cudaStream_t st) {
   return dispatch_n(p->N, [&](auto nc) { return Chain<decltype(nc)::value>::forward(p, w, disp, phig, phi, st); });

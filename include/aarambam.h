@@ -362,7 +362,8 @@ int aar_adj_displacement(aar_plan* plan, const void* d_w, float* d_disp, void* d
    scratch from the caller, 16-byte aligned (aar_adj_gradient_scratch_bytes with
    the plan's present tables; 0 before tables are set); the plan's own spectrum
    and fields are not touched.  The first call after a table change makes the plan's
-   gradient tables and synchronises the device. */
+   gradient tables and synchronises the device; later ones may overlap on
+   streams of their own with buffers and scratch of their own. */
 size_t aar_adj_gradient_scratch_bytes(const aar_plan* plan);
 int aar_adj_gradient(aar_plan* plan, const void* d_phig, const void* d_phi, const float* d_gdisp, void* d_gw,
                      double* d_galpha, void* d_scratch, size_t scratch_bytes, void* stream);

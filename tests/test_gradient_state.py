@@ -1,6 +1,6 @@
 """What a gradient takes from its plan and from its caller: the table of its own
-forward pass, whatever table the plan holds by then, and scratch that its 16-byte
-copies can read."""
+forward pass, whatever table the plan holds by then, scratch that its 16-byte
+copies can read, and nothing that another gradient of the plan writes."""
 import numpy as np
 import pytest
 import torch
@@ -77,3 +77,31 @@ def test_misaligned_scratch_is_refused(cuda):
     assert gradient(g, phi, phi, gd, scratch[16:], gw, galpha) == _lib.AAR_OK
     torch.cuda.synchronize()
     assert gw.any() and galpha.any()
+
+
+def test_gradients_of_one_plan_on_two_streams(cuda):
+    """Buffers and scratch of their own: what they give one after the other, the
+    sums of alpha's gradient (atomic adds in FP64) to the order of summation."""
+    N, alpha = 64, symmetric(4, [(0, 0, 3, 1.0), (0, 1, 2, 6.0), (1, 1, 1, -2.0)])
+    g = generator(N, alpha)
+    need = g.L.aar_adj_gradient_scratch_bytes(g.h)
+
+    def buffers(i):
+        phi, gen = white_noise(N, 7 + i, cuda), torch.Generator(device="cuda").manual_seed(2 + i)
+        return [phi, phi, torch.randn((3, N, N, N), generator=gen, device=cuda),
+                torch.empty(need, dtype=torch.uint8, device=cuda), torch.zeros_like(phi),
+                torch.zeros((4, 4, 4), dtype=torch.float64, device=cuda)]
+
+    want = [buffers(i) for i in range(2)]
+    for b in want:
+        assert gradient(g, *b) == _lib.AAR_OK
+    torch.cuda.synchronize()
+    got, streams = [buffers(i) for i in range(2)], [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for b, s in zip(got, streams):
+            with torch.cuda.stream(s):
+                assert gradient(g, *b) == _lib.AAR_OK
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a[4], b[4]) and rel(a[5], b[5]) < 1e-12
