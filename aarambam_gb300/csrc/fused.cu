@@ -1404,6 +1404,37 @@ struct Chain {
   using L = Launch<N>;
   static constexpr int64_t kTiles = TileCfg<N>::TILES;
   static constexpr size_t kLineSmem = pair_line_smem<N>(kC2rThreads);
+  static constexpr size_t kSevenSmem = L::pair_smem(7 * (32 / PairCfg<N>::T));
+  // shared memory of the products' kernels; shares of a chunk that the threads
+  // of k_chain_sums split into, as many as its items leave
+  static constexpr int sums_share(int M, int nrb) {
+    const int items = M * (M + 1) / 2 * nrb;
+    return items <= 32 ? 4 : items <= 64 ? 2 : 1;
+  }
+  static constexpr size_t sums_smem(int M, int share) {
+    return sizeof(double) * ((share * chain_ntrip(M) + 1) / 2 * 2) + sizeof(float) * 2 * M * kChainLd;
+  }
+  static constexpr size_t gf_smem(int M, int nent, int ngrp) {
+    return sizeof(float2) * 2 * M * kChainThreads + sizeof(AdjEntry) * ((nent + 1) / 2 * 2) + sizeof(AdjGroup) * ngrp;
+  }
+  // The limits belong to the functions, which all plans of a grid size share:
+  // set to what the largest table takes, never to a plan's own need (one thread
+  // could lower it between another's setting and its launch).
+  static int configure(Plan* p) {
+    auto limit = [&](auto kern, size_t smem) {
+      AAR_CUDA_TRY(p, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      return AAR_OK;
+    };
+    constexpr size_t sums = sums_smem(kMaxModes, 1), gf = gf_smem(kMaxModes, 2 * kMaxTerms, kMaxModes * kMaxModes);
+    static_assert(sums >= sums_smem(10, 2) && sums >= sums_smem(7, 4) && sums_share(kMaxModes, 2) == 1 &&
+                  sums_share(11, 1) == 1 && sums_share(8, 1) == 2 && gf <= 227 * 1024);
+    int rc;
+    if ((rc = limit(k_chain_sums<N, 4>, sums)) || (rc = limit(k_chain_sums<N, 8>, sums)) ||
+        (rc = limit(k_chain_sums<N, 12>, sums)) || (rc = limit(k_chain_sums<N, 16>, sums)) ||
+        (rc = limit(k_chain_gf<N>, gf)) || (rc = limit(k_rows_source_adj<N>, kSevenSmem)))
+      return rc;
+    return limit(k_xacc<N, true>, XaccCfg<N>::SMEM);
+  }
   static unsigned cells(Plan* p) { return (unsigned)(p->num_sms * 8); }
   static int done(Plan* p) {
     AAR_CUDA_TRY(p, cudaGetLastError());
@@ -1459,9 +1490,7 @@ struct Chain {
     {
       ProfScope ps_(p, "grad_rows_source", st);
       constexpr int per = 2 * (32 / PairCfg<N>::T);  // rows of a block
-      constexpr size_t smem = L::pair_smem(7 * (32 / PairCfg<N>::T));
-      AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_source_adj<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_rows_source_adj<N><<<(unsigned)((rows + per - 1) / per), kSevenThreads, smem, st>>>(
+      k_rows_source_adj<N><<<(unsigned)((rows + per - 1) / per), kSevenThreads, kSevenSmem, st>>>(
           SourceAdjRowOp{-1, kF, a.isinc2}, W, fs, p->HP, rows, p->d_tw2);
     }
     if ((rc = done(p))) return rc;
@@ -1487,27 +1516,22 @@ struct Chain {
       // r in as few blocks of at most 16 as hold them, the threads in as many
       // shares of a chunk as the items leave
       const int nrb = (M + 15) / 16, rb = (M + nrb - 1) / nrb;
-      const int items = M * (M + 1) / 2 * nrb, share = items <= 32 ? 4 : items <= 64 ? 2 : 1;
-      const size_t smem = sizeof(double) * ((share * chain_ntrip(M) + 1) / 2 * 2) + sizeof(float) * 2 * M * kChainLd;
+      const int share = sums_share(M, nrb);
+      const size_t smem = sums_smem(M, share);
       const unsigned blocks = (unsigned)std::min<int64_t>((int64_t)N * N * N / kChainChunk, (int64_t)p->num_sms * 8);
       auto go = [&](auto rbc) {
-        auto kern = k_chain_sums<N, decltype(rbc)::value>;
-        AAR_CUDA_TRY(p, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<blocks, kChainThreads, smem, st>>>((const float*)W, 2 * fs, p->HP, M, share, sum);
-        return AAR_OK;
+        k_chain_sums<N, decltype(rbc)::value>
+            <<<blocks, kChainThreads, smem, st>>>((const float*)W, 2 * fs, p->HP, M, share, sum);
       };
-      if ((rc = rb <= 4 ? go(std::integral_constant<int, 4>{})
-                : rb <= 8 ? go(std::integral_constant<int, 8>{})
-                : rb <= 12 ? go(std::integral_constant<int, 12>{})
-                           : go(std::integral_constant<int, 16>{})))
-        return rc;
+      if (rb <= 4) go(std::integral_constant<int, 4>{});
+      else if (rb <= 8) go(std::integral_constant<int, 8>{});
+      else if (rb <= 12) go(std::integral_constant<int, 12>{});
+      else go(std::integral_constant<int, 16>{});
     }
     if ((rc = done(p))) return rc;
     {
       ProfScope ps_(p, "grad_gf", st);
-      const size_t smem = sizeof(float2) * 2 * M * kChainThreads + sizeof(AdjEntry) * ((ct.nent + 1) / 2 * 2) +
-                          sizeof(AdjGroup) * ct.ngrp;
-      AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_chain_gf<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const size_t smem = gf_smem(M, ct.nent, ct.ngrp);
       const int64_t n2 = (int64_t)N * N * N / 2;
       k_chain_gf<N><<<(unsigned)std::min<int64_t>((n2 + kChainThreads - 1) / kChainThreads, (int64_t)p->num_sms * 16),
                       kChainThreads, smem, st>>>((float*)W, 2 * fs, p->HP, M, ct.ent, ct.nent, ct.grp, ct.ngrp);
@@ -1523,8 +1547,6 @@ struct Chain {
     if ((rc = done(p))) return rc;
     if ((rc = L::template axis_pass<1, -1>(p, W, M, run(0, M), st, "grad_y"))) return rc;
     const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), plane, cube, sc, p->d_amp, gw};
-    AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)XaccCfg<N>::SMEM));
     {
       ProfScope ps_(p, "grad_xacc", st);
       k_xacc<N, true><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);
@@ -1554,7 +1576,8 @@ int fused_configure_xform(Plan* p) {
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_c2r<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_rows_r2c<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    return Launch<N>::configure(p);
+    const int rc = Chain<N>::configure(p);
+    return rc ? rc : Launch<N>::configure(p);
   });
 }
 

@@ -1,6 +1,8 @@
 """What a gradient takes from its plan and from its caller: the table of its own
 forward pass, whatever table the plan holds by then, scratch that its 16-byte
 copies can read, and nothing that another gradient of the plan writes."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -105,3 +107,34 @@ def test_gradients_of_one_plan_on_two_streams(cuda):
         torch.cuda.synchronize()
         for a, b in zip(got, want):
             assert torch.equal(a[4], b[4]) and rel(a[5], b[5]) < 1e-12
+
+
+def test_gradients_of_two_plans_in_two_threads(cuda):
+    """Plans of one grid size whose products take different amounts of shared
+    memory, each thread on a stream of its own: every launch goes through."""
+    N, full = 16, np.zeros((20, 20, 20))
+    for p in range(20):
+        for q in range(p, 20):
+            full[p, q, q:] = 1.0
+    rc = [[], []]
+
+    def work(i, g, bufs, stream):
+        with torch.cuda.stream(stream):
+            for _ in range(400):
+                rc[i].append(gradient(g, *bufs))
+
+    threads = []
+    for i, alpha in enumerate((symmetric(4, [(0, 0, 3, 1.0)]), full)):
+        g, phi, M = generator(N, alpha), white_noise(N, 7, cuda), alpha.shape[0]
+        bufs = [phi, phi, torch.randn((3, N, N, N), device=cuda),
+                torch.empty(g.L.aar_adj_gradient_scratch_bytes(g.h), dtype=torch.uint8, device=cuda),
+                torch.zeros_like(phi), torch.zeros((M, M, M), dtype=torch.float64, device=cuda)]
+        assert gradient(g, *bufs) == _lib.AAR_OK
+        threads.append(threading.Thread(target=work, args=(i, g, bufs, torch.cuda.Stream())))
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert len(rc[0]) == len(rc[1]) == 400 and not any(rc[0]) and not any(rc[1])
