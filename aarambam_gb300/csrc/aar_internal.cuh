@@ -154,6 +154,10 @@ struct ProfScope {
 };
 
 int plan_alloc(Plan* p, void** ptr, size_t bytes);
+// Host table to device memory, complete when it returns: cudaMemcpy may return
+// while the last of a pageable source is on its way, and kernels on a stream
+// that does not wait for the legacy one would read in between.
+int upload(Plan* p, void* dst, const void* src, size_t bytes);
 
 const char* set_err(Plan* p, const std::string& e);
 

@@ -210,8 +210,8 @@ static int set_transfer(Plan* p, const double* k, const double* t, int n) {
                    : 0.f;
       twb[n2] = (float)(cz.transfer(km) / p->Dplus / p->Beta);
     }
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_amp, amp.data(), sizeof(float) * nsq, cudaMemcpyHostToDevice));
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_twb, twb.data(), sizeof(float) * nsq, cudaMemcpyHostToDevice));
+    if (int rc_ = upload(p, p->d_amp, amp.data(), sizeof(float) * nsq)) return rc_;
+    if (int rc_ = upload(p, p->d_twb, twb.data(), sizeof(float) * nsq)) return rc_;
     // a cube that exists follows at once (a captured run reads it); the first
     // is made with the fields
     p->tcube_stale = true;
@@ -231,6 +231,13 @@ int plan_alloc(Plan* p, void** ptr, size_t bytes) {
     return set_err(p, std::string("cudaMalloc: ") + cudaGetErrorString(e)), AAR_ERR_OOM;
   }
   p->used_bytes += bytes;
+  return AAR_OK;
+}
+
+int upload(Plan* p, void* dst, const void* src, size_t bytes) {
+  if (bytes == 0) return AAR_OK;
+  AAR_CUDA_TRY(p, cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+  AAR_CUDA_TRY(p, cudaStreamSynchronize(cudaStreamLegacy));
   return AAR_OK;
 }
 
@@ -370,8 +377,8 @@ static int mode_tables(Plan* p) {
     }
   }
   for (int n = 0; n < M; ++n) qt[(size_t)n * nsq] = 0.f;
-  AAR_CUDA_TRY(p, cudaMemcpy(p->d_qtab, qt.data(), sizeof(float) * qt.size(), cudaMemcpyHostToDevice));
-  AAR_CUDA_TRY(p, cudaMemcpy(p->d_rtab, rt.data(), sizeof(float) * rt.size(), cudaMemcpyHostToDevice));
+  if (int rc_ = upload(p, p->d_qtab, qt.data(), sizeof(float) * qt.size())) return rc_;
+  if (int rc_ = upload(p, p->d_rtab, rt.data(), sizeof(float) * rt.size())) return rc_;
   return AAR_OK;
 }
 
@@ -421,7 +428,7 @@ static int create(Plan* p) {
     std::vector<U576> pw;  // ranlux skip-ahead
     seedtable_powers(pw);
     if ((rc = plan_alloc(p, &p->d_rlxpow, sizeof(U576) * pw.size()))) return rc;
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_rlxpow, pw.data(), sizeof(U576) * pw.size(), cudaMemcpyHostToDevice));
+    if (int rc_ = upload(p, p->d_rlxpow, pw.data(), sizeof(U576) * pw.size())) return rc_;
   }
   if (is_fp32(q)) {
     std::vector<float2> twN(N), twH(N / 2);
@@ -432,8 +439,8 @@ static int create(Plan* p) {
     for (int m = 0; m < N / 2; ++m) twH[m] = twN[2 * m];
     if ((rc = plan_alloc(p, (void**)&p->d_twN, sizeof(float2) * N))) return rc;
     if ((rc = plan_alloc(p, (void**)&p->d_twH, sizeof(float2) * (N / 2)))) return rc;
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_twN, twN.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_twH, twH.data(), sizeof(float2) * (N / 2), cudaMemcpyHostToDevice));
+    if (int rc_ = upload(p, p->d_twN, twN.data(), sizeof(float2) * N)) return rc_;
+    if (int rc_ = upload(p, p->d_twH, twH.data(), sizeof(float2) * (N / 2))) return rc_;
     if (q.precision == AAR_FUSED_FP32) {
       // second-stage twiddles of the tile passes: [r][j], r < N / R1, j < R1
       const int R1 = fused_tile_r1(N);
@@ -441,7 +448,7 @@ static int create(Plan* p) {
       for (int r = 0; r < N / R1; ++r)
         for (int j = 0; j < R1; ++j) tw2[r * R1 + j] = twN[r * j];
       if ((rc = plan_alloc(p, (void**)&p->d_tw2, sizeof(float2) * N))) return rc;
-      AAR_CUDA_TRY(p, cudaMemcpy(p->d_tw2, tw2.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+      if (int rc_ = upload(p, p->d_tw2, tw2.data(), sizeof(float2) * N)) return rc_;
     }
     int64_t nsq = 3LL * (N / 2) * (N / 2) + 1;
     if ((rc = plan_alloc(p, (void**)&p->d_amp, sizeof(float) * nsq))) return rc;
@@ -457,7 +464,7 @@ static int create(Plan* p) {
       sinc[i] = (float)f;
     }
     if ((rc = plan_alloc(p, (void**)&p->d_sinc, sizeof(float) * N))) return rc;
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_sinc, sinc.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
+    if (int rc_ = upload(p, p->d_sinc, sinc.data(), sizeof(float) * N)) return rc_;
     // its inverse square, the per-axis CIC deconvolution factor of the
     // separable 2LPT passes
     std::vector<float> is2(N);
@@ -470,7 +477,7 @@ static int create(Plan* p) {
       is2[i] = (float)(1.0 / (f * f));
     }
     if ((rc = plan_alloc(p, (void**)&p->d_isinc2, sizeof(float) * N))) return rc;
-    AAR_CUDA_TRY(p, cudaMemcpy(p->d_isinc2, is2.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
+    if (int rc_ = upload(p, p->d_isinc2, is2.data(), sizeof(float) * N)) return rc_;
   }
   return AAR_OK;
 }

@@ -1363,7 +1363,7 @@ static int chain_tables(Plan* p, ChainTables& ct) {
     std::vector<char> host(need);
     std::copy(grp.begin(), grp.end(), (AdjGroup*)host.data());
     std::copy(ent.begin(), ent.end(), (AdjEntry*)(host.data() + o_ent));
-    if (need) AAR_CUDA_TRY(p, cudaMemcpy(p->d_chain, host.data(), need, cudaMemcpyHostToDevice));
+    if (int rc_ = upload(p, p->d_chain, host.data(), need)) return rc_;
     p->chain_nent = (int)ent.size();
     p->chain_ngrp = (int)grp.size();
     p->chain_stale = false;

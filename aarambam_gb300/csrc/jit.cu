@@ -224,7 +224,7 @@ int jit_prepare(Plan* p) {
     p->jit_status = "shared-memory attribute refused";
     return AAR_OK;
   }
-  if (!coef.empty()) AAR_CUDA_TRY(p, cudaMemcpy(j->coef, coef.data(), sizeof(float) * coef.size(), cudaMemcpyHostToDevice));
+  if (int rc_ = upload(p, j->coef, coef.data(), sizeof(float) * coef.size())) return rc_;
   p->jit_status = "on";
   return AAR_OK;
 }

@@ -395,10 +395,10 @@ int plain_setup(Plan* p) {
     }
     sinc[i] = f;
   }
-  AAR_CUDA_TRY(p, cudaMemcpy(s->qin, qin.data(), sizeof(double) * qin.size(), cudaMemcpyHostToDevice));
-  AAR_CUDA_TRY(p, cudaMemcpy(s->qout, qout.data(), sizeof(double) * qout.size(), cudaMemcpyHostToDevice));
-  AAR_CUDA_TRY(p, cudaMemcpy(s->twb, twb.data(), sizeof(double) * twb.size(), cudaMemcpyHostToDevice));
-  AAR_CUDA_TRY(p, cudaMemcpy(s->sinc, sinc.data(), sizeof(double) * N, cudaMemcpyHostToDevice));
+  if (int rc_ = upload(p, s->qin, qin.data(), sizeof(double) * qin.size())) return rc_;
+  if (int rc_ = upload(p, s->qout, qout.data(), sizeof(double) * qout.size())) return rc_;
+  if (int rc_ = upload(p, s->twb, twb.data(), sizeof(double) * twb.size())) return rc_;
+  if (int rc_ = upload(p, s->sinc, sinc.data(), sizeof(double) * N)) return rc_;
   if (cufftPlan3d(&s->z2d, N, N, N, CUFFT_Z2D) != CUFFT_SUCCESS) return set_err(p, "cufftPlan3d Z2D failed"), AAR_ERR_CUDA;
   if (cufftPlan3d(&s->d2z, N, N, N, CUFFT_D2Z) != CUFFT_SUCCESS) {
     cufftDestroy(s->z2d);
