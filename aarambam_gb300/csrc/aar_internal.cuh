@@ -67,18 +67,15 @@ struct Plan {
   int rtab_stride = 0;
   int64_t nsq = 0;            // 3 (N/2)^2 + 1
   int qtab_m = 0;             // modes the tables were allocated for
-  // field filters of the first modal pass over |ky|, kz, |kx|, M (N/2+1)^2 HP
-  // floats (qcube_build); made on first use after each table change
+  // field filters over |ky|, kz, |kx|, M (N/2+1)^2 HP floats (qcube_build); made
+  // on first use after each table change
   float* d_qcube = nullptr;
   int qcube_m = 0;
   bool qcube_stale = true;
   float* d_tcube = nullptr;  // T/(D Beta) likewise (tcube_build), after each transfer change
   bool tcube_stale = true;
-  // gradient (chain.cuh): the cube of all modes where the one above is not,
-  // and the products' tables, made on the first gradient after a table change
-  float* d_qfull = nullptr;
-  int qfull_m = 0;
-  bool qfull_stale = true;
+  // gradient (chain.cuh): the products' tables, made on the first gradient
+  // after a table change
   void* d_chain = nullptr;
   size_t chain_bytes = 0;
   int chain_nent = 0, chain_ngrp = 0;

@@ -249,7 +249,7 @@ static void plan_release(Plan* p) {
   p->prof.clear();
   for (auto e : p->event_pool) cudaEventDestroy(e);
   p->event_pool.clear();
-  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_tcube, p->d_qfull, p->d_chain};
+  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_tcube, p->d_chain};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   p->d_phik = p->d_work = nullptr;
@@ -259,10 +259,10 @@ static void plan_release(Plan* p) {
   p->d_rlxpow = nullptr;
   p->d_qtab = p->d_rtab = nullptr;
   p->d_sinc = p->d_isinc2 = nullptr;
-  p->d_qcube = p->d_tcube = p->d_qfull = nullptr;
+  p->d_qcube = p->d_tcube = nullptr;
   p->tcube_stale = true;
-  p->qcube_m = p->qfull_m = 0;
-  p->qcube_stale = p->qfull_stale = p->chain_stale = true;
+  p->qcube_m = 0;
+  p->qcube_stale = p->chain_stale = true;
   p->d_chain = nullptr;
   p->chain_bytes = 0;
   p->d_io = nullptr;
@@ -1088,7 +1088,6 @@ int aar_set_modal_partition(aar_plan* h, int32_t part, int32_t nparts) {
   p->modal_nparts = nparts;
   if (!p->have_tables) return AAR_OK;
   AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // the term list is rewritten below
-  p->qcube_stale = true;                     // the part may read other modes
   return fused_prepare(p);
 }
 

@@ -713,10 +713,7 @@ struct Launch {
     const int64_t fs = fstride(p);
     const TermList& tl = terms(p);
     const Slots in = slots(tl.in_mode, tl.nin), out = slots(tl.r_of_slot, tl.nr);
-    Slots in_line{}, out_line{};
-    for (int i = 0; i < tl.nin; ++i) in_line.s[i] = tl.line[tl.in_mode[i]];
-    for (int i = 0; i < tl.nr; ++i) out_line.s[i] = tl.line[tl.r_of_slot[i]];
-    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), in_line, p->d_qcube};
+    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), 0, p->d_qcube};
     int rc = run_pass<N, 0, +1>(p, xo, kTiles * tl.nin, st, "modal_xinv");
     if (rc) return rc;
     if ((rc = axis_pass<1, +1>(p, p->d_work, tl.nin, in, st, "modal_ypass_inv"))) return rc;
@@ -730,11 +727,11 @@ struct Launch {
     if constexpr (TileCfg<N>::R1 == 32) {
       if (tl.nr == 1) {
         const int64_t plane = (int64_t)(N / 2 + 1) * p->HP * (N / 2 + 1);
-        const XaddOp<N> xo1{a.g, p->d_phik, p->d_work + out.s[0] * fs, p->d_qcube + out_line.s[0] * plane, sc};
+        const XaddOp<N> xo1{a.g, p->d_phik, p->d_work + out.s[0] * fs, p->d_qcube + out.s[0] * plane, sc};
         return run_pass<N, 0, -1>(p, xo1, kTiles, st, "modal_xacc");
       }
     }
-    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, out_line, p->d_qcube, sc, nullptr, nullptr};
+    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, p->d_qcube, sc, nullptr, nullptr};
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XaccCfg<N>::SMEM));
     {
       ProfScope ps_(p, "modal_xacc", st);
@@ -949,18 +946,19 @@ static int build_terms(Plan* p) {
   p->host_terms.insert(p->host_terms.end(), (const char*)fac.data(), (const char*)(fac.data() + fac.size()));
   p->nterms = tl.nterms;
   p->nr_active = nr;
-  p->chain_stale = p->qfull_stale = true;
+  p->chain_stale = true;
   return AAR_OK;
 }
 
-// The filter cube of the first modal pass: the plan's per-|k|^2 filters
+// The filter cube of the modal passes: the plan's per-|k|^2 filters
 // (mode_tables: FP64 formulas rounded once to float) over 0 <= |kx|, |ky| <=
 // N/2 and the padded kz columns, zero on the cut, at k = 0 and on the padding
 // (keep_cell depends on |k_a| only).  Index (((p K + |ky|) NCOL + kz / 8) K +
-// |kx|) 8 + kz % 8, p the row-kernel line of a read mode or active r (TermList),
-// K = N/2 + 1, NCOL = HP / 8.
-__global__ void __launch_bounds__(256) k_qcube(Grid g, int nl, const __grid_constant__ Slots mode,
-                                               const float* __restrict__ qtab, int64_t nsq, float* __restrict__ q) {
+// |kx|) 8 + kz % 8, p the mode, K = N/2 + 1, NCOL = HP / 8.  Every mode has its
+// plane, read by a term or not: the products' gradients take them all, and the
+// cube keeps its address while the mode count does.
+__global__ void __launch_bounds__(256) k_qcube(Grid g, int M, const float* __restrict__ qtab, int64_t nsq,
+                                               float* __restrict__ q) {
   const int K = g.N / 2 + 1, ncol = g.HP / 8;
   const int64_t per = (int64_t)K * g.HP * K;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (int64_t)gridDim.x * blockDim.x) {
@@ -970,29 +968,30 @@ __global__ void __launch_bounds__(256) k_qcube(Grid g, int nl, const __grid_cons
     const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
     const int n2 = ax * ax + ay * ay + kz * kz;
     const bool on = kz <= g.N / 2 && n2 != 0 && keep_cell(g, ax, ay, kz);
-    for (int c = 0; c < nl; ++c) q[(int64_t)c * per + i] = on ? __ldg(qtab + (int64_t)mode.s[c] * nsq + n2) : 0.f;
+    for (int c = 0; c < M; ++c) q[(int64_t)c * per + i] = on ? __ldg(qtab + (int64_t)c * nsq + n2) : 0.f;
   }
 }
 
-// The cube of n modes into `cube` (plan-owned, `have` planes of it allocated)
-static int make_cube(Plan* p, int n, const Slots& mode, float*& cube, int& have) {
+int qcube_build(Plan* p) {
+  if (!p->have_tables || (!p->qcube_stale && p->d_qcube)) return AAR_OK;  // no tables yet: nothing reads filters
   const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
-  if (!cube || have != n) {
-    if (cube) {
+  if (!p->d_qcube || p->qcube_m != p->M) {
+    if (p->d_qcube) {
       AAR_CUDA_TRY(p, cudaDeviceSynchronize());
-      cudaFree(cube), p->used_bytes -= sizeof(float) * (size_t)per * have;
+      cudaFree(p->d_qcube), p->used_bytes -= sizeof(float) * (size_t)per * p->qcube_m;
     }
-    cube = nullptr;
-    have = 0;
-    int rc = plan_alloc(p, (void**)&cube, sizeof(float) * (size_t)per * n);
+    p->d_qcube = nullptr;
+    p->qcube_m = 0;
+    int rc = plan_alloc(p, (void**)&p->d_qcube, sizeof(float) * (size_t)per * p->M);
     if (rc) return rc;
-    have = n;
+    p->qcube_m = p->M;
   }
-  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, n, mode, p->d_qtab, p->nsq, cube);
+  k_qcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, p->M, p->d_qtab, p->nsq, p->d_qcube);
   AAR_CUDA_TRY(p, cudaGetLastError());
   // made on the legacy stream once per table set; runs on the caller's
   // streams read it afterwards
   AAR_CUDA_TRY(p, cudaDeviceSynchronize());
+  p->qcube_stale = false;
   return AAR_OK;
 }
 
@@ -1020,32 +1019,7 @@ int tcube_build(Plan* p) {
   if (!p->d_tcube && plan_alloc(p, (void**)&p->d_tcube, sizeof(float) * (size_t)per)) return AAR_OK;
   k_tcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, p->d_twb, p->d_tcube);
   AAR_CUDA_TRY(p, cudaGetLastError());
-  AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // as make_cube
-  return AAR_OK;
-}
-
-// Planes of the filter cube: the lines that the products read first, then the
-// modes that only their gradients read.
-static Slots cube_planes(const Plan* p, const TermList& tl) {
-  Slots plane{};
-  for (int m = 0, n = tl.nlines; m < p->M; ++m) plane.s[m] = tl.line[m] >= 0 ? tl.line[m] : n++;
-  return plane;
-}
-
-// The lines' planes; all M in a plan with a memory limit, which leaves the
-// gradient no second cube to allocate (chain_cube).
-int qcube_build(Plan* p) {
-  if (p->host_terms.empty()) return AAR_OK;  // no tables yet: nothing reads filters
-  const TermList& tl = *(const TermList*)p->host_terms.data();
-  const int n = p->prm.mem_limit_bytes > 0 ? p->M : tl.nlines;
-  if ((!p->qcube_stale && p->d_qcube) || n == 0) return AAR_OK;
-  const Slots plane = cube_planes(p, tl);
-  Slots mode{};
-  for (int m = 0; m < p->M; ++m)
-    if (plane.s[m] < n) mode.s[plane.s[m]] = m;
-  int rc = make_cube(p, n, mode, p->d_qcube, p->qcube_m);
-  if (rc) return rc;
-  p->qcube_stale = false;
+  AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // as qcube_build
   return AAR_OK;
 }
 
@@ -1375,24 +1349,6 @@ static int chain_tables(Plan* p, ChainTables& ct) {
   return AAR_OK;
 }
 
-// The filter cube of all M modes (the products' gradients need the ones that
-// the products do not read, too): the plan's own where it holds them all, else
-// a second one made on the first gradient after a table change.
-static int chain_cube(Plan* p, const float*& cube, Slots& plane) {
-  plane = cube_planes(p, *(const TermList*)p->host_terms.data());
-  cube = p->d_qcube;
-  if (p->qcube_m == p->M && !p->qcube_stale) return AAR_OK;
-  if (p->qfull_stale || !p->d_qfull) {
-    Slots mode{};
-    for (int m = 0; m < p->M; ++m) mode.s[plane.s[m]] = m;
-    int rc = make_cube(p, p->M, mode, p->d_qfull, p->qfull_m);
-    if (rc) return rc;
-    p->qfull_stale = false;
-  }
-  cube = p->d_qfull;
-  return AAR_OK;
-}
-
 // Fields of the gradient's scratch: G, T, then the larger of the Hessian
 // stage's nine and the products' 2 M; the sums of the products follow them (in
 // the caller's scratch, not the plan's memory: calls on different streams may
@@ -1468,10 +1424,8 @@ struct Chain {
     const AccScale sc{(float)(p->prm.primordial_index - 4), ra.log2kF, (float)(p->prm.fnl / ((double)N * N * N))};
     double* sum = (double*)(scratch + chain_fields(M) * fs);
     ChainTables ct;
-    Slots plane{};
-    const float* cube = nullptr;
     int rc;
-    if ((rc = chain_tables(p, ct)) || (rc = chain_cube(p, cube, plane))) return rc;
+    if ((rc = chain_tables(p, ct))) return rc;
     AAR_CUDA_TRY(p, cudaMemsetAsync(sum, 0, sizeof(double) * chain_ntrip(M), st));
     // displacement fields
     k_rows_r2c<N, true><<<dim3(c2r_blocks<N>(), 3), kC2rThreads, kLineSmem, st>>>(gdisp, W, fs, p->HP, rows, p->d_tw2);
@@ -1499,9 +1453,9 @@ struct Chain {
     k_chain_hess<N><<<cells(p), 256, 0, st>>>(a, W, fs, sc, G, T);
     if ((rc = done(p))) return rc;
     // the modal products, their fields made again from phig
-    const XinvOp<N> xg{T, W, fs, M, run(M, M), 1, plane, cube};
+    const XinvOp<N> xg{T, W, fs, M, run(0, M), 1, M, p->d_qcube};
     if ((rc = run_pass<N, 0, +1>(p, xg, kTiles * M, st, "grad_xinv"))) return rc;
-    const XinvNatOp<N> xf{{phig, W, fs, M, run(0, M), 1, plane, cube}};
+    const XinvNatOp<N> xf{{phig, W, fs, M, run(0, M), 1, 0, p->d_qcube}};
     if ((rc = run_pass<N, 0, +1>(p, xf, kTiles * M, st, "grad_xinv"))) return rc;
     for (int h = 0; h < 2; ++h)
       if ((rc = L::template axis_pass<1, +1>(p, W, M, run(h * M, M), st, "grad_y"))) return rc;
@@ -1546,7 +1500,7 @@ struct Chain {
     }
     if ((rc = done(p))) return rc;
     if ((rc = L::template axis_pass<1, -1>(p, W, M, run(0, M), st, "grad_y"))) return rc;
-    const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), plane, cube, sc, p->d_amp, gw};
+    const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), p->d_qcube, sc, p->d_amp, gw};
     {
       ProfScope ps_(p, "grad_xacc", st);
       k_xacc<N, true><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);

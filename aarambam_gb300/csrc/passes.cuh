@@ -134,8 +134,8 @@ __device__ __forceinline__ void group_order(unsigned item, unsigned nc, unsigned
 }
 
 // First modal pass: phi tile times q_p(k) (zero on the cut, DC and padding
-// columns), inverse x FFT, into field p, for the modes p = mode.s[c] that the
-// products read.  The factors come from the plan's
+// columns), inverse x FFT, into field dst0 + p, for the modes p = mode.s[c] that
+// the products read.  The factors come from the plan's
 // filter cube (qcube_build), laid out so that a warp's 32 factors of a
 // value index are 4 rows of 8 consecutive floats; they load together with
 // the tile.
@@ -148,20 +148,20 @@ struct XinvOp {
   int nin;
   Slots mode;
   unsigned grp;
-  Slots line;          // a mode's plane of the cube
-  const float* qcube;  // [line][|ky|][kz / 8][|kx|][8]
+  int dst0;
+  const float* qcube;  // [mode][|ky|][kz / 8][|kx|][8]
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     unsigned t;
     group_order<N>(item, (unsigned)nin, grp, t, c);
     tile_coords<N>(t, o, c0);
   }
   __device__ const float2* src(int) const { return phi; }
-  __device__ float2* dst(int c) const { return work + (int64_t)mode.s[c] * fs; }
+  __device__ float2* dst(int c) const { return work + (int64_t)(dst0 + mode.s[c]) * fs; }
   __device__ void pre(float2* v, int o, int kz, int c, int t) const {
     using C = TileCfg<N>;
     constexpr int K = N / 2 + 1;
     const int ay = o <= N / 2 ? o : N - o;
-    const float* q = qcube + ((((int64_t)line.s[c] * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
+    const float* q = qcube + ((((int64_t)mode.s[c] * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
     float f[C::R1];
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) {
@@ -352,7 +352,7 @@ struct XaccArgs {
   const float2* work;
   int64_t fs;
   int nr;
-  Slots slot, line;  // field and cube plane of an active r
+  Slots slot;  // the active r: field and cube plane
   const float* qcube;
   AccScale sc;
   // gradient form (k_xacc<N, true>): gw = amp (phi + w sum) in natural order,
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
   float* qs = reinterpret_cast<float*>(stage + N * C::W);  // two buffers
   auto issue = [&](int s) {
     tile_stage_load<N, 0>(stage, a.work + (int64_t)a.slot.s[s] * a.fs, o, c0);
-    const float* q = qb + a.line.s[s] * plane;
+    const float* q = qb + a.slot.s[s] * plane;
     float* d = qs + (s & 1) * X::QROWS;
     for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
     cp_async_commit();
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
 #pragma unroll
       for (int r = 0; r < C::R1; ++r) v[r] = src[TileMap<N, 0>::off(C::T * r)];
       if (s) __syncthreads();  // the exchange has been read
-      q = qb + a.line.s[s] * plane + w;
+      q = qb + a.slot.s[s] * plane + w;
     }
     tile_fft2<N, -1>(v, ex, t, w, tw2);
 #pragma unroll
