@@ -35,6 +35,7 @@ def _stale(obj: str, src: str) -> bool:
     if not os.path.exists(obj):
         return True
     deps = [src] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    deps += [os.path.join(OUT, f) for f in os.listdir(OUT) if f.endswith(".h")]
     deps.append(os.path.join(os.path.dirname(HERE), "include", "aarambam.h"))
     t = os.path.getmtime(obj)
     return any(os.path.getmtime(d) > t for d in deps)
@@ -51,16 +52,36 @@ def _embed_headers() -> None:
         if ")AARJIT\"" in text:
             raise RuntimeError(name + " contains the raw-string delimiter")
         parts.append("static const char* " + var + " = R\"AARJIT(" + text + ")AARJIT\";\n")
-    new = "".join(parts)
-    old = open(out).read() if os.path.exists(out) else None
-    if new != old:
-        with open(out, "w") as f:
-            f.write(new)
+    _write(out, "".join(parts))
+
+
+def _ranlux_powers() -> None:
+    """_build/ranlux_powers.h: the skip-ahead powers b^{-202 d 256^l} mod m of the
+    seed table (csrc/ranlux.cuh: b = 2^48, m = b^12 - b^5 + 1; nine 64-bit limbs,
+    the lowest first), levels l < 3, digits d < 256.  Constants of the library's
+    image: a plan holds no copy."""
+    b = 1 << 48
+    m = b ** 12 - b ** 5 + 1
+    rows = []
+    for level in range(3):
+        a = pow(b, -202 * 256 ** level, m)
+        v = 1
+        for _ in range(256):
+            rows.append("{{" + ",".join(f"{v >> (64 * i) & (1 << 64) - 1:#x}ull" for i in range(9)) + "}},\n")
+            v = v * a % m
+    _write(os.path.join(OUT, "ranlux_powers.h"), "// generated by build.py\n" + "".join(rows))
+
+
+def _write(path: str, text: str) -> None:
+    if not os.path.exists(path) or open(path).read() != text:
+        with open(path, "w") as f:
+            f.write(text)
 
 
 def build(verbose: bool = False) -> str:
     os.makedirs(OUT, exist_ok=True)
     _embed_headers()
+    _ranlux_powers()
     flags = ["-std=c++20", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
              "-I" + os.path.join(os.path.dirname(HERE), "include"), "-I" + OUT] + ARCH
     procs = []

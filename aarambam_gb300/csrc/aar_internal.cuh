@@ -67,8 +67,8 @@ struct Plan {
   int rtab_stride = 0;
   int64_t nsq = 0;            // 3 (N/2)^2 + 1
   int qtab_m = 0;             // modes the tables were allocated for
-  // field filters over |ky|, kz, |kx|, M (N/2+1)^2 HP floats (qcube_build); made
-  // on first use after each table change
+  // field filters over |ky|, kz, |kx|, M (N/2+1)^3 floats (qcube_build); made on
+  // first use after each table change
   float* d_qcube = nullptr;
   int qcube_m = 0;
   bool qcube_stale = true;
@@ -80,7 +80,6 @@ struct Plan {
   size_t chain_bytes = 0;
   int chain_nent = 0, chain_ngrp = 0;
   bool chain_stale = true;
-  void* d_rlxpow = nullptr;   // skip-ahead powers (seedtable_powers)
   std::vector<char> host_terms;  // the modal term list (a TermList, then its Terms)
   void* jit = nullptr;           // run-time specialised modal row kernel (jit.cu), or null
   int jit_mode = 1;              // 0 off, 1 for N >= 256, 2 always
@@ -160,8 +159,6 @@ const char* set_err(Plan* p, const std::string& e);
 
 // launchers (return 0 or an error code; errors leave a message on the plan)
 int launch_seedtable(Plan* p, uint32_t* d_out, cudaStream_t st);
-struct U576;
-void seedtable_powers(std::vector<U576>& pw);
 int launch_noise_fp32(Plan* p, const uint32_t* d_seed, float2* d_phik, cudaStream_t st);
 int launch_noise_fp64(Plan* p, const uint32_t* d_seed, double2* d_phik, int hp, cudaStream_t st);
 int fused_prepare(Plan* p);

@@ -16,7 +16,6 @@
 #include <vector>
 
 #include "aar_internal.cuh"
-#include "ranlux.cuh"
 #include "spectral.cuh"
 
 struct aar_plan {
@@ -249,14 +248,13 @@ static void plan_release(Plan* p) {
   p->prof.clear();
   for (auto e : p->event_pool) cudaEventDestroy(e);
   p->event_pool.clear();
-  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_rlxpow, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_tcube, p->d_chain};
+  void* ptrs[] = {p->d_phik, p->d_work, p->d_seed, p->d_twN, p->d_twH, p->d_tw2, p->d_amp, p->d_twb, p->d_io, p->d_qtab, p->d_rtab, p->d_sinc, p->d_isinc2, p->d_adj_scratch, p->d_qcube, p->d_tcube, p->d_chain};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   p->d_phik = p->d_work = nullptr;
   p->d_seed = nullptr;
   p->d_twN = p->d_twH = p->d_tw2 = nullptr;
   p->d_amp = p->d_twb = nullptr;
-  p->d_rlxpow = nullptr;
   p->d_qtab = p->d_rtab = nullptr;
   p->d_sinc = p->d_isinc2 = nullptr;
   p->d_qcube = p->d_tcube = nullptr;
@@ -424,12 +422,6 @@ static int create(Plan* p) {
 
   int rc;
   if ((rc = plan_alloc(p, (void**)&p->d_seed, sizeof(uint32_t) * (size_t)N * N))) return rc;
-  {
-    std::vector<U576> pw;  // ranlux skip-ahead
-    seedtable_powers(pw);
-    if ((rc = plan_alloc(p, &p->d_rlxpow, sizeof(U576) * pw.size()))) return rc;
-    if (int rc_ = upload(p, p->d_rlxpow, pw.data(), sizeof(U576) * pw.size())) return rc_;
-  }
   if (is_fp32(q)) {
     std::vector<float2> twN(N), twH(N / 2);
     for (int m = 0; m < N; ++m) {

@@ -713,7 +713,7 @@ struct Launch {
     const int64_t fs = fstride(p);
     const TermList& tl = terms(p);
     const Slots in = slots(tl.in_mode, tl.nin), out = slots(tl.r_of_slot, tl.nr);
-    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), 0, p->d_qcube};
+    XinvOp<N> xo{p->d_phik, p->d_work, fs, tl.nin, in, group(p), 0, p->M, p->d_qcube};
     int rc = run_pass<N, 0, +1>(p, xo, kTiles * tl.nin, st, "modal_xinv");
     if (rc) return rc;
     if ((rc = axis_pass<1, +1>(p, p->d_work, tl.nin, in, st, "modal_ypass_inv"))) return rc;
@@ -726,12 +726,11 @@ struct Launch {
     // (0.0122 against 0.0132 ms at 128^3)
     if constexpr (TileCfg<N>::R1 == 32) {
       if (tl.nr == 1) {
-        const int64_t plane = (int64_t)(N / 2 + 1) * p->HP * (N / 2 + 1);
-        const XaddOp<N> xo1{a.g, p->d_phik, p->d_work + out.s[0] * fs, p->d_qcube + out.s[0] * plane, sc};
+        const XaddOp<N> xo1{a.g, p->d_phik, p->d_work + out.s[0] * fs, out.s[0], p->M, p->d_qcube, sc};
         return run_pass<N, 0, -1>(p, xo1, kTiles, st, "modal_xacc");
       }
     }
-    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, p->d_qcube, sc, nullptr, nullptr};
+    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, p->M, p->d_qcube, sc, nullptr, nullptr};
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XaccCfg<N>::SMEM));
     {
       ProfScope ps_(p, "modal_xacc", st);
@@ -952,29 +951,26 @@ static int build_terms(Plan* p) {
 
 // The filter cube of the modal passes: the plan's per-|k|^2 filters
 // (mode_tables: FP64 formulas rounded once to float) over 0 <= |kx|, |ky| <=
-// N/2 and the padded kz columns, zero on the cut, at k = 0 and on the padding
-// (keep_cell depends on |k_a| only).  Index (((p K + |ky|) NCOL + kz / 8) K +
-// |kx|) 8 + kz % 8, p the mode, K = N/2 + 1, NCOL = HP / 8.  Every mode has its
+// N/2 and 0 <= kz <= N/2, zero on the cut and at k = 0 (keep_cell depends on
+// |k_a| only), in the order of CubeMap (passes.cuh), p the mode.  Every mode has its
 // plane, read by a term or not: the products' gradients take them all, and the
 // cube keeps its address while the mode count does.
 __global__ void __launch_bounds__(256) k_qcube(Grid g, int M, const float* __restrict__ qtab, int64_t nsq,
                                                float* __restrict__ q) {
-  const int K = g.N / 2 + 1, ncol = g.HP / 8;
-  const int64_t per = (int64_t)K * g.HP * K;
+  const CubeMap cm{g.N / 2 + 1, M};
+  const int64_t per = (int64_t)cm.K * cm.K * cm.K;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / 8;
-    const int ax = (int)(r % K);
-    const int64_t s = r / K;
-    const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
+    int ax, ay, kz;
+    cm.cell(i, ax, ay, kz);
     const int n2 = ax * ax + ay * ay + kz * kz;
-    const bool on = kz <= g.N / 2 && n2 != 0 && keep_cell(g, ax, ay, kz);
-    for (int c = 0; c < M; ++c) q[(int64_t)c * per + i] = on ? __ldg(qtab + (int64_t)c * nsq + n2) : 0.f;
+    const bool on = n2 != 0 && keep_cell(g, ax, ay, kz);
+    for (int c = 0; c < M; ++c) q[cm.at(c, ay, kz, ax)] = on ? __ldg(qtab + (int64_t)c * nsq + n2) : 0.f;
   }
 }
 
 int qcube_build(Plan* p) {
   if (!p->have_tables || (!p->qcube_stale && p->d_qcube)) return AAR_OK;  // no tables yet: nothing reads filters
-  const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
+  const int64_t K = p->N / 2 + 1, per = K * K * K;
   if (!p->d_qcube || p->qcube_m != p->M) {
     if (p->d_qcube) {
       AAR_CUDA_TRY(p, cudaDeviceSynchronize());
@@ -996,28 +992,26 @@ int qcube_build(Plan* p) {
 }
 
 // The transfer cube of the 2LPT x passes: T/(D Beta) in the filter cube's
-// layout, no cut, zero on the padding columns.  It takes an eighth of a field
+// layout, no cut.  It takes an eighth of a field
 // that a caller's memory limit does not know of, so plans with a limit, and
 // those whose device has no room, read the per-|n|^2 table in its place.
-__global__ void __launch_bounds__(256) k_tcube(Grid g, const float* __restrict__ twb, float* __restrict__ q) {
-  const int K = g.N / 2 + 1, ncol = g.HP / 8;
-  const int64_t per = (int64_t)K * g.HP * K;
+__global__ void __launch_bounds__(256) k_tcube(int K, const float* __restrict__ twb, float* __restrict__ q) {
+  const CubeMap cm{K, 1};
+  const int64_t per = (int64_t)K * K * K;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / 8;
-    const int ax = (int)(r % K);
-    const int64_t s = r / K;
-    const int kz = (int)(s % ncol) * 8 + (int)(i % 8), ay = (int)(s / ncol);
-    q[i] = kz <= g.N / 2 ? __ldg(twb + ax * ax + ay * ay + kz * kz) : 0.f;
+    int ax, ay, kz;
+    cm.cell(i, ax, ay, kz);
+    q[cm.at(0, ay, kz, ax)] = __ldg(twb + ax * ax + ay * ay + kz * kz);
   }
 }
 
 int tcube_build(Plan* p) {
   if (!p->tcube_stale || !p->have_transfer) return AAR_OK;
-  const int64_t K = p->N / 2 + 1, per = K * p->HP * K;
+  const int64_t K = p->N / 2 + 1, per = K * K * K;
   p->tcube_stale = false;
   if (p->prm.mem_limit_bytes > 0) return AAR_OK;
   if (!p->d_tcube && plan_alloc(p, (void**)&p->d_tcube, sizeof(float) * (size_t)per)) return AAR_OK;
-  k_tcube<<<(unsigned)(p->num_sms * 8), 256>>>(p->grid, p->d_twb, p->d_tcube);
+  k_tcube<<<(unsigned)(p->num_sms * 8), 256>>>((int)K, p->d_twb, p->d_tcube);
   AAR_CUDA_TRY(p, cudaGetLastError());
   AAR_CUDA_TRY(p, cudaDeviceSynchronize());  // as qcube_build
   return AAR_OK;
@@ -1453,9 +1447,9 @@ struct Chain {
     k_chain_hess<N><<<cells(p), 256, 0, st>>>(a, W, fs, sc, G, T);
     if ((rc = done(p))) return rc;
     // the modal products, their fields made again from phig
-    const XinvOp<N> xg{T, W, fs, M, run(0, M), 1, M, p->d_qcube};
+    const XinvOp<N> xg{T, W, fs, M, run(0, M), 1, M, M, p->d_qcube};
     if ((rc = run_pass<N, 0, +1>(p, xg, kTiles * M, st, "grad_xinv"))) return rc;
-    const XinvNatOp<N> xf{{phig, W, fs, M, run(0, M), 1, 0, p->d_qcube}};
+    const XinvNatOp<N> xf{{phig, W, fs, M, run(0, M), 1, 0, M, p->d_qcube}};
     if ((rc = run_pass<N, 0, +1>(p, xf, kTiles * M, st, "grad_xinv"))) return rc;
     for (int h = 0; h < 2; ++h)
       if ((rc = L::template axis_pass<1, +1>(p, W, M, run(h * M, M), st, "grad_y"))) return rc;
@@ -1500,7 +1494,7 @@ struct Chain {
     }
     if ((rc = done(p))) return rc;
     if ((rc = L::template axis_pass<1, -1>(p, W, M, run(0, M), st, "grad_y"))) return rc;
-    const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), p->d_qcube, sc, p->d_amp, gw};
+    const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), M, p->d_qcube, sc, p->d_amp, gw};
     {
       ProfScope ps_(p, "grad_xacc", st);
       k_xacc<N, true><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);

@@ -58,12 +58,15 @@ __device__ __forceinline__ int shell_pos(int d, int N) {
 // digits; the binary powers took up to 17), and a thread does one refill.
 // N = 64 0.023 ms, N = 1024 0.065 ms; with 8 refills per thread, seeding on
 // the device and binary powers 0.137 and 0.161 ms.
+static __device__ const U576 kSkip[kRlxLevels * kRlxRadix] = {
+#include "ranlux_powers.h"  // level l, digit d: b^{-202 d 256^l} mod m (generated by build.py)
+};
 struct SeedStart {
   Rlx s;   // the seeded state
   U576 r;  // its residue
 };
 __global__ void __launch_bounds__(32) k_seedtable(const __grid_constant__ SeedStart st, int N,
-                                                  const U576* __restrict__ pw, uint32_t* __restrict__ table) {
+                                                  uint32_t* __restrict__ table) {
   const int g = blockIdx.x * 32 + threadIdx.x;
   const int total = N * N, d0 = 12 * g;
   if (d0 >= total) return;
@@ -73,7 +76,7 @@ __global__ void __launch_bounds__(32) k_seedtable(const __grid_constant__ SeedSt
   } else {
     U576 r = st.r;
     for (int l = 0, h = g; h; ++l, h >>= 8)
-      if (h & 255) r = modmul576(r, pw[l * kRlxRadix + (h & 255)]);
+      if (h & 255) r = modmul576(r, kSkip[l * kRlxRadix + (h & 255)]);
     rlx_from_residue(r, s);
   }
   rlx_refill(s);
@@ -85,23 +88,12 @@ __global__ void __launch_bounds__(32) k_seedtable(const __grid_constant__ SeedSt
   }
 }
 
-// Table of the skip-ahead powers, level l, digit d: b^{-202 d 256^l} mod m.
-void seedtable_powers(std::vector<U576>& pw) {
-  static_assert(kRlxRadix == 256 && kRlxLevels == 3, "the threads' numbers have three base-256 digits");
-  pw.assign(kRlxLevels * kRlxRadix, u576_one());
-  U576 a = modpow576(u576_binv(), (uint64_t)kRlxLux);
-  for (int l = 0; l < kRlxLevels; ++l) {
-    for (int d = 1; d < kRlxRadix; ++d) pw[l * kRlxRadix + d] = modmul576(pw[l * kRlxRadix + d - 1], a);
-    a = modmul576(pw[l * kRlxRadix + kRlxRadix - 1], a);
-  }
-}
-
 static void run_seedtable(Plan* p, uint32_t* d_out, cudaStream_t st) {
   SeedStart s0;
   rlx_seed(s0.s, (uint32_t)p->prm.seed);
   s0.r = rlx_window_residue(s0.s);
   const int64_t nthr = ((int64_t)p->N * p->N + 11) / 12;
-  k_seedtable<<<(unsigned)((nthr + 31) / 32), 32, 0, st>>>(s0, p->N, (const U576*)p->d_rlxpow, d_out);
+  k_seedtable<<<(unsigned)((nthr + 31) / 32), 32, 0, st>>>(s0, p->N, d_out);
 }
 
 int launch_seedtable(Plan* p, uint32_t* d_out, cudaStream_t st) {

@@ -133,12 +133,62 @@ __device__ __forceinline__ void group_order(unsigned item, unsigned nc, unsigned
   t = g * grp + (r - (unsigned)c * gs);
 }
 
+// Order of a cube of per-cell factors over |kx|, |ky|, kz <= N/2 (K = N/2 + 1
+// each), `planes` of them: the columns kz < N/2 as [p][|ky|][kz / 8][|kx|][8], so
+// that a warp's factors of a value index are 4 rows of 8 consecutive floats on
+// 32-byte boundaries, then the columns kz = N/2 as [p][|ky|][|kx|].  (With that
+// column padded to a block of its own a cube took 1.4 % more at N = 1024, 21 %
+// at 64, which a plan's memory limit may not have.)
+struct CubeMap {
+  int K, planes;
+  __host__ __device__ __forceinline__ int64_t at(int p, int ay, int kz, int ax) const {
+    const int NB = (K - 1) / 8;
+    const int64_t row = (int64_t)p * K + ay;
+    return kz < K - 1 ? ((row * NB + kz / 8) * K + ax) * 8 + kz % 8 : ((int64_t)planes * K * NB * 8 + row) * K + ax;
+  }
+  // the cell of index i < K^3 of a one-plane cube
+  __host__ __device__ __forceinline__ void cell(int64_t i, int& ax, int& ay, int& kz) const {
+    const int NB = (K - 1) / 8;
+    const int64_t blocks = (int64_t)K * NB * K * 8;
+    if (i < blocks) {
+      const int64_t r = i / 8, s = r / K;
+      ax = (int)(r % K), kz = (int)(s % NB) * 8 + (int)(i % 8), ay = (int)(s / NB);
+    } else {
+      ax = (int)((i - blocks) % K), kz = K - 1, ay = (int)((i - blocks) / K);
+    }
+  }
+};
+
+// A thread's factors f[i] at kx of line value i, |ky| = ay and column kz of
+// plane p; zero on the padding columns.
+template <int N>
+__device__ __forceinline__ void cube_load(float* f, const float* __restrict__ cube, int planes, int p, int ay, int kz,
+                                          int t) {
+  using C = TileCfg<N>;
+  const float* q = cube + CubeMap{N / 2 + 1, planes}.at(p, ay, min(kz, N / 2), 0);
+  auto load = [&](auto step) {
+#pragma unroll
+    for (int i = 0; i < C::R1; ++i) {
+      // value i < R1 / 2 has kx = t + T i < N / 2, the others |kx| = N - n
+      const int n = tile_n<N>(t, i);
+      f[i] = __ldg(q + (i < C::R1 / 2 ? n : N - n) * decltype(step)::value);
+    }
+  };
+  if (kz < N / 2) {
+    load(std::integral_constant<int, 8>{});
+  } else {
+    load(std::integral_constant<int, 1>{});
+    if (kz > N / 2) {
+#pragma unroll
+      for (int i = 0; i < C::R1; ++i) f[i] = 0.f;
+    }
+  }
+}
+
 // First modal pass: phi tile times q_p(k) (zero on the cut, DC and padding
 // columns), inverse x FFT, into field dst0 + p, for the modes p = mode.s[c] that
 // the products read.  The factors come from the plan's
-// filter cube (qcube_build), laid out so that a warp's 32 factors of a
-// value index are 4 rows of 8 consecutive floats; they load together with
-// the tile.
+// filter cube (qcube_build); they load together with the tile.
 template <int N>
 struct XinvOp {
   static constexpr bool kPre = true, kPost = false;
@@ -148,8 +198,8 @@ struct XinvOp {
   int nin;
   Slots mode;
   unsigned grp;
-  int dst0;
-  const float* qcube;  // [mode][|ky|][kz / 8][|kx|][8]
+  int dst0, planes;
+  const float* qcube;
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     unsigned t;
     group_order<N>(item, (unsigned)nin, grp, t, c);
@@ -159,16 +209,8 @@ struct XinvOp {
   __device__ float2* dst(int c) const { return work + (int64_t)(dst0 + mode.s[c]) * fs; }
   __device__ void pre(float2* v, int o, int kz, int c, int t) const {
     using C = TileCfg<N>;
-    constexpr int K = N / 2 + 1;
-    const int ay = o <= N / 2 ? o : N - o;
-    const float* q = qcube + ((((int64_t)mode.s[c] * K + ay) * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
     float f[C::R1];
-#pragma unroll
-    for (int i = 0; i < C::R1; ++i) {
-      // value i < R1 / 2 has kx = t + T i < N / 2, the others |kx| = N - n
-      const int n = tile_n<N>(t, i);
-      f[i] = __ldg(q + (i < C::R1 / 2 ? n : N - n) * C::W);
-    }
+    cube_load<N>(f, qcube, planes, mode.s[c], o <= N / 2 ? o : N - o, kz, t);
 #pragma unroll
     for (int i = 0; i < C::R1; ++i) v[i] = cscale(v[i], f[i]);
   }
@@ -205,7 +247,7 @@ struct LptXOp {
   unsigned grp;
   float kF;
   const float* isinc2;
-  const float* tcube;  // [|ky|][kz / 8][|kx|][8], zero on the padding columns; null: twb by |n|^2
+  const float* tcube;  // one plane; null: twb by |n|^2
   const float* twb;
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     unsigned t;
@@ -216,20 +258,20 @@ struct LptXOp {
   __device__ float2* dst(int c) const { return work + (int64_t)out[c] * fs; }
   __device__ void pre(float2* v, int o, int kz, int c, int t) const {
     using C = TileCfg<N>;
-    constexpr int K = N / 2 + 1;
     const int ay = o <= N / 2 ? o : N - o;
-    const float* q = tcube + (((int64_t)ay * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
     const bool psi2 = KIND == 1 && c >= 2;
     float f[C::R1];
     if (psi2 || kz > N / 2) {
 #pragma unroll
       for (int i = 0; i < C::R1; ++i) f[i] = kz <= N / 2 ? 1.f : 0.f;
+    } else if (tcube) {
+      cube_load<N>(f, tcube, 1, 0, ay, kz, t);
     } else {
       const int b = ay * ay + kz * kz;
 #pragma unroll
       for (int i = 0; i < C::R1; ++i) {
         const int n = tile_n<N>(t, i), ax = i < C::R1 / 2 ? n : N - n;
-        f[i] = tcube ? __ldg(q + ax * C::W) : __ldg(twb + b + ax * ax);
+        f[i] = __ldg(twb + b + ax * ax);
       }
     }
 #pragma unroll
@@ -353,6 +395,7 @@ struct XaccArgs {
   int64_t fs;
   int nr;
   Slots slot;  // the active r: field and cube plane
+  int planes;
   const float* qcube;
   AccScale sc;
   // gradient form (k_xacc<N, true>): gw = amp (phi + w sum) in natural order,
@@ -365,7 +408,7 @@ struct XaccCfg {
   using C = TileCfg<N>;
   static constexpr bool kStaged = N >= 256;
   static constexpr int K = N / 2 + 1;
-  static constexpr size_t QROWS = (size_t)K * C::W;  // floats of a plane's column block
+  static constexpr size_t QROWS = (size_t)K * C::W;  // floats of a plane's block of columns
   static constexpr size_t SMEM = C::SMEM + (kStaged ? sizeof(float2) * N * C::W + 2 * sizeof(float) * QROWS : 0);
   static constexpr int MINB = C::R1 == 32 ? 256 / C::THREADS : C::R1 == 16 ? 512 / C::THREADS : 8;
 };
@@ -380,15 +423,21 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
   tile_coords<N>(blockIdx.x, o, c0);
   const int64_t base = TileMap<N, 0>(o, c0, t, w).base;
   const int ay = o <= N / 2 ? o : N - o;
-  const float* qb = a.qcube + ((int64_t)ay * C::NCOL + c0 / C::W) * X::QROWS;
-  constexpr int64_t plane = (int64_t)X::K * C::NCOL * X::QROWS;
+  // a block of eight columns, or (last) the column kz = N/2 alone: the sums of
+  // the padding columns beside it are not stored
+  const bool last = c0 == N / 2;
+  const int qw = last ? 0 : w;
+  auto qplane = [&](int s) { return a.qcube + CubeMap{X::K, a.planes}.at(a.slot.s[s], ay, c0, 0); };
   float2* stage = ex + C::SMEM / sizeof(float2);
   float* qs = reinterpret_cast<float*>(stage + N * C::W);  // two buffers
   auto issue = [&](int s) {
     tile_stage_load<N, 0>(stage, a.work + (int64_t)a.slot.s[s] * a.fs, o, c0);
-    const float* q = qb + a.slot.s[s] * plane;
+    const float* q = qplane(s);
     float* d = qs + (s & 1) * X::QROWS;
-    for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
+    if (last)
+      for (int i = threadIdx.x; i < X::K; i += C::THREADS) cp_async4(d + C::W * i, q + i);
+    else
+      for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
     cp_async_commit();
   };
   float2 sum[C::R1], cmp[C::R1];
@@ -406,13 +455,13 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       for (int r = 0; r < C::R1; ++r) v[r] = stage[tile_n<N>(t, r) * C::W + w];
       __syncthreads();  // the stage is free, and the exchange of the slot before has been read
       if (s + 1 < a.nr) issue(s + 1);
-      q = qs + (s & 1) * X::QROWS + w;
+      q = qs + (s & 1) * X::QROWS + qw;
     } else {
       const float2* src = a.work + (int64_t)a.slot.s[s] * a.fs + base;
 #pragma unroll
       for (int r = 0; r < C::R1; ++r) v[r] = src[TileMap<N, 0>::off(C::T * r)];
       if (s) __syncthreads();  // the exchange has been read
-      q = qb + a.slot.s[s] * plane + w;
+      q = qplane(s) + qw;
     }
     tile_fft2<N, -1>(v, ex, t, w, tw2);
 #pragma unroll
@@ -420,7 +469,8 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
 #pragma unroll
       for (int r = 0; r < C::R2; ++r) {
         const int i = tile_out_i<N>(b, r), n = tile_n<N>(t, i);
-        const float f = q[(i < C::R1 / 2 ? n : N - n) * C::W];
+        const int ax = i < C::R1 / 2 ? n : N - n;
+        const float f = q[X::kStaged || !last ? ax * C::W : ax];
         two_sum2(sum[i], cmp[i], cscale(v[b * C::R2 + r], f));
       }
   }
@@ -458,7 +508,8 @@ struct XaddOp {
   Grid g;
   float2* phi;
   const float2* slot;
-  const float* q;  // the cube's plane of r
+  int r, planes;
+  const float* qcube;
   AccScale sc;
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     tile_coords<N>(item, o, c0);
@@ -468,9 +519,9 @@ struct XaddOp {
   __device__ float2* dst(int) const { return phi; }
   __device__ void post(float2* v, int o, int kz, int, int t) const {
     using C = TileCfg<N>;
-    constexpr int K = N / 2 + 1;
     const int ay = o <= N / 2 ? o : N - o, ky = sidx(o, N);
-    const float* qb = q + (((int64_t)ay * C::NCOL + kz / C::W) * K) * C::W + kz % C::W;
+    const float* qb = qcube + CubeMap{N / 2 + 1, planes}.at(r, ay, min(kz, N / 2), 0);
+    const int step = kz < N / 2 ? C::W : 1;
     const float2* ph = phi + TileMap<N, 0>(o, kz, t, 0).base;
     constexpr int H = 8 < C::R1 ? 8 : C::R1;  // values whose loads go out together
 #pragma unroll
@@ -481,7 +532,7 @@ struct XaddOp {
       for (int j = 0; j < H; ++j) {
         const int i = h + j, n = tile_n<N>(t, i);
         u[j] = ph[TileMap<N, 0>::off(C::T * i)];
-        f[j] = __ldg(qb + (i < C::R1 / 2 ? n : N - n) * C::W);
+        f[j] = __ldg(qb + (i < C::R1 / 2 ? n : N - n) * step);
       }
 #pragma unroll
       for (int j = 0; j < H; ++j) {

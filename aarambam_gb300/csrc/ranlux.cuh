@@ -31,7 +31,7 @@ namespace aar {
 
 constexpr int kRlxLux = 202;  // ranlxd1
 // skip-ahead powers: kRlxLevels base-kRlxRadix digits of the refill number
-// (Nmesh <= 4096: N^2 / 12 refills < 2^24)
+// (Nmesh <= 4096: N^2 / 12 refills < 2^24); build.py makes the table
 constexpr int kRlxRadix = 256, kRlxLevels = 3;
 constexpr uint64_t kMask48 = (uint64_t(1) << 48) - 1;
 
@@ -314,40 +314,6 @@ AAR_HD void rlx_from_residue(const U576& R, Rlx& s) {
   // x_{t+12} = x_{t+7} - x_t - c_{t+11} + b c_{t+12}  =>  c_{t+11} = (x_{t+7} - x_t - x_{t+12}) mod b
   s.carry = (uint32_t)((dig[7] - dig[0] - dig[12]) & kMask48);
   s.pos = 12;
-}
-
-// b^{-1} mod m = m - b^11 + b^4  (b (b^11 - b^4) = b^12 - b^5 = -1 mod m)
-AAR_HD U576 u576_binv() {
-  U576 m = u576_m();
-  uint64_t mm[10], t[10] = {0}, r[10];
-  for (int i = 0; i < 9; ++i) mm[i] = m.w[i];
-  mm[9] = 0;
-  // b^11 = 2^528: limb 8 bit 16; b^4 = 2^192: limb 3 bit 0
-  t[8] = uint64_t(1) << 16;
-  limbs_sub(r, mm, t, 10);
-  uint64_t b4[10] = {0};
-  b4[3] = 1;
-  limbs_add(r, r, b4, 10);
-  U576 o;
-  for (int i = 0; i < 9; ++i) o.w[i] = r[i];
-  return o;
-}
-
-AAR_HD U576 u576_one() {
-  U576 o;
-  for (int i = 0; i < 9; ++i) o.w[i] = 0;
-  o.w[0] = 1;
-  return o;
-}
-
-AAR_HD U576 modpow576(U576 a, uint64_t e) {
-  U576 r = u576_one();
-  while (e) {
-    if (e & 1) r = modmul576(r, a);
-    a = modmul576(a, a);
-    e >>= 1;
-  }
-  return r;
 }
 
 }  // namespace aar
