@@ -63,8 +63,7 @@ struct Plan {
   float* d_sinc = nullptr;    // per grid index: CIC window sin(x)/x
   float* d_isinc2 = nullptr;  // per grid index: 1 / (sin(x)/x)^2
   float* d_qtab = nullptr;    // [M][nsq] field filters q_p per n^2
-  float* d_rtab = nullptr;    // [nsq][rtab_stride] radial parts rho_r per n^2 (r fastest)
-  int rtab_stride = 0;
+  float* d_rtab = nullptr;    // [M][nsq] radial parts rho_r per n^2
   int64_t nsq = 0;            // 3 (N/2)^2 + 1
   int qtab_m = 0;             // modes the tables were allocated for
   // field filters over |ky|, kz, |kx|, M (N/2+1)^3 floats (qcube_build); made on

@@ -30,9 +30,8 @@ struct SpecArgs {
   LptArgs l;
   const float* amp;   // per n^2 noise amplitude
   const float* qtab;  // [M][nsq]
-  const float* rtab;  // [nsq][rstride]
+  const float* rtab;  // [M][nsq]
   int64_t nsq;
-  int rstride;
   float fnl_n3;       // Fnl / N^3
 };
 
@@ -57,7 +56,7 @@ __device__ __forceinline__ float2 spec_factor(const SpecArgs& s, int op, int com
     }
     case AAR_ADJ_OP_RHO: {
       const bool on = n2 != 0 && keep_cell(g, kx, ky, kz);
-      return make_float2(on ? s.fnl_n3 * __ldg(s.rtab + (int64_t)n2 * s.rstride + comp) : 0.f, 0.f);
+      return make_float2(on ? s.fnl_n3 * __ldg(s.rtab + (int64_t)comp * s.nsq + n2) : 0.f, 0.f);
     }
     case AAR_ADJ_OP_HESS:
       return lpt_factor<0>(s.l, comp, i, j, kz, kx, ky, n2);
@@ -174,7 +173,6 @@ static SpecArgs spec_args(Plan* p) {
   s.qtab = p->d_qtab;
   s.rtab = p->d_rtab;
   s.nsq = p->nsq;
-  s.rstride = p->rtab_stride;
   s.fnl_n3 = (float)(p->prm.fnl / ((double)p->N * p->N * p->N));
   return s;
 }

@@ -326,9 +326,8 @@ static int alloc_fused(Plan* p, int M) {
 //                                         (P_{n-1}(kbar) - X0[n-1]) k^{2-ns}
 //   rho_n (radial part, main.c:833-860):  k^{s(n-3)} (n <= 3),  (P_{n-1}(kbar) - X0[n-1]) / k^2
 // with s = (4-ns)/3, kbar = -1 + 2 (k^s - kmin^s)/(kmax^s - kmin^s).
-// q is stored per mode ([M][nsq]: a filter pass reads one mode); rho per
-// |k|^2 ([nsq][rtab_stride], mode fastest: the accumulation reads every mode
-// of one cell, a few sectors instead of one per mode).
+// Both are stored per mode ([M][nsq]): a filter pass reads one mode's q, the
+// accumulation rho_0 = k^(ns-4) or one slot's rho.
 static int mode_tables(Plan* p) {
   int N = p->N, M = p->M;
   int64_t nsq = 3LL * (N / 2) * (N / 2) + 1;
@@ -336,12 +335,11 @@ static int mode_tables(Plan* p) {
     // reuse the allocation
   } else {
     if (p->d_qtab) cudaFree(p->d_qtab), p->used_bytes -= sizeof(float) * p->nsq * p->qtab_m;
-    if (p->d_rtab) cudaFree(p->d_rtab), p->used_bytes -= sizeof(float) * p->nsq * p->rtab_stride;
+    if (p->d_rtab) cudaFree(p->d_rtab), p->used_bytes -= sizeof(float) * p->nsq * p->qtab_m;
     p->d_qtab = p->d_rtab = nullptr;
     int rc;
     if ((rc = plan_alloc(p, (void**)&p->d_qtab, sizeof(float) * nsq * M))) return rc;
-    p->rtab_stride = (M + 3) / 4 * 4;
-    if ((rc = plan_alloc(p, (void**)&p->d_rtab, sizeof(float) * nsq * p->rtab_stride))) return rc;
+    if ((rc = plan_alloc(p, (void**)&p->d_rtab, sizeof(float) * nsq * M))) return rc;
     p->qtab_m = M;
   }
   p->nsq = nsq;
@@ -349,8 +347,7 @@ static int mode_tables(Plan* p) {
   const double kmin = 2 * kPi / box, kmax = 2 * kPi / box * p->prm.nmax;
   const double sx = (4 - ns) / 3, kmin_ns = pow(kmin, sx), kmax_ns = pow(kmax, sx);
   const double kF = 2 * kPi / box;
-  const int rs = p->rtab_stride;
-  std::vector<float> qt((size_t)nsq * M), rt((size_t)nsq * rs, 0.f);
+  std::vector<float> qt((size_t)nsq * M), rt((size_t)nsq * M);
   std::vector<double> P(std::max(M, 2));
   for (int64_t n2 = 1; n2 < nsq; ++n2) {
     double k1 = kF * sqrt((double)n2), k2 = k1 * k1;
@@ -371,10 +368,10 @@ static int mode_tables(Plan* p) {
         in = d * p2n;
       }
       qt[(size_t)n * nsq + n2] = (float)in;
-      rt[(size_t)n2 * rs + n] = (float)out;
+      rt[(size_t)n * nsq + n2] = (float)out;
     }
   }
-  for (int n = 0; n < M; ++n) qt[(size_t)n * nsq] = 0.f;
+  for (int n = 0; n < M; ++n) qt[(size_t)n * nsq] = rt[(size_t)n * nsq] = 0.f;
   if (int rc_ = upload(p, p->d_qtab, qt.data(), sizeof(float) * qt.size())) return rc_;
   if (int rc_ = upload(p, p->d_rtab, rt.data(), sizeof(float) * rt.size())) return rc_;
   return AAR_OK;

@@ -180,10 +180,11 @@ struct XSumOp {
 };
 
 // G -= w kF^2 T/(D Beta) (kx^2 P + kx Q + R), the Hessians' gradients P, Q, R
-// (fields 0, 1, 3 of X), and T = k^(ns - 4) Fnl / N^3 G / w: what the filters
-// q_r take to the gradients of the products g_r.
+// (fields 0, 1, 3 of X), and T = rho_0 Fnl / N^3 G / w, rho_0 = k^(ns - 4): what
+// the filters q_r take to the gradients of the products g_r (XinvGradOp).
 template <int N>
-__global__ void __launch_bounds__(256) k_chain_hess(LptArgs a, const float2* __restrict__ X, int64_t fs, AccScale sc,
+__global__ void __launch_bounds__(256) k_chain_hess(LptArgs a, const float2* __restrict__ X, int64_t fs,
+                                                    const float* __restrict__ rho0, float fnl_n3,
                                                     float2* __restrict__ G, float2* __restrict__ T) {
   constexpr int64_t total = (int64_t)N * N * (N / 2 + 1);
   const float kF = a.m.g.kF;
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(256) k_chain_hess(LptArgs a, const float2* __r
     g.x = fmaf(f, fmaf(fx, fmaf(fx, P.x, Q.x), R.x), g.x);
     g.y = fmaf(f, fmaf(fx, fmaf(fx, P.y, Q.y), R.y), g.y);
     G[e] = g;
-    const float s = n2 ? sc.at(n2) / w : 0.f;
+    const float s = fnl_n3 * __ldg(rho0 + n2) / w;  // 0 at k = 0
     T[e] = cscale(g, s);
   }
 }

@@ -719,18 +719,26 @@ struct Launch {
     if ((rc = axis_pass<1, +1>(p, p->d_work, tl.nin, in, st, "modal_ypass_inv"))) return rc;
     if ((rc = p->jit ? jit_modal_rows(p, p->d_work, fs, st) : modal_rows(p, p->d_work, fs, (int64_t)N * N, st))) return rc;
     if ((rc = axis_pass<1, -1>(p, p->d_work, tl.nr, out, st, "modal_ypass_fwd"))) return rc;
-    const RhoArgs ra = rho_args(p);
-    const AccScale sc{(float)(p->prm.primordial_index - 4), ra.log2kF, (float)(p->prm.fnl / ((double)N * N * N))};
+    const float fnl_n3 = (float)(p->prm.fnl / ((double)N * N * N));
     // one slot: 2.83 ms against k_xacc's 4.39 at 1024^3, whose registers leave
     // one block per SM; with 16 values per lane and fewer k_xacc is as fast
     // (0.0122 against 0.0132 ms at 128^3)
     if constexpr (TileCfg<N>::R1 == 32) {
       if (tl.nr == 1) {
-        const XaddOp<N> xo1{a.g, p->d_phik, p->d_work + out.s[0] * fs, out.s[0], p->M, p->d_qcube, sc};
-        return run_pass<N, 0, -1>(p, xo1, kTiles, st, "modal_xacc");
+        const int r = out.s[0];
+        auto add = [&](auto one) {
+          const XaddOp<N, decltype(one)::value> xo1{a.g, p->d_phik, p->d_work + r * fs, p->d_rtab + r * p->nsq, fnl_n3};
+          return run_pass<N, 0, -1>(p, xo1, kTiles, st, "modal_xacc");
+        };
+        return r == 3 ? add(std::true_type{}) : add(std::false_type{});
       }
     }
-    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, out, p->M, p->d_qcube, sc, nullptr, nullptr};
+    Slots order{};  // r = 3 last
+    int nw = 0;
+    for (int i = 0; i < tl.nr; ++i)
+      if (out.s[i] != 3) order.s[nw++] = out.s[i];
+    if (nw < tl.nr) order.s[nw] = 3;
+    const XaccArgs<N> xa{a.g, p->d_phik, p->d_work, fs, tl.nr, nw, order, p->M, p->d_qcube, p->d_rtab, fnl_n3, nullptr, nullptr};
     AAR_CUDA_TRY(p, cudaFuncSetAttribute(k_xacc<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XaccCfg<N>::SMEM));
     {
       ProfScope ps_(p, "modal_xacc", st);
@@ -1414,8 +1422,7 @@ struct Chain {
     const LptArgs a = lpt_args(p);
     const float kF = a.m.g.kF;
     const ZTypes none{{0, 0, 0, 0, 0, 0}, 0.f, nullptr};
-    const RhoArgs ra = rho_args(p);
-    const AccScale sc{(float)(p->prm.primordial_index - 4), ra.log2kF, (float)(p->prm.fnl / ((double)N * N * N))};
+    const float fnl_n3 = (float)(p->prm.fnl / ((double)N * N * N));
     double* sum = (double*)(scratch + chain_fields(M) * fs);
     ChainTables ct;
     int rc;
@@ -1444,10 +1451,10 @@ struct Chain {
     if ((rc = done(p))) return rc;
     if ((rc = run_pass<N, 1, -1>(p, YAdjOp<N>{W, fs, Slots{{0, 1, 0, 2, 1, 0}}}, kTiles * 6, st, "grad_y"))) return rc;
     if ((rc = run_pass<N, 0, -1>(p, XSumOp<N>{W, fs, {0, 1, 3}, {1, 2, 3}}, kTiles * 3, st, "grad_x"))) return rc;
-    k_chain_hess<N><<<cells(p), 256, 0, st>>>(a, W, fs, sc, G, T);
+    k_chain_hess<N><<<cells(p), 256, 0, st>>>(a, W, fs, p->d_rtab, fnl_n3, G, T);
     if ((rc = done(p))) return rc;
     // the modal products, their fields made again from phig
-    const XinvOp<N> xg{T, W, fs, M, run(0, M), 1, M, M, p->d_qcube};
+    const XinvGradOp<N> xg{{T, W, fs, M, run(0, M), 1, M, M, p->d_qcube}, G, fnl_n3};
     if ((rc = run_pass<N, 0, +1>(p, xg, kTiles * M, st, "grad_xinv"))) return rc;
     const XinvNatOp<N> xf{{phig, W, fs, M, run(0, M), 1, 0, M, p->d_qcube}};
     if ((rc = run_pass<N, 0, +1>(p, xf, kTiles * M, st, "grad_xinv"))) return rc;
@@ -1494,7 +1501,7 @@ struct Chain {
     }
     if ((rc = done(p))) return rc;
     if ((rc = L::template axis_pass<1, -1>(p, W, M, run(0, M), st, "grad_y"))) return rc;
-    const XaccArgs<N> xa{p->grid, G, W, fs, M, run(0, M), M, p->d_qcube, sc, p->d_amp, gw};
+    const XaccArgs<N> xa{p->grid, G, W, fs, M, M, run(0, M), M, p->d_qcube, nullptr, 0.f, p->d_amp, gw};
     {
       ProfScope ps_(p, "grad_xacc", st);
       k_xacc<N, true><<<(unsigned)kTiles, TileCfg<N>::THREADS, XaccCfg<N>::SMEM, st>>>(xa, p->d_tw2);

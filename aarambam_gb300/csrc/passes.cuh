@@ -220,6 +220,24 @@ template <int N>
 struct XinvNatOp : XinvOp<N> {  // phi in the caller's natural order
   static constexpr bool kNatIn = true;
 };
+// The transposed chain's passes from T, which carries rho_0 Fnl / N^3 (w the
+// weights of the half spectrum): rho_r = q_r rho_0 but for r = 3, which takes G
+// itself on the kept cells, where q_3 > 0.
+template <int N>
+struct XinvGradOp : XinvOp<N> {
+  const float2* G;
+  float fnl_n3;
+  __device__ const float2* src(int c) const { return this->mode.s[c] == 3 ? G : this->phi; }
+  __device__ void pre(float2* v, int o, int kz, int c, int t) const {
+    using C = TileCfg<N>;
+    float f[C::R1];
+    cube_load<N>(f, this->qcube, this->planes, this->mode.s[c], o <= N / 2 ? o : N - o, kz, t);
+    const bool one = this->mode.s[c] == 3;
+    const float s = fnl_n3 / half_weight(kz, N);
+#pragma unroll
+    for (int i = 0; i < C::R1; ++i) v[i] = cscale(v[i], !one ? f[i] : f[i] > 0.f ? s : 0.f);
+  }
+};
 
 // 2LPT x passes.  The spectral factors of main.c:1180-1368 are products of
 // one factor per axis, except T/(D Beta), which the transfer cube brings (laid
@@ -361,19 +379,12 @@ struct XfwdInvK2Op {
   }
 };
 
-// k^(ns - 4) Fnl / N^3 at a cell of |k|^2 = n2 (grid units): the factor of the
-// modal sum's cube-weighted terms (rho_r = q_r k^(ns - 4))
-struct AccScale {
-  float e, log2kF, fnl_n3;  // e = ns - 4
-  __device__ __forceinline__ float at(int n2) const {
-    return fnl_n3 * exp2f(e * fmaf(0.5f, log2f((float)n2), log2kF));
-  }
-};
-
 // Last modal step: forward x pass of every active slot and the accumulation,
 // phi <- phi + fnl_n3 sum_r rho_r(k) g_r(k), DC = 0 (main.c:825-867,
 // 1101-1126).  rho_r = q_r k^(ns - 4) for every r (main.c:580-637, 833-860), so
-// the sum takes the filter cube's factors and one power of k at its end.  One
+// the sum takes the filter cube's factors and then rho_0 = k^(ns - 4), both
+// rounded once from 64 bits; rho_3 = 1, so r = 3 comes last and takes neither.
+// (k^(ns - 4) as an FP32 power of |k|^2 was up to 1.7e-6 off.)  One
 // block per tile walks the slots: the tile of the next slot comes in through
 // shared memory (from N = 256 on) while one is transformed, the compensated
 // sums (two_sum2) stay in registers -- the transformed slots never go back to
@@ -393,11 +404,12 @@ struct XaccArgs {
   float2* phi;
   const float2* work;
   int64_t fs;
-  int nr;
+  int nr, nw;  // active r; the first nw of them are weighted (all but r = 3)
   Slots slot;  // the active r: field and cube plane
   int planes;
   const float* qcube;
-  AccScale sc;
+  const float* rho0;  // per |k|^2
+  float fnl_n3;
   // gradient form (k_xacc<N, true>): gw = amp (phi + w sum) in natural order,
   // w = 1 on the kz = 0 and N/2 planes, else 2
   const float* amp;
@@ -434,7 +446,9 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
     tile_stage_load<N, 0>(stage, a.work + (int64_t)a.slot.s[s] * a.fs, o, c0);
     const float* q = qplane(s);
     float* d = qs + (s & 1) * X::QROWS;
-    if (last)
+    if (!GRAD && s >= a.nw)
+      ;  // r = 3
+    else if (last)
       for (int i = threadIdx.x; i < X::K; i += C::THREADS) cp_async4(d + C::W * i, q + i);
     else
       for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
@@ -444,8 +458,33 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) sum[i] = cmp[i] = make_float2(0.f, 0.f);
   if constexpr (X::kStaged) issue(0);
+  const int kz = c0 + w, ky = sidx(o, N);
 #pragma unroll 1
-  for (int s = 0; s < a.nr; ++s) {
+  for (int s = 0;; ++s) {
+    if (!GRAD && s == a.nw) {
+      // the sums so far, as the exact products' leading and trailing parts
+      constexpr int H = 8 < C::R1 ? 8 : C::R1;  // values whose loads go out together
+      int tt = t;
+      asm volatile("" : "+r"(tt));  // keeps the indices out of the loop over slots (they would spill)
+#pragma unroll
+      for (int h = 0; h < C::R1; h += H) {
+        float f[H];
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+          const int i = h + j, n = tile_n<N>(tt, i), kx = i < C::R1 / 2 ? n : n - N;
+          f[j] = kz <= N / 2 ? __ldg(a.rho0 + (kx * kx + ky * ky + kz * kz)) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+          const int i = h + j;
+          const float2 u = cscale(sum[i], f[j]);
+          cmp[i] = make_float2(fmaf(cmp[i].x, f[j], fmaf(sum[i].x, f[j], -u.x)),
+                               fmaf(cmp[i].y, f[j], fmaf(sum[i].y, f[j], -u.y)));
+          sum[i] = u;
+        }
+      }
+    }
+    if (s == a.nr) break;
     float2 v[C::R1];
     const float* q;
     if constexpr (X::kStaged) {
@@ -470,13 +509,11 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       for (int r = 0; r < C::R2; ++r) {
         const int i = tile_out_i<N>(b, r), n = tile_n<N>(t, i);
         const int ax = i < C::R1 / 2 ? n : N - n;
-        const float f = q[X::kStaged || !last ? ax * C::W : ax];
+        const float f = !GRAD && s >= a.nw ? 1.f : q[X::kStaged || !last ? ax * C::W : ax];
         two_sum2(sum[i], cmp[i], cscale(v[b * C::R2 + r], f));
       }
   }
-  const int kz = c0 + w;
   if (kz > N / 2) return;
-  const int ky = sidx(o, N);
   float2* phi = a.phi + base;
   float2 u[C::R1];  // all loads first: behind one another's stores they cost 9 ms at 1024^3
 #pragma unroll
@@ -492,8 +529,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       a.gw[NatMap<N>::base(o, c0, n, w)] = make_float2(m * fmaf(h, d.x, u[i].x), m * fmaf(h, d.y, u[i].y));
       continue;
     }
-    const float g = a.sc.at(n2);
-    float2 r = make_float2(fmaf(g, d.x, u[i].x), fmaf(g, d.y, u[i].y));
+    float2 r = make_float2(fmaf(a.fnl_n3, d.x, u[i].x), fmaf(a.fnl_n3, d.y, u[i].y));
     if (!keep_cell(a.g, kx, ky, kz)) r = u[i];
     if (n2 == 0) r = make_float2(0.f, 0.f);
     phi[TileMap<N, 0>::off(C::T * i)] = r;
@@ -501,16 +537,15 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
 }
 
 // The same with a single active r (Local templates): nothing to accumulate,
-// so a pass of its own with the plain passes' occupancy.
-template <int N>
+// so a pass of its own with the plain passes' occupancy.  ONE: r = 3, rho = 1.
+template <int N, bool ONE>
 struct XaddOp {
   static constexpr bool kPre = false, kPost = true;
   Grid g;
   float2* phi;
   const float2* slot;
-  int r, planes;
-  const float* qcube;
-  AccScale sc;
+  const float* rho;  // per |k|^2
+  float fnl_n3;
   __device__ void coords(unsigned item, int& o, int& c0, int& c) const {
     tile_coords<N>(item, o, c0);
     c = 0;
@@ -519,9 +554,7 @@ struct XaddOp {
   __device__ float2* dst(int) const { return phi; }
   __device__ void post(float2* v, int o, int kz, int, int t) const {
     using C = TileCfg<N>;
-    const int ay = o <= N / 2 ? o : N - o, ky = sidx(o, N);
-    const float* qb = qcube + CubeMap{N / 2 + 1, planes}.at(r, ay, min(kz, N / 2), 0);
-    const int step = kz < N / 2 ? C::W : 1;
+    const int ky = sidx(o, N);
     const float2* ph = phi + TileMap<N, 0>(o, kz, t, 0).base;
     constexpr int H = 8 < C::R1 ? 8 : C::R1;  // values whose loads go out together
 #pragma unroll
@@ -530,20 +563,18 @@ struct XaddOp {
       float f[H];
 #pragma unroll
       for (int j = 0; j < H; ++j) {
-        const int i = h + j, n = tile_n<N>(t, i);
+        const int i = h + j, n = tile_n<N>(t, i), kx = i < C::R1 / 2 ? n : n - N;
         u[j] = ph[TileMap<N, 0>::off(C::T * i)];
-        f[j] = __ldg(qb + (i < C::R1 / 2 ? n : N - n) * step);
+        f[j] = ONE ? 1.f : __ldg(rho + (kz <= N / 2 ? kx * kx + ky * ky + kz * kz : 0));
       }
 #pragma unroll
       for (int j = 0; j < H; ++j) {
         const int i = h + j, n = tile_n<N>(t, i);
         const int kx = i < C::R1 / 2 ? n : n - N;
-        const int n2 = kx * kx + ky * ky + kz * kz;
         float2& x = v[(i % C::G) * C::R2 + i / C::G];  // tile_out_i
-        const float s = sc.at(n2);
-        float2 r = make_float2(fmaf(s, x.x * f[j], u[j].x), fmaf(s, x.y * f[j], u[j].y));
+        float2 r = make_float2(fmaf(fnl_n3, x.x * f[j], u[j].x), fmaf(fnl_n3, x.y * f[j], u[j].y));
         if (kz > N / 2 || !keep_cell(g, kx, ky, kz)) r = u[j];
-        if (n2 == 0) r = make_float2(0.f, 0.f);
+        if (kx == 0 && ky == 0 && kz == 0) r = make_float2(0.f, 0.f);
         x = r;
       }
     }
