@@ -331,15 +331,21 @@ static int alloc_fused(Plan* p, int M) {
 static int mode_tables(Plan* p) {
   int N = p->N, M = p->M;
   int64_t nsq = 3LL * (N / 2) * (N / 2) + 1;
-  if (p->d_qtab && p->nsq == nsq && p->qtab_m >= M) {
+  if (p->nsq == nsq && p->qtab_m >= M) {
     // reuse the allocation
   } else {
-    if (p->d_qtab) cudaFree(p->d_qtab), p->used_bytes -= sizeof(float) * p->nsq * p->qtab_m;
-    if (p->d_rtab) cudaFree(p->d_rtab), p->used_bytes -= sizeof(float) * p->nsq * p->qtab_m;
-    p->d_qtab = p->d_rtab = nullptr;
-    int rc;
-    if ((rc = plan_alloc(p, (void**)&p->d_qtab, sizeof(float) * nsq * M))) return rc;
-    if ((rc = plan_alloc(p, (void**)&p->d_rtab, sizeof(float) * nsq * M))) return rc;
+    for (float** tab : {&p->d_qtab, &p->d_rtab}) {
+      if (*tab) cudaFree(*tab), p->used_bytes -= sizeof(float) * p->nsq * p->qtab_m;
+      *tab = nullptr;
+    }
+    p->qtab_m = 0;
+    int rc = plan_alloc(p, (void**)&p->d_qtab, sizeof(float) * nsq * M);
+    if (rc) return rc;
+    if ((rc = plan_alloc(p, (void**)&p->d_rtab, sizeof(float) * nsq * M))) {
+      cudaFree(p->d_qtab), p->used_bytes -= sizeof(float) * nsq * M;
+      p->d_qtab = nullptr;
+      return rc;
+    }
     p->qtab_m = M;
   }
   p->nsq = nsq;
@@ -571,6 +577,7 @@ int aar_set_tables(aar_plan* h, const double* alpha, const double* x0, int32_t M
   // with synchronous copies that are ordered only against the legacy stream:
   // wait for runs still in flight on other streams (or in batch graphs)
   AAR_CUDA_TRY(p, cudaDeviceSynchronize());
+  p->have_tables = false;  // until everything below has been made
   p->alpha.assign(alpha, alpha + n3);
   p->x0.assign(x0, x0 + M);
   p->M = M;

@@ -74,6 +74,8 @@ def _dptr(a: np.ndarray):
 class ICGenerator:
     """One plan: grid, cosmology, coefficient tables and transfer function."""
 
+    _set = False  # the plan holds _alpha and _x0 (not after a set_tables that failed)
+
     def __init__(self, cfg: dict, alpha: np.ndarray, x0: np.ndarray, k: np.ndarray, T: np.ndarray,
                  precision: str = "fp32", device=None, mem_limit_bytes: int = 0, noise_fp64: bool = False,
                  nslab: int = 8):
@@ -105,6 +107,7 @@ class ICGenerator:
             raise AarError(rc, msg.decode() if msg else "")
         M = self._alpha.shape[0]
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(self._alpha), _dptr(self._x0), M))
+        self._set = True
         kk = np.ascontiguousarray(k, dtype=np.float64)
         tt = np.ascontiguousarray(T, dtype=np.float64)
         check(self.L, self.h, self.L.aar_set_transfer(self.h, _dptr(kk), _dptr(tt), len(kk)))
@@ -158,13 +161,14 @@ class ICGenerator:
     def set_tables(self, alpha: np.ndarray, x0: np.ndarray = None) -> None:
         """Replace the coefficient tables (no-op when they are unchanged)."""
         x0 = self._x0 if x0 is None else x0
-        if (alpha is self._alpha or np.array_equal(alpha, self._alpha)) and \
+        if self._set and (alpha is self._alpha or np.array_equal(alpha, self._alpha)) and \
                 (x0 is self._x0 or np.array_equal(x0, self._x0)):
             return
         alpha, x0 = _kept(alpha), _kept(x0)
         _check_tables(alpha, x0)
+        self._set = False
         check(self.L, self.h, self.L.aar_set_tables(self.h, _dptr(alpha), _dptr(x0), alpha.shape[0]))
-        self._alpha, self._x0 = alpha, x0
+        self._alpha, self._x0, self._set = alpha, x0, True
 
     def set_jit(self, mode: int) -> str:
         """Run-time specialised modal row kernel: 0 off, 1 for N >= 256 (the
