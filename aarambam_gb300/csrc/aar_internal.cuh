@@ -82,8 +82,8 @@ struct Plan {
   std::vector<char> host_terms;  // the modal term list (a TermList, then its Terms)
   void* jit = nullptr;           // run-time specialised modal row kernel (jit.cu), or null
   int jit_mode = 1;              // 0 off, 1 for N >= 256, 2 always
-  int jit_minb = 0;              // resident row blocks per SM of the NVRTC kernel (0: by N)
-  int jit_threads = 0;           // threads per block of the NVRTC folded row kernel (0: by the lines)
+  int jit_minb = 0;              // resident row blocks per SM of the NVRTC kernel (0: by N and the lines)
+  int jit_threads = 0;           // threads per block of the NVRTC row kernel (0: by N and the lines)
   int64_t xpass_group = 1;       // tiles per item group of the multi-output x passes (passes.cuh)
   int noise_one_draw = 0;        // noise columns one draw at a time (AAR_NOISE_ONE_DRAW=1, a check)
   std::string jit_status = "off";
@@ -212,6 +212,8 @@ int copy_rows(Plan* p, void* dst, int64_t dst_ld, int dst_xb, const void* src, i
               size_t elem, cudaStream_t st);
 int noalloc_gaussian(Plan* p, void* d_out, cudaStream_t st);
 int jit_prepare(Plan* p);
+// Blocks of the kernel that jit_prepare makes; true: rows in pairs, false: folded.
+bool jit_row_shape(const Plan* p, int& minb, int& threads);
 int jit_modal_rows(Plan* p, float2* work, int64_t fs, cudaStream_t st, int64_t nrows = -1);
 int profile_modal_rows(Plan* p, float2* work, int64_t nrows, cudaStream_t st);
 void jit_free(Plan* p);

@@ -1110,10 +1110,11 @@ const char* aar_jit_status(const aar_plan* h) { return h ? h->p.jit_status.c_str
 // ------------------------------------------------------------- autotuner
 // Times the field stages (noise, modal, 2LPT) of this plan on its device for
 // each schedule candidate and keeps the fastest: row kernel generic or
-// NVRTC-specialised with 2 or 3 resident blocks per SM of 256 threads or 2
-// of 320 (ten warps: one round of line transforms fewer when the plan has
-// 17 to 20 modes), and the item
-// grouping of the multi-output x passes (1, one y row of tiles, four rows).
+// NVRTC-specialised, and the item grouping of the multi-output x passes (1, one
+// y row of tiles, four rows).  The specialised kernel comes in the shape that
+// the plan takes by itself (jit_row_shape) and with 3 resident blocks per SM of
+// 256 threads, 2 of 320 (rows in pairs) or 2 of 256 (folded rows, which take 320
+// by themselves where that saves a round over the lines).
 // Each candidate runs twice (the first run compiles and warms up); the
 // second is timed with CUDA events on the stream.  The plan's spectrum and
 // fields are overwritten, as by a realisation.
@@ -1125,21 +1126,37 @@ int aar_autotune(aar_plan* h, char* report, int32_t len, void* stream) {
   if (p->prm.precision != AAR_FUSED_FP32) return set_err(p, "the autotuner is for the fused form"), AAR_ERR_ARG;
   cudaStream_t st = S(stream);
   struct Cand {
-    int jit, minb, threads;
+    int jit, minb, threads;    // what the plan is set to
     int64_t grp;
     float ms;
+    int blocks, block_threads;  // what the kernel is compiled for
   };
   const int64_t row_tiles = p->HP / 8;
-  // (row kernel, blocks per SM, threads per block); 320 threads only where
-  // ten warps take the input lines in fewer rounds than eight
-  std::vector<int3> rows = {{0, 2, 256}, {2, 2, 256}, {2, 3, 256}};
-  const int nin = p->host_terms.empty() ? 0 : ((const TermList*)p->host_terms.data())->nin;
-  if ((nin + 9) / 10 < (nin + 7) / 8) rows.push_back({2, 2, 320});
-  std::vector<Cand> cands;
-  for (const int3& r : rows)
-    for (int64_t g : {(int64_t)1, row_tiles, 4 * row_tiles}) cands.push_back(Cand{r.x, r.y, r.z, g, -1.f});
   const int saved_mode = p->jit_mode, saved_minb = p->jit_minb, saved_threads = p->jit_threads;
   const int64_t saved_grp = p->xpass_group;
+  std::vector<Cand> cands;
+  auto add = [&](int jit, int minb, int threads) {  // true: specialised rows in pairs
+    Cand c{jit, minb, threads, 1, -1.f, 0, 256};
+    bool pairs = false;
+    if (jit) {
+      p->jit_minb = minb;
+      p->jit_threads = threads;
+      pairs = jit_row_shape(p, c.blocks, c.block_threads);
+      for (const Cand& o : cands)
+        if (o.jit && o.blocks == c.blocks && o.block_threads == c.block_threads) return pairs;
+    }
+    for (int64_t g : {(int64_t)1, row_tiles, 4 * row_tiles}) c.grp = g, cands.push_back(c);
+    return pairs;
+  };
+  add(0, 0, 0);
+  if (p->nr_active > 0) {
+    const bool pairs = add(2, 0, 0);
+    add(2, 3, 256);
+    if (pairs) add(2, 2, 320);
+    else add(2, 2, 256);
+  }
+  p->jit_minb = saved_minb;
+  p->jit_threads = saved_threads;
   // every candidate may unload and reload the NVRTC module (jit_prepare), so
   // graphs captured before this call are stale whatever the outcome
   ++p->generation;
@@ -1189,7 +1206,7 @@ int aar_autotune(aar_plan* h, char* report, int32_t len, void* stream) {
     for (size_t i = 0; i < cands.size(); ++i) {
       const Cand& c = cands[i];
       snprintf(line, sizeof(line), "%s rows=%s minb=%d threads=%d group=%lld %.3f ms\n", (int)i == best ? "*" : " ",
-               c.jit ? "nvrtc" : "generic", c.jit ? c.minb : 0, c.threads, (long long)c.grp, c.ms);
+               c.jit ? "nvrtc" : "generic", c.blocks, c.block_threads, (long long)c.grp, c.ms);
       out += line;
     }
     if ((int)out.size() + 1 > len) return set_err(p, "autotune report buffer too small"), AAR_ERR_ARG;

@@ -125,6 +125,45 @@ void jit_free(Plan* p) {
   p->jit = nullptr;
 }
 
+// Blocks of the specialised kernel: what the plan asks for (jit_minb,
+// jit_threads), else by its lines.
+struct RowShape {
+  int minb, threads, pr;
+  size_t smem;
+};
+static RowShape row_shape(const Plan* p, const TermList& tl) {
+  const int N = p->N;
+  RowShape s{};
+  if (rows_use_pairs(N, tl.nlines)) {
+    // a line per T threads: as many row pairs as fill 192 threads within 72
+    // KB, one or more rounds of at most 512 threads where a pair has more lines
+    const int R1 = two_stage_r1(N), T = N / R1, m = std::max(tl.nin, tl.nr);
+    const size_t pair = sizeof(float2) * (size_t)tl.nlines * (N + T);
+    s.pr = std::max(1, (p->jit_threads > 0 ? p->jit_threads : 192) / (m * T));
+    while (s.pr > 1 && s.pr * pair > 72 * 1024) --s.pr;
+    const int want = s.pr * m * T, rounds = (want + 511) / 512;
+    s.threads = p->jit_threads > 0 ? p->jit_threads : ((want + rounds - 1) / rounds + 31) / 32 * 32;
+    s.minb = p->jit_minb > 0 ? p->jit_minb : std::max(1, 65536 / (R1 == 32 ? 112 : 64) / s.threads);
+    s.minb = std::min(s.minb, 65536 / 64 / s.threads);
+    s.smem = s.pr * pair;
+  } else {
+    s.minb = p->jit_minb > 0 ? p->jit_minb : 2;
+    // 320 threads (ten warps) where they take the input lines in fewer rounds
+    // than eight warps (measured at 1024^3, 20 modes: 362 vs 372 ms per step);
+    // the autotuner may choose otherwise
+    s.threads = p->jit_threads > 0 ? p->jit_threads : (tl.nin + 9) / 10 < (tl.nin + 7) / 8 ? 320 : kRowThreads;
+    s.smem = sizeof(float2) * ((size_t)tl.nlines * FoldCfg<1024>::LS + FoldCfg<1024>::LT);
+  }
+  return s;
+}
+
+bool jit_row_shape(const Plan* p, int& minb, int& threads) {
+  const RowShape s = row_shape(p, *(const TermList*)p->host_terms.data());
+  minb = s.minb;
+  threads = s.threads;
+  return s.pr > 0;
+}
+
 // Build (or reuse) the specialised kernel for the plan's current term list.
 // Returns AAR_OK with p->jit set, or AAR_OK with p->jit == nullptr and the
 // reason in p->jit_status when the generic kernel stays in use.
@@ -139,28 +178,9 @@ int jit_prepare(Plan* p) {
   const Term* ft = (const Term*)(p->host_terms.data() + sizeof(TermList));
   std::vector<Term> terms(ft, ft + tl.nterms);
   const int N = p->N, M = p->M;
-  int minb, threads, pr = 0;
-  size_t smem;
-  if (rows_use_pairs(N, tl.nlines)) {
-    // a line per T threads: as many row pairs as fill 192 threads within 72
-    // KB, one or more rounds of at most 512 threads where a pair has more lines
-    const int R1 = two_stage_r1(N), T = N / R1, m = std::max(tl.nin, tl.nr);
-    const size_t pair = sizeof(float2) * (size_t)tl.nlines * (N + T);
-    pr = std::max(1, 192 / (m * T));
-    while (pr > 1 && pr * pair > 72 * 1024) --pr;
-    const int want = pr * m * T, rounds = (want + 511) / 512;
-    threads = ((want + rounds - 1) / rounds + 31) / 32 * 32;
-    minb = p->jit_minb > 0 ? p->jit_minb : std::max(1, 65536 / (R1 == 32 ? 112 : 64) / threads);
-    minb = std::min(minb, 65536 / 64 / threads);
-    smem = pr * pair;
-  } else {
-    minb = p->jit_minb > 0 ? p->jit_minb : 2;
-    // 320 threads (ten warps) where they take the input lines in fewer rounds
-    // than eight warps (measured at 1024^3, 20 modes: 362 vs 372 ms per step);
-    // the autotuner may choose otherwise
-    threads = p->jit_threads > 0 ? p->jit_threads : (tl.nin + 9) / 10 < (tl.nin + 7) / 8 ? 320 : kRowThreads;
-    smem = sizeof(float2) * ((size_t)tl.nlines * FoldCfg<1024>::LS + FoldCfg<1024>::LT);
-  }
+  const RowShape rs = row_shape(p, tl);
+  const int minb = rs.minb, threads = rs.threads, pr = rs.pr;
+  const size_t smem = rs.smem;
   const int regcap = 65536 / (threads * minb);
   const int pairs = 2 * 2 * tl.nin + 16 <= regcap * 3 / 4;  // f values of two positions fit the register budget
   std::string key = std::to_string(N) + ":" + std::to_string(M) + ":" + std::to_string(minb) + ":" +

@@ -416,9 +416,8 @@ const char* aar_jit_status(const aar_plan* plan);
 
 /* Schedule autotuner (no counterpart in the reference): times the field
    stages of this plan on its device for each candidate schedule -- the row
-   kernel generic or NVRTC-specialised with 2 or 3 resident blocks per SM of
-   256 threads (or 2 of 320 where ten warps need fewer rounds over the modes),
-   and the item grouping of the multi-output x passes -- and keeps the
+   kernel generic or NVRTC-specialised in the blocks that the plan takes by
+   itself and two others, and the item grouping of the multi-output x passes -- and keeps the
    fastest for the plan's later runs.  Needs tables and transfer function;
    overwrites the plan's spectrum and fields.  `report` (may be NULL)
    receives one line per candidate, the chosen one marked '*'. */
