@@ -120,6 +120,17 @@ def active_r(alpha: np.ndarray) -> int:
     return len(rs)
 
 
+def read_modes(alpha: np.ndarray) -> int:
+    """Modes whose field some product reads: the ones that are filtered,
+    transformed and loaded by the rows (the counter-terms of main.c:1045-1050
+    read the first three)."""
+    M = alpha.shape[0]
+    ms = {m for p in range(M) for q in range(p, M) if np.any(alpha[p, q, q:] != 0) for m in (p, q)}
+    if M > 2 and alpha[0, 1, 2] != 0:
+        ms |= {0, 1, 2}
+    return len(ms)
+
+
 def active_pairs(alpha: np.ndarray) -> int:
     """(N_i, N_j) pairs whose FFTs the reference does not skip (main.c:747-759)."""
     M = alpha.shape[0]
@@ -188,13 +199,14 @@ class Clocks:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def alg_bytes(name: str, N: int, M: int, R: int, npart: int) -> float:
+def alg_bytes(name: str, N: int, Q: int, R: int, npart: int) -> float:
     """Algorithmic HBM bytes of one launch of each kernel: every field it must
-    read and write once (complex half spectrum, F = 8 N^2 (N/2+1) bytes)."""
+    read and write once (complex half spectrum, F = 8 N^2 (N/2+1) bytes); Q modes
+    read by the products (read_modes), R active slots."""
     F = 8.0 * N * N * (N // 2 + 1)
     table = {
         "seedtable": 4.0 * N * N, "noise": F + 4.0 * N * N,
-        "modal_xinv": (1 + M) * F, "modal_ypass_inv": 2 * M * F, "modal_rows": (M + R) * F,
+        "modal_xinv": (1 + Q) * F, "modal_ypass_inv": 2 * Q * F, "modal_rows": (Q + R) * F,
         "modal_ypass_fwd": 2 * R * F, "modal_xacc": (R + 2) * F,
         # 2LPT: x passes write one field per distinct x factor (Hessians 3,
         # displacements 2 + 2) and the y passes fan them out to 6
@@ -206,6 +218,11 @@ def alg_bytes(name: str, N: int, M: int, R: int, npart: int) -> float:
         "lpt_rows_readout": 6 * F + 24.0 * npart,
     }
     return table.get(name, float("nan"))
+
+
+def path_bytes(N: int, Q: int) -> float:
+    """Algorithmic bytes of a realisation, 4 N^3 (46 + 9 per mode that is read)."""
+    return 4.0 * N ** 3 * (46 + 9 * Q)
 
 
 def peaks() -> dict:
@@ -377,7 +394,7 @@ def gpu_arm(args):
     cfg = make_cfg(args.workload, replica_seed(rank))
     N, M = cfg["Nmesh"], cfg["N_modes"]
     alpha, x0, k, t = load_tables(cfg["table"], M)
-    R = active_r(alpha)
+    R, Q = active_r(alpha), read_modes(alpha)
     gen = ICGenerator(cfg, alpha, x0, k, t)
     # the plan's schedule, chosen by timing the candidates on this GPU
     tuned = [] if args.no_autotune else [l for l in gen.autotune().splitlines() if l.strip()]
@@ -445,14 +462,13 @@ def gpu_arm(args):
     for nm, v in kernels.items():
         per = v["ms"] / v["launches"] / 1e3
         v["share"] = round(v["ms"] / tot, 4)
-        v["gbs"] = round(alg_bytes(nm, N, M, R, npart) / per / 1e9, 1)
+        v["gbs"] = round(alg_bytes(nm, N, Q, R, npart) / per / 1e9, 1)
     d_per = kernels[dom]["ms"] / kernels[dom]["launches"] / 1e3
-    achieved = alg_bytes(dom, N, M, R, npart) / d_per / 1e9
+    achieved = alg_bytes(dom, N, Q, R, npart) / d_per / 1e9
     roofline = {"kernel": dom, "bound": "hbm", "achieved": round(achieved, 1), "peak": pk["hbm_gbs"],
                 "unit": "GB/s", "frac": round(achieved / pk["hbm_gbs"], 4),
                 "traffic": traffic_for(dom, N), "peak_source": pk["source"]}
-    # whole path against the algorithmic byte count 4 N^3 (46 + 9 M)
-    b_path = 4.0 * N ** 3 * (46 + 9 * M)
+    b_path = path_bytes(N, Q)
     path_roof = {"bytes_per_step": b_path, "achieved": round(b_path / (elapsed / args.steps) / 1e9, 1),
                  "frac": round(b_path / (elapsed / args.steps) / 1e9 / pk["hbm_gbs"], 4)}
 
@@ -810,7 +826,7 @@ def rows_arm(args):
     e1.record(stream)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / args.steps
-    byts = (M + R) * 8.0 * nrows * HP
+    byts = (read_modes(alpha) + R) * 8.0 * nrows * HP
     print(json.dumps({"case": f"modal rows of {args.workload}, {nrows} rows", "jit": gen.jit_status,
                       "ms_per_launch": ms, "alg_bytes": byts, "gbs": byts / ms / 1e6,
                       "device_bytes": int(work.numel() * 4 + gen.device_bytes)}))
@@ -833,7 +849,7 @@ def batch_arm(args):
         cfg = dict(base, Nmesh=N, Nsample=N, Nmax=256, Box=box, Seed=1234 + i, Fnl=fnl, N_modes=M, table=tab)
         alpha, x0, k, t = load_tables(tab, M)
         gens.append(ICGenerator(cfg, alpha, x0, k, t))
-        bytes_step += 4.0 * N ** 3 * (46 + 9 * M)
+        bytes_step += path_bytes(N, read_modes(alpha))
     lagr = lattice_positions(N, box, dev)
     npart = lagr.shape[0]
     lagrs = [lagr] * nreal
