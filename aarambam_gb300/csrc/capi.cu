@@ -313,6 +313,7 @@ static int alloc_fused(Plan* p, int M) {
     cudaFree(p->d_work);
     p->used_bytes -= fbytes * p->nwork;
     p->d_work = nullptr;
+    p->disp_real = false;
   }
   int rc = plan_alloc(p, (void**)&p->d_work, fbytes * nwork);
   if (rc) return rc;

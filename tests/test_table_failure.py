@@ -1,5 +1,6 @@
-"""A set_tables that runs out of memory half way: the plan refuses to compute
-until tables are set again, and then gives what it gave before."""
+"""What a plan holds after other tables: after a set_tables that ran out of
+memory half way it refuses to compute until tables are set again, and then gives
+what it gave before; fields that more modes have moved are not handed out."""
 import numpy as np
 import pytest
 import torch
@@ -38,3 +39,16 @@ def test_plan_after_tables_that_did_not_fit(cuda, spare):
     again = g.run(lagr)
     assert torch.equal(again[0], pos) and torch.equal(again[1], vel)
     assert g.device_bytes == held
+
+
+def test_fields_are_gone_with_their_memory(cuda):
+    g = plan(32, 4)
+    for stage in ("noise", "modal", "lpt"):
+        g.stage(stage)
+    g.field(0)
+    g.set_tables(symmetric(16, [(0, 0, 3, 1.0)]), np.linspace(1.0, 0.5, 16))  # more work fields than before
+    g.prepare()
+    with pytest.raises(AarError, match="run the field stages first"):
+        g.field(0)
+    g.stage("lpt")
+    g.field(0)
