@@ -266,12 +266,12 @@ __device__ __forceinline__ void rows_pairs(const Op& op, float2* work, int64_t f
 // E_k - e^{-2 pi i k/H} O_k, then the post-step X_k from Z_k, Z_{H-k}.
 template <int N>
 struct FoldCfg {
-  static_assert(N == 1024, "folded rows: one warp per 512-point half line");
+  static_assert(N == 1024 && N / 4 == kLineR * kLineR, "folded rows: one warp per 512-point half line");
   static constexpr int LS = spad_len(N / 2);
   // float2 slots of the lane twiddle table (fft.cuh) of the H/2-point
   // half-line transforms, at the start of the shared memory, filled once per
   // block (the modal rows at 1024^3 with 20 modes 67.9 -> 60.8 ms)
-  static constexpr int LT = lt_slots(N / 4, 16);
+  static constexpr int LT = kLineTw;
 };
 
 // Z_j of the c2r pre-step from a = X_j, b = X_{H-j}, w = e^{+2 pi i j/N}:
@@ -402,13 +402,13 @@ __device__ __forceinline__ void rows_fold(const Op& op, float2* work, int64_t fs
   constexpr int nwarps = THREADS / 32;
   const int half = lane >> 4, t16 = lane & 15;
   const float2* lt = sm_all;
-  lt_fill<h, 16, 2>(sm_all, twH, threadIdx.x, THREADS);
+  lt_fill<2>(sm_all, twH, threadIdx.x, THREADS);
   __syncthreads();
   for (int l = warp; l < op.nin(); l += nwarps) {
     float2* line = sm + op.in_line(l) * C::LS;
     row_c2r_pre_fold<N>(line, lane, twN, twH, work + (int64_t)op.in_slot(l) * fs + row * HP);
     __syncwarp();
-    line_fft_smem<h, 16, +1, 0, 2, true>(line + half * HO, t16, lt, true);
+    line_fft<+1>(line + half * HO, t16, lt);
   }
   __syncthreads();
   for (int n = threadIdx.x; n < H; n += (Op::kPairs ? 2 : 1) * THREADS) {
@@ -423,7 +423,7 @@ __device__ __forceinline__ void rows_fold(const Op& op, float2* work, int64_t fs
   __syncthreads();
   for (int l = warp; l < op.nout(); l += nwarps) {
     float2* line = sm + op.out_line(l) * C::LS;
-    line_fft_smem<h, 16, -1, 0, 2, true>(line + half * HO, t16, lt, true);
+    line_fft<-1>(line + half * HO, t16, lt);
     row_r2c_post_fold<N>(line, work + (int64_t)op.out_slot(l) * fs + row * HP, lane, twN, twH);
     __syncwarp();
   }
