@@ -24,7 +24,7 @@ pytestmark = pytest.mark.gpu
                                       (256, 500.0, [0, 5]), (512, 1000.0, [3]), (512, 1000.0, [5]),
                                       (512, 1000.0, [0, 1, 3, 4])])
 def test_weights_of_the_modal_sum(cuda, N, box, rs):
-    M, ns, nmax = 6, 0.965, 512
+    M, ns, nmax = 6, 0.965, max(512, N)
     x0 = np.linspace(1.0, 0.5, M)
     s, kF = (4 - ns) / 3, 2 * np.pi / box
     i = torch.arange(N, device=cuda)
