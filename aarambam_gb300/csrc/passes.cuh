@@ -459,6 +459,17 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
   for (int i = 0; i < C::R1; ++i) sum[i] = cmp[i] = make_float2(0.f, 0.f);
   if constexpr (X::kStaged) issue(0);
   const int kz = c0 + w, ky = sidx(o, N);
+  auto weight = [&](int t0, int i) {
+    const int n = tile_n<N>(t0, i), kx = i < C::R1 / 2 ? n : n - N;
+    return kz <= N / 2 ? __ldg(a.rho0 + (kx * kx + ky * ky + kz * kz)) : 0.f;
+  };
+  // where registers are left the weights are on their way before the slots
+  constexpr bool kAhead = !GRAD && C::R1 <= 8;
+  float ahead[kAhead ? C::R1 : 1];
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int i = 0; i < C::R1; ++i) ahead[i] = weight(t, i);
+  }
 #pragma unroll 1
   for (int s = 0;; ++s) {
     if (!GRAD && s == a.nw) {
@@ -470,10 +481,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       for (int h = 0; h < C::R1; h += H) {
         float f[H];
 #pragma unroll
-        for (int j = 0; j < H; ++j) {
-          const int i = h + j, n = tile_n<N>(tt, i), kx = i < C::R1 / 2 ? n : n - N;
-          f[j] = kz <= N / 2 ? __ldg(a.rho0 + (kx * kx + ky * ky + kz * kz)) : 0.f;
-        }
+        for (int j = 0; j < H; ++j) f[j] = kAhead ? ahead[kAhead ? h + j : 0] : weight(tt, h + j);
 #pragma unroll
         for (int j = 0; j < H; ++j) {
           const int i = h + j;
