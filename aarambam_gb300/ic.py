@@ -47,10 +47,14 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
-def _dense(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
-    """t as plain contiguous memory of dtype: a conjugate or negated view
+def _dense(t: torch.Tensor, dtype: torch.dtype = None) -> torch.Tensor:
+    """t as plain contiguous memory (of dtype): a conjugate or negated view
     (x.conj(), its imag) says so in a flag, which the address does not carry."""
-    return t.to(dtype).resolve_conj().resolve_neg().contiguous()
+    if dtype is not None and t.dtype != dtype:
+        t = t.to(dtype)
+    if t.is_conj() or t.is_neg():
+        t = t.resolve_conj().resolve_neg()
+    return t.contiguous()
 
 
 def _kept(a) -> np.ndarray:
@@ -246,7 +250,7 @@ class ICGenerator:
         check(self.L, self.h, self.L.aar_set_spectrum(self.h, _ptr(spec), self._stream()))
 
     def readout(self, lagr: torch.Tensor, pos: torch.Tensor = None, vel: torch.Tensor = None):
-        lagr = lagr.resolve_neg().contiguous()
+        lagr = _dense(lagr)
         pos = torch.empty_like(lagr) if pos is None else pos
         vel = torch.empty_like(lagr) if vel is None else vel
         check(self.L, self.h, self.L.aar_stage_readout(self.h, _ptr(lagr), lagr.shape[0], _ptr(pos), _ptr(vel),
@@ -255,7 +259,7 @@ class ICGenerator:
 
     def run(self, lagr: torch.Tensor, pos: torch.Tensor = None, vel: torch.Tensor = None):
         """Whole path on device-resident Lagrangian positions float32 [n, 3]."""
-        lagr = lagr.resolve_neg().contiguous()
+        lagr = _dense(lagr)
         pos = torch.empty_like(lagr) if pos is None else pos
         vel = torch.empty_like(lagr) if vel is None else vel
         check(self.L, self.h, self.L.aar_run(self.h, _ptr(lagr), lagr.shape[0], _ptr(pos), _ptr(vel),
