@@ -194,7 +194,6 @@ inline bool is_plain(const aar_params& q) {
 // the FP32 forms share the plan's field layout (x-blocked rows of HP complex)
 inline bool is_fp32(const aar_params& q) { return q.precision == AAR_FUSED_FP32 || q.precision == AAR_SLAB_FP32; }
 int build_term_list(Plan* p);  // the regrouped term list (fused.cu)
-RhoArgs rho_args(const Plan* p);
 int slab_check(const aar_params& q, std::string& why);
 int slab_setup(Plan* p);
 int slab_run(Plan* p, cudaStream_t st);

@@ -1,7 +1,6 @@
-// Per-cell geometry of the half spectrum, shared by the library's kernels
-// and the run-time specialised ones (jit.cu, NVRTC): row order, signed
-// wavenumbers, the reference's keep/cut rule and the per-cell mode
-// functions of the modal accumulation.  Device code and plain structs only.
+// Per-cell geometry of the half spectrum, shared by the library's kernels: row
+// order, signed wavenumbers, the reference's keep/cut rule and the slab form's
+// per-cell mode functions.  Device code and plain structs only.
 #pragma once
 #include "fft.cuh"
 
@@ -61,7 +60,8 @@ __device__ __forceinline__ bool keep_cell(const Grid& g, int kx, int ky, int kz)
   return !(__ddiv_rn(__dmul_rn(km, g.box), __dmul_rn(2.0, kPi)) > (double)g.nsample_half);
 }
 
-// rho_n(k) of the accumulation evaluated per cell (main.c:825-860):
+// The mode functions as the slab form evaluates them per cell, rho_n(k) of the
+// accumulation (main.c:825-860) and the field filters (slab.cu):
 // k^(s (n-3)) for n <= 3, (P_{n-1}(kbar) - X0[n-1]) / k^2 above, with
 // kbar = -1 + 2 (k^s - kmin^s)/(kmax^s - kmin^s); kmin = kF, so
 // k^s - kmin^s = kmin^s expm1(s ln(sqrt(n^2))) (no cancellation near kmin),

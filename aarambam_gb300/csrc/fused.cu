@@ -6,9 +6,9 @@
 // three passes, each reading and writing a field once:
 //   x pass / y pass  -- strided complex FFTs on tiles of 8 consecutive kz
 //                       columns x N rows, held in registers (tile.cuh);
-//   z pass (rows)    -- the real<->half-complex transform of contiguous rows
-//                       as an N/2-point complex FFT plus the usual
-//                       even/odd split twiddle step.
+//   z pass (rows)    -- the real<->half-complex transform of contiguous rows,
+//                       two real rows as one N-point complex line (N = 1024
+//                       with many lines: folded single rows; rows.cuh).
 // The reference's per-pass work is fused into these passes:
 //   modal potential (Aarambam/LPT/Basis/main.c:564-1151) regrouped exactly by
 //   linearity of the DFT: acc = sum_r rho_r(k) r2c[ g_r ],
@@ -17,9 +17,8 @@
 //   main.c:1045-1050.  The x pass that starts every f_p reads phi once and
 //   applies q_p; one row kernel does all c2r's, products and r2c's of a row;
 //   the last x pass applies rho_r, sums over r and adds Fnl acc / N^3.
-//   2LPT (main.c:1156-1381): Hessians straight from phi (-k_a k_b T/(D Beta)),
-//   the source in the row kernel, Poisson + CIC deconvolution fused into the
-//   x pass that also starts the six displacement c2r's.
+//   2LPT (main.c:1156-1381): one factor per axis (x passes, fan-out y passes,
+//   c2r rows), the source in the row kernel, 1/k^2 in its forward x pass.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -601,25 +600,6 @@ static int run_pass(Plan* p, const Op& op, int64_t nitems, cudaStream_t st, cons
   return AAR_OK;
 }
 
-RhoArgs rho_args(const Plan* p) {
-  RhoArgs r{};
-  const double ns = p->prm.primordial_index, box = p->prm.box;
-  const double kF = 2 * kPi / box, kmin = kF, kmax = kF * p->prm.nmax;
-  const double sx = (4 - ns) / 3, kmin_s = pow(kmin, sx), kmax_s = pow(kmax, sx);
-  r.s = (float)sx;
-  r.c1 = (float)(2 * kmin_s / (kmax_s - kmin_s));
-  r.log2kF = (float)log2(kF);
-  r.inv_kF2 = (float)(1 / (kF * kF));
-  r.e4 = (float)(4 - ns);
-  r.e2 = (float)(2 - ns);
-  for (int n = 0; n < kMaxModes; ++n) r.x0[n] = n < (int)p->x0.size() ? (float)p->x0[n] : 0.f;
-  for (int l = 1; l < kMaxModes; ++l) {
-    r.A[l] = (float)((2.0 * l - 1) / l);
-    r.B[l] = (float)((l - 1.0) / l);
-  }
-  return r;
-}
-
 template <int N>
 struct Launch {
   static constexpr int64_t kTiles = TileCfg<N>::TILES;
@@ -720,8 +700,8 @@ struct Launch {
     if ((rc = p->jit ? jit_modal_rows(p, p->d_work, fs, st) : modal_rows(p, p->d_work, fs, (int64_t)N * N, st))) return rc;
     if ((rc = axis_pass<1, -1>(p, p->d_work, tl.nr, out, st, "modal_ypass_fwd"))) return rc;
     const float fnl_n3 = (float)(p->prm.fnl / ((double)N * N * N));
-    // one slot: 2.83 ms against k_xacc's 4.39 at 1024^3, whose registers leave
-    // one block per SM; with 16 values per lane and fewer k_xacc is as fast
+    // one slot (r = 3): 2.53 ms against k_xacc's 4.39 at 1024^3, whose registers
+    // leave one block per SM; with 16 values per lane and fewer k_xacc is as fast
     // (0.0122 against 0.0132 ms at 128^3)
     if constexpr (TileCfg<N>::R1 == 32) {
       if (tl.nr == 1) {

@@ -1,10 +1,10 @@
 // Run-time specialised modal row kernel.
 //
-// The generic row kernel (fused.cu, ModalRowOp) reads its term list at run
-// time, so every term costs four shared-memory loads (f_p and f_q at two
-// positions).  Here the kernel is generated for the plan's term structure
+// The generic row kernel (fused.cu, ModalRowOp) walks its term list at run
+// time: in factored order a term costs a shared-memory load at each of two
+// positions, its address and the loop.  Here the kernel is generated for the plan's term structure
 // and compiled with NVRTC for sm_103a: a thread loads the M values f_p of
-// its positions into registers once and every term is two multiply-adds with
+// its positions into registers once and a term is a multiply-add per component with
 // compile-time register indices; the coefficients sit in the module's
 // __constant__ memory, so a new alpha table with the same nonzero pattern
 // (same terms) only rewrites them.  The FFT and row code are the same

@@ -412,7 +412,9 @@ static int run_noise32(Plan* p, const uint32_t* d_seed, float2* out, int hp, int
   }
   // columns per warp: fewer lanes run the generator where there are few warps
   // to hide its latency, at the price of its issue slots: 64^3 0.0226 ms with
-  // 8, 0.0275 with 16; 128^3 0.049 with 16, 0.058 with 32
+  // 8, 0.0275 with 16; 128^3 0.049 with 16, 0.058 with 32.  That is one plan by
+  // itself; the rule knows nothing of other plans on the device.  Six 128^3
+  // plans in one graph took 2615 us with 16 and 2584 with 32.
   auto go = [&](auto c) {
     constexpr int COLS = decltype(c)::value, per = COLS * kNoiseWarps;
     k_noise32<COLS><<<(unsigned)((cols + per - 1) / per), 32 * kNoiseWarps, 0, st>>>(noise_args(p, xb), d_seed, out, hp);

@@ -379,6 +379,37 @@ struct XfwdInvK2Op {
   }
 };
 
+// The values of a thread's line that the cut keeps, bit i value i (keep_cell).
+// The sphere's boundary takes FP64 and is rare: unrolled over 32 values it made
+// k_xacc slower (512^3, three slots: 0.96 against 0.78 ms); with 16 values the mask
+// costs more (256^3, a potential with 19 slots: 2255 against 2245 us).
+template <int N>
+__device__ __forceinline__ unsigned keep_mask(const Grid& g, int t, int ky, int kz) {
+  using C = TileCfg<N>;
+  auto kx = [&](int i) { return i < C::R1 / 2 ? tile_n<N>(t, i) : tile_n<N>(t, i) - N; };
+  unsigned m = 0;
+  if (!g.sphere) {
+    if (abs(ky) > g.kcut || kz > g.kcut) return 0;
+#pragma unroll
+    for (int i = 0; i < C::R1; ++i) m |= (abs(kx(i)) <= g.kcut ? 1u : 0u) << i;
+    return m;
+  }
+  const int b = g.nsq_bnd - ky * ky - kz * kz;
+  bool edge = false;
+#pragma unroll
+  for (int i = 0; i < C::R1; ++i) {
+    const int k2 = kx(i) * kx(i);
+    m |= (k2 < b ? 1u : 0u) << i;
+    edge |= k2 == b;
+  }
+  if (edge) {
+#pragma unroll 1
+    for (int i = 0; i < C::R1; ++i)
+      if (kx(i) * kx(i) == b && keep_cell(g, kx(i), ky, kz)) m |= 1u << i;
+  }
+  return m;
+}
+
 // Last modal step: forward x pass of every active slot and the accumulation,
 // phi <- phi + fnl_n3 sum_r rho_r(k) g_r(k), DC = 0 (main.c:825-867,
 // 1101-1126).  rho_r = q_r k^(ns - 4) for every r (main.c:580-637, 833-860), so
@@ -396,7 +427,7 @@ struct XfwdInvK2Op {
 // What bounds it: instruction issue of the 8 (N >= 512) to 16 warps that
 // 32 values, their sums and compensations leave room for.  Against the forward
 // x pass and the specialised pointwise accumulation: 0.39 -> 0.23 ms (256^3, 12
-// slots), 0.71 -> 0.33 (256^3, 19), 3.39 -> 1.95 (512^3, 11), 48.1 -> 35.0
+// slots), 0.71 -> 0.33 (256^3, 19), 3.39 -> 1.88 (512^3, 11), 48.1 -> 35.3
 // (1024^3, 19).
 template <int N>
 struct XaccArgs {
@@ -419,6 +450,9 @@ template <int N>
 struct XaccCfg {
   using C = TileCfg<N>;
   static constexpr bool kStaged = N >= 256;
+  // the weights, too: 512^3 with 11 slots 1.91 -> 1.88 ms; at 256^3, where more warps
+  // hide a thread's own gather, a potential with 19 slots 2251 against 2243 us
+  static constexpr bool kStagedW = kStaged && C::R1 == 32;
   static constexpr int K = N / 2 + 1;
   static constexpr size_t QROWS = (size_t)K * C::W;  // floats of a plane's block of columns
   static constexpr size_t SMEM = C::SMEM + (kStaged ? sizeof(float2) * N * C::W + 2 * sizeof(float) * QROWS : 0);
@@ -442,29 +476,40 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
   auto qplane = [&](int s) { return a.qcube + CubeMap{X::K, a.planes}.at(a.slot.s[s], ay, c0, 0); };
   float2* stage = ex + C::SMEM / sizeof(float2);
   float* qs = reinterpret_cast<float*>(stage + N * C::W);  // two buffers
+  const int kz = c0 + w, ky = sidx(o, N);
+  // rho_0 is taken into the sums behind the last weighted slot
+  const bool weighted = !GRAD && a.nw > 0;
   auto issue = [&](int s) {
-    tile_stage_load<N, 0>(stage, a.work + (int64_t)a.slot.s[s] * a.fs, o, c0);
-    const float* q = qplane(s);
+    if (s < a.nr) tile_stage_load<N, 0>(stage, a.work + (int64_t)a.slot.s[s] * a.fs, o, c0);
     float* d = qs + (s & 1) * X::QROWS;
-    if (!GRAD && s >= a.nw)
-      ;  // r = 3
-    else if (last)
-      for (int i = threadIdx.x; i < X::K; i += C::THREADS) cp_async4(d + C::W * i, q + i);
-    else
-      for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
+    if (GRAD || s < a.nw) {
+      const float* q = qplane(s);
+      if (last)
+        for (int i = threadIdx.x; i < X::K; i += C::THREADS) cp_async4(d + C::W * i, q + i);
+      else
+        for (int i = threadIdx.x; i < (int)X::QROWS / 4; i += C::THREADS) cp_async16(d + 4 * i, q + 4 * i);
+    } else if (X::kStagedW && weighted) {
+      // s = nw, r = 3 or none: the buffer takes the tile's weights, a gather per
+      // |kx| and column while the slot before is transformed
+      const int b = ky * ky;
+      for (int i = threadIdx.x; i < (int)X::QROWS; i += C::THREADS) {
+        const int ax = i / C::W, z = c0 + i % C::W;
+        cp_async4(d + i, a.rho0 + (z <= N / 2 ? ax * ax + b + z * z : 0));
+      }
+    }
     cp_async_commit();
   };
   float2 sum[C::R1], cmp[C::R1];
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) sum[i] = cmp[i] = make_float2(0.f, 0.f);
   if constexpr (X::kStaged) issue(0);
-  const int kz = c0 + w, ky = sidx(o, N);
   auto weight = [&](int t0, int i) {
-    const int n = tile_n<N>(t0, i), kx = i < C::R1 / 2 ? n : n - N;
-    return kz <= N / 2 ? __ldg(a.rho0 + (kx * kx + ky * ky + kz * kz)) : 0.f;
+    const int n = tile_n<N>(t0, i), ax = i < C::R1 / 2 ? n : N - n;
+    if constexpr (X::kStagedW) return qs[(a.nw & 1) * X::QROWS + ax * C::W + w];
+    else return kz <= N / 2 ? __ldg(a.rho0 + (ax * ax + ky * ky + kz * kz)) : 0.f;
   };
   // where registers are left the weights are on their way before the slots
-  constexpr bool kAhead = !GRAD && C::R1 <= 8;
+  constexpr bool kAhead = !GRAD && !X::kStaged && C::R1 <= 8;
   float ahead[kAhead ? C::R1 : 1];
   if constexpr (kAhead) {
 #pragma unroll
@@ -472,7 +517,12 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
   }
 #pragma unroll 1
   for (int s = 0;; ++s) {
-    if (!GRAD && s == a.nw) {
+    if constexpr (X::kStaged)
+      if (s < a.nr || (X::kStagedW && weighted)) {
+        cp_async_wait<0>();
+        __syncthreads();
+      }
+    if (weighted && s == a.nw) {
       // the sums so far, as the exact products' leading and trailing parts
       constexpr int H = 8 < C::R1 ? 8 : C::R1;  // values whose loads go out together
       int tt = t;
@@ -496,12 +546,10 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
     float2 v[C::R1];
     const float* q;
     if constexpr (X::kStaged) {
-      cp_async_wait<0>();
-      __syncthreads();
 #pragma unroll
       for (int r = 0; r < C::R1; ++r) v[r] = stage[tile_n<N>(t, r) * C::W + w];
       __syncthreads();  // the stage is free, and the exchange of the slot before has been read
-      if (s + 1 < a.nr) issue(s + 1);
+      if (s + 1 < a.nr || (X::kStagedW && weighted && s + 1 == a.nw)) issue(s + 1);
       q = qs + (s & 1) * X::QROWS + qw;
     } else {
       const float2* src = a.work + (int64_t)a.slot.s[s] * a.fs + base;
@@ -526,11 +574,12 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
   float2 u[C::R1];  // all loads first: behind one another's stores they cost 9 ms at 1024^3
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) u[i] = phi[TileMap<N, 0>::off(C::T * i)];
+  constexpr bool kMask = !GRAD && C::R1 == 32;
+  const unsigned keep = kMask ? keep_mask<N>(a.g, t, ky, kz) : 0u;
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) {
     const int n = tile_n<N>(t, i);
     const int kx = i < C::R1 / 2 ? n : n - N;
-    const int n2 = kx * kx + ky * ky + kz * kz;
     const float2 d = add2(sum[i], cmp[i]);
     if constexpr (GRAD) {
       const float h = half_weight(kz, N), m = gauss_amp(a.g, a.amp, n, o, kx, ky, kz);
@@ -538,8 +587,8 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       continue;
     }
     float2 r = make_float2(fmaf(a.fnl_n3, d.x, u[i].x), fmaf(a.fnl_n3, d.y, u[i].y));
-    if (!keep_cell(a.g, kx, ky, kz)) r = u[i];
-    if (n2 == 0) r = make_float2(0.f, 0.f);
+    if (kMask ? !(keep >> i & 1u) : !keep_cell(a.g, kx, ky, kz)) r = u[i];
+    if (kx == 0 && ky == 0 && kz == 0) r = make_float2(0.f, 0.f);
     phi[TileMap<N, 0>::off(C::T * i)] = r;
   }
 }

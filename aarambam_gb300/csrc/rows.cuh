@@ -36,9 +36,10 @@ struct ZFac {
 // N-point spectrum is C_k = A_k + i B_k, C_{N-k} = conj A_k + i conj B_k, so
 // a c2r of both is one complex inverse transform of C and an r2c of both one
 // forward transform and C's even / odd split -- no half-length twiddle steps.
-// The rows of a pair are neighbours of the same field (memory rows m, m + 1),
-// so both have the same magnitude and the FP32 rounding of the line is that
-// of each row.
+// The rows of a pair are neighbours of the same field (memory rows m, m + 1).
+// The FP32 rounding of a line is relative to the larger of the two; the x and y
+// passes mix all rows anyway, so the error of a 3-D transform relative to its
+// norm is that of single rows, whatever the field.
 //
 // A line is transformed by T threads with R1 = N / T values each in two
 // register stages and one exchange through the line's own shared memory

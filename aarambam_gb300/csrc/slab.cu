@@ -119,6 +119,25 @@ __global__ void __launch_bounds__(256) k_slab_herm(float2* F, int nf, int64_t sf
   }
 }
 
+static RhoArgs rho_args(const Plan* p) {
+  RhoArgs r{};
+  const double ns = p->prm.primordial_index, box = p->prm.box;
+  const double kF = 2 * kPi / box, kmin = kF, kmax = kF * p->prm.nmax;
+  const double sx = (4 - ns) / 3, kmin_s = pow(kmin, sx), kmax_s = pow(kmax, sx);
+  r.s = (float)sx;
+  r.c1 = (float)(2 * kmin_s / (kmax_s - kmin_s));
+  r.log2kF = (float)log2(kF);
+  r.inv_kF2 = (float)(1 / (kF * kF));
+  r.e4 = (float)(4 - ns);
+  r.e2 = (float)(2 - ns);
+  for (int n = 0; n < kMaxModes; ++n) r.x0[n] = n < (int)p->x0.size() ? (float)p->x0[n] : 0.f;
+  for (int l = 1; l < kMaxModes; ++l) {
+    r.A[l] = (float)((2.0 * l - 1) / l);
+    r.B[l] = (float)((l - 1.0) / l);
+  }
+  return r;
+}
+
 // Field filters q_p(k) of main.c:580-637, p < M, at one cell (n2 = |k|^2 in
 // grid units, > 0) in FP32: k^(s (p-3)) k^(4-ns) for p <= 3, (P_{p-1}(kbar) -
 // X0[p-1]) k^(2-ns) above, one Legendre recurrence for all modes.  With k = kF

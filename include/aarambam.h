@@ -67,7 +67,11 @@ typedef struct aar_params {
   double input_spectrum_unit_length_in_cm;
   int32_t fixed_amplitude, phase_flip, sphere_mode;
   int32_t precision;        /* AAR_FUSED_FP32, AAR_PLAIN_FP64, AAR_PLAIN_FP64_REGROUPED or AAR_SLAB_FP32 */
-  int64_t mem_limit_bytes;  /* refuse plan allocations beyond this (0 = no cap) */
+  /* Refuse plan allocations beyond this (0 = no cap).  The fused form's: 1 +
+     max(M, 9) fields of 8 N^2 HP bytes (HP = N/2+1 rounded up to 8), the filter
+     cube, 4 M (N/2+1)^3, and tables per |k|^2, 4 (2 + 2 M) (3 (N/2)^2 + 1); with no
+     cap also the transfer cube, 4 (N/2+1)^3, where the device has room for it. */
+  int64_t mem_limit_bytes;
   int32_t variant;          /* AAR_VARIANT_BASIS or AAR_VARIANT_RESBASIS */
   int32_t which_spectrum;   /* WhichSpectrum: 0 for Basis; 0, 1 or 2 for ResBasis */
   double a_res, w_res, phi_res; /* ResBasis oscillation (ResBasis/read_param.c:88-99) */
