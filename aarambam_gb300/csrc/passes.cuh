@@ -379,12 +379,24 @@ struct XfwdInvK2Op {
   }
 };
 
-// The values of a thread's line that the cut keeps, bit i value i (keep_cell).
-// The sphere's boundary takes FP64 and is rare: unrolled over 32 values it made
-// k_xacc slower (512^3, three slots: 0.96 against 0.78 ms); with 16 values the mask
-// costs more (256^3, a potential with 19 slots: 2255 against 2245 us).
+// keep_cell with the cells on the sphere's boundary, which take FP64, looked up in
+// the filter cube: q_0 is 1 inside the cut and 0 outside.  (Unrolled over the
+// values the FP64 code made k_xacc slower: 512^3, three slots, 0.96 ms against 0.78;
+// 64^3 and 32^3, 2 to 4 us.)
 template <int N>
-__device__ __forceinline__ unsigned keep_mask(const Grid& g, int t, int ky, int kz) {
+__device__ __forceinline__ bool keep_cube(const Grid& g, const float* __restrict__ qcube, int planes, int kx, int ky,
+                                          int kz) {
+  if (!g.sphere) return abs(kx) <= g.kcut && abs(ky) <= g.kcut && kz <= g.kcut;
+  const int n2 = kx * kx + ky * ky + kz * kz;
+  if (n2 != g.nsq_bnd) return n2 < g.nsq_bnd;
+  return __ldg(qcube + CubeMap{N / 2 + 1, planes}.at(0, abs(ky), kz, abs(kx))) > 0.f;
+}
+// The same for a thread's line, bit i value i, the lookups out of line: with 32
+// values keep_cube at each spills (512^3, 11 slots: 2.01 ms against 1.88), with 16 the
+// mask does (256^3, a potential with 19 slots: 2255 us against 2245).
+template <int N>
+__device__ __forceinline__ unsigned keep_mask(const Grid& g, const float* __restrict__ qcube, int planes, int t, int ky,
+                                              int kz) {
   using C = TileCfg<N>;
   auto kx = [&](int i) { return i < C::R1 / 2 ? tile_n<N>(t, i) : tile_n<N>(t, i) - N; };
   unsigned m = 0;
@@ -405,7 +417,7 @@ __device__ __forceinline__ unsigned keep_mask(const Grid& g, int t, int ky, int 
   if (edge) {
 #pragma unroll 1
     for (int i = 0; i < C::R1; ++i)
-      if (kx(i) * kx(i) == b && keep_cell(g, kx(i), ky, kz)) m |= 1u << i;
+      if (kx(i) * kx(i) == b && keep_cube<N>(g, qcube, planes, kx(i), ky, kz)) m |= 1u << i;
   }
   return m;
 }
@@ -575,7 +587,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) u[i] = phi[TileMap<N, 0>::off(C::T * i)];
   constexpr bool kMask = !GRAD && C::R1 == 32;
-  const unsigned keep = kMask ? keep_mask<N>(a.g, t, ky, kz) : 0u;
+  const unsigned keep = kMask ? keep_mask<N>(a.g, a.qcube, a.planes, t, ky, kz) : 0u;
 #pragma unroll
   for (int i = 0; i < C::R1; ++i) {
     const int n = tile_n<N>(t, i);
@@ -587,7 +599,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       continue;
     }
     float2 r = make_float2(fmaf(a.fnl_n3, d.x, u[i].x), fmaf(a.fnl_n3, d.y, u[i].y));
-    if (kMask ? !(keep >> i & 1u) : !keep_cell(a.g, kx, ky, kz)) r = u[i];
+    if (kMask ? !(keep >> i & 1u) : !keep_cube<N>(a.g, a.qcube, a.planes, kx, ky, kz)) r = u[i];
     if (kx == 0 && ky == 0 && kz == 0) r = make_float2(0.f, 0.f);
     phi[TileMap<N, 0>::off(C::T * i)] = r;
   }
