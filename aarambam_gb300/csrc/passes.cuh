@@ -520,13 +520,6 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
     if constexpr (X::kStagedW) return qs[(a.nw & 1) * X::QROWS + ax * C::W + w];
     else return kz <= N / 2 ? __ldg(a.rho0 + (ax * ax + ky * ky + kz * kz)) : 0.f;
   };
-  // where registers are left the weights are on their way before the slots
-  constexpr bool kAhead = !GRAD && !X::kStaged && C::R1 <= 8;
-  float ahead[kAhead ? C::R1 : 1];
-  if constexpr (kAhead) {
-#pragma unroll
-    for (int i = 0; i < C::R1; ++i) ahead[i] = weight(t, i);
-  }
 #pragma unroll 1
   for (int s = 0;; ++s) {
     if constexpr (X::kStaged)
@@ -543,7 +536,7 @@ __global__ void __launch_bounds__(TileCfg<N>::THREADS, XaccCfg<N>::MINB)
       for (int h = 0; h < C::R1; h += H) {
         float f[H];
 #pragma unroll
-        for (int j = 0; j < H; ++j) f[j] = kAhead ? ahead[kAhead ? h + j : 0] : weight(tt, h + j);
+        for (int j = 0; j < H; ++j) f[j] = weight(tt, h + j);
 #pragma unroll
         for (int j = 0; j < H; ++j) {
           const int i = h + j;
